@@ -60,6 +60,22 @@ def test_chain_add_special_values(host):
     assert same.all()
 
 
+@pytest.mark.parametrize("mantissa_bits", [3, 24])
+def test_chain_add_long_chains(host, mantissa_bits):
+    """Chains over several binades, with few mantissa bits (ties at every step) and with full ones;
+    lengths from those stepped plainly up to whole rows of the widest target."""
+    r = np.random.default_rng(mantissa_bits)
+    N = 3000
+    mantissa = lambda: np.ldexp(r.integers(1 << (mantissa_bits - 1), 1 << mantissa_bits, N), -mantissa_bits)
+    e = r.integers(-60, 60, N)
+    s = np.ldexp(mantissa(), e) * r.choice([1, -1], N)
+    d = np.ldexp(mantissa(), e - r.integers(0, 28, N)) * r.choice([1, -1], N)
+    n = np.where(np.arange(N) < 64, np.arange(N) % 16, r.integers(0, 16384, N))
+    s, d, n = s.astype(np.float32), d.astype(np.float32), n.astype(np.int32)
+    a, b = _chain(host, s, d, n), _serial(s, d, n)
+    assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
+
+
 def _rows(host, flat, y0, rows, L, R):
     fl = np.ascontiguousarray(flat, np.int32)
     lefts, rights = np.zeros(rows, np.int32), np.zeros(rows, np.int32)
