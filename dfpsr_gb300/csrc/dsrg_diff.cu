@@ -145,8 +145,7 @@ __global__ void normals_kernel(DiffModel m, const float *__restrict__ modelToWor
 // One thread per pixel of every view: the winning fragment's vertex weights, re-evaluated
 // exactly as the resolve pass does, then the float shading and the visibility buffer.
 __global__ void __launch_bounds__(256) diff_forward_kernel(BatchParams b, const DrawRecord *__restrict__ records,
-                                                           const uint32_t *__restrict__ rowOffsets, const uint32_t *__restrict__ rows,
-                                                           const unsigned long long *__restrict__ keys, DiffModel m, DiffParams q,
+                                                           const uint32_t *__restrict__ rows, const unsigned long long *__restrict__ keys, DiffModel m, DiffParams q,
                                                            int32_t width, int32_t height, uint64_t pixels, float4 *images,
                                                            uint32_t *visibility) {
 	for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < pixels; i += (uint64_t)gridDim.x * blockDim.x) {
@@ -162,12 +161,11 @@ __global__ void __launch_bounds__(256) diff_forward_kernel(BatchParams b, const 
 			visibility[i * 3 + 2] = 0u;
 			continue;
 		}
-		const uint32_t ri = key_record(key, true);
-		const DrawRecord r = records[ri];
+		const DrawRecord r = records[record_slot(b, key_record(key, true))];
 		const bool affine = b.frames[view].affine != 0;
 		const int32_t y1 = py & ~1, x = px & ~1;
 		const int lane4 = ((py & 1) << 1) | (px & 1);
-		const RowPair pair = record_row_pair(r, rows + rowOffsets[ri], y1, height);
+		const RowPair pair = record_row_pair(r, rows, y1, height);
 		float w[3][4], wa[4], wb[4], wc[4];
 		for (int c = 0; c < 3; c++) quad_lanes(r.start[c], r.dx[c], r.dy[c], pair, y1, x, w[c]);
 		lane_weights(w, affine, wa, wb, wc);
@@ -640,8 +638,8 @@ int dsrg_diff_forward(dsrg_diff d, int32_t views, const dsrg_camera *cameras, co
 	q.log2H = d->log2H;
 	q.ambient = d->ambient;
 	const unsigned long long *keys = totals.pixels ? ctx->keys.ptr : nullptr;
-	diff_forward_kernel<<<grid_for(pixels, 256), 256, 0, stream>>>(outputs.params, outputs.fb.records, outputs.fb.rowOffsets,
-	                                                               outputs.fb.rows, keys, diff_model(d), q, width, height, pixels,
+	diff_forward_kernel<<<grid_for(pixels, 256), 256, 0, stream>>>(outputs.params, outputs.fb.records, outputs.fb.rows,
+	                                                               keys, diff_model(d), q, width, height, pixels,
 	                                                               reinterpret_cast<float4 *>(images), visibility);
 	add_launches(1);
 	TRY(cudaGetLastError());

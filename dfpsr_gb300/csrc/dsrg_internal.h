@@ -172,6 +172,10 @@ struct PhaseGraph {
 	}
 };
 
+// Words of a context's control buffer, all zeroed by a batch's first launch.
+enum ControlWord : uint32_t { CONTROL_TILE_QUEUE = 0, CONTROL_ERROR = 1, CONTROL_EMIT = 2, CONTROL_BIG_RECORDS = 5, CONTROL_LISTED_TILES = 6, CONTROL_WORDS = 7 };
+static_assert(CONTROL_BIG_RECORDS == CONTROL_EMIT + EMIT_COUNTERS, "control words");
+
 struct BatchTotals {
 	uint32_t points = 0, triangles = 0, tiles = 0;
 	size_t pixels = 0;
@@ -204,18 +208,21 @@ struct dsrg_context_s {
 	DeviceBuffer<unsigned char> tables;  // the batch's task, frame and texture tables
 	unsigned char *pinnedTables = nullptr; // host staging of the tables (page-locked)
 	size_t pinnedCapacity = 0;
-	DeviceBuffer<uint32_t> control;      // [0] tile queue, [1] error flag, [4..7] a batch's gathered totals, [9] listed tiles
+	DeviceBuffer<uint32_t> control;      // a batch's counters (ControlWord)
 	DeviceBuffer<uint32_t> tileList;     // the tiles of a batch that have tile-list entries
 	uint32_t *pinnedReadback = nullptr;  // page-locked: the gathered totals (written there by the GPU), the fragment count,
-	                                     // [8] the entries a deterministic adjoint's sums keep
+	                                     // [8] the entries a deterministic adjoint's sums keep, [9] TOTALS_EXTRAS
 	uint32_t *readbackDevice = nullptr;  // its device address
 	bool timingPending = false;          // stats' times not yet read from the events of the last call
 	bool timingHasRaster = false;
 	bool stopRecorded = false;           // the last batch recorded eventStop before its host wait
 	// capacities of the buffers sized before their totals are known (largest totals seen, with slack)
-	uint64_t recordCapacity = 0, rowCapacity = 0, binCapacity = 0;
+	uint64_t extraCapacity = 0, recordCapacity = 0, rowCapacity = 0, binCapacity = 0;
 	DeviceBuffer<uint32_t> binCounts, binOffsets, binCursors, binLists;
-	DeviceBuffer<uint32_t> bigList;      // records binned a warp each (their count lives in control[8])
+	DeviceBuffer<uint32_t> bigList;      // records over more than four tiles
+	DeviceBuffer<uint32_t> drawnSlots, extraBase, extraIds, segmentSlots; // the one-pass setup (EmitBuffers)
+	DeviceBuffer<uint2> tileHeads;
+	DeviceBuffer<uint4> tileRanks;
 	DeviceBuffer<TextureData> textureTable;
 	DeviceBuffer<uint32_t> stagingColor;
 	DeviceBuffer<uint32_t> textureStaging;      // texture creation: host images and two-step resize halves

@@ -1,17 +1,16 @@
 // CUDA kernels of the DFPSR triangle path for sm_103a.
 //
 // Every launch covers a whole batch of frames (see dsrg_kernels.h).  Per batch:
-//   A  project_kernel       Camera::worldToScreen for every model point (implementation/render/Camera.h:157-190)
-//      setup_kernel<false>  per fan triangle: cull, clip, front-face; counts its draw records
-//      scan                 record offsets, so that records land in submission order
-//      setup_kernel<true>   writes the DrawRecords (bound, sub-pixel corners, projection)
-//   B  row_count_kernel     + scan: where each record's row intervals go
-//      bin_kernel<false>    + scan: (tile, record) pair counts per tile
-//   C  rows_kernel          row intervals of every record (rasterizeTriangle)
-//      bin_kernel<true>     per-tile record lists
-//      raster_kernel        persistent CTAs pull tiles from a queue; every fragment competes for
-//                           64-bit depth keys in shared memory; the winners go to the key image
-//      resolve_kernel       every pixel re-evaluates and shades its winning fragment
+//   A  project_kernel       Camera::worldToScreen for every model point (implementation/render/Camera.h:157-190),
+//                           and the counters of the launches behind it zeroed
+//      setup_emit_kernel    per fan triangle: cull, clip, front-face; writes the DrawRecords (bound, sub-pixel
+//                           corners, projection), takes their rows and counts their tiles
+//   B  bin_big_kernel       (tile, record) pairs of the records over more than four tiles
+//      scan                 where each tile's list begins
+//   C  rows_*_kernel        row intervals of every record (rasterizeTriangle)
+//      bin_fill_kernel      per-tile record lists
+//   D  raster_kernel        persistent CTAs pull tiles from a queue; every fragment competes for
+//                           64-bit depth keys in shared memory; every pixel re-evaluates and shades its winner
 //
 // Why the depth test can run out of order: the reference writes a fragment when its depth is
 // strictly greater (1/W, perspective) or smaller (linear, orthogonal) than the stored one
@@ -19,7 +18,7 @@
 // triangles the stored value is the extreme depth over all fragments that beat the initial
 // value, and the colour is the earliest fragment reaching it.  Packing (depth, ~record index)
 // into one 64-bit key and taking the maximum reproduces exactly that, in any order, because
-// the records of a frame are stored in submission order.
+// record numbers grow in submission order.
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <string.h>
@@ -122,8 +121,20 @@ __device__ __forceinline__ bool overflowed(const BatchParams &b) {
 
 // ------------------------------------------------------------------ projection
 
-__global__ void project_kernel(BatchParams b, ProjectedPoints out) {
+// The counters of a batch's later launches, zeroed by its first one (`clear`, see ClearedCounters):
+// no launch or memset of their own sits in the chain.
+__device__ __forceinline__ void clear_counters(const ClearedCounters &c) {
+	const uint32_t at = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+	for (uint32_t i = at; i < c.tileSlots; i += stride) {
+		c.tileCounts[i] = 0u;
+		c.tileCursors[i] = 0u;
+	}
+	for (uint32_t i = at; i < c.words; i += stride) c.control[i] = 0u;
+}
+
+__global__ void project_kernel(BatchParams b, ProjectedPoints out, ClearedCounters clear) {
 	chain_enter();
+	clear_counters(clear);
 	for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < b.totalPoints; i += gridDim.x * blockDim.x) {
 		const TaskParams &task = b.tasks[find_segment(b.taskPointBase, b.taskCount, i)];
 		const uint32_t local = i - task.pointBase;
@@ -142,10 +153,13 @@ __global__ void project_kernel(BatchParams b, ProjectedPoints out) {
 	}
 }
 
-void launch_project(const BatchParams &b, const FrameBuffers &fb, cudaStream_t stream) {
-	if (b.totalPoints == 0) return;
+void launch_project(const BatchParams &b, const FrameBuffers &fb, cudaStream_t stream, const ClearedCounters *clear) {
+	ClearedCounters none;
+	memset(&none, 0, sizeof(none));
+	if (!clear) clear = &none;
+	if (b.totalPoints == 0 && clear->words == 0) return;
 	COUNT_LAUNCH();
-	launch_chained(project_kernel, grid_for(b.totalPoints, 256), 256, stream, b, fb.points);
+	launch_chained(project_kernel, grid_for(std::max(b.totalPoints, clear->tileSlots), 256), 256, stream, b, fb.points, *clear);
 }
 
 // ------------------------------------------------------------------ triangle setup
@@ -185,8 +199,8 @@ __device__ void occlude_cells(const FrameTarget &f, const int64_t *fx, const int
 
 template <int MODE>
 __device__ void emit_record(const TaskParams &task, uint32_t taskIndex, const FrameTarget &frame, const FrameBuffers &fb,
-                            uint32_t recordCapacity, const Corner *c, const float *subB, const float *subC, uint32_t order,
-                            uint32_t tri, uint32_t base, uint32_t &emitted) {
+                            uint32_t recordCapacity, const Corner *c, const float *subB, const float *subC, uint32_t tri,
+                            uint32_t base, uint32_t &emitted) {
 	const int32_t width = frame.width, height = frame.height;
 	int64_t fx[3] = {c[0].fx, c[1].fx, c[2].fx}, fy[3] = {c[0].fy, c[1].fy, c[2].fy};
 	int32_t bd[4];
@@ -221,30 +235,37 @@ __device__ void emit_record(const TaskParams &task, uint32_t taskIndex, const Fr
 			float isx[3] = {c[0].isx, c[1].isx, c[2].isx}, isy[3] = {c[0].isy, c[1].isy, c[2].isy};
 			float csz[3] = {c[0].cs.z, c[1].cs.z, c[2].cs.z};
 			triangle_projection(isx, isy, csz, subB, subC, task.camera.perspective != 0, r.start, r.dx, r.dy);
-			r.order = order;
+			r.rowStart = 0; // written with the rows (rows_group_kernel)
 			r.tri = tri;
 			r.task = taskIndex;
 			r.frame = (uint32_t)task.frame;
 			r.source = task.triSource[tri];
 			fb.records[index] = r;
-			if (fb.counts.rowCounts) {
-				// the record's rows, and its tiles as bin_kernel<false> counts them
-				fb.counts.rowCounts[index] = (uint32_t)(r.bottom - r.top);
-				const uint32_t large = (fb.counts.depthOnly || !record_is_small(r, fb.counts.smallRows, fb.counts.smallWidth)) ? 1u : 0u;
-				const int32_t tx0 = r.left >> 4, ty0 = r.top >> 4;
-				const int32_t tx1 = min((r.right - 1) >> 4, frame.tilesX - 1), ty1 = min((r.bottom - 1) >> 4, frame.tilesY - 1);
-				const int32_t w = tx1 - tx0 + 1, h = ty1 - ty0 + 1;
-				const int32_t tiles = (w > 0 && h > 0) ? w * h : 0;
-				if (tiles > 4) {
-					fb.counts.bigList[atomicAdd(fb.counts.bigCount, 1u)] = index;
-				} else {
-					for (int32_t i = 0; i < tiles; i++)
-						atomicAdd(&fb.counts.binCounts[2u * (frame.tileBase + (uint32_t)((ty0 + i / w) * frame.tilesX + tx0 + i % w)) + large], 1u);
-				}
-			}
 		}
 	}
 	emitted++;
+}
+
+// The projected corners of fan triangle t of a task, and whether it is drawn at all: seen by the
+// camera, and not an alpha-filtered triangle whose three alphas are almost zero (renderCore.cpp:319).
+__device__ __forceinline__ bool load_triangle(const TaskParams &task, uint32_t t, const ProjectedPoints &points, Corner *c) {
+	const int32_t src = task.triSource[t];
+	const int32_t p = src >> 1, fan = src & 1;
+	const int corner[3] = {0, 1 + fan, 2 + fan}; // fan 0-1-2, 0-2-3 (model/Model.cpp:135-162, 164-183)
+	for (int i = 0; i < 3; i++) {
+		const uint32_t pi = task.pointBase + (uint32_t)task.polygons[p * 4 + corner[i]];
+		const float4 a = points.csis[pi];
+		const longlong2 f = points.flat[pi];
+		c[i].cs = vec3(a.x, a.y, a.z);
+		c[i].isx = a.w; c[i].isy = points.isy[pi];
+		c[i].fx = f.x; c[i].fy = f.y;
+	}
+	if (triangle_visibility(task.camera, c[0].cs, c[1].cs, c[2].cs, false) == 0) return false;
+	if (!task.depthOnly && task.filter == 1) {
+		const float *col = task.colors + p * 16;
+		if (almost_zero(col[corner[0] * 4 + 3]) && almost_zero(col[corner[1] * 4 + 3]) && almost_zero(col[corner[2] * 4 + 3])) return false;
+	}
+	return true;
 }
 
 // renderTriangleFromData / renderTriangleFromDataDepth for one fan triangle (renderCore.cpp:220-341, 400-443).
@@ -261,26 +282,8 @@ __global__ void __launch_bounds__(256) setup_kernel(BatchParams b, FrameBuffers 
 		uint32_t emitted = 0;
 		const uint32_t base = WRITE ? fb.triOffsets[g] : 0u;
 		if (WRITE && fb.triOffsets[g + 1] == base) continue; // the count pass emitted nothing for it
-		const int32_t src = task.triSource[t];
-		const int32_t p = src >> 1, fan = src & 1;
-		const int corner[3] = {0, 1 + fan, 2 + fan}; // fan 0-1-2, 0-2-3 (model/Model.cpp:135-162, 164-183)
 		Corner c[3];
-		for (int i = 0; i < 3; i++) {
-			const uint32_t pi = task.pointBase + (uint32_t)task.polygons[p * 4 + corner[i]];
-			const float4 a = fb.points.csis[pi];
-			const longlong2 f = fb.points.flat[pi];
-			c[i].cs = vec3(a.x, a.y, a.z);
-			c[i].isx = a.w; c[i].isy = fb.points.isy[pi];
-			c[i].fx = f.x; c[i].fy = f.y;
-		}
-		const uint32_t order = (task.orderBase + t) * 8u;
-		bool visible = triangle_visibility(task.camera, c[0].cs, c[1].cs, c[2].cs, false) != 0;
-		if (visible && !task.depthOnly && task.filter == 1) {
-			// renderTriangleFromData skips alpha-filtered triangles whose three alphas are almost zero (renderCore.cpp:319)
-			const float *col = task.colors + p * 16;
-			if (almost_zero(col[corner[0] * 4 + 3]) && almost_zero(col[corner[1] * 4 + 3]) && almost_zero(col[corner[2] * 4 + 3]))
-				visible = false;
-		}
+		const bool visible = load_triangle(task, t, fb.points, c);
 		if (visible && hasTarget) {
 			const float defaultB[3] = {0.0f, 1.0f, 0.0f}, defaultC[3] = {0.0f, 0.0f, 1.0f};
 			const float zero3[3] = {0.0f, 0.0f, 0.0f};
@@ -288,7 +291,7 @@ __global__ void __launch_bounds__(256) setup_kernel(BatchParams b, FrameBuffers 
 				int64_t fx[3] = {c[0].fx, c[1].fx, c[2].fx}, fy[3] = {c[0].fy, c[1].fy, c[2].fy};
 				if (is_frontfacing(fx, fy)) {
 					emit_record<MODE>(task, k, frame, fb, recordCapacity, c, task.depthOnly ? zero3 : defaultB,
-					                   task.depthOnly ? zero3 : defaultC, order, t, base, emitted);
+					                   task.depthOnly ? zero3 : defaultC, t, base, emitted);
 				}
 			} else {
 				ClippedPolygon poly;
@@ -310,7 +313,7 @@ __global__ void __launch_bounds__(256) setup_kernel(BatchParams b, FrameBuffers 
 						float sb[3] = {sv[0]->subB, sv[1]->subB, sv[2]->subB};
 						float scc[3] = {sv[0]->subC, sv[1]->subC, sv[2]->subC};
 						emit_record<MODE>(task, k, frame, fb, recordCapacity, sc, task.depthOnly ? zero3 : sb,
-						                   task.depthOnly ? zero3 : scc, order + (uint32_t)f, t, base, emitted);
+						                   task.depthOnly ? zero3 : scc, t, base, emitted);
 					}
 				}
 			}
@@ -339,6 +342,230 @@ void launch_setup_occlude(const BatchParams &b, const FrameBuffers &fb, cudaStre
 	if (b.totalTriangles == 0) return;
 	COUNT_LAUNCH();
 	launch_chained(setup_kernel<SETUP_OCCLUDE>, grid_for(b.totalTriangles, 256), 256, stream, b, fb, 0u);
+}
+
+// ------------------------------------------------------------------ one-pass triangle setup
+
+// One draw command on its way to a record: its corners and its raster bound.
+struct Command {
+	float isx[3], isy[3], csz[3];
+	int32_t flat[6];
+	int32_t left, top, right, bottom;
+};
+
+// Takes the corners over and cuts their bound to the target with rows aligned to pairs
+// (ITriangle2D.cpp:70-75); false when the command faces away, lies outside or lies behind every
+// cell of the occlusion grid.
+__device__ __forceinline__ bool make_command(const FrameTarget &f, const Corner *c, int32_t *errorFlag, Command &m) {
+	const int64_t fx[3] = {c[0].fx, c[1].fx, c[2].fx}, fy[3] = {c[0].fy, c[1].fy, c[2].fy};
+	if (!is_frontfacing(fx, fy)) return false;
+	int32_t bd[4];
+	triangle_bound(fx, fy, bd);
+	if (f.occlusion &&
+	    !command_survives(f.occlusion, f.gridWidth, f.gridHeight, f.gridStride, bd, nearest_corner(c[0].cs.z, c[1].cs.z, c[2].cs.z)))
+		return false;
+	if (!(bd[0] < f.width && bd[2] > 0 && bd[1] < f.height && bd[3] > 0)) return false;
+	bool inRange = true;
+	for (int i = 0; i < 3; i++) {
+		if (fx[i] < -(1ll << 30) || fx[i] > (1ll << 30) || fy[i] < -(1ll << 30) || fy[i] > (1ll << 30)) inRange = false;
+		m.flat[2 * i] = (int32_t)fx[i];
+		m.flat[2 * i + 1] = (int32_t)fy[i];
+		m.isx[i] = c[i].isx;
+		m.isy[i] = c[i].isy;
+		m.csz[i] = c[i].cs.z;
+	}
+	if (!inRange) atomicOr(errorFlag, ERROR_COORDINATE_RANGE);
+	m.left = bd[0] > 0 ? bd[0] : 0;
+	m.top = (bd[1] > 0 ? bd[1] : 0) & ~1;                           // roundDown(top, 2)
+	m.right = bd[2] < f.width ? bd[2] : f.width;
+	m.bottom = ((bd[3] < f.height ? bd[3] : f.height) + 1) & ~1;    // roundUp(bottom, 2)
+	return true;
+}
+
+// Rows the command takes: its bound's, in whole segments where segments are listed.
+__device__ __forceinline__ uint32_t command_rows(const Command &m, const EmitBuffers &emit) {
+	const uint32_t rows = (uint32_t)(m.bottom - m.top);
+	return emit.segmentSlots ? (rows + ROW_SEGMENT - 1) / ROW_SEGMENT * ROW_SEGMENT : rows;
+}
+
+__device__ __forceinline__ int32_t command_tiles(const Command &m, const FrameTarget &f, int32_t &tx0, int32_t &ty0, int32_t &w) {
+	tx0 = m.left >> 4;
+	ty0 = m.top >> 4;
+	w = min((m.right - 1) >> 4, f.tilesX - 1) - tx0 + 1;
+	const int32_t h = min((m.bottom - 1) >> 4, f.tilesY - 1) - ty0 + 1;
+	return (w > 0 && h > 0) ? w * h : 0;
+}
+
+// Writes a command's record and what the launches behind it need.  subB, subC: its corners' places
+// in the fan triangle.
+__device__ __forceinline__ void store_command(const BatchParams &b, const FrameBuffers &fb, const TaskParams &task, uint32_t taskIndex,
+                                              const FrameTarget &f, uint32_t tri, const Command &m, const float *subB, const float *subC,
+                                              uint32_t slot, uint32_t rowStart, uint32_t drawnAt, uint32_t bigAt) {
+	const EmitBuffers &emit = fb.emit;
+	int32_t tx0, ty0, w;
+	const int32_t tiles = command_tiles(m, f, tx0, ty0, w);
+	emit.drawn[drawnAt] = slot;
+	if (tiles > 4) {
+		emit.tileHeads[drawnAt] = make_uint2(0u, 0u);
+		emit.bigList[bigAt] = slot;
+	} else {
+		// a place in each tile's list: the atomics' answers arrive while the record is made
+		const uint32_t large = (b.depthOnly || !bound_is_small(m.left, m.top, m.right, m.bottom, b.smallRows, b.smallWidth)) ? 1u : 0u;
+		const uint32_t first = 2u * (f.tileBase + (uint32_t)(ty0 * f.tilesX + tx0)) + large;
+		uint32_t rank[4] = {0u, 0u, 0u, 0u};
+		// tile i at column i % w, row i / w (w at most 4)
+#pragma unroll
+		for (int32_t i = 0; i < 4; i++) {
+			const int32_t row = w == 1 ? i : (w == 2 ? i >> 1 : (i >= w ? 1 : 0));
+			if (i < tiles) rank[i] = atomicAdd(&emit.tileCursors[first + 2u * (uint32_t)(row * f.tilesX + i - row * w)], 1u);
+		}
+		emit.tileHeads[drawnAt] = make_uint2(first, (uint32_t)f.tilesX | ((uint32_t)w << 16) | ((uint32_t)tiles << 24));
+		emit.tileRanks[drawnAt] = make_uint4(rank[0], rank[1], rank[2], rank[3]);
+	}
+	const uint32_t rows = command_rows(m, emit);
+	if (rowStart + rows > fb.rowCapacity) atomicOr(fb.errorFlag, ERROR_ROW_OVERFLOW);
+	if (emit.segmentSlots)
+		for (uint32_t s = rowStart / ROW_SEGMENT; s < (rowStart + rows) / ROW_SEGMENT && s < fb.rowCapacity / ROW_SEGMENT; s++)
+			emit.segmentSlots[s] = slot;
+	DrawRecord r;
+	for (int i = 0; i < 6; i++) r.flat[i] = m.flat[i];
+	r.left = m.left; r.top = m.top; r.right = m.right; r.bottom = m.bottom;
+	triangle_projection(m.isx, m.isy, m.csz, subB, subC, task.camera.perspective != 0, r.start, r.dx, r.dy);
+	r.rowStart = rowStart;
+	r.tri = tri;
+	r.task = taskIndex;
+	r.frame = (uint32_t)task.frame;
+	r.source = task.triSource[tri];
+	fb.records[slot] = r;
+}
+
+// A fan triangle that crosses a clipping plane: every piece is stored on its own, the first at the
+// triangle's slot (renderTriangleFromData, renderCore.cpp:220-341).  Out of line: few triangles come
+// here, and the polygon would cost the others their registers.
+__device__ __noinline__ void emit_clipped(const BatchParams &b, const FrameBuffers &fb, uint32_t g, uint32_t k, const Corner *corners) {
+	const TaskParams &task = b.tasks[k];
+	const FrameTarget &f = b.frames[task.frame];
+	const EmitBuffers &emit = fb.emit;
+	const uint32_t t = g - task.triangleBase;
+	ClippedPolygon poly;
+	poly.count = 3;
+	for (int i = 0; i < 3; i++) { poly.v[i].cs = corners[i].cs; poly.v[i].state = 0; poly.v[i].value = 0.0f; }
+	poly.v[0].subB = 0.0f; poly.v[0].subC = 0.0f;
+	poly.v[1].subB = 1.0f; poly.v[1].subC = 0.0f;
+	poly.v[2].subB = 0.0f; poly.v[2].subC = 1.0f;
+	for (int s = 0; s < task.camera.clipCount; s++) poly.clip(task.camera.clip[s]);
+	uint32_t pieces = 0, base = 0;
+	for (int n = 0; n < poly.count - 2; n++) {
+		const SubVertex *sv[3] = {&poly.v[0], &poly.v[1 + n], &poly.v[2 + n]};
+		Corner c[3];
+		float subB[3], subC[3];
+		for (int i = 0; i < 3; i++) {
+			const Projected pr = camera_to_screen(task.camera, sv[i]->cs);
+			c[i].cs = pr.cs; c[i].isx = pr.isx; c[i].isy = pr.isy; c[i].fx = pr.flatx; c[i].fy = pr.flaty;
+			subB[i] = task.depthOnly ? 0.0f : sv[i]->subB;
+			subC[i] = task.depthOnly ? 0.0f : sv[i]->subC;
+		}
+		Command m;
+		if (!make_command(f, c, fb.errorFlag, m)) continue;
+		uint64_t slot = g;
+		if (pieces == 1) { // extra slots for this piece and all that can follow it
+			base = atomicAdd(&emit.counters[EMIT_EXTRAS], (uint32_t)(poly.count - 2 - n));
+			emit.extraBase[g] = base;
+		}
+		if (pieces > 0) {
+			slot = (uint64_t)b.totalTriangles + base + (pieces - 1);
+			if (slot < emit.capacity) emit.extraIds[base + (pieces - 1)] = (g << 3) | pieces;
+		}
+		pieces++;
+		if (slot >= emit.capacity) {
+			atomicOr(fb.errorFlag, ERROR_RECORD_OVERFLOW);
+			continue;
+		}
+		int32_t tx0, ty0, w;
+		const bool big = command_tiles(m, f, tx0, ty0, w) > 4;
+		store_command(b, fb, task, k, f, t, m, subB, subC, (uint32_t)slot, atomicAdd(&emit.counters[EMIT_ROWS], command_rows(m, emit)),
+		              atomicAdd(&emit.counters[EMIT_DRAWN], 1u), big ? atomicAdd(emit.bigCount, 1u) : 0u);
+	}
+}
+
+// One thread per fan triangle (renderTriangleFromData, renderCore.cpp:220-341, 400-443).  The record
+// of triangle g goes to slot g and is numbered 8 * g; further pieces of a clipped triangle go to
+// extra slots as numbers 8 * g + 1 .. 8 * g + 6 (record_slot), so that record numbers grow in
+// submission order wherever the records lie, and nothing has to be counted and scanned before they
+// can be written.  The rows, the list of drawn records and the list of big ones are taken from
+// counters, one atomic of each per block of 256 triangles; a record over at most four tiles takes
+// its place in their lists at once (what the atomic on the list's cursor returns).
+// This pass takes the place of a counting pass over the same triangles, two scans (of the
+// triangles' records and of the records' rows) and the atomics of the list-filling pass:
+// a terrain frame of 522,242 triangles went from 304 to 290 us, 64 views of 50,000 triangles (forward,
+// loss and adjoint) from 960 to 938 us, a frame of 400 triangles (64x64) from 114 to 107 us with 7 launches
+// less.  It is bound by the latency of its gathers and atomics, so four blocks per SM with a few
+// spilled registers beat two with none (128 registers: 1,015 us for the 64 views).
+__global__ void __launch_bounds__(256, 4) setup_emit_kernel(BatchParams b, FrameBuffers fb) {
+	chain_enter();
+	__shared__ uint32_t warpRows[8], warpDrawn[8], warpBig[8], taken[3];
+	const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+	const EmitBuffers &emit = fb.emit;
+	for (uint32_t g0 = blockIdx.x * 256u; g0 < b.totalTriangles; g0 += gridDim.x * 256u) { // uniform per block
+		const uint32_t g = g0 + threadIdx.x;
+		Command m;
+		bool drawn = false, big = false;
+		uint32_t k = 0, rows = 0;
+		if (g < b.totalTriangles) {
+			k = (uint32_t)find_segment(b.taskTriangleBase, b.taskCount, g);
+			const TaskParams &task = b.tasks[k];
+			const FrameTarget &f = b.frames[task.frame];
+			Corner c[3];
+			if (load_triangle(task, g - task.triangleBase, fb.points, c) && (f.color != nullptr || f.depth != nullptr)) {
+				if (triangle_visibility(task.camera, c[0].cs, c[1].cs, c[2].cs, true) == 1) {
+					drawn = make_command(f, c, fb.errorFlag, m);
+				} else {
+					Corner copy[3] = {c[0], c[1], c[2]};
+					emit_clipped(b, fb, g, k, copy);
+				}
+			}
+			if (drawn) {
+				int32_t tx0, ty0, w;
+				rows = command_rows(m, emit);
+				big = command_tiles(m, f, tx0, ty0, w) > 4;
+			}
+		}
+		// this block's share of the counters, then each thread's place in it
+		const uint32_t drawnMask = __ballot_sync(0xFFFFFFFFu, drawn), bigMask = __ballot_sync(0xFFFFFFFFu, big);
+		uint32_t inclusive = rows;
+		for (int o = 1; o < 32; o <<= 1) {
+			const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, inclusive, o);
+			if (lane >= (uint32_t)o) inclusive += v;
+		}
+		if (lane == 31) { warpRows[warp] = inclusive; warpDrawn[warp] = __popc(drawnMask); warpBig[warp] = __popc(bigMask); }
+		__syncthreads();
+		if (threadIdx.x < 3) {
+			const uint32_t *of = threadIdx.x == 0 ? warpRows : (threadIdx.x == 1 ? warpDrawn : warpBig);
+			uint32_t total = 0;
+			for (int i = 0; i < 8; i++) total += of[i];
+			uint32_t *counter = threadIdx.x == 0 ? &emit.counters[EMIT_ROWS] : (threadIdx.x == 1 ? &emit.counters[EMIT_DRAWN] : emit.bigCount);
+			taken[threadIdx.x] = total ? atomicAdd(counter, total) : 0u;
+		}
+		__syncthreads();
+		if (drawn) {
+			uint32_t rowStart = taken[0] + inclusive - rows, drawnAt = taken[1], bigAt = taken[2];
+			for (uint32_t i = 0; i < warp; i++) { rowStart += warpRows[i]; drawnAt += warpDrawn[i]; bigAt += warpBig[i]; }
+			const uint32_t before = (1u << lane) - 1u;
+			drawnAt += __popc(drawnMask & before);
+			bigAt += __popc(bigMask & before);
+			const TaskParams &task = b.tasks[k];
+			const float one = task.depthOnly ? 0.0f : 1.0f; // depth only: no weights
+			const float subB[3] = {0.0f, one, 0.0f}, subC[3] = {0.0f, 0.0f, one};
+			store_command(b, fb, task, k, b.frames[task.frame], g - task.triangleBase, m, subB, subC, g, rowStart, drawnAt, bigAt);
+		}
+		__syncthreads(); // the shared totals are read before the next round writes them
+	}
+}
+
+void launch_setup_emit(const BatchParams &b, const FrameBuffers &fb, cudaStream_t stream) {
+	if (b.totalTriangles == 0) return;
+	COUNT_LAUNCH();
+	launch_chained(setup_emit_kernel, grid_for(b.totalTriangles, 256), 256, stream, b, fb);
 }
 
 // One thread per cell of the grid: the cell's run of the top pixel row of its cell row.  The
@@ -380,7 +607,8 @@ void launch_occlusion_top_rows(float *grid, int32_t gridWidth, int32_t gridHeigh
 // Exclusive scan in two launches and no host round trip: the first writes one sum per chunk of
 // SCAN_CHUNK values, the second gives every chunk the sum of the chunk sums before it (read by
 // the whole block) and scans the chunk through shared memory.  The length may live on the
-// device (a count written by an earlier kernel), with `capacity` bounding it for the grid.
+// device (a count written by an earlier kernel), with `capacity` bounding it for the grid.  With
+// `plus` the scan is over in[i] + plus[i].
 static const int SCAN_THREADS = 256;
 static const int SCAN_PER_THREAD = 16;
 static const uint32_t SCAN_CHUNK = SCAN_THREADS * SCAN_PER_THREAD;
@@ -401,19 +629,21 @@ __device__ __forceinline__ uint32_t block_sum(uint32_t v, uint32_t *shared) {
 	return total;
 }
 
-__global__ void __launch_bounds__(SCAN_THREADS) scan_reduce_kernel(const uint32_t *__restrict__ in, uint32_t n, const uint32_t *nDevice,
+__global__ void __launch_bounds__(SCAN_THREADS) scan_reduce_kernel(const uint32_t *__restrict__ in, const uint32_t *__restrict__ plus,
+                                                                   uint32_t n, const uint32_t *nDevice,
                                                                    uint32_t capacity, uint32_t *chunkSums) {
 	chain_enter();
 	__shared__ uint32_t warpSums[SCAN_THREADS / 32];
 	const uint32_t count = scan_length(n, nDevice, capacity);
 	const uint32_t begin = blockIdx.x * SCAN_CHUNK;
 	uint32_t v = 0;
-	for (uint32_t i = begin + threadIdx.x; i < begin + SCAN_CHUNK && i < count; i += SCAN_THREADS) v += in[i];
+	for (uint32_t i = begin + threadIdx.x; i < begin + SCAN_CHUNK && i < count; i += SCAN_THREADS) v += in[i] + (plus ? plus[i] : 0u);
 	const uint32_t total = block_sum(v, warpSums);
 	if (threadIdx.x == 0) chunkSums[blockIdx.x] = total;
 }
 
-__global__ void __launch_bounds__(SCAN_THREADS) scan_apply_kernel(const uint32_t *__restrict__ in, uint32_t *out, uint32_t n,
+__global__ void __launch_bounds__(SCAN_THREADS) scan_apply_kernel(const uint32_t *__restrict__ in, const uint32_t *__restrict__ plus, uint32_t *out,
+                                                                  uint32_t n,
                                                                   const uint32_t *nDevice, uint32_t capacity,
                                                                   const uint32_t *__restrict__ chunkSums) {
 	chain_enter();
@@ -429,7 +659,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) scan_apply_kernel(const uint32_t
 	for (int k = 0; k < SCAN_PER_THREAD; k++) {
 		const uint32_t i = begin + k * SCAN_THREADS + threadIdx.x;
 		const uint32_t at = k * SCAN_THREADS + threadIdx.x;
-		values[at + (at >> 5)] = i < count ? in[i] : 0u;
+		values[at + (at >> 5)] = i < count ? in[i] + (plus ? plus[i] : 0u) : 0u;
 	}
 	__syncthreads();
 	uint32_t local[SCAN_PER_THREAD];
@@ -470,7 +700,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) scan_apply_kernel(const uint32_t
 
 size_t scan_scratch_elems(uint32_t n) { return (size_t)(n / SCAN_CHUNK) + 16; }
 
-static void scan_launch(const uint32_t *in, uint32_t *out, uint32_t n, const uint32_t *nDevice, uint32_t *scratch, size_t scratchElems,
+static void scan_launch(const uint32_t *in, const uint32_t *plus, uint32_t *out, uint32_t n, const uint32_t *nDevice, uint32_t *scratch, size_t scratchElems,
                         cudaStream_t stream) {
 	const uint32_t blocks = n / SCAN_CHUNK + 1; // n = the length, or the capacity bounding a device length
 	if (blocks > scratchElems) {
@@ -478,36 +708,36 @@ static void scan_launch(const uint32_t *in, uint32_t *out, uint32_t n, const uin
 		return;
 	}
 	COUNT_LAUNCH();
-	launch_chained(scan_reduce_kernel, blocks, SCAN_THREADS, stream, in, n, nDevice, n, scratch);
+	launch_chained(scan_reduce_kernel, blocks, SCAN_THREADS, stream, in, plus, n, nDevice, n, scratch);
 	COUNT_LAUNCH();
-	launch_chained(scan_apply_kernel, blocks, SCAN_THREADS, stream, in, out, n, nDevice, n, scratch);
+	launch_chained(scan_apply_kernel, blocks, SCAN_THREADS, stream, in, plus, out, n, nDevice, n, scratch);
 }
 
 
 void launch_scan(const uint32_t *in, uint32_t *out, uint32_t n, uint32_t *scratch, size_t scratchElems, cudaStream_t stream) {
-	scan_launch(in, out, n, nullptr, scratch, scratchElems, stream);
+	scan_launch(in, nullptr, out, n, nullptr, scratch, scratchElems, stream);
 }
 
 void launch_scan_device(const uint32_t *in, uint32_t *out, const uint32_t *nDevice, uint32_t capacity, uint32_t *scratch,
                         size_t scratchElems, cudaStream_t stream) {
-	scan_launch(in, out, capacity, nDevice, scratch, scratchElems, stream);
+	scan_launch(in, nullptr, out, capacity, nDevice, scratch, scratchElems, stream);
 }
 
-// The totals a batch's host side reads once its phases ran: records, rows, tile-list entries and
-// the error bits, gathered into one small block for a single copy.  The same launch lists the
-// tiles that have entries (one thread per tile, warp-aggregated appends), so that the persistent
-// tile kernel pulls only those: frames that are mostly empty (shadow-cube faces) no longer send
-// every CTA through thousands of empty tiles.
-__global__ void gather_totals_kernel(const uint32_t *triOffsets, uint32_t triangles, const uint32_t *rowOffsets, uint32_t recordCapacity,
-                                     const uint32_t *binOffsets, uint32_t tiles, const int32_t *errorFlag, uint32_t *out,
-                                     uint32_t *tileList, uint32_t *tileListCount) {
+// The totals a batch's host side reads once its phases ran: records, rows, tile-list entries, the
+// error bits and the extra records of clipped triangles, gathered into one small block.  The same
+// launch lists the tiles that have entries (one thread per tile, warp-aggregated appends), so that
+// the persistent tile kernel pulls only those: frames that are mostly empty (shadow-cube faces) no
+// longer send every CTA through thousands of empty tiles.
+__global__ void gather_totals_kernel(TotalsSources from, const uint32_t *binOffsets, uint32_t tiles, uint32_t *out, uint32_t *tileList,
+                                     uint32_t *tileListCount) {
 	chain_enter();
 	if (blockIdx.x == 0 && threadIdx.x == 0) {
-		const uint32_t records = triOffsets[triangles];
+		const uint32_t records = *from.records;
 		out[0] = records;
-		out[1] = rowOffsets[records < recordCapacity ? records : recordCapacity];
+		out[1] = from.rowOffsets ? from.rowOffsets[records < from.recordCapacity ? records : from.recordCapacity] : *from.rows;
 		out[2] = binOffsets[2 * tiles];
-		out[3] = (uint32_t)*errorFlag;
+		out[3] = (uint32_t)*from.errorFlag;
+		out[TOTALS_EXTRAS] = from.extras ? *from.extras : 0u;
 	}
 	if (!tileList) return;
 	const uint32_t lane = threadIdx.x & 31u;
@@ -524,12 +754,11 @@ __global__ void gather_totals_kernel(const uint32_t *triOffsets, uint32_t triang
 	}
 }
 
-void launch_gather_totals(const uint32_t *triOffsets, uint32_t triangles, const uint32_t *rowOffsets, uint32_t recordCapacity,
-                          const uint32_t *binOffsets, uint32_t tiles, const int32_t *errorFlag, uint32_t *out, uint32_t *tileList,
+void launch_gather_totals(const TotalsSources &from, const uint32_t *binOffsets, uint32_t tiles, uint32_t *out, uint32_t *tileList,
                           uint32_t *tileListCount, cudaStream_t stream) {
 	COUNT_LAUNCH();
-	launch_chained(gather_totals_kernel, tileList ? grid_for(tiles, 256) : 1u, tileList ? 256u : 1u, stream, triOffsets, triangles, rowOffsets,
-	               recordCapacity, binOffsets, tiles, errorFlag, out, tileList, tileListCount);
+	launch_chained(gather_totals_kernel, tileList ? grid_for(tiles, 256) : 1u, tileList ? 256u : 1u, stream, from, binOffsets, tiles, out,
+	               tileList, tileListCount);
 }
 
 // ------------------------------------------------------------------ row intervals
@@ -553,127 +782,8 @@ void launch_row_offsets(const FrameBuffers &fb, uint32_t recordCount, uint32_t *
 		launch_scan(rowCounts, fb.rowOffsets, recordCount, fb.scanScratch, fb.scanScratchElems, stream);
 }
 
-// Row interval of row y for corners held in registers (row_interval without the corner array).
-__device__ __forceinline__ void row_interval_regs(int32_t x0, int32_t y0, int32_t x1, int32_t y1, int32_t x2, int32_t y2,
-                                                  int32_t y, int32_t L, int32_t R, int32_t &left, int32_t &right) {
-	if ((x0 == x1 && y0 == y1) || (x1 == x2 && y1 == y2) || (x2 == x0 && y2 == y0)) { left = R; right = L; return; }
-	left = L; right = R;
-	cut_row(make_edge(x0, y0, x1, y1), y, L, R, left, right);
-	cut_row(make_edge(x1, y1, x2, y2), y, L, R, left, right);
-	cut_row(make_edge(x2, y2, x0, y0), y, L, R, left, right);
-}
-
-// The row intervals of every record (rasterizeTriangle, ITriangle2D.cpp:150-176), balanced by rows:
-// each CTA takes ROWS_CHUNK consecutive rows of the concatenation of all records' rows (one warp
-// finds the records they belong to with a 32-way search over the row offsets), stages those
-// records' corners in shared memory, gives each thread ROWS_PER_THREAD consecutive rows and
-// writes the chunk back coalesced.  Every record has at least two rows (raster bounds cover row
-// pairs), so a chunk spans at most ROWS_CHUNK / 2 + 2 records.
-static const int ROWS_THREADS = 256;
-static const int ROWS_PER_THREAD = 4;
-static const uint32_t ROWS_CHUNK = ROWS_THREADS * ROWS_PER_THREAD;
-static const uint32_t ROWS_MAX_RECORDS = ROWS_CHUNK / 2 + 2;
-
-// The largest r in [0, n) with offsets[r] <= v (offsets non-decreasing, offsets[0] = 0 <= v), by one warp.
-__device__ __forceinline__ uint32_t warp_search(const uint32_t *offsets, uint32_t n, uint32_t v) {
-	const uint32_t lane = threadIdx.x & 31;
-	uint32_t lo = 0, hi = n;
-	while (hi - lo > 32) {
-		const uint32_t step = (hi - lo + 31) / 32;
-		const uint32_t probe = lo + lane * step;
-		const bool below = probe < hi && offsets[probe] <= v;
-		const uint32_t k = 31 - __clz(__ballot_sync(0xFFFFFFFFu, below));
-		lo += k * step;
-		hi = min(lo + step, hi);
-	}
-	const uint32_t probe = lo + lane;
-	const bool below = probe < hi && offsets[probe] <= v;
-	return lo + (31 - __clz(__ballot_sync(0xFFFFFFFFu, below)));
-}
-
-__global__ void __launch_bounds__(ROWS_THREADS) rows_chunk_kernel(const DrawRecord *__restrict__ records, uint32_t capacity,
-                                                            const uint32_t *countDevice, const uint32_t *__restrict__ rowOffsets,
-                                                            uint32_t *rows, uint32_t rowCapacity, int32_t *errorFlag) {
-	chain_enter();
-	__shared__ uint32_t first, last;
-	__shared__ uint32_t offsets[ROWS_MAX_RECORDS + 1];
-	__shared__ int4 cornersA[ROWS_MAX_RECORDS];   // flat 0..3
-	__shared__ int4 cornersB[ROWS_MAX_RECORDS];   // flat 4..5, left, top
-	__shared__ int32_t rights[ROWS_MAX_RECORDS];
-	__shared__ uint32_t out[ROWS_CHUNK + ROWS_CHUNK / 32];
-	const uint32_t n = device_count(capacity, countDevice);
-	if (n == 0) return;
-	const uint32_t total = rowOffsets[n];
-	for (uint32_t begin = blockIdx.x * ROWS_CHUNK; begin < total; begin += gridDim.x * ROWS_CHUNK) {
-		const uint32_t end = min(begin + ROWS_CHUNK, total);
-		if (threadIdx.x < 32) {
-			const uint32_t f = warp_search(rowOffsets, n, begin);
-			const uint32_t l = warp_search(rowOffsets, n, end - 1);
-			if (threadIdx.x == 0) { first = f; last = l; }
-		}
-		__syncthreads();
-		uint32_t count = last - first + 1;
-		if (count > ROWS_MAX_RECORDS) { // only records without rows could do this, and none are made
-			if (threadIdx.x == 0) atomicOr(errorFlag, ERROR_INTERNAL);
-			count = ROWS_MAX_RECORDS;
-		}
-		for (uint32_t k = threadIdx.x; k < count; k += ROWS_THREADS) {
-			const DrawRecord &r = records[first + k];
-			cornersA[k] = __ldg(reinterpret_cast<const int4 *>(&r.flat[0]));
-			cornersB[k] = __ldg(reinterpret_cast<const int4 *>(&r.flat[4]));
-			rights[k] = r.right;
-			offsets[k] = rowOffsets[first + k];
-		}
-		if (threadIdx.x == 0) offsets[count] = rowOffsets[first + count];
-		__syncthreads();
-		// this thread's rows: [j0, j0 + ROWS_PER_THREAD) within the chunk
-		const uint32_t j0 = begin + threadIdx.x * ROWS_PER_THREAD;
-		if (j0 < end) {
-			uint32_t lo = 0, hi = count; // the record holding row j0
-			while (hi - lo > 1) {
-				const uint32_t mid = (lo + hi) >> 1;
-				if (offsets[mid] <= j0) lo = mid; else hi = mid;
-			}
-			uint32_t k = lo;
-			const uint32_t jEnd = min(j0 + (uint32_t)ROWS_PER_THREAD, end);
-			if (offsets[k + 1] >= jEnd) {
-				// all of this thread's rows belong to one record: stepped from the first (two divisions
-				// per edge instead of one per edge and row; rows past jEnd are stepped but not kept)
-				const int4 a = cornersA[k], c = cornersB[k];
-				const int32_t flat[6] = {a.x, a.y, a.z, a.w, c.x, c.y};
-				int32_t lefts[ROWS_PER_THREAD], rightsOut[ROWS_PER_THREAD];
-				row_intervals_stepped(flat, c.w + (int32_t)(j0 - offsets[k]), ROWS_PER_THREAD, c.z, rights[k], lefts, rightsOut);
-#pragma unroll
-				for (int i = 0; i < ROWS_PER_THREAD; i++) {
-					const uint32_t j = j0 + i;
-					if (j >= jEnd) break;
-					const uint32_t at = j - begin;
-					out[at + (at >> 5)] = (uint32_t)(lefts[i] & 0xFFFF) | ((uint32_t)rightsOut[i] << 16);
-				}
-			} else {
-				for (int i = 0; i < ROWS_PER_THREAD; i++) {
-					const uint32_t j = j0 + i;
-					if (j >= end) break;
-					while (offsets[k + 1] <= j) k++;
-					const int4 a = cornersA[k], c = cornersB[k];
-					int32_t left, right;
-					row_interval_regs(a.x, a.y, a.z, a.w, c.x, c.y, c.w + (int32_t)(j - offsets[k]), c.z, rights[k], left, right);
-					const uint32_t at = j - begin;
-					out[at + (at >> 5)] = (uint32_t)(left & 0xFFFF) | ((uint32_t)right << 16);
-				}
-			}
-		}
-		__syncthreads();
-		for (uint32_t at = threadIdx.x; at < end - begin; at += ROWS_THREADS) {
-			const uint32_t j = begin + at;
-			if (j < rowCapacity) rows[j] = out[at + (at >> 5)];
-			else atomicOr(errorFlag, ERROR_ROW_OVERFLOW);
-		}
-		__syncthreads();
-	}
-}
-
 static const int32_t ROWS_STEPPED_MAX = 16; // records of at most this many rows are stepped by one lane each
+static_assert(ROWS_STEPPED_MAX == ROW_SEGMENT, "a segment is what one lane steps");
 
 // The row intervals of every record, stepped exactly (row_intervals_stepped: two floor divisions
 // per edge start a segment of rows, then one carry step per edge and row).  Each warp takes 32
@@ -681,26 +791,31 @@ static const int32_t ROWS_STEPPED_MAX = 16; // records of at most this many rows
 // own record; otherwise the records are cut into segments of up to ROWS_STEPPED_MAX rows that are
 // spread over the lanes (a lane finds its record by a search over the warp's prefix sums of
 // segment counts and fetches its corners with shuffles), so tall triangles keep every lane busy.
-__global__ void __launch_bounds__(256, 3) rows_group_kernel(const DrawRecord *__restrict__ records, uint32_t capacity,
-                                                   const uint32_t *countDevice, const uint32_t *__restrict__ rowOffsets,
+// `drawn` lists the records (null: all of the first recordCount).  With rowOffsets (the two-pass
+// setup) the rows lie where that scan put them and rowStart is written; otherwise rowStart holds
+// where setup_emit_kernel put them.
+__global__ void __launch_bounds__(256, 3) rows_group_kernel(DrawRecord *records, uint32_t capacity, const uint32_t *countDevice,
+                                                   const uint32_t *__restrict__ drawn, const uint32_t *__restrict__ rowOffsets,
                                                    uint32_t *rows, uint32_t rowCapacity, int32_t *errorFlag) {
 	chain_enter();
 	const uint32_t recordCount = device_count(capacity, countDevice);
 	const int lane = threadIdx.x & 31;
 	const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
 	for (uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w * 32u < recordCount; w += warps) {
-		const uint32_t i = w * 32u + (uint32_t)lane;
+		uint32_t i = w * 32u + (uint32_t)lane;
 		int32_t count = 0, top = 0, L = 0, R = 0;
 		int32_t f0 = 0, f1 = 0, f2 = 0, f3 = 0, f4 = 0, f5 = 0;
 		uint32_t out = 0;
 		if (i < recordCount) {
-			const int4 a = __ldg(reinterpret_cast<const int4 *>(&records[i].flat[0]));   // flat[0..3]
-			const int4 b = __ldg(reinterpret_cast<const int4 *>(&records[i].flat[4]));   // flat[4..5], left, top
-			const int2 c = __ldg(reinterpret_cast<const int2 *>(&records[i].right));     // right, bottom
+			if (drawn) i = drawn[i];
+			const int4 a = *reinterpret_cast<const int4 *>(&records[i].flat[0]);   // flat[0..3]
+			const int4 b = *reinterpret_cast<const int4 *>(&records[i].flat[4]);   // flat[4..5], left, top
+			const int2 c = *reinterpret_cast<const int2 *>(&records[i].right);     // right, bottom
 			f0 = a.x; f1 = a.y; f2 = a.z; f3 = a.w; f4 = b.x; f5 = b.y;
 			L = b.z; top = b.w; R = c.x;
 			count = c.y - top;
-			out = rowOffsets[i];
+			if (rowOffsets) records[i].rowStart = rowOffsets[i];
+			out = rowOffsets ? rowOffsets[i] : records[i].rowStart;
 		}
 		const bool short_ = __all_sync(0xFFFFFFFFu, count <= ROWS_STEPPED_MAX);
 		const int32_t segments = short_ ? 1 : (count + ROWS_STEPPED_MAX - 1) / ROWS_STEPPED_MAX;
@@ -757,16 +872,60 @@ __global__ void __launch_bounds__(256, 3) rows_group_kernel(const DrawRecord *__
 	}
 }
 
-void launch_rows(const FrameBuffers &fb, uint32_t recordCount, bool tallRecords, cudaStream_t stream) {
+// The rows of frames of tall triangles: one thread per segment of ROW_SEGMENT rows, whose record
+// setup_emit_kernel wrote down (segmentSlots) as it took the rows.  Two floor divisions per edge
+// start the segment and each row then steps, so the work is spread evenly whatever the records'
+// heights and no thread searches for its record.  A kernel that cut the concatenated rows into
+// chunks of 1,024, searched the records of each chunk with one warp and stepped four rows per thread
+// took 43 us for the 2.5 M rows of 20,000 random triangles at 800x600; this one takes 17 us.
+__global__ void __launch_bounds__(128) rows_segment_kernel(const DrawRecord *__restrict__ records, const uint32_t *__restrict__ segmentSlots,
+                                                           const uint32_t *rowTotal, uint32_t rowCapacity, uint32_t *rows) {
+	chain_enter();
+	const uint32_t total = min(*rowTotal, rowCapacity) / ROW_SEGMENT; // rows past the capacity: the frame is redone
+	for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < total; s += gridDim.x * blockDim.x) {
+		const DrawRecord &r = records[segmentSlots[s]];
+		const int4 a = __ldg(reinterpret_cast<const int4 *>(&r.flat[0]));   // flat[0..3]
+		const int4 b = __ldg(reinterpret_cast<const int4 *>(&r.flat[4]));   // flat[4..5], left, top
+		const int2 c = __ldg(reinterpret_cast<const int2 *>(&r.right));     // right, bottom
+		const int32_t first = (int32_t)(s * ROW_SEGMENT - __ldg(&r.rowStart));
+		const int32_t count = min((int32_t)ROW_SEGMENT, c.y - b.w - first);
+		const bool degenerate = (a.x == a.z && a.y == a.w) || (a.z == b.x && a.w == b.y) || (b.x == a.x && b.y == a.y);
+		EdgeStepper st[3];
+		if (!degenerate) {
+			st[0] = edge_stepper(make_edge(a.x, a.y, a.z, a.w), b.w + first);
+			st[1] = edge_stepper(make_edge(a.z, a.w, b.x, b.y), b.w + first);
+			st[2] = edge_stepper(make_edge(b.x, b.y, a.x, a.y), b.w + first);
+		}
+		uint32_t *out = rows + (size_t)s * ROW_SEGMENT;
+		// rows come in pairs (raster bounds cover row pairs)
+		for (int32_t k = 0; k < count; k += 2) {
+			uint32_t packed[2];
+#pragma unroll
+			for (int j = 0; j < 2; j++) {
+				int32_t left = c.x, right = b.z;
+				if (!degenerate) {
+					left = b.z; right = c.x;
+					edge_step(st[0], b.z, c.x, left, right);
+					edge_step(st[1], b.z, c.x, left, right);
+					edge_step(st[2], b.z, c.x, left, right);
+				}
+				packed[j] = (uint32_t)(left & 0xFFFF) | ((uint32_t)right << 16);
+			}
+			*reinterpret_cast<uint2 *>(out + k) = make_uint2(packed[0], packed[1]);
+		}
+	}
+}
+
+void launch_rows(const FrameBuffers &fb, uint32_t recordCount, cudaStream_t stream) {
 	if (recordCount == 0) return;
 	COUNT_LAUNCH();
 	const uint32_t rowCapacity = fb.rowCapacity ? fb.rowCapacity : 0xFFFFFFFFu;
-	if (tallRecords)
-		launch_chained(rows_chunk_kernel, sm_count() * 6, ROWS_THREADS, stream, fb.records, recordCount, fb.recordCountDevice, fb.rowOffsets,
-		                                                               fb.rows, rowCapacity, fb.errorFlag);
+	if (fb.emit.segmentSlots)
+		launch_chained(rows_segment_kernel, grid_for(fb.rowCapacity / ROW_SEGMENT, 128), 128, stream, fb.records, fb.emit.segmentSlots,
+		               fb.emit.counters + EMIT_ROWS, rowCapacity, fb.rows);
 	else
-		launch_chained(rows_group_kernel, grid_for((uint64_t)((recordCount + 31) / 32) * 32, 256), 256, stream,
-			fb.records, recordCount, fb.recordCountDevice, fb.rowOffsets, fb.rows, rowCapacity, fb.errorFlag);
+		launch_chained(rows_group_kernel, grid_for((uint64_t)((recordCount + 31) / 32) * 32, 256), 256, stream, fb.records, recordCount,
+		               fb.recordCountDevice, fb.emit.drawn, fb.emit.drawn ? nullptr : fb.rowOffsets, fb.rows, rowCapacity, fb.errorFlag);
 }
 
 // ------------------------------------------------------------------ binning
@@ -815,6 +974,7 @@ __device__ __forceinline__ bool tile_test_is_exact(const DrawRecord &r) {
 // their own thread, with the atomics of threads that hit the same slot merged into one; larger
 // ones by the whole warp, tested tile by tile.  A list keeps submission order only per warp, which
 // the order-free depth keys do not need.
+// This is the two-pass setup's binning (its records are stored one after another).
 template <bool FILL>
 __global__ void bin_kernel(BatchParams b, const DrawRecord *__restrict__ records, uint32_t capacity, const uint32_t *countDevice,
                            TileBins bins, int32_t *errorFlag) {
@@ -857,17 +1017,6 @@ __global__ void bin_kernel(BatchParams b, const DrawRecord *__restrict__ records
 			}
 		}
 		uint32_t bigMask = __ballot_sync(0xFFFFFFFFu, big);
-		if (bins.bigList) {
-			// deferred to bin_big_kernel, which gives every big record a warp of its own
-			if (!FILL && bigMask) {
-				const uint32_t leader = __ffs(bigMask) - 1;
-				uint32_t base = 0;
-				if (lane == leader) base = atomicAdd(bins.bigCount, (uint32_t)__popc(bigMask));
-				base = __shfl_sync(0xFFFFFFFFu, base, leader);
-				if (big) bins.bigList[base + __popc(bigMask & ((1u << lane) - 1u))] = r;
-			}
-			continue;
-		}
 		while (bigMask) {
 			const uint32_t src = __ffs(bigMask) - 1;
 			bigMask &= bigMask - 1;
@@ -893,21 +1042,20 @@ __global__ void bin_kernel(BatchParams b, const DrawRecord *__restrict__ records
 	}
 }
 
-// The records bin_kernel deferred.  A block takes BIG_GROUP of them at a time and its threads share
+// The records over more than four tiles, which setup_emit_kernel listed.  A block takes BIG_GROUP of them at a time and its threads share
 // the (record, tile) pairs of their bounds evenly, so that one record spanning a whole frame is
 // spread over the block instead of keeping a single warp busy while the rest of the grid idles.
 static const int BIG_GROUP = 8;
 
 struct BigRecord {
 	DrawRecord rec;
-	uint32_t index, tileBase, large;
+	uint32_t id, tileBase, large;
 	int32_t tx0, ty0, bw, tilesX, exact;
 };
 
 template <bool FILL>
-__global__ void __launch_bounds__(256) bin_big_kernel(BatchParams b, const DrawRecord *__restrict__ records, TileBins bins,
-                                                      int32_t *errorFlag) {
-	chain_enter();
+__device__ __forceinline__ void bin_big(const BatchParams &b, const DrawRecord *__restrict__ records, const TileBins &bins,
+                                        const uint32_t *extraIds, int32_t *errorFlag) {
 	__shared__ BigRecord held[BIG_GROUP];
 	__shared__ int32_t firstPair[BIG_GROUP + 1];
 	const uint32_t count = *bins.bigCount;
@@ -917,8 +1065,9 @@ __global__ void __launch_bounds__(256) bin_big_kernel(BatchParams b, const DrawR
 			int32_t pairs = 0;
 			if (w < count) {
 				BigRecord &h = held[threadIdx.x];
-				h.index = bins.bigList[w];
-				h.rec = records[h.index];
+				const uint32_t slot = bins.bigList[w];
+				h.id = record_id(b, extraIds, slot);
+				h.rec = records[slot];
 				const FrameTarget &f = b.frames[h.rec.frame];
 				h.large = (b.depthOnly || !record_is_small(h.rec, b.smallRows, b.smallWidth)) ? 1u : 0u;
 				h.tx0 = h.rec.left >> 4;
@@ -952,98 +1101,70 @@ __global__ void __launch_bounds__(256) bin_big_kernel(BatchParams b, const DrawR
 			uint32_t slot = atomicAdd(FILL ? &bins.cursors[tile] : &bins.counts[tile], 1u);
 			if (FILL) {
 				slot += bins.offsets[tile];
-				if (slot < bins.listCapacity) bins.lists[slot] = h.index; else atomicOr(errorFlag, ERROR_BIN_OVERFLOW);
+				if (slot < bins.listCapacity) bins.lists[slot] = h.id; else atomicOr(errorFlag, ERROR_BIN_OVERFLOW);
 			}
 		}
 		__syncthreads(); // the group is done with before the next one is loaded
 	}
 }
 
-// Zeroes a batch's tile counters (per-tile counts and cursors, the big-record count, the tile
-// queue) and its error bits in one launch at the start of its phases, so that no memset node sits
-// in the chain of dependent launches behind it.
-__global__ void clear_tiles_kernel(TileBins bins, uint32_t slots, uint32_t *tileQueue, uint32_t *tileListCount, int32_t *errorFlag) {
+__global__ void __launch_bounds__(256) bin_big_kernel(BatchParams b, const DrawRecord *__restrict__ records, TileBins bins,
+                                                      const uint32_t *extraIds, int32_t *errorFlag) {
 	chain_enter();
-	for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < slots; i += gridDim.x * blockDim.x) {
-		bins.counts[i] = 0u;
-		bins.cursors[i] = 0u;
-	}
-	if (blockIdx.x == 0 && threadIdx.x == 0) {
-		if (bins.bigCount) *bins.bigCount = 0u;
-		if (tileQueue) *tileQueue = 0u;
-		if (tileListCount) *tileListCount = 0u;
-		if (errorFlag) *errorFlag = 0;
-	}
+	bin_big<false>(b, records, bins, extraIds, errorFlag);
 }
 
-void launch_clear_tiles(const BatchParams &b, const TileBins &bins, int32_t *errorFlag, cudaStream_t stream) {
-	const uint32_t slots = 2 * b.totalTiles;
-	COUNT_LAUNCH();
-	launch_chained(clear_tiles_kernel, grid_for(slots, 256), 256, stream, bins, slots, b.tileQueue, b.tileListCount, errorFlag);
-}
-
-void launch_setup_write_counting(const BatchParams &b, FrameBuffers fb, uint32_t recordCapacity, uint32_t *rowCounts, TileBins &bins,
-                                 cudaStream_t stream, cudaStream_t rowStream, cudaEvent_t fork) {
-	if (!bins.cleared) {
-		memset_async(bins.counts, 0, sizeof(uint32_t) * 2 * b.totalTiles, stream);
-		memset_async(bins.bigCount, 0, sizeof(uint32_t), stream);
+// The tile lists once their offsets are known.  A record over at most four tiles took its place in
+// each of them in setup_emit_kernel, so listing it is plain stores; the big records, whose places
+// follow (the cursors go on), are listed in the same launch.
+__global__ void __launch_bounds__(256) bin_fill_kernel(BatchParams b, const DrawRecord *__restrict__ records, TileBins bins, EmitBuffers emit,
+                                                       int32_t *errorFlag) {
+	chain_enter();
+	const uint32_t count = min(emit.counters[EMIT_DRAWN], emit.capacity);
+	for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
+		const uint2 head = emit.tileHeads[i];
+		if (head.y == 0u) continue; // a big record
+		const uint4 rank4 = emit.tileRanks[i];
+		const uint32_t id = record_id(b, emit.extraIds, emit.drawn[i]);
+		const uint32_t tilesX = head.y & 0xFFFFu, w = (head.y >> 16) & 0xFFu, tiles = head.y >> 24;
+		const uint32_t rank[4] = {rank4.x, rank4.y, rank4.z, rank4.w};
+#pragma unroll
+		for (uint32_t k = 0; k < 4; k++) {
+			if (k >= tiles) break;
+			const uint32_t slot = bins.offsets[head.x + 2u * (k / w * tilesX + k % w)] + rank[k];
+			if (slot < bins.listCapacity) bins.lists[slot] = id; else atomicOr(errorFlag, ERROR_BIN_OVERFLOW);
+		}
 	}
-	fb.counts.rowCounts = rowCounts;
-	fb.counts.binCounts = bins.counts;
-	fb.counts.bigList = bins.bigList;
-	fb.counts.bigCount = bins.bigCount;
-	fb.counts.smallRows = b.smallRows;
-	fb.counts.smallWidth = b.smallWidth;
-	fb.counts.depthOnly = b.depthOnly;
-	launch_setup_write(b, fb, recordCapacity, stream);
-	const uint32_t rowBlocks = recordCapacity / SCAN_CHUNK + 1, tileBlocks = (2 * b.totalTiles) / SCAN_CHUNK + 1;
-	if (rowStream && (size_t)rowBlocks + tileBlocks <= fb.scanScratchElems) {
-		// the row offsets on the second stream right after the records (each scan with its own part
-		// of the scratch), the big records' tile counts and the tile-list offsets on this one
-		enqueue_join(stream, rowStream, fork);
-		scan_launch(rowCounts, fb.rowOffsets, recordCapacity, fb.recordCountDevice, fb.scanScratch, rowBlocks, rowStream);
-	}
-	if (recordCapacity > 0) {
-		COUNT_LAUNCH();
-		launch_chained(bin_big_kernel<false>, sm_count() * 8, 256, stream, b, fb.records, bins, fb.errorFlag);
-	}
-	if (rowStream && (size_t)rowBlocks + tileBlocks <= fb.scanScratchElems) {
-		scan_launch(bins.counts, bins.offsets, 2 * b.totalTiles, nullptr, fb.scanScratch + rowBlocks, fb.scanScratchElems - rowBlocks, stream);
-		return;
-	}
-	// one after the other on this stream, sharing the scratch (rowStream, if given, waits for both)
-	scan_launch(rowCounts, fb.rowOffsets, recordCapacity, fb.recordCountDevice, fb.scanScratch, fb.scanScratchElems, stream);
-	scan_launch(bins.counts, bins.offsets, 2 * b.totalTiles, nullptr, fb.scanScratch, fb.scanScratchElems, stream);
-	if (rowStream) enqueue_join(stream, rowStream, fork);
+	bin_big<true>(b, records, bins, emit.extraIds, errorFlag);
 }
 
 void launch_bin_count(const BatchParams &b, const FrameBuffers &fb, uint32_t recordCount, TileBins &bins, cudaStream_t stream) {
-	if (!bins.cleared) {
-		memset_async(bins.counts, 0, sizeof(uint32_t) * 2 * b.totalTiles, stream);
-		if (bins.bigCount) memset_async(bins.bigCount, 0, sizeof(uint32_t), stream);
-	}
-	if (recordCount > 0) {
+	if (fb.emit.drawn) { // the others were counted as they were written
 		COUNT_LAUNCH();
-		launch_chained(bin_kernel<false>, grid_for(recordCount, 256), 256, stream, b, fb.records, recordCount, fb.recordCountDevice, bins,
-		                                                                  fb.errorFlag);
-		if (bins.bigList) {
+		launch_chained(bin_big_kernel, sm_count() * 8, 256, stream, b, fb.records, bins, fb.emit.extraIds, fb.errorFlag);
+	} else {
+		memset_async(bins.counts, 0, sizeof(uint32_t) * 2 * b.totalTiles, stream);
+		if (recordCount > 0) {
 			COUNT_LAUNCH();
-			launch_chained(bin_big_kernel<false>, sm_count() * 8, 256, stream, b, fb.records, bins, fb.errorFlag);
+			launch_chained(bin_kernel<false>, grid_for(recordCount, 256), 256, stream, b, fb.records, recordCount, fb.recordCountDevice, bins,
+			               fb.errorFlag);
 		}
 	}
-	launch_scan(bins.counts, bins.offsets, 2 * b.totalTiles, fb.scanScratch, fb.scanScratchElems, stream);
+	scan_launch(bins.counts, fb.emit.drawn ? bins.cursors : nullptr, bins.offsets, 2 * b.totalTiles, nullptr, fb.scanScratch,
+	            fb.scanScratchElems, stream);
 }
 
 void launch_bin_fill(const BatchParams &b, const FrameBuffers &fb, uint32_t recordCount, TileBins &bins, cudaStream_t stream) {
-	if (!bins.cleared) memset_async(bins.cursors, 0, sizeof(uint32_t) * 2 * b.totalTiles, stream);
+	if (fb.emit.drawn) {
+		COUNT_LAUNCH();
+		launch_chained(bin_fill_kernel, sm_count() * 8, 256, stream, b, fb.records, bins, fb.emit, fb.errorFlag);
+		return;
+	}
+	memset_async(bins.cursors, 0, sizeof(uint32_t) * 2 * b.totalTiles, stream);
 	if (recordCount > 0) {
 		COUNT_LAUNCH();
 		launch_chained(bin_kernel<true>, grid_for(recordCount, 256), 256, stream, b, fb.records, recordCount, fb.recordCountDevice, bins,
-		                                                                 fb.errorFlag);
-		if (bins.bigList) {
-			COUNT_LAUNCH();
-			launch_chained(bin_big_kernel<true>, sm_count() * 8, 256, stream, b, fb.records, bins, fb.errorFlag);
-		}
+		               fb.errorFlag);
 	}
 }
 
@@ -1164,11 +1285,11 @@ __device__ __forceinline__ void write_lane(const BatchParams &b, const FrameTarg
 
 // The depth model_renderDepth leaves at (px, py) when record ri wins the pixel: the reference's
 // 1 x 1 walk from its row's left end (executeTriangleDrawingDepth, renderCore.cpp:343-387).
-__device__ __forceinline__ float depth_walk_value(const DrawRecord *__restrict__ records, const uint32_t *__restrict__ rowOffsets,
+__device__ __forceinline__ float depth_walk_value(const BatchParams &b, const DrawRecord *__restrict__ records,
                                                   const uint32_t *__restrict__ rows, uint32_t ri, int32_t px, int32_t py) {
-	const DrawRecord r = records[ri];
+	const DrawRecord r = records[record_slot(b, ri)];
 	int32_t left, right;
-	unpack_row(rows[rowOffsets[ri] + (py - r.top)], left, right);
+	unpack_row(rows[r.rowStart + (uint32_t)(py - r.top)], left, right);
 	const float value = fadd(fadd(r.start[0], fmul(r.dx[0], (float)left + 0.5f)), fmul(r.dy[0], (float)py + 0.5f));
 	return chain_add(value, r.dx[0], px - left);
 }
@@ -1176,12 +1297,12 @@ __device__ __forceinline__ float depth_walk_value(const DrawRecord *__restrict__
 // The depth of a depth-only winner from its key: the key's upper word is the ordered bits of the
 // very value the walk wrote (make_key), so it decodes to that value, except that +0 and -0 share
 // one key word; that word is walked again.
-__device__ __forceinline__ float depth_from_key(unsigned long long key, bool affine, const DrawRecord *__restrict__ records,
-                                                const uint32_t *__restrict__ rowOffsets, const uint32_t *__restrict__ rows,
+__device__ __forceinline__ float depth_from_key(const BatchParams &b, unsigned long long key, bool affine,
+                                                const DrawRecord *__restrict__ records, const uint32_t *__restrict__ rows,
                                                 int32_t px, int32_t py) {
 	uint32_t hi = (uint32_t)(key >> 32);
 	if (affine) hi = ~hi;
-	if (hi == 0x80000000u) return depth_walk_value(records, rowOffsets, rows, key_record(key, true), px, py);
+	if (hi == 0x80000000u) return depth_walk_value(b, records, rows, key_record(key, true), px, py);
 	return bitsf((hi & 0x80000000u) ? (hi & 0x7FFFFFFFu) : ~hi);
 }
 
@@ -1191,15 +1312,13 @@ __device__ __forceinline__ float depth_from_key(unsigned long long key, bool aff
 // on the order of the triangles); without a depth buffer the last triangle drawn wins there as
 // anywhere, with its lower lane's value where the pixel lies in its run of full quads.
 __device__ __forceinline__ void resolve_pixel(const BatchParams &b, const FrameTarget &f, const DrawRecord *__restrict__ records,
-                                              const uint32_t *__restrict__ rowOffsets, const uint32_t *__restrict__ rows,
-                                              int32_t px, int32_t py, unsigned long long key) {
+                                              const uint32_t *__restrict__ rows, int32_t px, int32_t py, unsigned long long key) {
 	const bool depthTest = f.depth != nullptr, affine = f.affine != 0;
 	const bool oddRow = odd_last_row(py, f.height);
 	if (oddRow && depthTest) return;
-	const uint32_t ri = key_record(key, depthTest);
-	const DrawRecord r = records[ri];
+	const DrawRecord r = records[record_slot(b, key_record(key, depthTest))];
 	const int32_t y1 = py & ~1, x = px & ~1;
-	const RowPair pair = record_row_pair(r, rows + rowOffsets[ri], y1, f.height);
+	const RowPair pair = record_row_pair(r, rows, y1, f.height);
 	const int lane4 = ((py & 1) << 1) | (px & 1) | ((oddRow && full_quad(pair, x)) ? 2 : 0);
 	write_lane(b, f, r, pair, y1, x, lane4, px, py, affine);
 }
@@ -1211,13 +1330,11 @@ __device__ __forceinline__ void resolve_pixel(const BatchParams &b, const FrameT
 // lanes by shuffles.  The values are those of resolve_pixel; the quad's sums are evaluated once
 // instead of four times.
 __device__ __forceinline__ void resolve_shared_quad(const BatchParams &b, const FrameTarget &f, const DrawRecord *__restrict__ records,
-                                                    const uint32_t *__restrict__ rowOffsets, const uint32_t *__restrict__ rows,
-                                                    int32_t px, int32_t py, unsigned long long key, int l4, unsigned quadLanes) {
+                                                    const uint32_t *__restrict__ rows, int32_t px, int32_t py, unsigned long long key, int l4, unsigned quadLanes) {
 	const bool depthTest = f.depth != nullptr, affine = f.affine != 0;
-	const uint32_t ri = key_record(key, depthTest);
-	const DrawRecord r = records[ri];
+	const DrawRecord r = records[record_slot(b, key_record(key, depthTest))];
 	const int32_t y1 = py & ~1, x = px & ~1;
-	const RowPair pair = record_row_pair(r, rows + rowOffsets[ri], y1, f.height);
+	const RowPair pair = record_row_pair(r, rows, y1, f.height);
 	const float depthValue = quad_lane(r.start[0], r.dx[0], r.dy[0], pair, y1, x, l4);
 	if (f.color) {
 		float a, bw, c;
@@ -1252,8 +1369,7 @@ static const int SHARED_FRAMES = 256;
 
 template <bool DEPTH_ONLY_1X1, int THREADS, bool RESOLVE>
 __global__ void __launch_bounds__(THREADS, 1024 / THREADS) raster_kernel(BatchParams b, const DrawRecord *__restrict__ records,
-                                                                         TileBins bins, const uint32_t *__restrict__ rowOffsets,
-                                                                         const uint32_t *__restrict__ rows) {
+                                                                         TileBins bins, const uint32_t *__restrict__ rows) {
 	chain_enter();
 	constexpr int WARPS = THREADS / 32;
 	if (overflowed(b)) return; // the lists or rows are incomplete: the frame is redone
@@ -1326,12 +1442,12 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) raster_kernel(BatchPa
 			float s0 = 0.0f, dx0 = 0.0f, dy0 = 0.0f;
 			if (e < smallEnd) {
 				ri = bins.lists[e];
-				const DrawRecord &r = records[ri];
+				const DrawRecord &r = records[record_slot(b, ri)];
 				const int32_t left = r.left, right = r.right;
 				top = r.top;
 				const int32_t bottom = r.bottom;
 				s0 = r.start[0]; dx0 = r.dx[0]; dy0 = r.dy[0];
-				rowOffset = rowOffsets[ri];
+				rowOffset = r.rowStart;
 				rowStart = max(top, ty0);
 				const int32_t rowEnd = min(bottom, ty0 + TILE_H);
 				colStart = max(left & ~1, tx0);
@@ -1393,7 +1509,7 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) raster_kernel(BatchPa
 			uint32_t myBest = 0u;
 			if (cull) tileMin = warp_tile_threshold(keys, initialDepth, lane, validW, validH, affine);
 			if (valid && cull) {
-				myBest = record_best_hi(records[myRecord], tx0, ty0, affine, DEPTH_ONLY_1X1);
+				myBest = record_best_hi(records[record_slot(b, myRecord)], tx0, ty0, affine, DEPTH_ONLY_1X1);
 				culled = myBest < tileMin;
 			}
 			uint32_t largeMask = __ballot_sync(0xFFFFFFFFu, valid && !culled);
@@ -1410,11 +1526,11 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) raster_kernel(BatchPa
 					if (__shfl_sync(0xFFFFFFFFu, myBest, src) < tileMin) continue;
 				}
 				const uint32_t ri = __shfl_sync(0xFFFFFFFFu, myRecord, src);
-				const DrawRecord r = records[ri];
+				const DrawRecord r = records[record_slot(b, ri)];
 				// every lane reads one of the tile's 16 rows (lanes 16..31 repeat 0..15)
 				int32_t rowLeft = 0, rowRight = 0;
 				const int32_t ry = ty0 + (lane & 15);
-				if (ry >= r.top && ry < r.bottom) unpack_row(rows[rowOffsets[ri] + (ry - r.top)], rowLeft, rowRight);
+				if (ry >= r.top && ry < r.bottom) unpack_row(rows[r.rowStart + (uint32_t)(ry - r.top)], rowLeft, rowRight);
 				if (DEPTH_ONLY_1X1) {
 					// executeTriangleDrawingDepth (renderCore.cpp:343-387): depth starts at the row's left
 					// pixel and grows by dx one pixel at a time.
@@ -1508,7 +1624,7 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) raster_kernel(BatchPa
 				if (!RESOLVE) keyImage[(size_t)py * width + px] = key;
 				// model_renderDepth: the winner's depth straight from its key, written by the tile pass itself
 				else if (DEPTH_ONLY_1X1 && key != 0ull)
-					f.depth[(size_t)py * f.depthStride + px] = depth_from_key(key, affine, records, rowOffsets, rows, px, py);
+					f.depth[(size_t)py * f.depthStride + px] = depth_from_key(b, key, affine, records, rows, px, py);
 			}
 			if (!RESOLVE || DEPTH_ONLY_1X1) continue;
 			// the tile's winners shaded right away (resolve_pixels_kernel fused into the tile pass): a
@@ -1520,9 +1636,9 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) raster_kernel(BatchPa
 			                       __shfl_xor_sync(0xFFFFFFFFu, same, 3)) != 0;
 			const unsigned drawn = __ballot_sync(0xFFFFFFFFu, key != 0ull);
 			if (__all_sync(0xFFFFFFFFu, quadSame || key == 0ull)) {
-				if (key != 0ull) resolve_shared_quad(b, f, records, rowOffsets, rows, px, py, key, l4, drawn);
+				if (key != 0ull) resolve_shared_quad(b, f, records, rows, px, py, key, l4, drawn);
 			} else if (key != 0ull) {
-				resolve_pixel(b, f, records, rowOffsets, rows, px, py, key);
+				resolve_pixel(b, f, records, rows, px, py, key);
 			}
 		}
 		if (tid == 0 && fragmentSum) {
@@ -1538,8 +1654,7 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) raster_kernel(BatchPa
 // frames of small triangles, where the pixels of a quad mostly have different winners.  One CTA
 // of 256 threads per 16x16 tile.
 __global__ void __launch_bounds__(256, 4) resolve_pixels_kernel(BatchParams b, const DrawRecord *__restrict__ records,
-                                                                const uint32_t *__restrict__ binOffsets,
-                                                                const uint32_t *__restrict__ rowOffsets, const uint32_t *__restrict__ rows) {
+                                                                const uint32_t *__restrict__ binOffsets, const uint32_t *__restrict__ rows) {
 	chain_enter();
 	if (overflowed(b)) return;
 	const uint32_t tile = blockIdx.x;
@@ -1549,7 +1664,7 @@ __global__ void __launch_bounds__(256, 4) resolve_pixels_kernel(BatchParams b, c
 	const int32_t px = (local % f.tilesX) * TILE_W + (threadIdx.x & 15), py = (local / f.tilesX) * TILE_H + (threadIdx.x >> 4);
 	if (px >= f.width || py >= f.height) return;
 	const unsigned long long key = f.keys[(size_t)py * f.width + px];
-	if (key != 0ull) resolve_pixel(b, f, records, rowOffsets, rows, px, py, key);
+	if (key != 0ull) resolve_pixel(b, f, records, rows, px, py, key);
 }
 
 // One thread per 2x2 quad: the winners of its pixels are grouped by record, and for each record
@@ -1558,8 +1673,7 @@ __global__ void __launch_bounds__(256, 4) resolve_pixels_kernel(BatchParams b, c
 // (deferred shading: only winners are shaded).  Used for frames of larger triangles, where a
 // quad's pixels mostly share their winner.  One CTA of 64 threads per 16x16 tile.
 __global__ void __launch_bounds__(64) resolve_quads_kernel(BatchParams b, const DrawRecord *__restrict__ records,
-                                                     const uint32_t *__restrict__ binOffsets,
-                                                     const uint32_t *__restrict__ rowOffsets, const uint32_t *__restrict__ rows) {
+                                                     const uint32_t *__restrict__ binOffsets, const uint32_t *__restrict__ rows) {
 	chain_enter();
 	if (overflowed(b)) return;
 	const uint32_t tile = blockIdx.x;
@@ -1591,8 +1705,8 @@ __global__ void __launch_bounds__(64) resolve_quads_kernel(BatchParams b, const 
 		for (int l = first; l < 4; l++)
 			if ((pending & (1u << l)) && record[l] == ri) mask |= 1u << l;
 		pending &= ~mask;
-		const DrawRecord r = records[ri];
-		const RowPair pair = record_row_pair(r, rows + rowOffsets[ri], y1, height);
+		const DrawRecord r = records[record_slot(b, ri)];
+		const RowPair pair = record_row_pair(r, rows, y1, height);
 		float w[3][4];
 		const int components = f.color ? 3 : 1;
 		for (int c = 0; c < components; c++) quad_lanes(r.start[c], r.dx[c], r.dy[c], pair, y1, x, w[c]);
@@ -1627,14 +1741,16 @@ static const int ODD_SORT = 512; // ODD_WINDOW rounded up to a power of two, for
 
 // Whether a record can touch row y of the 16 columns from tx0 (its bound, which holds every pixel
 // it writes, the lower lanes of the last row's full quads included).
-__device__ __forceinline__ bool odd_row_relevant(const DrawRecord *__restrict__ records, uint32_t ri, int32_t y, int32_t tx0) {
-	const int4 bound = *reinterpret_cast<const int4 *>(&records[ri].flat[4]); // flat[4], flat[5], left, top
-	const int2 rb = *reinterpret_cast<const int2 *>(&records[ri].right);
+__device__ __forceinline__ bool odd_row_relevant(const BatchParams &b, const DrawRecord *__restrict__ records, uint32_t ri, int32_t y,
+                                                 int32_t tx0) {
+	const DrawRecord &r = records[record_slot(b, ri)];
+	const int4 bound = *reinterpret_cast<const int4 *>(&r.flat[4]); // flat[4], flat[5], left, top
+	const int2 rb = *reinterpret_cast<const int2 *>(&r.right);
 	return bound.w <= y && rb.y > y && bound.z < tx0 + TILE_W && rb.x > tx0;
 }
 
 // Relevant records of the tile's list with index in [lo, hi): counted, and the largest one.
-__device__ __forceinline__ void odd_row_count(const DrawRecord *__restrict__ records, const uint32_t *__restrict__ lists,
+__device__ __forceinline__ void odd_row_count(const BatchParams &b, const DrawRecord *__restrict__ records, const uint32_t *__restrict__ lists,
                                               uint32_t begin, uint32_t end, uint32_t lo, uint32_t hi, int32_t y, int32_t tx0,
                                               uint32_t *count, uint32_t *largest) {
 	__syncthreads(); // every thread has read the previous totals
@@ -1643,7 +1759,7 @@ __device__ __forceinline__ void odd_row_count(const DrawRecord *__restrict__ rec
 	uint32_t n = 0, m = 0;
 	for (uint32_t e = begin + threadIdx.x; e < end; e += blockDim.x) {
 		const uint32_t ri = lists[e];
-		if (ri >= lo && ri < hi && odd_row_relevant(records, ri, y, tx0)) { n++; m = max(m, ri); }
+		if (ri >= lo && ri < hi && odd_row_relevant(b, records, ri, y, tx0)) { n++; m = max(m, ri); }
 	}
 	if (n) { atomicAdd(count, n); atomicMax(largest, m); }
 	__syncthreads();
@@ -1662,7 +1778,7 @@ __device__ __forceinline__ void odd_row_count(const DrawRecord *__restrict__ rec
 // stored depth, else the upper one if it does.  The winner is shaded once at the end.
 __global__ void __launch_bounds__(256) odd_row_kernel(BatchParams b, const DrawRecord *__restrict__ records,
                                                       const uint32_t *__restrict__ binOffsets, const uint32_t *__restrict__ lists,
-                                                      const uint32_t *__restrict__ rowOffsets, const uint32_t *__restrict__ rows) {
+                                                      const uint32_t *__restrict__ rows) {
 	chain_enter();
 	if (overflowed(b)) return;
 	__shared__ uint32_t ids[ODD_SORT];
@@ -1690,7 +1806,7 @@ __global__ void __launch_bounds__(256) odd_row_kernel(BatchParams b, const DrawR
 		}
 		uint32_t lo = 0;
 		for (;;) {
-			odd_row_count(records, lists, begin, end, lo, 0xFFFFFFFFu, y, tx0, &count, &largest);
+			odd_row_count(b, records, lists, begin, end, lo, 0xFFFFFFFFu, y, tx0, &count, &largest);
 			uint32_t n = count;
 			if (n == 0) break;
 			uint32_t hi = 0xFFFFFFFFu;
@@ -1700,7 +1816,7 @@ __global__ void __launch_bounds__(256) odd_row_kernel(BatchParams b, const DrawR
 				uint32_t good = lo + 1, bad = largest + 1;
 				while (bad - good > 1) {
 					const uint32_t mid = good + (bad - good) / 2;
-					odd_row_count(records, lists, begin, end, lo, mid, y, tx0, &count, &largest);
+					odd_row_count(b, records, lists, begin, end, lo, mid, y, tx0, &count, &largest);
 					if (count <= (uint32_t)ODD_WINDOW) good = mid; else bad = mid;
 				}
 				hi = good;
@@ -1711,7 +1827,7 @@ __global__ void __launch_bounds__(256) odd_row_kernel(BatchParams b, const DrawR
 			__syncthreads();
 			for (uint32_t e = begin + tid; e < end; e += blockDim.x) {
 				const uint32_t ri = lists[e];
-				if (ri >= lo && ri < hi && odd_row_relevant(records, ri, y, tx0)) {
+				if (ri >= lo && ri < hi && odd_row_relevant(b, records, ri, y, tx0)) {
 					const uint32_t slot = atomicAdd(&count, 1u);
 					if (slot < (uint32_t)ODD_WINDOW) ids[slot] = ri; // always true: the window was sized by the same test
 				}
@@ -1741,8 +1857,8 @@ __global__ void __launch_bounds__(256) odd_row_kernel(BatchParams b, const DrawR
 				float2 cand = make_float2(none, none);
 				if (cx < width) {
 					const uint32_t ri = ids[j];
-					const DrawRecord r = records[ri];
-					const RowPair pair = record_row_pair(r, rows + rowOffsets[ri], y, f.height);
+					const DrawRecord r = records[record_slot(b, ri)];
+					const RowPair pair = record_row_pair(r, rows, y, f.height);
 					const int32_t x = cx & ~1;
 					if (pair.any && x >= pair.obs && x < pair.obe) {
 						float v[4];
@@ -1768,9 +1884,9 @@ __global__ void __launch_bounds__(256) odd_row_kernel(BatchParams b, const DrawR
 			lo = hi;
 		}
 		if (tid < TILE_W && px < width && winner != 0xFFFFFFFFu) {
-			const DrawRecord r = records[winner];
+			const DrawRecord r = records[record_slot(b, winner)];
 			const int32_t x = px & ~1;
-			const RowPair pair = record_row_pair(r, rows + rowOffsets[winner], y, f.height);
+			const RowPair pair = record_row_pair(r, rows, y, f.height);
 			write_lane(b, f, r, pair, y, x, (px & 1) + (winnerLower ? 2 : 0), px, y, affine);
 		}
 		__syncthreads(); // the next frame reuses the shared arrays
@@ -1803,7 +1919,7 @@ __global__ void tile_keys_kernel(const uint32_t *__restrict__ entryTile, const u
 // re-evaluated exactly as the resolve pass does.  One CTA of 256 threads per 16x16 tile.
 __global__ void __launch_bounds__(256) alpha_kernel(BatchParams b, const DrawRecord *__restrict__ records,
                                                     const uint32_t *__restrict__ binOffsets, const uint32_t *__restrict__ sorted,
-                                                    const uint32_t *__restrict__ rowOffsets, const uint32_t *__restrict__ rows) {
+                                                    const uint32_t *__restrict__ rows) {
 	if (overflowed(b)) return;
 	const uint32_t tile = blockIdx.x;
 	const uint32_t begin = binOffsets[2 * tile], end = binOffsets[2 * tile + 2];
@@ -1821,14 +1937,13 @@ __global__ void __launch_bounds__(256) alpha_kernel(BatchParams b, const DrawRec
 	const bool oddRow = odd_last_row(py, f.height);
 	uint32_t fragments = 0;
 	for (uint32_t e = begin; e < end; e++) {
-		const uint32_t ri = sorted[e];
-		const DrawRecord r = records[ri];
+		const DrawRecord r = records[record_slot(b, sorted[e])];
 		if (py < r.top || py >= r.bottom || px < r.left || px >= r.right) continue;
 		int32_t left, right;
-		unpack_row(rows[rowOffsets[ri] + (py - r.top)], left, right);
+		unpack_row(rows[r.rowStart + (uint32_t)(py - r.top)], left, right);
 		if (px < left || px >= right) continue;
 		fragments++;
-		const RowPair pair = record_row_pair(r, rows + rowOffsets[ri], y1, f.height);
+		const RowPair pair = record_row_pair(r, rows, y1, f.height);
 		float w[3][4];
 		for (int c = 0; c < 3; c++) quad_lanes(r.start[c], r.dx[c], r.dy[c], pair, y1, x, w[c]);
 		const float z = (lane4 == 0) ? w[0][0] : (lane4 == 1) ? w[0][1] : (lane4 == 2) ? w[0][2] : w[0][3];
@@ -1861,9 +1976,9 @@ __global__ void __launch_bounds__(256) alpha_kernel(BatchParams b, const DrawRec
 	if (b.walked && fragments) atomicAdd(b.walked, (unsigned long long)fragments);
 }
 
-void launch_alpha(const BatchParams &b, const FrameBuffers &fb, const TileBins &bins, uint32_t entries, uint32_t recordCount,
-                  const AlphaBuffers &a, cudaStream_t stream) {
+void launch_alpha(const BatchParams &b, const FrameBuffers &fb, const TileBins &bins, uint32_t entries, const AlphaBuffers &a, cudaStream_t stream) {
 	if (b.totalTiles == 0) return;
+	const uint64_t recordNumbers = (uint64_t)b.totalTriangles * 8u; // both setups number records below this
 	const uint32_t *sorted = bins.lists;
 	if (entries > 1) {
 		// every tile's list in submission order: a stable sort of the entries by record, then a
@@ -1872,7 +1987,7 @@ void launch_alpha(const BatchParams &b, const FrameBuffers &fb, const TileBins &
 		COUNT_LAUNCH();
 		entry_tile_kernel<<<b.totalTiles, 128, 0, stream>>>(bins.offsets, a.entryTile);
 		int recordBits = 1, tileBits = 1;
-		while ((1ull << recordBits) < (uint64_t)recordCount) recordBits++;
+		while ((1ull << recordBits) < recordNumbers) recordBits++;
 		while ((1ull << tileBits) < (uint64_t)b.totalTiles) tileBits++;
 		const uint32_t *records = nullptr, *order = nullptr;
 		launch_stable_sort(bins.lists, nullptr, entries, recordBits, a.sort, stream, &records, &order);
@@ -1882,7 +1997,7 @@ void launch_alpha(const BatchParams &b, const FrameBuffers &fb, const TileBins &
 		launch_stable_sort(a.tileKeys, a.records, entries, tileBits, a.sort, stream, &tiles, &sorted);
 	}
 	COUNT_LAUNCH();
-	alpha_kernel<<<b.totalTiles, 256, 0, stream>>>(b, fb.records, bins.offsets, sorted, fb.rowOffsets, fb.rows);
+	alpha_kernel<<<b.totalTiles, 256, 0, stream>>>(b, fb.records, bins.offsets, sorted, fb.rows);
 }
 
 void launch_odd_rows(const BatchParams &b, const FrameBuffers &fb, const TileBins &bins, cudaStream_t stream) {
@@ -1890,7 +2005,7 @@ void launch_odd_rows(const BatchParams &b, const FrameBuffers &fb, const TileBin
 	COUNT_LAUNCH();
 	const unsigned frames = (unsigned)std::min<int32_t>(b.frameCount, 65535);
 	launch_chained(odd_row_kernel, dim3((unsigned)b.maxTilesX, frames), 256, stream, b, fb.records, bins.offsets,
-	               bins.lists, fb.rowOffsets, fb.rows);
+	               bins.lists, fb.rows);
 }
 
 void launch_raster(const BatchParams &b, const FrameBuffers &fb, const TileBins &bins, const RasterConfig &config, bool resolve,
@@ -1906,10 +2021,10 @@ void launch_raster(const BatchParams &b, const FrameBuffers &fb, const TileBins 
 	// small triangles resolve per pixel inside the tile pass; the keys then never leave the chip
 	const bool fused = resolve && !b.depthOnly && config.resolveMode == 1;
 #define DSRG_RASTER(T)                                                                                            \
-	if (b.depthOnly && resolve) launch_chained(raster_kernel<true, T, true>, ctas, T, stream, b, fb.records, bins, fb.rowOffsets, fb.rows); \
-	else if (b.depthOnly) launch_chained(raster_kernel<true, T, false>, ctas, T, stream, b, fb.records, bins, fb.rowOffsets, fb.rows); \
-	else if (fused) launch_chained(raster_kernel<false, T, true>, ctas, T, stream, b, fb.records, bins, fb.rowOffsets, fb.rows); \
-	else launch_chained(raster_kernel<false, T, false>, ctas, T, stream, b, fb.records, bins, fb.rowOffsets, fb.rows);
+	if (b.depthOnly && resolve) launch_chained(raster_kernel<true, T, true>, ctas, T, stream, b, fb.records, bins, fb.rows); \
+	else if (b.depthOnly) launch_chained(raster_kernel<true, T, false>, ctas, T, stream, b, fb.records, bins, fb.rows); \
+	else if (fused) launch_chained(raster_kernel<false, T, true>, ctas, T, stream, b, fb.records, bins, fb.rows); \
+	else launch_chained(raster_kernel<false, T, false>, ctas, T, stream, b, fb.records, bins, fb.rows);
 	if (threads == 64) { DSRG_RASTER(64) }
 	else if (threads == 128) { DSRG_RASTER(128) }
 	else { DSRG_RASTER(256) }
@@ -1917,8 +2032,8 @@ void launch_raster(const BatchParams &b, const FrameBuffers &fb, const TileBins 
 	if (!resolve) return;
 	if (!fused && !b.depthOnly) { // depth-only batches resolve inside the tile pass (depth_from_key)
 		COUNT_LAUNCH();
-		if (config.resolveMode == 2) launch_chained(resolve_quads_kernel, b.totalTiles, 64, stream, b, fb.records, bins.offsets, fb.rowOffsets, fb.rows);
-		else launch_chained(resolve_pixels_kernel, b.totalTiles, 256, stream, b, fb.records, bins.offsets, fb.rowOffsets, fb.rows);
+		if (config.resolveMode == 2) launch_chained(resolve_quads_kernel, b.totalTiles, 64, stream, b, fb.records, bins.offsets, fb.rows);
+		else launch_chained(resolve_pixels_kernel, b.totalTiles, 256, stream, b, fb.records, bins.offsets, fb.rows);
 	}
 	// the last rows of depth-tested odd-height frames, which every resolve above leaves alone
 	launch_odd_rows(b, fb, bins, stream);

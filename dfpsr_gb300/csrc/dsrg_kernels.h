@@ -71,6 +71,8 @@ struct BatchParams {
 	uint32_t *tileQueue;              // work counter of the persistent tile kernel
 	uint32_t *tileList;               // the tiles that have list entries (written at the end of phase C), or null: every tile
 	uint32_t *tileListCount;          // their number
+	uint32_t recordShift;             // 3: records numbered 8 * fan triangle + piece, 0: as they are stored (record_slot)
+	const uint32_t *extraBase;        // per fan triangle: where the further pieces of a clipped triangle begin
 	const int32_t *errorFlag;         // device error bits; tile and resolve kernels return when an overflow is set
 };
 
@@ -83,12 +85,30 @@ struct ProjectedPoints {
 	longlong2 *flat;  // flat x, flat y
 };
 
+// What setup_emit_kernel writes beside the records.  Counters in device memory, zeroed by the
+// batch's first launch: draw records, row intervals taken, extra slots taken.
+enum EmitCounter : uint32_t { EMIT_DRAWN = 0, EMIT_ROWS = 1, EMIT_EXTRAS = 2, EMIT_COUNTERS = 3 };
+static const uint32_t ROW_SEGMENT = 16; // rows one thread of rows_segment_kernel computes
+
+struct EmitBuffers {
+	uint32_t *counters;      // EMIT_COUNTERS values
+	uint32_t *drawn;         // the slots of the records, in no order; null: the two-pass setup
+	uint32_t capacity;       // slots: one per fan triangle, then the extra ones
+	uint32_t *extraBase;     // per fan triangle with further pieces: their first extra slot
+	uint32_t *extraIds;      // per extra slot: its record's number
+	uint2 *tileHeads;        // per drawn record: its first tile-list slot, and tilesX | columns << 16 | tiles << 24 (0: a big record)
+	uint4 *tileRanks;        // per drawn record over at most four tiles: its place in each tile's list
+	uint32_t *segmentSlots;  // tall triangles: the record of every segment of ROW_SEGMENT rows; null: rows are packed in pairs
+	uint32_t *tileCursors;   // 2 * totalTiles: the places taken in each tile's lists
+	uint32_t *bigList, *bigCount; // records over more than four tiles, for bin_big_kernel
+};
+
 struct FrameBuffers {
 	ProjectedPoints points;
-	uint32_t *triCounts;      // per fan triangle: draw records it emits
-	uint32_t *triOffsets;     // exclusive scan of triCounts, total at [totalTriangles]
+	uint32_t *triCounts;      // two-pass setup: draw records that each fan triangle emits,
+	uint32_t *triOffsets;     // their exclusive scan, total at [totalTriangles],
+	uint32_t *rowOffsets;     // and per record its first row interval (+ total at [recordCount])
 	DrawRecord *records;
-	uint32_t *rowOffsets;     // per record: first entry of its rows in `rows` (+ total at [recordCount])
 	uint32_t *rows;           // row intervals of every record, left | right << 16
 	int32_t *errorFlag;       // device error bits
 	uint32_t *scanScratch;
@@ -97,37 +117,39 @@ struct FrameBuffers {
 	// launches, which then bounds the grids), and rows hold at most rowCapacity entries
 	const uint32_t *recordCountDevice;
 	uint32_t rowCapacity;
-	// when rowCounts is set, the record-writing setup pass also writes every record's row count and
-	// counts its tiles (bins of up to four tiles; larger records go to bigList for bin_big_kernel)
-	struct {
-		uint32_t *rowCounts;
-		uint32_t *binCounts;
-		uint32_t *bigList;
-		uint32_t *bigCount;
-		int32_t smallRows, smallWidth, depthOnly;
-	} counts;
+	EmitBuffers emit;         // the one-pass setup (emit.drawn set)
+};
+
+// Counters zeroed by a batch's first launch (launch_project).
+struct ClearedCounters {
+	uint32_t *tileCounts, *tileCursors; // tileSlots values each
+	uint32_t tileSlots;
+	uint32_t *control;                  // words values: tile queue, error bits, emit counters, list lengths
+	uint32_t words;
 };
 
 // Two lists per tile: slot 2 * tile holds the records walked one lane each (small), slot
 // 2 * tile + 1 the ones walked by a whole warp (large).
 struct TileBins {
-	uint32_t *counts;   // 2 * totalTiles
+	uint32_t *counts;   // 2 * totalTiles: entries of each list (one-pass setup: of its big records)
 	uint32_t *offsets;  // 2 * totalTiles + 1
-	uint32_t *cursors;  // 2 * totalTiles
+	uint32_t *cursors;  // 2 * totalTiles: places taken in each list
 	uint32_t *lists;
 	size_t listCapacity;
-	// records over more than four tiles, binned by whole warps in a second launch (room for every
-	// record; the count pass fills the list, the fill pass reads it); null: binned in the same launch
+	// records over more than four tiles, listed by setup_emit_kernel and binned by whole blocks
 	uint32_t *bigList;
 	uint32_t *bigCount;
-	// counts, cursors, bigCount, the tile queue and the error bits are zeroed by launch_clear_tiles
-	// at the start of the batch's phases (0: each launcher zeroes what it uses with memsets)
+	// the tile queue is zeroed by the batch's first launch (0: launch_raster zeroes it with a memset)
 	int32_t cleared;
 };
 
 // True when one lane walks the whole record inside a tile (small-triangle path).
+__host__ __device__ inline bool bound_is_small(int32_t left, int32_t top, int32_t right, int32_t bottom, int32_t smallRows,
+                                               int32_t smallWidth) {
+	return (bottom - top) <= smallRows && (right - left) <= smallWidth;
+}
 __host__ __device__ inline bool record_is_small(const DrawRecord &r, int32_t smallRows, int32_t smallWidth) {
-	return (r.bottom - r.top) <= smallRows && (r.right - r.left) <= smallWidth;
+	return bound_is_small(r.left, r.top, r.right, r.bottom, smallRows, smallWidth);
 }
 
 enum ErrorBits : int32_t {
@@ -141,21 +163,17 @@ enum ErrorBits : int32_t {
 	ERROR_OVERFLOW_BITS = ERROR_RECORD_OVERFLOW | ERROR_BIN_OVERFLOW | ERROR_ROW_OVERFLOW,
 };
 
-// Phase A: projection and the count of draw records per fan triangle, scanned so that the record
-// count ends at triOffsets[totalTriangles].
-void launch_project(const BatchParams &b, const FrameBuffers &fb, cudaStream_t stream);
+// Phase A: projection (zeroing the counters of the launches behind it when `clear` is given).
+void launch_project(const BatchParams &b, const FrameBuffers &fb, cudaStream_t stream, const ClearedCounters *clear = nullptr);
+// The one-pass setup (fb.emit): every fan triangle's records with their rows taken and their tiles
+// counted.  Needs fewer than MAX_EMIT_TRIANGLES fan triangles.
+static const uint32_t MAX_EMIT_TRIANGLES = 1u << 29;
+void launch_setup_emit(const BatchParams &b, const FrameBuffers &fb, cudaStream_t stream);
+// The two-pass setup: the count of draw records per fan triangle, scanned so that the record count
+// ends at triOffsets[totalTriangles], then the records in submission order (per frame: the order of
+// its tasks, then of their triangles), row offsets (total at rowOffsets[recordCount]).
 void launch_setup_count(const BatchParams &b, const FrameBuffers &fb, cudaStream_t stream);
-// Phase B: the records, in submission order (per frame: the order of its tasks, then of their
-// triangles), row offsets (total at rowOffsets[recordCount]) and tile counts (total at offsets[2 * totalTiles]).
 void launch_setup_write(const BatchParams &b, const FrameBuffers &fb, uint32_t recordCapacity, cudaStream_t stream);
-// launch_setup_write with the row and tile counting folded in (fb.counts is filled from rowCounts and
-// bins here), then the big records' tile counts and the scans of row counts and tile counts: the
-// work of launch_setup_write + launch_row_offsets + launch_bin_count in one pass over the records.
-void launch_clear_tiles(const BatchParams &b, const TileBins &bins, int32_t *errorFlag, cudaStream_t stream);
-// With rowStream, the row-offset scan runs there (forked with `fork` right after the records) and
-// the caller's row-interval launch on rowStream follows it; the tile counts stay on `stream`.
-void launch_setup_write_counting(const BatchParams &b, FrameBuffers fb, uint32_t recordCapacity, uint32_t *rowCounts, TileBins &bins,
-                                 cudaStream_t stream, cudaStream_t rowStream = nullptr, cudaEvent_t fork = nullptr);
 // occludeFromExistingTriangles (api/rendererAPI.cpp:240-255): every solid draw command of the batch
 // whose bound exceeds one cell lowers the occlusion grid of its frame over the cells it covers.
 void launch_setup_occlude(const BatchParams &b, const FrameBuffers &fb, cudaStream_t stream);
@@ -163,10 +181,10 @@ void launch_setup_occlude(const BatchParams &b, const FrameBuffers &fb, cudaStre
 void launch_occlusion_top_rows(float *grid, int32_t gridWidth, int32_t gridHeight, int32_t gridStride, const float *depth,
                                int32_t depthStride, int32_t width, bool perspective, cudaStream_t stream);
 void launch_row_offsets(const FrameBuffers &fb, uint32_t recordCount, uint32_t *rowCounts, cudaStream_t stream);
+// Phase B: tile counts and where each tile's lists begin (total at offsets[2 * totalTiles]).
 void launch_bin_count(const BatchParams &b, const FrameBuffers &fb, uint32_t recordCount, TileBins &bins, cudaStream_t stream);
 // Phase C: row intervals, tile lists, the persistent tile raster and the per-pixel resolve.
-// tallRecords: records average many rows (large triangles); rows are then balanced by row, not by record.
-void launch_rows(const FrameBuffers &fb, uint32_t recordCount, bool tallRecords, cudaStream_t stream);
+void launch_rows(const FrameBuffers &fb, uint32_t recordCount, cudaStream_t stream);
 void launch_bin_fill(const BatchParams &b, const FrameBuffers &fb, uint32_t recordCount, TileBins &bins, cudaStream_t stream);
 // Launch shape of the persistent tile kernel.
 struct RasterConfig {
@@ -198,16 +216,23 @@ struct AlphaBuffers {
 };
 // The alpha filter over the binned records (in place of launch_raster): colour blends in
 // submission order, depth read only.
-void launch_alpha(const BatchParams &b, const FrameBuffers &fb, const TileBins &bins, uint32_t entries, uint32_t recordCount,
-                  const AlphaBuffers &a, cudaStream_t stream);
+void launch_alpha(const BatchParams &b, const FrameBuffers &fb, const TileBins &bins, uint32_t entries, const AlphaBuffers &a,
+                  cudaStream_t stream);
 // Debug overlays: the three edges of every record as lines in pixels (flat / 256), and draw_line
 // (api/drawAPI.cpp:176-279) of many lines of one packed colour into a device image.
-void launch_wire_lines(const DrawRecord *records, uint32_t count, int4 *lines, cudaStream_t stream);
+void launch_wire_lines(const DrawRecord *records, const uint32_t *drawn, uint32_t count, int4 *lines, cudaStream_t stream);
 void launch_draw_lines(uint32_t *image, int32_t stride, int32_t width, int32_t height, const int4 *lines, uint32_t count,
                        uint32_t color, cudaStream_t stream);
-// out[0..3] = record count, row count, tile-list entry count, error bits of a batch.
-void launch_gather_totals(const uint32_t *triOffsets, uint32_t triangles, const uint32_t *rowOffsets, uint32_t recordCapacity,
-                          const uint32_t *binOffsets, uint32_t tiles, const int32_t *errorFlag, uint32_t *out, uint32_t *tileList,
+// out[0..3] = record count, row count, tile-list entry count, error bits of a batch, and the extra
+// slots at out[TOTALS_EXTRAS].
+static const uint32_t TOTALS_EXTRAS = 9;
+struct TotalsSources {
+	const uint32_t *records, *rows, *extras;
+	const uint32_t *rowOffsets;   // the two-pass setup: the row count is rowOffsets[records]
+	uint32_t recordCapacity;
+	const int32_t *errorFlag;
+};
+void launch_gather_totals(const TotalsSources &from, const uint32_t *binOffsets, uint32_t tiles, uint32_t *out, uint32_t *tileList,
                           uint32_t *tileListCount, cudaStream_t stream);
 // Exclusive scan of n uint32 values into out (out[n] = total); two launches, scratch of
 // scan_scratch_elems(n) values.

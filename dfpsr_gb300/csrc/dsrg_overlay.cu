@@ -16,9 +16,9 @@ namespace dsrg {
 
 namespace {
 
-__global__ void wire_lines_kernel(const DrawRecord *__restrict__ records, uint32_t count, int4 *lines) {
+__global__ void wire_lines_kernel(const DrawRecord *__restrict__ records, const uint32_t *__restrict__ drawn, uint32_t count, int4 *lines) {
 	for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
-		const DrawRecord &r = records[i];
+		const DrawRecord &r = records[drawn ? drawn[i] : i];
 		int32_t x[3], y[3];
 		for (int c = 0; c < 3; c++) { x[c] = r.flat[2 * c] / 256; y[c] = r.flat[2 * c + 1] / 256; } // flat / unitsPerPixel
 		for (int e = 0; e < 3; e++) {
@@ -76,9 +76,9 @@ int grid_of(uint64_t threads) {
 
 } // namespace
 
-void launch_wire_lines(const DrawRecord *records, uint32_t count, int4 *lines, cudaStream_t stream) {
+void launch_wire_lines(const DrawRecord *records, const uint32_t *drawn, uint32_t count, int4 *lines, cudaStream_t stream) {
 	if (count == 0) return;
-	wire_lines_kernel<<<grid_of(count), 256, 0, stream>>>(records, count, lines);
+	wire_lines_kernel<<<grid_of(count), 256, 0, stream>>>(records, drawn, count, lines);
 	add_launches(1);
 }
 

@@ -175,12 +175,12 @@ static int enqueue_phases(dsrg_context ctx, BatchJob &job, BatchTotals &totals, 
 	if (!job.resolve && totals.pixels > 0) TRY(cudaMemsetAsync(ctx->keys.ptr, 0, totals.pixels * sizeof(unsigned long long), stream));
 	params.smallRows = ctx->smallRows;
 	params.smallWidth = ctx->smallWidth;
-	params.tileQueue = ctx->control.ptr;
+	params.tileQueue = ctx->control.ptr + CONTROL_TILE_QUEUE;
 	// depth-only batches (shadow-cube faces) are mostly empty tiles: their tile kernel pulls only
 	// the listed ones.  Colour frames pull every tile in order, which measured faster for them
 	// (the listed order is not the tile order, and the list costs a wider totals launch).
 	params.tileList = job.depthOnly ? ctx->tileList.ptr : nullptr;
-	params.tileListCount = job.depthOnly ? ctx->control.ptr + 9 : nullptr;
+	params.tileListCount = job.depthOnly ? ctx->control.ptr + CONTROL_LISTED_TILES : nullptr;
 	params.fragments = nullptr;
 	params.walked = ctx->fragmentCounter.ptr + 1;
 	if (ctx->counting && !job.clearCounters) {
@@ -192,7 +192,7 @@ static int enqueue_phases(dsrg_context ctx, BatchJob &job, BatchTotals &totals, 
 			if (f.coverage) TRY(cudaMemsetAsync(f.coverage, 0, (size_t)f.width * f.height * sizeof(uint32_t), stream));
 	}
 	if (totals.triangles == 0) return DSRG_OK; // nothing reaches the tiles: the targets stay as they are
-	params.errorFlag = (const int32_t *)(ctx->control.ptr + 1);
+	params.errorFlag = (const int32_t *)(ctx->control.ptr + CONTROL_ERROR);
 	RasterConfig config;
 	config.threadsPerTile = ctx->threadsPerTile;
 	config.ctasPerSm = ctx->ctasPerSm;
@@ -207,38 +207,66 @@ static int enqueue_phases(dsrg_context ctx, BatchJob &job, BatchTotals &totals, 
 	// A total above its capacity sets an overflow bit, the tile and resolve kernels return at once,
 	// and batch_enqueue redoes the batch with the capacities the totals asked for.
 	const size_t np = totals.points, nt = totals.triangles;
-	const uint32_t recordCap = (uint32_t)std::max<uint64_t>(ctx->recordCapacity, nt + nt / 8 + 1024);
+	// the one-pass setup keeps a slot per fan triangle and extra ones for the pieces of clipped
+	// triangles; beyond its record numbers' range the two-pass setup counts first
+	const bool onePass = nt < MAX_EMIT_TRIANGLES;
+	const uint32_t recordCap = onePass ? (uint32_t)(nt + std::max<uint64_t>(ctx->extraCapacity, nt / 8 + 1024))
+	                                   : (uint32_t)std::max<uint64_t>(ctx->recordCapacity, nt + nt / 8 + 1024);
 	const uint32_t rowCap = (uint32_t)std::max<uint64_t>(ctx->rowCapacity, (uint64_t)recordCap * 4);
 	const uint32_t binCap = (uint32_t)std::max<uint64_t>(ctx->binCapacity, (uint64_t)recordCap * 2);
 	TRY(ctx->pointCsis.reserve(np)); TRY(ctx->pointIsy.reserve(np)); TRY(ctx->pointFlat.reserve(np));
-	TRY(ctx->triCounts.reserve(nt + 1));
-	TRY(ctx->triOffsets.reserve(nt + 1));
 	TRY(ctx->records.reserve((size_t)recordCap + 1));
-	TRY(ctx->rowCounts.reserve((size_t)recordCap + 1));
-	TRY(ctx->rowOffsets.reserve((size_t)recordCap + 1));
+	if (onePass) {
+		TRY(ctx->drawnSlots.reserve((size_t)recordCap + 1));
+		TRY(ctx->extraBase.reserve(nt + 1));
+		TRY(ctx->extraIds.reserve((size_t)recordCap - nt + 1));
+		TRY(ctx->tileHeads.reserve((size_t)recordCap + 1));
+		TRY(ctx->tileRanks.reserve((size_t)recordCap + 1));
+		if (tallTriangles) TRY(ctx->segmentSlots.reserve((size_t)rowCap / ROW_SEGMENT + 1));
+	} else {
+		TRY(ctx->triCounts.reserve(nt + 1));
+		TRY(ctx->triOffsets.reserve(nt + 1));
+		TRY(ctx->rowCounts.reserve((size_t)recordCap + 1));
+		TRY(ctx->rowOffsets.reserve((size_t)recordCap + 1));
+	}
 	TRY(ctx->rows.reserve((size_t)rowCap + 2));
 	TRY(ctx->binCounts.reserve(2 * (size_t)totals.tiles + 1));
 	TRY(ctx->binOffsets.reserve(2 * (size_t)totals.tiles + 1));
 	TRY(ctx->binCursors.reserve(2 * (size_t)totals.tiles + 1));
 	TRY(ctx->binLists.reserve((size_t)binCap + 1));
 	TRY(ctx->bigList.reserve((size_t)recordCap + 1));
-	const uint64_t largest = std::max<uint64_t>(std::max<uint64_t>(nt, recordCap), 2 * (uint64_t)totals.tiles);
-	// the row and tile-list scans share one launch pair, with both arrays' chunk sums in the scratch
-	TRY(ctx->scanScratch.reserve(std::max(scan_scratch_elems((uint32_t)largest + 1),
-	                                      scan_scratch_elems(recordCap + 1) + scan_scratch_elems(2 * (uint32_t)totals.tiles + 1))));
+	const uint64_t scanned = std::max<uint64_t>(onePass ? 0 : recordCap, 2 * (uint64_t)totals.tiles);
+	TRY(ctx->scanScratch.reserve(scan_scratch_elems((uint32_t)scanned + 1)));
 	FrameBuffers fb;
 	memset(&fb, 0, sizeof(fb));
 	fb.points.csis = ctx->pointCsis.ptr; fb.points.isy = ctx->pointIsy.ptr; fb.points.flat = ctx->pointFlat.ptr;
-	fb.triCounts = ctx->triCounts.ptr;
-	fb.triOffsets = ctx->triOffsets.ptr;
 	fb.records = ctx->records.ptr;
-	fb.rowOffsets = ctx->rowOffsets.ptr;
 	fb.rows = ctx->rows.ptr;
-	fb.errorFlag = (int32_t *)(ctx->control.ptr + 1);
+	fb.errorFlag = (int32_t *)(ctx->control.ptr + CONTROL_ERROR);
 	fb.scanScratch = ctx->scanScratch.ptr;
 	fb.scanScratchElems = ctx->scanScratch.capacity;
-	fb.recordCountDevice = fb.triOffsets + nt;
 	fb.rowCapacity = rowCap;
+	if (onePass) {
+		fb.emit.counters = ctx->control.ptr + CONTROL_EMIT;
+		fb.emit.drawn = ctx->drawnSlots.ptr;
+		fb.emit.capacity = recordCap;
+		fb.emit.extraBase = ctx->extraBase.ptr;
+		fb.emit.extraIds = ctx->extraIds.ptr;
+		fb.emit.tileHeads = ctx->tileHeads.ptr;
+		fb.emit.tileRanks = ctx->tileRanks.ptr;
+		fb.emit.segmentSlots = tallTriangles ? ctx->segmentSlots.ptr : nullptr;
+		fb.emit.tileCursors = ctx->binCursors.ptr;
+		fb.emit.bigList = ctx->bigList.ptr;
+		fb.emit.bigCount = ctx->control.ptr + CONTROL_BIG_RECORDS;
+		fb.recordCountDevice = fb.emit.counters + EMIT_DRAWN;
+		params.recordShift = 3;
+		params.extraBase = ctx->extraBase.ptr;
+	} else {
+		fb.triCounts = ctx->triCounts.ptr;
+		fb.triOffsets = ctx->triOffsets.ptr;
+		fb.rowOffsets = ctx->rowOffsets.ptr;
+		fb.recordCountDevice = fb.triOffsets + nt;
+	}
 	TileBins bins;
 	memset(&bins, 0, sizeof(bins));
 	bins.counts = ctx->binCounts.ptr;
@@ -247,8 +275,23 @@ static int enqueue_phases(dsrg_context ctx, BatchJob &job, BatchTotals &totals, 
 	bins.lists = ctx->binLists.ptr;
 	bins.listCapacity = binCap;
 	bins.bigList = ctx->bigList.ptr;
-	bins.bigCount = ctx->control.ptr + 8;
+	bins.bigCount = ctx->control.ptr + CONTROL_BIG_RECORDS;
 	bins.cleared = 1; // by the first launch of phase A
+	ClearedCounters clear;
+	memset(&clear, 0, sizeof(clear));
+	clear.tileCounts = bins.counts;
+	clear.tileCursors = bins.cursors;
+	clear.tileSlots = 2 * totals.tiles;
+	clear.control = ctx->control.ptr;
+	clear.words = CONTROL_WORDS;
+	TotalsSources from;
+	memset(&from, 0, sizeof(from));
+	from.records = fb.recordCountDevice;
+	from.rows = onePass ? fb.emit.counters + EMIT_ROWS : nullptr;
+	from.extras = onePass ? fb.emit.counters + EMIT_EXTRAS : nullptr;
+	from.rowOffsets = fb.rowOffsets;
+	from.recordCapacity = recordCap;
+	from.errorFlag = fb.errorFlag;
 	uint32_t *rowCounts = ctx->rowCounts.ptr;
 	uint32_t *gathered = ctx->readbackDevice; // records, rows, bin entries, error bits: written into host memory
 	PhaseKey key;
@@ -262,20 +305,28 @@ static int enqueue_phases(dsrg_context ctx, BatchJob &job, BatchTotals &totals, 
 	key.rowCounts = rowCounts;
 	key.recordCount = recordCap;
 	key.phase = 0;
-	// phases A (projection, record counts), B (records, row offsets, tile counts) and C (row
-	// intervals, tile lists) as one graph, then D (tiles and resolve) for solid batches as another
+	// phases A (projection, records), B (tile counts and list offsets) and C (row intervals, tile
+	// lists) as one graph, then D (tiles and resolve) for solid batches as another
 	TRY(run_phase(ctx, ctx->graphs[0], key, [&] {
-		launch_clear_tiles(params, bins, fb.errorFlag, stream);
-		launch_project(params, fb, stream);
-		launch_setup_count(params, fb, stream);
-		// the row offsets and intervals on a second branch right after the records, the tile counts,
-		// offsets and lists on this one: neither needs the other; joined before the totals
-		launch_setup_write_counting(params, fb, recordCap, rowCounts, bins, stream, ctx->branchStream, ctx->branchFork);
-		launch_rows(fb, recordCap, tallTriangles, ctx->branchStream);
-		launch_bin_fill(params, fb, recordCap, bins, stream);
-		enqueue_join(ctx->branchStream, stream, ctx->branchJoin);
-		launch_gather_totals(fb.triOffsets, (uint32_t)nt, fb.rowOffsets, recordCap, bins.offsets, totals.tiles, fb.errorFlag,
-		                     gathered, params.tileList, params.tileListCount, stream);
+		launch_project(params, fb, stream, &clear);
+		if (onePass) {
+			launch_setup_emit(params, fb, stream);
+			// the row intervals on a second branch right after the records, the tile counts, offsets
+			// and lists on this one: neither needs the other; joined before the totals
+			enqueue_join(stream, ctx->branchStream, ctx->branchFork);
+			launch_rows(fb, recordCap, ctx->branchStream);
+			launch_bin_count(params, fb, recordCap, bins, stream);
+			launch_bin_fill(params, fb, recordCap, bins, stream);
+			enqueue_join(ctx->branchStream, stream, ctx->branchJoin);
+		} else {
+			launch_setup_count(params, fb, stream);
+			launch_setup_write(params, fb, recordCap, stream);
+			launch_row_offsets(fb, recordCap, rowCounts, stream);
+			launch_rows(fb, recordCap, stream);
+			launch_bin_count(params, fb, recordCap, bins, stream);
+			launch_bin_fill(params, fb, recordCap, bins, stream);
+		}
+		launch_gather_totals(from, bins.offsets, totals.tiles, gathered, params.tileList, params.tileListCount, stream);
 	}));
 	if (!job.alpha) {
 		// phase D right behind, timed on the stream between the two graphs; after an overflow its
@@ -298,8 +349,10 @@ static int enqueue_phases(dsrg_context ctx, BatchJob &job, BatchTotals &totals, 
 	const uint32_t errorBits = ctx->pinnedReadback[3];
 	if (errorBits & ERROR_OVERFLOW_BITS) {
 		// the capacities the totals ask for; a total counted past an overflowed buffer is a lower bound
-		const bool recordsOver = totals.records > recordCap;
-		ctx->recordCapacity = std::max<uint64_t>(ctx->recordCapacity, (uint64_t)totals.records + totals.records / 4 + 1024);
+		const uint64_t extras = onePass ? ctx->pinnedReadback[TOTALS_EXTRAS] : 0;
+		const bool recordsOver = onePass ? nt + extras > recordCap : totals.records > recordCap;
+		if (onePass) ctx->extraCapacity = std::max<uint64_t>(ctx->extraCapacity, extras + extras / 4 + 1024);
+		else ctx->recordCapacity = std::max<uint64_t>(ctx->recordCapacity, (uint64_t)totals.records + totals.records / 4 + 1024);
 		if (!recordsOver) {
 			ctx->rowCapacity = std::max<uint64_t>(ctx->rowCapacity, (uint64_t)totals.rows + totals.rows / 4 + 1024);
 			ctx->binCapacity = std::max<uint64_t>(ctx->binCapacity, (uint64_t)totals.binEntries + totals.binEntries / 4 + 1024);
@@ -328,7 +381,7 @@ static int enqueue_phases(dsrg_context ctx, BatchJob &job, BatchTotals &totals, 
 		key.entries = totals.binEntries;
 		key.alphaBuffers = a;
 		key.recordCount = totals.records;
-		TRY(run_phase(ctx, ctx->graphs[3], key, [&] { launch_alpha(params, fb, bins, totals.binEntries, totals.records, a, stream); }));
+		TRY(run_phase(ctx, ctx->graphs[3], key, [&] { launch_alpha(params, fb, bins, totals.binEntries, a, stream); }));
 		TRY(cudaEventRecord(ctx->eventRasterStop, stream));
 	}
 	if (outputs) {
@@ -372,7 +425,7 @@ int occlude_enqueue(dsrg_context ctx, BatchJob &job) {
 	FrameBuffers fb;
 	memset(&fb, 0, sizeof(fb));
 	fb.points.csis = ctx->pointCsis.ptr; fb.points.isy = ctx->pointIsy.ptr; fb.points.flat = ctx->pointFlat.ptr;
-	fb.errorFlag = (int32_t *)(ctx->control.ptr + 1);
+	fb.errorFlag = (int32_t *)(ctx->control.ptr + CONTROL_ERROR);
 	launch_project(params, fb, stream);
 	launch_setup_occlude(params, fb, stream);
 	TRY(take_enqueue_error());

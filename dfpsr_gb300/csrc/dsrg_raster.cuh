@@ -5,6 +5,7 @@
 #define DSRG_RASTER_CUH
 
 #include "dsrg_exact.h"
+#include "dsrg_kernels.h"
 #include "dsrg_types.h"
 
 namespace dsrg {
@@ -55,11 +56,11 @@ __device__ __forceinline__ RowPair make_row_pair(int32_t uL, int32_t uR, int32_t
 	return rp;
 }
 
-// Row pair of a record for the rows y1, y1 + 1 from its row intervals (recordRows = its first row;
-// row offsets are even because raster bounds are row-pair aligned, so two rows load as one uint2).
-__device__ __forceinline__ RowPair record_row_pair(const DrawRecord &r, const uint32_t *recordRows, int32_t y1, int32_t height) {
+// Row pair of a record for the rows y1, y1 + 1 from the row intervals (rowStart is even because
+// raster bounds are row-pair aligned, so two rows load as one uint2).
+__device__ __forceinline__ RowPair record_row_pair(const DrawRecord &r, const uint32_t *rows, int32_t y1, int32_t height) {
 	int32_t uL, uR, lL, lR;
-	const uint2 two = *reinterpret_cast<const uint2 *>(recordRows + (y1 - r.top));
+	const uint2 two = *reinterpret_cast<const uint2 *>(rows + r.rowStart + (uint32_t)(y1 - r.top));
 	unpack_row(two.x, uL, uR);
 	unpack_row(two.y, lL, lR);
 	return make_row_pair(uL, uR, lL, lR, y1 + 1, height);
@@ -75,6 +76,22 @@ __device__ __forceinline__ float chain_add_short(float s, float d, int32_t n) {
 		return s;
 	}
 	return chain_add(s, d, n);
+}
+
+// Where record `id` is stored.  Record numbers of setup_emit_kernel are 8 * fan triangle + piece (a
+// clipped triangle is drawn as up to seven pieces): the first piece of triangle g lies at slot g,
+// further pieces after all triangles from extraBase[g].  The two-pass setup numbers its records as
+// they are stored (recordShift 0).
+__device__ __forceinline__ uint32_t record_slot(const BatchParams &b, uint32_t id) {
+	if (b.recordShift == 0) return id;
+	const uint32_t triangle = id >> 3, piece = id & 7u;
+	return piece == 0u ? triangle : b.totalTriangles + __ldg(&b.extraBase[triangle]) + piece - 1u;
+}
+
+// The number of the record stored at `slot` (extraIds: the numbers of the further pieces).
+__device__ __forceinline__ uint32_t record_id(const BatchParams &b, const uint32_t *extraIds, uint32_t slot) {
+	if (b.recordShift == 0) return slot;
+	return slot < b.totalTriangles ? slot << 3 : extraIds[slot - b.totalTriangles];
 }
 
 // The four lane values of one component (1/W or W, U/W, V/W) for the quad at x, following the

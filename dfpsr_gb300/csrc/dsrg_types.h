@@ -81,7 +81,7 @@ struct __align__(16) DrawRecord {
 	int32_t flat[6];
 	int32_t left, top, right, bottom; // getAlignedRasterBound against the whole target
 	float start[3], dx[3], dy[3];     // pWeightStart, pWeightDx, pWeightDy
-	uint32_t order;                   // submission order: triangle index * 8 + clipped sub-triangle index
+	uint32_t rowStart;                // the first of its row intervals (even)
 	uint32_t tri;                     // fan triangle of its task (polygon data for shading)
 	uint32_t task;                    // index into the batch's task table
 	uint32_t frame;                   // index into the batch's frame table
