@@ -62,19 +62,6 @@ DSRG_HD bool plane_inside(const Plane &pl, const Vec3 &p) { // math/FPlane3D.h:3
 	return fadd(dot3(p, pl.nx, pl.ny, pl.nz), -pl.offset) <= 0.0f;
 }
 
-// getTriangleVisibility (implementation/render/renderCore.cpp:172-198): 0 hidden, 1 full, 2 partial.
-DSRG_HD int triangle_visibility(const CameraData &c, const Vec3 &a, const Vec3 &b, const Vec3 &d, bool clipFrustum) {
-	const int count = clipFrustum ? c.clipCount : c.cullCount;
-	const Plane *planes = clipFrustum ? c.clip : c.cull;
-	bool anyOutside = false;
-	for (int s = 0; s < count; s++) {
-		bool oa = !plane_inside(planes[s], a), ob = !plane_inside(planes[s], b), od = !plane_inside(planes[s], d);
-		if (oa && ob && od) return 0;
-		anyOutside = anyOutside || oa || ob || od;
-	}
-	return anyOutside ? 2 : 1;
-}
-
 // ITriangle2D::isFrontfacing (implementation/render/ITriangle2D.cpp:55-60).
 DSRG_HD bool is_frontfacing(const int64_t *fx, const int64_t *fy) {
 	return ((fx[2] - fx[0]) * (fy[1] - fy[0])) + ((fy[2] - fy[0]) * (fx[0] - fx[1])) < 0;

@@ -199,7 +199,7 @@ struct dsrg_context_s {
 	std::string lastError;
 	// frame scratch, grown on demand and reused
 	DeviceBuffer<float4> pointCsis;      // projected points (ProjectedPoints)
-	DeviceBuffer<float> pointIsy;
+	DeviceBuffer<uint2> pointIsyOut;
 	DeviceBuffer<longlong2> pointFlat;
 	DeviceBuffer<uint32_t> triCounts, triOffsets, scanScratch;
 	DeviceBuffer<unsigned long long> denseKeys; // per-pixel winners of dsrg_dense_render

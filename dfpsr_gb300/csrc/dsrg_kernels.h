@@ -77,11 +77,12 @@ struct BatchParams {
 };
 
 // Projected corners (implementation/render/ProjectedPoint.h:33-49): the camera-space position and
-// the image x in one 16-byte vector, the image y, and both sub-pixel coordinates in one 16-byte
-// vector, so that the triangle setup gathers a corner with three loads.
+// the image x in one 16-byte vector, the image y with the camera planes that the point lies outside
+// of, and both sub-pixel coordinates in one 16-byte vector, so that the triangle setup gathers a
+// corner with three loads.
 struct ProjectedPoints {
 	float4 *csis;     // cs.x, cs.y, cs.z, is.x
-	float *isy;       // is.y
+	uint2 *isyOut;    // is.y (bits) and the planes the point is outside of (outside_planes)
 	longlong2 *flat;  // flat x, flat y
 };
 

@@ -214,7 +214,7 @@ static int enqueue_phases(dsrg_context ctx, BatchJob &job, BatchTotals &totals, 
 	                                   : (uint32_t)std::max<uint64_t>(ctx->recordCapacity, nt + nt / 8 + 1024);
 	const uint32_t rowCap = (uint32_t)std::max<uint64_t>(ctx->rowCapacity, (uint64_t)recordCap * 4);
 	const uint32_t binCap = (uint32_t)std::max<uint64_t>(ctx->binCapacity, (uint64_t)recordCap * 2);
-	TRY(ctx->pointCsis.reserve(np)); TRY(ctx->pointIsy.reserve(np)); TRY(ctx->pointFlat.reserve(np));
+	TRY(ctx->pointCsis.reserve(np)); TRY(ctx->pointIsyOut.reserve(np)); TRY(ctx->pointFlat.reserve(np));
 	TRY(ctx->records.reserve((size_t)recordCap + 1));
 	if (onePass) {
 		TRY(ctx->drawnSlots.reserve((size_t)recordCap + 1));
@@ -239,7 +239,7 @@ static int enqueue_phases(dsrg_context ctx, BatchJob &job, BatchTotals &totals, 
 	TRY(ctx->scanScratch.reserve(scan_scratch_elems((uint32_t)scanned + 1)));
 	FrameBuffers fb;
 	memset(&fb, 0, sizeof(fb));
-	fb.points.csis = ctx->pointCsis.ptr; fb.points.isy = ctx->pointIsy.ptr; fb.points.flat = ctx->pointFlat.ptr;
+	fb.points.csis = ctx->pointCsis.ptr; fb.points.isyOut = ctx->pointIsyOut.ptr; fb.points.flat = ctx->pointFlat.ptr;
 	fb.records = ctx->records.ptr;
 	fb.rows = ctx->rows.ptr;
 	fb.errorFlag = (int32_t *)(ctx->control.ptr + CONTROL_ERROR);
@@ -421,10 +421,10 @@ int occlude_enqueue(dsrg_context ctx, BatchJob &job) {
 	layout_tables(job, nullptr, ctx->pinnedTables, ctx->tables.ptr, params, totals);
 	TRY(cudaMemcpyAsync(ctx->tables.ptr, ctx->pinnedTables, tableBytes, cudaMemcpyHostToDevice, stream));
 	const size_t np = totals.points;
-	TRY(ctx->pointCsis.reserve(np)); TRY(ctx->pointIsy.reserve(np)); TRY(ctx->pointFlat.reserve(np));
+	TRY(ctx->pointCsis.reserve(np)); TRY(ctx->pointIsyOut.reserve(np)); TRY(ctx->pointFlat.reserve(np));
 	FrameBuffers fb;
 	memset(&fb, 0, sizeof(fb));
-	fb.points.csis = ctx->pointCsis.ptr; fb.points.isy = ctx->pointIsy.ptr; fb.points.flat = ctx->pointFlat.ptr;
+	fb.points.csis = ctx->pointCsis.ptr; fb.points.isyOut = ctx->pointIsyOut.ptr; fb.points.flat = ctx->pointFlat.ptr;
 	fb.errorFlag = (int32_t *)(ctx->control.ptr + CONTROL_ERROR);
 	launch_project(params, fb, stream);
 	launch_setup_occlude(params, fb, stream);
