@@ -220,6 +220,7 @@ struct dsrg_context_s {
 	uint64_t extraCapacity = 0, recordCapacity = 0, rowCapacity = 0, binCapacity = 0;
 	DeviceBuffer<uint32_t> binCounts, binOffsets, binCursors, binLists;
 	DeviceBuffer<uint32_t> bigList;      // records over more than four tiles
+	DeviceBuffer<uint32_t> binThresholds; // per tile: the key that large records must reach to be listed
 	DeviceBuffer<uint32_t> drawnSlots, extraBase, extraIds, segmentSlots; // the one-pass setup (EmitBuffers)
 	DeviceBuffer<uint2> tileHeads;
 	DeviceBuffer<uint4> tileRanks;

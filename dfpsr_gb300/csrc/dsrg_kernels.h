@@ -124,6 +124,7 @@ struct FrameBuffers {
 // Counters zeroed by a batch's first launch (launch_project).
 struct ClearedCounters {
 	uint32_t *tileCounts, *tileCursors; // tileSlots values each
+	uint32_t *thresholds;               // tileSlots / 2 values, or null
 	uint32_t tileSlots;
 	uint32_t *control;                  // words values: tile queue, error bits, emit counters, list lengths
 	uint32_t words;
@@ -140,6 +141,9 @@ struct TileBins {
 	// records over more than four tiles, listed by setup_emit_kernel and binned by whole blocks
 	uint32_t *bigList;
 	uint32_t *bigCount;
+	// per tile: a key (upper word) that every pixel of the tile reaches, from the big records covering it
+	// completely; large records below it are not listed.  null: nothing is culled while binning
+	uint32_t *thresholds;
 	// the tile queue is zeroed by the batch's first launch (0: launch_raster zeroes it with a memset)
 	int32_t cleared;
 };

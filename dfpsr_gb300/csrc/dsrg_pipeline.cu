@@ -235,6 +235,7 @@ static int enqueue_phases(dsrg_context ctx, BatchJob &job, BatchTotals &totals, 
 	TRY(ctx->binCursors.reserve(2 * (size_t)totals.tiles + 1));
 	TRY(ctx->binLists.reserve((size_t)binCap + 1));
 	TRY(ctx->bigList.reserve((size_t)recordCap + 1));
+	TRY(ctx->binThresholds.reserve((size_t)totals.tiles + 1));
 	const uint64_t scanned = std::max<uint64_t>(onePass ? 0 : recordCap, 2 * (uint64_t)totals.tiles);
 	TRY(ctx->scanScratch.reserve(scan_scratch_elems((uint32_t)scanned + 1)));
 	FrameBuffers fb;
@@ -277,11 +278,15 @@ static int enqueue_phases(dsrg_context ctx, BatchJob &job, BatchTotals &totals, 
 	bins.bigList = ctx->bigList.ptr;
 	bins.bigCount = ctx->control.ptr + CONTROL_BIG_RECORDS;
 	bins.cleared = 1; // by the first launch of phase A
+	// records are culled while binning where only the best key of a pixel counts: not where every
+	// fragment is counted, nor for the alpha filter, which blends them all
+	bins.thresholds = (job.alpha || params.fragments) ? nullptr : ctx->binThresholds.ptr;
 	ClearedCounters clear;
 	memset(&clear, 0, sizeof(clear));
 	clear.tileCounts = bins.counts;
 	clear.tileCursors = bins.cursors;
 	clear.tileSlots = 2 * totals.tiles;
+	clear.thresholds = bins.thresholds;
 	clear.control = ctx->control.ptr;
 	clear.words = CONTROL_WORDS;
 	TotalsSources from;

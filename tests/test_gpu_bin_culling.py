@@ -1,0 +1,65 @@
+"""GPU parity of frames whose large triangles are culled while binning, against the oracle, bit for bit.
+
+A tile's threshold is the worst key of the large records that cover it completely; records whose
+best key lies below it are not listed.  The scenes put many screen-filling triangles over one
+another: parallel layers with exact depth ties (the earliest must win), planes crossing inside
+tiles, an initial depth image in front of some of them; targets with partial tiles, odd heights
+(whose bottom tile row is not culled) and large records over at most four tiles.
+"""
+import dataclasses
+
+import numpy as np
+import pytest
+
+from dfpsr_gb300 import scenes
+from test_gpu_render import run_case
+
+pytestmark = pytest.mark.gpu
+
+
+def _layers(w, h, n, seed, tilt, perspective):
+    rng = np.random.default_rng(seed)
+    s = scenes.random_triangles(seed=seed, triangles=n, width=w, height=h, texture_size=32)
+    depth = rng.integers(-4, 5, size=(n, 1)) * 0.125  # few distinct depths: exact ties between layers
+    corners = np.array([[-9.0, -7.0], [0.0, 9.0], [9.0, -7.0]])
+    p = np.zeros((n, 3, 3))
+    p[:, :, :2] = corners * rng.uniform(0.1, 1.0, size=(n, 1, 1)) + rng.uniform(-1.0, 1.0, size=(n, 1, 2))
+    p[:, :, 2] = depth + tilt * rng.uniform(-1.0, 1.0, size=(n, 3))
+    s.positions = p.reshape(-1, 3).astype(np.float32)
+    if not perspective:
+        s = dataclasses.replace(s, perspective=False, slope=2.0)
+    return s
+
+
+@pytest.mark.parametrize("perspective", [True, False])
+@pytest.mark.parametrize("tilt", [0.0, 0.4])
+@pytest.mark.parametrize("w,h", [(48, 32), (80, 75), (129, 64), (40, 17)])
+def test_layers_over_one_another(ctx, w, h, tilt, perspective):
+    s = _layers(w, h, 400, seed=w + h, tilt=tilt, perspective=perspective)
+    run_case(ctx, s, f"{w}x{h} tilt {tilt}")
+    rng = np.random.default_rng(1)
+    depth = (rng.uniform(0.25, 0.4, (h, w)) if perspective else rng.uniform(2.4, 3.4, (h, w))).astype(np.float32)
+    depth[::3, ::5] = 0.0 if perspective else 1000.0
+    _prefilled(ctx, s, depth)
+
+
+def _prefilled(ctx, s, depth):
+    import dfpsr_gb300 as d
+    from oracle import port
+    color = np.full(depth.shape, 0x40302010, np.uint32)
+    c, z = d.render_scene(ctx, s, color, depth)
+    rc, rz, _ = port.render(s, color, depth)
+    assert np.array_equal(c, rc)
+    assert np.array_equal(z.view(np.uint32), rz.view(np.uint32))
+
+
+@pytest.mark.parametrize("w,h", [(64, 48), (95, 33)])
+def test_depth_only_layers(ctx, w, h):
+    import dfpsr_gb300 as d
+    from oracle import port
+    s = _layers(w, h, 300, seed=w, tilt=0.3, perspective=True)
+    z = np.zeros((h, w), np.float32)
+    m = d.Model(ctx, s)
+    ctx.render_depth(m, m.camera, z)
+    rz = port.render_depth(s)[0]
+    assert np.array_equal(z.view(np.uint32), rz.view(np.uint32))
