@@ -111,6 +111,7 @@ int dsrg_context_destroy(dsrg_context ctx) {
 	if (ctx->branchJoin) cudaEventDestroy(ctx->branchJoin);
 	if (ctx->branchStream) cudaStreamDestroy(ctx->branchStream);
 	ctx->tileList.release(); ctx->bigList.release(); ctx->binThresholds.release();
+	ctx->tileParts.release(); ctx->tilePartsDone.release();
 	ctx->drawnSlots.release(); ctx->extraBase.release(); ctx->extraIds.release(); ctx->tileHeads.release(); ctx->tileRanks.release();
 	ctx->segmentSlots.release();
 	for (PhaseGraph &g : ctx->graphs) g.reset();

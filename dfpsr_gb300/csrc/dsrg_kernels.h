@@ -144,9 +144,24 @@ struct TileBins {
 	// per tile: a key (upper word) that every pixel of the tile reaches, from the big records covering it
 	// completely; large records below it are not listed.  null: nothing is culled while binning
 	uint32_t *thresholds;
+	// tiles weighing more than PART_WEIGHT as (tile, part) items, and per tile the parts done; null: every
+	// tile is drawn by one CTA
+	uint2 *parts;
+	uint32_t *partCount;
+	uint32_t partCapacity;
+	uint32_t *partsDone;
 	// the tile queue is zeroed by the batch's first launch (0: launch_raster zeroes it with a memset)
 	int32_t cleared;
 };
+
+// What a tile's lists cost to draw, and the share of it that one CTA takes.  A large entry is walked by
+// a whole warp, small ones 32 at a time: about eight times the time.  Shares of 2,048 to 8,192 take a
+// batch of small frames of many triangles the same time; dense terrain seen from afar (a thousand
+// small entries in a tile of the horizon) should not be cut, which cost 3 to 10 % of its frame.
+static const uint32_t LARGE_WEIGHT = 8, PART_WEIGHT = 4096;
+__host__ __device__ inline uint32_t part_weight(uint32_t smalls, uint32_t larges) { return smalls + LARGE_WEIGHT * larges; }
+// At most this many parts for lists of `entries` entries in all: a cut tile weighs more than PART_WEIGHT.
+inline uint32_t max_parts(uint64_t entries) { return (uint32_t)(2 * LARGE_WEIGHT * entries / PART_WEIGHT) + 1u; }
 
 // True when one lane walks the whole record inside a tile (small-triangle path).
 __host__ __device__ inline bool bound_is_small(int32_t left, int32_t top, int32_t right, int32_t bottom, int32_t smallRows,
@@ -237,8 +252,7 @@ struct TotalsSources {
 	uint32_t recordCapacity;
 	const int32_t *errorFlag;
 };
-void launch_gather_totals(const TotalsSources &from, const uint32_t *binOffsets, uint32_t tiles, uint32_t *out, uint32_t *tileList,
-                          uint32_t *tileListCount, cudaStream_t stream);
+void launch_gather_totals(const BatchParams &b, const TotalsSources &from, const TileBins &bins, uint32_t *out, cudaStream_t stream);
 // Exclusive scan of n uint32 values into out (out[n] = total); two launches, scratch of
 // scan_scratch_elems(n) values.
 void launch_scan(const uint32_t *in, uint32_t *out, uint32_t n, uint32_t *scratch, size_t scratchElems, cudaStream_t stream);

@@ -236,6 +236,8 @@ static int enqueue_phases(dsrg_context ctx, BatchJob &job, BatchTotals &totals, 
 	TRY(ctx->binLists.reserve((size_t)binCap + 1));
 	TRY(ctx->bigList.reserve((size_t)recordCap + 1));
 	TRY(ctx->binThresholds.reserve((size_t)totals.tiles + 1));
+	TRY(ctx->tileParts.reserve((size_t)max_parts(binCap) + 1));
+	TRY(ctx->tilePartsDone.reserve((size_t)totals.tiles + 1));
 	const uint64_t scanned = std::max<uint64_t>(onePass ? 0 : recordCap, 2 * (uint64_t)totals.tiles);
 	TRY(ctx->scanScratch.reserve(scan_scratch_elems((uint32_t)scanned + 1)));
 	FrameBuffers fb;
@@ -281,6 +283,12 @@ static int enqueue_phases(dsrg_context ctx, BatchJob &job, BatchTotals &totals, 
 	// records are culled while binning where only the best key of a pixel counts: not where every
 	// fragment is counted, nor for the alpha filter, which blends them all
 	bins.thresholds = (job.alpha || params.fragments) ? nullptr : ctx->binThresholds.ptr;
+	if (!job.alpha) {
+		bins.parts = ctx->tileParts.ptr;
+		bins.partCount = ctx->control.ptr + CONTROL_TILE_PARTS;
+		bins.partCapacity = max_parts(binCap);
+		bins.partsDone = ctx->tilePartsDone.ptr;
+	}
 	ClearedCounters clear;
 	memset(&clear, 0, sizeof(clear));
 	clear.tileCounts = bins.counts;
@@ -331,7 +339,7 @@ static int enqueue_phases(dsrg_context ctx, BatchJob &job, BatchTotals &totals, 
 			launch_bin_count(params, fb, recordCap, bins, stream);
 			launch_bin_fill(params, fb, recordCap, bins, stream);
 		}
-		launch_gather_totals(from, bins.offsets, totals.tiles, gathered, params.tileList, params.tileListCount, stream);
+		launch_gather_totals(params, from, bins, gathered, stream);
 	}));
 	if (!job.alpha) {
 		// phase D right behind, timed on the stream between the two graphs; after an overflow its

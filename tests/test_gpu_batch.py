@@ -313,3 +313,54 @@ def test_batch_with_a_tuning_of_its_own(ctx):
         ctx.set_tuning(**{k: v for k, v in before.items()})
         for m in models:
             m.destroy()
+
+
+@pytest.mark.parametrize("w,h,triangles,smalls", [(16, 16, 9000, False), (33, 17, 12000, False), (20, 31, 30000, True), (64, 64, 40000, False)])
+@pytest.mark.parametrize("resolve", [0, 1])
+def test_tiles_drawn_in_parts(ctx, w, h, triangles, smalls, resolve):
+    """Small frames of many triangles: each tile's lists are cut into parts that several blocks draw at
+    once (large entries, then a frame of tiny triangles, whose small lists are cut); counting every
+    fragment and not, bit for bit, beside a frame with nothing to cut in the same batch."""
+    import torch
+    import dfpsr_gb300 as d
+    from oracle import port
+    s = scenes.random_triangles(seed=w * h, triangles=triangles, width=w, height=h, texture_size=32)
+    if smalls:
+        p = s.positions.reshape(-1, 3, 3)
+        s.positions = (p.mean(axis=1, keepdims=True) + 0.1 * (p - p.mean(axis=1, keepdims=True))).reshape(-1, 3)
+    other = scenes.random_triangles(seed=5, triangles=200, width=80, height=49, texture_size=32)
+    saved = ctx.tuning()
+    try:
+        ctx.set_tuning(resolve=resolve)
+        for counting in (True, False):
+            batch = ctx.batch()
+            images = []
+            for scene in (s, other):
+                c = torch.zeros((scene.height, scene.width), dtype=torch.int32, device="cuda")
+                z = torch.zeros((scene.height, scene.width), dtype=torch.float32, device="cuda")
+                batch.give_task(batch.add_frame(c, z), d.Model(ctx, scene))
+                images.append((c, z))
+            ctx.set_counting(counting)
+            batch.render()
+            fragments = ctx.stats()["fragments"]
+            ctx.set_counting(False)
+            total = 0
+            for scene, (c, z) in zip((s, other), images):
+                rc, rz, info = port.render(scene)
+                total += info["fragments"]
+                assert np.array_equal(c.cpu().numpy().view(np.uint32), rc)
+                assert np.array_equal(z.cpu().numpy().view(np.uint32), rz.view(np.uint32))
+            assert not counting or fragments == total
+            batch.destroy()
+    finally:
+        ctx.set_tuning(resolve=saved["resolve"])
+
+
+def test_depth_only_tiles_drawn_in_parts(ctx):
+    import dfpsr_gb300 as d
+    from oracle import port
+    s = scenes.random_triangles(seed=8, triangles=15000, width=35, height=18)
+    z = np.zeros((18, 35), np.float32)
+    m = d.Model(ctx, s)
+    ctx.render_depth(m, m.camera, z)
+    assert np.array_equal(z.view(np.uint32), port.render_depth(s)[0].view(np.uint32))
