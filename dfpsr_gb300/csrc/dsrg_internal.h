@@ -242,14 +242,12 @@ struct dsrg_context_s {
 	DeviceBuffer<unsigned long long> fragmentCounter;
 	DeviceBuffer<unsigned long long> keys;
 	DeviceBuffer<uint32_t> rowCounts, rowOffsets, rows;
-	DeviceBuffer<uint32_t> alphaEntryTile, alphaTileKeys, alphaRecords; // the alpha filter's list order
-	DeviceBuffer<uint32_t> sortKeysA, sortKeysB, sortIdsA, sortIdsB, sortHist, sortOffsets;
 	int32_t smallRows = 8, smallWidth = 16; // one lane walks records whose raster bound is at most 8 x 16 pixels
 	int32_t ctasPerSm = 4;                  // resident CTAs per SM of the persistent tile kernel
 	int32_t threadsPerTile = 256;           // threads of one tile's CTA
 	int32_t useGraphs = 1;                  // replay unchanged phases as CUDA graphs
 	int32_t resolveMode = 1;                // 0 per pixel in its own pass, 1 per pixel in the tile kernel, 2 per quad
-	dsrg::PhaseGraph graphs[4];             // phases A, B, C (lists) and D (raster)
+	dsrg::PhaseGraph graphs[4];             // phases A to C and D of solid batches, then of alpha-filtered ones
 	int32_t counting = 0;
 	uint32_t *coverage = nullptr;
 	dsrg_stats stats;

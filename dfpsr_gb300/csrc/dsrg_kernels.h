@@ -228,16 +228,9 @@ uint32_t sort_blocks(uint64_t n);
 // their keys; *sortedKeys and *sortedIds point at the buffers holding the result (the inputs when n is 0).
 void launch_stable_sort(const uint32_t *keys, const uint32_t *ids, uint64_t n, int keyBits, const SortBuffers &b,
                         cudaStream_t stream, const uint32_t **sortedKeys, const uint32_t **sortedIds);
-// Scratch of launch_alpha for `entries` list entries: entryTile, tileKeys and records hold
-// `entries` values each; sort as launch_stable_sort needs for `entries` items.
-struct AlphaBuffers {
-	uint32_t *entryTile, *tileKeys, *records;
-	SortBuffers sort;
-};
 // The alpha filter over the binned records (in place of launch_raster): colour blends in
 // submission order, depth read only.
-void launch_alpha(const BatchParams &b, const FrameBuffers &fb, const TileBins &bins, uint32_t entries, const AlphaBuffers &a,
-                  cudaStream_t stream);
+void launch_alpha(const BatchParams &b, const FrameBuffers &fb, const TileBins &bins, cudaStream_t stream);
 // Debug overlays: the three edges of every record as lines in pixels (flat / 256), and draw_line
 // (api/drawAPI.cpp:176-279) of many lines of one packed colour into a device image.
 void launch_wire_lines(const DrawRecord *records, const uint32_t *drawn, uint32_t count, int4 *lines, cudaStream_t stream);

@@ -96,8 +96,6 @@ struct PhaseKey {
 	int32_t resolve;
 	int32_t alpha;
 	uint32_t recordCount;
-	uint32_t entries;
-	AlphaBuffers alphaBuffers;
 	RasterConfig config;
 	BatchParams params;
 	FrameBuffers fb;
@@ -319,8 +317,9 @@ static int enqueue_phases(dsrg_context ctx, BatchJob &job, BatchTotals &totals, 
 	key.recordCount = recordCap;
 	key.phase = 0;
 	// phases A (projection, records), B (tile counts and list offsets) and C (row intervals, tile
-	// lists) as one graph, then D (tiles and resolve) for solid batches as another
-	TRY(run_phase(ctx, ctx->graphs[0], key, [&] {
+	// lists) as one graph, then D (tiles and resolve, or the alpha filter) as another
+	const int graph = job.alpha ? 2 : 0; // a frame's solid and alpha-filtered runs each keep their graphs
+	TRY(run_phase(ctx, ctx->graphs[graph], key, [&] {
 		launch_project(params, fb, stream, &clear);
 		if (onePass) {
 			launch_setup_emit(params, fb, stream);
@@ -341,21 +340,22 @@ static int enqueue_phases(dsrg_context ctx, BatchJob &job, BatchTotals &totals, 
 		}
 		launch_gather_totals(params, from, bins, gathered, stream);
 	}));
-	if (!job.alpha) {
-		// phase D right behind, timed on the stream between the two graphs; after an overflow its
-		// kernels return at once and the targets stay untouched
-		TRY(cudaEventRecord(ctx->eventRasterStart, stream));
-		key.phase = 1;
-		TRY(run_phase(ctx, ctx->graphs[1], key, [&] { launch_raster(params, fb, bins, config, job.resolve, stream); }));
-		TRY(cudaEventRecord(ctx->eventRasterStop, stream));
-		// the batch's own work ends here: the one host wait below also completes the timing events
-		TRY(cudaEventRecord(ctx->eventStop, stream));
-		if (ctx->counting)
-			TRY(cudaMemcpyAsync(ctx->pinnedReadback + 4, ctx->fragmentCounter.ptr, sizeof(unsigned long long), cudaMemcpyDeviceToHost,
-			                    stream));
-	}
+	// phase D right behind, timed on the stream between the two graphs; after an overflow its
+	// kernels return at once and the targets stay untouched
+	TRY(cudaEventRecord(ctx->eventRasterStart, stream));
+	key.phase = 1;
+	TRY(run_phase(ctx, ctx->graphs[graph + 1], key, [&] {
+		if (job.alpha) launch_alpha(params, fb, bins, stream);
+		else launch_raster(params, fb, bins, config, job.resolve, stream);
+	}));
+	TRY(cudaEventRecord(ctx->eventRasterStop, stream));
+	// the batch's own work ends here: the one host wait below also completes the timing events
+	TRY(cudaEventRecord(ctx->eventStop, stream));
+	if (ctx->counting)
+		TRY(cudaMemcpyAsync(ctx->pinnedReadback + 4, ctx->fragmentCounter.ptr, sizeof(unsigned long long), cudaMemcpyDeviceToHost,
+		                    stream));
 	TRY(cudaStreamSynchronize(stream));
-	ctx->stopRecorded = !job.alpha;
+	ctx->stopRecorded = true;
 	totals.records = ctx->pinnedReadback[0];
 	totals.rows = ctx->pinnedReadback[1];
 	totals.binEntries = ctx->pinnedReadback[2];
@@ -373,30 +373,6 @@ static int enqueue_phases(dsrg_context ctx, BatchJob &job, BatchTotals &totals, 
 		return DSRG_RETRY;
 	}
 	if (errorBits != 0) return fail(ctx, DSRG_ERROR_DEVICE, "triangle setup reported device error bits " + std::to_string(errorBits));
-	if (job.alpha) {
-		// blending in submission order: sorted tile lists, one thread per pixel (needs the entry count)
-		TRY(cudaEventRecord(ctx->eventRasterStart, stream));
-		const uint64_t n = totals.binEntries;
-		const uint32_t blocks = sort_blocks(n);
-		TRY(ctx->alphaEntryTile.reserve(n + 1)); TRY(ctx->alphaTileKeys.reserve(n + 1)); TRY(ctx->alphaRecords.reserve(n + 1));
-		TRY(ctx->sortKeysA.reserve(n + 1)); TRY(ctx->sortKeysB.reserve(n + 1));
-		TRY(ctx->sortIdsA.reserve(n + 1)); TRY(ctx->sortIdsB.reserve(n + 1));
-		TRY(ctx->sortHist.reserve((size_t)256 * blocks + 1)); TRY(ctx->sortOffsets.reserve((size_t)256 * blocks + 1));
-		TRY(ctx->scanScratch.reserve(scan_scratch_elems((uint32_t)((size_t)256 * blocks) + 1)));
-		AlphaBuffers a;
-		memset(&a, 0, sizeof(a));
-		a.entryTile = ctx->alphaEntryTile.ptr; a.tileKeys = ctx->alphaTileKeys.ptr; a.records = ctx->alphaRecords.ptr;
-		a.sort.keysA = ctx->sortKeysA.ptr; a.sort.keysB = ctx->sortKeysB.ptr;
-		a.sort.idsA = ctx->sortIdsA.ptr; a.sort.idsB = ctx->sortIdsB.ptr;
-		a.sort.hist = ctx->sortHist.ptr; a.sort.offsets = ctx->sortOffsets.ptr;
-		a.sort.scanScratch = ctx->scanScratch.ptr; a.sort.scanScratchElems = ctx->scanScratch.capacity;
-		key.phase = 3;
-		key.entries = totals.binEntries;
-		key.alphaBuffers = a;
-		key.recordCount = totals.records;
-		TRY(run_phase(ctx, ctx->graphs[3], key, [&] { launch_alpha(params, fb, bins, totals.binEntries, a, stream); }));
-		TRY(cudaEventRecord(ctx->eventRasterStop, stream));
-	}
 	if (outputs) {
 		outputs->params = params;
 		outputs->fb = fb;

@@ -1,8 +1,7 @@
 // Stable LSD radix sort of (key, id) pairs, 8 bits per pass: per-block digit histograms, one scan
 // over (digit, block) in digit-major order, and a scatter that keeps each block's items in input
 // order (ranks within a warp from __match_any_sync, across warps from per-warp digit counts).
-// Used by the deterministic adjoint of the differentiable renderer and by the alpha filter, which
-// needs every tile's list in submission order.
+// Used by the deterministic adjoint of the differentiable renderer.
 #include <cuda_runtime.h>
 #include <stdint.h>
 

@@ -135,3 +135,18 @@ def test_frame_mixing_solid_and_alpha_tasks(ctx):
         assert np.array_equal(cov.cpu().numpy().view(np.uint32), coverage), f"repeat {repeat}: coverage differs"
         assert stats["fragments"] == fragments
         r.destroy()
+
+
+@pytest.mark.parametrize("w,h,triangles", [(16, 16, 2048), (17, 15, 2600), (33, 16, 9000), (20, 37, 40)])
+@pytest.mark.parametrize("perspective", [True, False])
+def test_alpha_lists_around_the_shared_sort(ctx, w, h, triangles, perspective):
+    """Tiles whose lists are shorter than one staged chunk, about as long as the sort in shared memory
+    holds, and longer (taken in windows), on odd and even heights."""
+    from oracle import port
+    s = _alpha_scene(w + h + triangles, triangles=2 * triangles, width=w, height=h)  # about half face the camera
+    if not perspective:
+        s = dataclasses.replace(s, perspective=False, slope=1.2)
+    color, depth = _prefilled(3, h, w)
+    if not perspective:
+        depth = (depth * 5.0 + 2.5).astype(np.float32)
+    _check(_gpu(ctx, s, color, depth), port.render(s, color, depth, coverage=True), f"{w}x{h} {triangles}")
