@@ -209,7 +209,7 @@ struct dsrg_context_s {
 	unsigned char *pinnedTables = nullptr; // host staging of the tables (page-locked)
 	size_t pinnedCapacity = 0;
 	DeviceBuffer<uint32_t> control;      // a batch's counters (ControlWord)
-	DeviceBuffer<uint32_t> tileList;     // the tiles of a batch that have tile-list entries
+	DeviceBuffer<uint4> tileList;        // the tiles of a batch that have tile-list entries
 	uint32_t *pinnedReadback = nullptr;  // page-locked: the gathered totals (written there by the GPU), the fragment count,
 	                                     // [8] the entries a deterministic adjoint's sums keep, [9] TOTALS_EXTRAS
 	uint32_t *readbackDevice = nullptr;  // its device address

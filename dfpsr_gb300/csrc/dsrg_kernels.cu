@@ -753,11 +753,12 @@ void launch_scan_device(const uint32_t *in, uint32_t *out, const uint32_t *nDevi
 // launch lists the tiles that have entries (one thread per tile, warp-aggregated appends), so that
 // the persistent tile kernel pulls only those: frames that are mostly empty (shadow-cube faces) no
 // longer send every CTA through thousands of empty tiles.  And it cuts tiles weighing more than
-// PART_WEIGHT into parts, which the tile kernel draws before the other tiles (raster_kernel).
+// bins.partWeight into parts, which the tile kernel draws before the other tiles (raster_kernel).
 __global__ void gather_totals_kernel(BatchParams b, TotalsSources from, TileBins bins, uint32_t *out) {
 	const uint32_t *binOffsets = bins.offsets;
 	const uint32_t tiles = b.totalTiles;
-	uint32_t *tileList = b.tileList, *tileListCount = b.tileListCount;
+	uint4 *tileList = b.tileList;
+	uint32_t *tileListCount = b.tileListCount;
 	chain_enter();
 	if (blockIdx.x == 0 && threadIdx.x == 0) {
 		const uint32_t records = *from.records;
@@ -772,11 +773,11 @@ __global__ void gather_totals_kernel(BatchParams b, TotalsSources from, TileBins
 		for (uint32_t first = blockIdx.x * blockDim.x; first < tiles; first += gridDim.x * blockDim.x) { // uniform per block
 			const uint32_t t = first + threadIdx.x;
 			const uint32_t weight = t < tiles ? part_weight(bins.cursors[2 * t], bins.cursors[2 * t + 1]) : 0u;
-			const bool cut = weight > PART_WEIGHT;
+			const bool cut = weight > bins.partWeight;
 			const uint32_t cutMask = __ballot_sync(0xFFFFFFFFu, cut);
 			if (!cutMask) continue;
 			// the warp's parts from one atomic
-			const uint32_t parts = cut ? (weight + PART_WEIGHT - 1) / PART_WEIGHT : 0u;
+			const uint32_t parts = cut ? (weight + bins.partWeight - 1) / bins.partWeight : 0u;
 			uint32_t inclusive = parts;
 			for (int o = 1; o < 32; o <<= 1) {
 				const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, inclusive, o);
@@ -820,7 +821,9 @@ __global__ void gather_totals_kernel(BatchParams b, TotalsSources from, TileBins
 		uint32_t at = 0;
 		if (lane == leader) at = atomicAdd(tileListCount, (uint32_t)__popc(mask));
 		at = __shfl_sync(0xFFFFFFFFu, at, leader);
-		if (drawn) tileList[at + __popc(mask & ((1u << lane) - 1u))] = t;
+		if (drawn) // large entries only: depth-only batches have no small ones
+			tileList[at + __popc(mask & ((1u << lane) - 1u))] =
+				make_uint4(t, binOffsets[2 * t + 1], bins.cursors[2 * t + 1], (uint32_t)find_segment(b.frameTileBase, b.frameCount, t));
 	}
 }
 
@@ -1521,7 +1524,7 @@ __device__ __forceinline__ void resolve_shared_quad(const BatchParams &b, const 
 // which evaluates the running sums once at the tile's left edge and then walks on.
 // All fragments compete for the tile's shared keys; the winners go to the frame's key image.
 // Tiles that nothing covers write nothing: the resolve pass skips them too.
-// A tile weighing more than PART_WEIGHT is drawn in parts by several CTAs at once: each draws its
+// A tile weighing more than bins.partWeight is drawn in parts by several CTAs at once: each draws its
 // share of the lists, merges its keys into the key image with 64-bit maxima (the same order-free
 // argument as inside a CTA) and counts itself done; the last part to finish resolves the tile.  No
 // CTA waits for another.  Small frames of many triangles have a few tiles with thousands of entries,
@@ -1563,7 +1566,7 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) raster_kernel(BatchPa
 				sharedPart = item.y;
 			} else {
 				ticket -= partItems;
-				sharedTile = !b.tileList ? ticket : (ticket < listed ? b.tileList[ticket] : 0xFFFFFFFFu);
+				sharedTile = !b.tileList ? ticket : (ticket < listed ? b.tileList[ticket].x : 0xFFFFFFFFu);
 			}
 			fragmentSum = 0ull;
 		}
@@ -1576,11 +1579,11 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) raster_kernel(BatchPa
 		const uint32_t smalls = smallEnd - smallBegin;
 		// nothing to draw, or drawn in parts
 		const uint32_t weight = part_weight(smalls, end - largeBegin);
-		if (weight == 0u || (sharedPart == WHOLE_TILE && bins.parts && weight > PART_WEIGHT)) { __syncthreads(); continue; }
+		if (weight == 0u || (sharedPart == WHOLE_TILE && bins.parts && weight > bins.partWeight)) { __syncthreads(); continue; }
 		if (sharedPart != WHOLE_TILE) { // (read where it is needed: a register for it costs the resolve spills)
 			// this part's share of the small list followed by the large one
-			if (tid == 0) sharedParts = (weight + PART_WEIGHT - 1) / PART_WEIGHT;
-			const uint32_t lo = sharedPart * PART_WEIGHT, hi = min(lo + PART_WEIGHT, weight);
+			if (tid == 0) sharedParts = (weight + bins.partWeight - 1) / bins.partWeight;
+			const uint32_t lo = sharedPart * bins.partWeight, hi = min(lo + bins.partWeight, weight);
 			end = largeBegin + (max(hi, smalls) - smalls) / LARGE_WEIGHT;
 			largeBegin += (max(lo, smalls) - smalls) / LARGE_WEIGHT;
 			smallEnd = smallBegin + min(hi, smalls);
@@ -1862,6 +1865,167 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) raster_kernel(BatchPa
 			if (b.walked) atomicAdd(b.walked, fragmentSum);
 		}
 		__syncthreads();
+	}
+}
+
+// Depth-only batches (shadow-cube faces, model_renderDepth): one warp per tile.  Lane l owns eight
+// pixels of row l / 2 (the left half of the tile for even lanes, the right one for odd), which is how the
+// reference's 1 x 1 walk runs along a row, so the tile's keys stay in the lanes' registers: no shared
+// memory, no barriers and no atomics.  A lane starts each pixel from the key of the depth already in
+// the image with the largest low word, which no record has, so a fragment replaces it exactly when it
+// passes the reference's strict test; a NaN in the image is never passed.  What bounds it is the latency
+// of a tile's few dependent loads (shadow faces have two or three entries per drawn tile), hence many
+// small independent warps, a descriptor per listed tile, the next ticket taken a tile ahead and each
+// record's row interval loaded one record ahead.  With a block of 64 threads per tile and keys in
+// shared memory the 96 faces of the 1080p light frame took 180 us; they now take 83 us (frame 710 -> 616 us).
+// Tiles cut into parts (raster_kernel) meet in the key image as there.
+static const int DEPTH_PIXELS = 8; // of one lane
+static const int DEPTH_BLOCKS = 8; // of four warps, per SM
+
+__global__ void __launch_bounds__(128) raster_depth_kernel(BatchParams b, const DrawRecord *__restrict__ records, TileBins bins,
+                                                           const uint32_t *__restrict__ rows) {
+	chain_enter();
+	if (overflowed(b)) return;
+	const int lane = threadIdx.x & 31;
+	const uint32_t partItems = bins.parts ? *bins.partCount : 0u, items = partItems + *b.tileListCount;
+	uint32_t walked = 0;
+	uint32_t ticket = 0;
+	if (lane == 0) ticket = atomicAdd(b.tileQueue, 1u);
+	ticket = __shfl_sync(0xFFFFFFFFu, ticket, 0);
+	while (ticket < items) { // every condition on the ticket's tile is the same for the whole warp
+		uint32_t following = 0;
+		if (lane == 0) following = atomicAdd(b.tileQueue, 1u);
+		uint32_t part = WHOLE_TILE, parts = 1;
+		uint4 item; // tile, first entry, entries, frame
+		if (ticket < partItems) {
+			const uint2 p = bins.parts[ticket];
+			part = p.y;
+			item.x = p.x;
+			item.y = bins.offsets[2 * p.x + 1];
+			item.z = bins.cursors[2 * p.x + 1];
+			item.w = (uint32_t)find_segment(b.frameTileBase, b.frameCount, p.x);
+			const uint32_t weight = part_weight(0u, item.z);
+			parts = (weight + bins.partWeight - 1) / bins.partWeight;
+			const uint32_t lo = part * bins.partWeight / LARGE_WEIGHT, hi = min((part + 1) * bins.partWeight, weight) / LARGE_WEIGHT;
+			item.y += lo;
+			item.z = hi - lo;
+		} else {
+			item = b.tileList[ticket - partItems];
+			if (bins.parts && part_weight(0u, item.z) > bins.partWeight) { // drawn in parts
+				ticket = __shfl_sync(0xFFFFFFFFu, following, 0);
+				continue;
+			}
+		}
+		const FrameTarget &f = b.frames[item.w];
+		const int32_t width = f.width, height = f.height, tilesX = f.tilesX;
+		const bool affine = f.affine != 0;
+		const int32_t local = (int32_t)(item.x - f.tileBase);
+		const int32_t y = (local / tilesX) * TILE_H + (lane >> 1), xs = (local % tilesX) * TILE_W + (lane & 1) * DEPTH_PIXELS;
+		float *pixels = f.depth + (size_t)y * f.depthStride + xs; // (used inside the image only)
+		const int32_t valid = y < height ? min(DEPTH_PIXELS, width - xs) : 0;
+		const bool vector = valid == DEPTH_PIXELS && (reinterpret_cast<unsigned long long>(pixels) & 15ull) == 0ull;
+		unsigned long long key[DEPTH_PIXELS];
+		{
+			float initial[DEPTH_PIXELS];
+			if (vector) {
+				const float4 a = reinterpret_cast<const float4 *>(pixels)[0], c = reinterpret_cast<const float4 *>(pixels)[1];
+				initial[0] = a.x; initial[1] = a.y; initial[2] = a.z; initial[3] = a.w;
+				initial[4] = c.x; initial[5] = c.y; initial[6] = c.z; initial[7] = c.w;
+			} else {
+#pragma unroll
+				for (int k = 0; k < DEPTH_PIXELS; k++) initial[k] = k < valid ? pixels[k] : 0.0f;
+			}
+#pragma unroll
+			for (int k = 0; k < DEPTH_PIXELS; k++) {
+				uint32_t hi = ordered_depth(initial[k]);
+				if (affine) hi = ~hi;
+				if (k >= valid || initial[k] != initial[k]) hi = 0xFFFFFFFFu;
+				key[k] = ((unsigned long long)hi << 32) | 0xFFFFFFFFull;
+			}
+		}
+		uint32_t drawn = 0; // pixels some record has won
+		for (uint32_t first = 0; first < item.z; first += 32u) {
+			const uint32_t count = min(32u, item.z - first);
+			uint32_t id = 0, rowStart = 0;
+			int32_t top = 0, bottom = 0;
+			float start = 0.0f, dx = 0.0f, dy = 0.0f;
+			if ((uint32_t)lane < count) {
+				id = bins.lists[item.y + first + (uint32_t)lane];
+				const DrawRecord &r = records[record_slot(b, id)];
+				top = r.top; bottom = r.bottom;
+				start = r.start[0]; dx = r.dx[0]; dy = r.dy[0];
+				rowStart = r.rowStart;
+			}
+			// this lane's row of record j
+			auto interval = [&](uint32_t j) -> uint32_t {
+				const int32_t t = __shfl_sync(0xFFFFFFFFu, top, j), o = __shfl_sync(0xFFFFFFFFu, bottom, j);
+				const uint32_t at = __shfl_sync(0xFFFFFFFFu, rowStart, j);
+				return (valid > 0 && y >= t && y < o) ? rows[at + (uint32_t)(y - t)] : 0u;
+			};
+			uint32_t ahead = interval(0);
+			for (uint32_t j = 0; j < count; j++) {
+				const uint32_t packed = ahead;
+				if (j + 1 < count) ahead = interval(j + 1);
+				const float s = __shfl_sync(0xFFFFFFFFu, start, j), sx = __shfl_sync(0xFFFFFFFFu, dx, j), sy = __shfl_sync(0xFFFFFFFFu, dy, j);
+				const uint32_t record = __shfl_sync(0xFFFFFFFFu, id, j);
+				int32_t left, right;
+				unpack_row(packed, left, right);
+				const int32_t x0 = max(xs, left), x1 = min(xs + valid, right);
+				if (x0 >= x1) continue;
+				walked += (uint32_t)(x1 - x0);
+				// executeTriangleDrawingDepth (renderCore.cpp:343-387): depth starts at the row's left pixel
+				// and grows by dx one pixel at a time
+				float z = fadd(fadd(s, fmul(sx, (float)left + 0.5f)), fmul(sy, (float)y + 0.5f));
+				z = chain_add(z, sx, x0 - left);
+#pragma unroll
+				for (int k = 0; k < DEPTH_PIXELS; k++) {
+					if (xs + k < x0 || xs + k >= x1) continue;
+					const unsigned long long candidate = make_key(z, record, true, affine);
+					if (z == z && candidate > key[k]) {
+						key[k] = candidate;
+						drawn |= 1u << k;
+					}
+					z = fadd(z, sx);
+				}
+			}
+		}
+		if (part != WHOLE_TILE) {
+			// the part's keys into the key image; the tile's last part writes the depths of all of them
+			unsigned long long *merged = f.keys + (size_t)y * width + xs;
+#pragma unroll
+			for (int k = 0; k < DEPTH_PIXELS; k++)
+				if ((drawn >> k) & 1u) atomicMax(merged + k, key[k]);
+			__threadfence();
+			__syncwarp();
+			uint32_t done = 0;
+			if (lane == 0) done = atomicAdd(&bins.partsDone[item.x], 1u) + 1u;
+			done = __shfl_sync(0xFFFFFFFFu, done, 0);
+			drawn = 0;
+			if (done == parts) {
+				__threadfence();
+#pragma unroll
+				for (int k = 0; k < DEPTH_PIXELS; k++) {
+					key[k] = k < valid ? __ldcg(merged + k) : 0ull;
+					if (key[k] != 0ull) drawn |= 1u << k;
+				}
+			}
+		}
+		if (vector && drawn == 0xFFu) {
+			float z[DEPTH_PIXELS];
+#pragma unroll
+			for (int k = 0; k < DEPTH_PIXELS; k++) z[k] = depth_from_key(b, key[k], affine, records, rows, xs + k, y);
+			reinterpret_cast<float4 *>(pixels)[0] = make_float4(z[0], z[1], z[2], z[3]);
+			reinterpret_cast<float4 *>(pixels)[1] = make_float4(z[4], z[5], z[6], z[7]);
+		} else {
+#pragma unroll
+			for (int k = 0; k < DEPTH_PIXELS; k++)
+				if ((drawn >> k) & 1u) pixels[k] = depth_from_key(b, key[k], affine, records, rows, xs + k, y);
+		}
+		ticket = __shfl_sync(0xFFFFFFFFu, following, 0);
+	}
+	if (b.walked) {
+		for (int o = 16; o > 0; o >>= 1) walked += __shfl_xor_sync(0xFFFFFFFFu, walked, o);
+		if (lane == 0 && walked) atomicAdd(b.walked, (unsigned long long)walked);
 	}
 }
 
@@ -2338,6 +2502,10 @@ void launch_raster(const BatchParams &b, const FrameBuffers &fb, const TileBins 
 	const uint64_t items = (uint64_t)b.totalTiles + (bins.parts ? bins.partCapacity : 0u);
 	if (ctas > items) ctas = (uint32_t)items;
 	COUNT_LAUNCH();
+	if (b.depthOnly && resolve && b.tileList && !b.fragments) { // counting fragments, and batches without a tile list: raster_kernel
+		launch_chained(raster_depth_kernel, sm_count() * DEPTH_BLOCKS, 128, stream, b, fb.records, bins, fb.rows);
+		return;
+	}
 	// small triangles resolve per pixel inside the tile pass; the keys then never leave the chip
 	const bool fused = resolve && !b.depthOnly && config.resolveMode == 1;
 #define DSRG_RASTER(T)                                                                                            \

@@ -69,7 +69,8 @@ struct BatchParams {
 	int32_t oddDepthFrames;           // frames of odd height with a depth buffer (their last row: odd_row_kernel)
 	int32_t maxTilesX;                // the widest frame's tile columns
 	uint32_t *tileQueue;              // work counter of the persistent tile kernel
-	uint32_t *tileList;               // the tiles that have list entries (written at the end of phase C), or null: every tile
+	uint4 *tileList;                  // the tiles that have list entries (written at the end of phase C) as tile, first
+	                                  // entry, entries and frame, or null: every tile
 	uint32_t *tileListCount;          // their number
 	uint32_t recordShift;             // 3: records numbered 8 * fan triangle + piece, 0: as they are stored (record_slot)
 	const uint32_t *extraBase;        // per fan triangle: where the further pieces of a clipped triangle begin
@@ -144,9 +145,10 @@ struct TileBins {
 	// per tile: a key (upper word) that every pixel of the tile reaches, from the big records covering it
 	// completely; large records below it are not listed.  null: nothing is culled while binning
 	uint32_t *thresholds;
-	// tiles weighing more than PART_WEIGHT as (tile, part) items, and per tile the parts done; null: every
+	// tiles weighing more than partWeight as (tile, part) items, and per tile the parts done; null: every
 	// tile is drawn by one CTA
 	uint2 *parts;
+	uint32_t partWeight;
 	uint32_t *partCount;
 	uint32_t partCapacity;
 	uint32_t *partsDone;
@@ -158,10 +160,11 @@ struct TileBins {
 // a whole warp, small ones 32 at a time: about eight times the time.  Shares of 2,048 to 8,192 take a
 // batch of small frames of many triangles the same time; dense terrain seen from afar (a thousand
 // small entries in a tile of the horizon) should not be cut, which cost 3 to 10 % of its frame.
-static const uint32_t LARGE_WEIGHT = 8, PART_WEIGHT = 4096;
+// Depth-only tiles are drawn by single warps, whose share is smaller.
+static const uint32_t LARGE_WEIGHT = 8, PART_WEIGHT = 4096, DEPTH_PART_WEIGHT = 1024;
 __host__ __device__ inline uint32_t part_weight(uint32_t smalls, uint32_t larges) { return smalls + LARGE_WEIGHT * larges; }
-// At most this many parts for lists of `entries` entries in all: a cut tile weighs more than PART_WEIGHT.
-inline uint32_t max_parts(uint64_t entries) { return (uint32_t)(2 * LARGE_WEIGHT * entries / PART_WEIGHT) + 1u; }
+// At most this many parts for lists of `entries` entries in all: a cut tile weighs more than partWeight.
+inline uint32_t max_parts(uint64_t entries, uint32_t partWeight) { return (uint32_t)(2 * LARGE_WEIGHT * entries / partWeight) + 1u; }
 
 // True when one lane walks the whole record inside a tile (small-triangle path).
 __host__ __device__ inline bool bound_is_small(int32_t left, int32_t top, int32_t right, int32_t bottom, int32_t smallRows,

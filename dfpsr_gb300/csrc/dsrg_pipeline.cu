@@ -234,7 +234,8 @@ static int enqueue_phases(dsrg_context ctx, BatchJob &job, BatchTotals &totals, 
 	TRY(ctx->binLists.reserve((size_t)binCap + 1));
 	TRY(ctx->bigList.reserve((size_t)recordCap + 1));
 	TRY(ctx->binThresholds.reserve((size_t)totals.tiles + 1));
-	TRY(ctx->tileParts.reserve((size_t)max_parts(binCap) + 1));
+	const uint32_t partWeight = job.depthOnly ? DEPTH_PART_WEIGHT : PART_WEIGHT;
+	TRY(ctx->tileParts.reserve((size_t)max_parts(binCap, partWeight) + 1));
 	TRY(ctx->tilePartsDone.reserve((size_t)totals.tiles + 1));
 	const uint64_t scanned = std::max<uint64_t>(onePass ? 0 : recordCap, 2 * (uint64_t)totals.tiles);
 	TRY(ctx->scanScratch.reserve(scan_scratch_elems((uint32_t)scanned + 1)));
@@ -284,7 +285,8 @@ static int enqueue_phases(dsrg_context ctx, BatchJob &job, BatchTotals &totals, 
 	if (!job.alpha) {
 		bins.parts = ctx->tileParts.ptr;
 		bins.partCount = ctx->control.ptr + CONTROL_TILE_PARTS;
-		bins.partCapacity = max_parts(binCap);
+		bins.partWeight = partWeight;
+		bins.partCapacity = max_parts(binCap, partWeight);
 		bins.partsDone = ctx->tilePartsDone.ptr;
 	}
 	ClearedCounters clear;

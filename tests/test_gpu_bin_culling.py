@@ -63,3 +63,32 @@ def test_depth_only_layers(ctx, w, h):
     ctx.render_depth(m, m.camera, z)
     rz = port.render_depth(s)[0]
     assert np.array_equal(z.view(np.uint32), rz.view(np.uint32))
+
+
+@pytest.mark.parametrize("w,h,stride", [(64, 64, 64), (33, 31, 33), (70, 50, 75), (16, 16, 20), (7, 3, 8)])
+@pytest.mark.parametrize("perspective", [True, False])
+def test_depth_only_images_of_any_shape(ctx, w, h, stride, perspective):
+    """Partial tiles, odd heights, row strides that are no multiple of 16 bytes, prefilled depths
+    with infinities and NaN (never passed), signed zeros; page-locked host memory and device memory."""
+    import torch
+    import dfpsr_gb300 as d
+    from oracle import port
+    s = scenes.random_triangles(seed=w * 31 + h, triangles=500, width=w, height=h)
+    if not perspective:
+        s = dataclasses.replace(s, perspective=False, slope=1.5)
+        s.positions = s.positions.copy()
+        s.positions[::7, 2] = -3.0  # at the camera: linear depth zero
+    rng = np.random.default_rng(w)
+    initial = (rng.uniform(0.2, 0.4, (h, w)) if perspective else rng.uniform(1.0, 4.0, (h, w))).astype(np.float32)
+    initial[0, ::3], initial[h // 2, 1::4], initial[-1, ::5], initial[h // 3, ::2] = np.inf, -np.inf, np.nan, -0.0
+    expected = port.render_depth(s, initial)[0]
+    m = d.Model(ctx, s)
+    host = torch.zeros((h, stride), dtype=torch.float32).pin_memory()
+    host[:, :w] = torch.from_numpy(initial)
+    device = host.cuda()
+    ctx.render_depth(m, m.camera, device[:, :w])
+    ctx.render_depth(m, m.camera, host.numpy()[:, :w])
+    for got in (device.cpu().numpy()[:, :w], host.numpy()[:, :w]):
+        same = (got.view(np.uint32) == expected.view(np.uint32)) | (np.isnan(got) & np.isnan(expected))
+        assert same.all(), np.argwhere(~same)[:5].tolist()
+    assert (host.numpy()[:, w:] == 0).all() and bool((device[:, w:] == 0).all())
