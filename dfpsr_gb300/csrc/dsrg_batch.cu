@@ -132,8 +132,9 @@ void batch_clear_depth(dsrg_batch b) {
 	// a cube map) are cleared as one rectangle
 	char *first = nullptr;
 	int32_t strideBytes = 0, width = 0, rows = 0;
+	std::vector<FillRect> rects;
 	auto flush = [&]() {
-		if (first) enqueue_fill_words(first, strideBytes / 4, width, rows, 0u, b->context->stream);
+		if (first) rects.push_back(fill_rect(first, strideBytes / 4, width, rows, 0u));
 		first = nullptr;
 	};
 	for (const auto &f : b->frames) {
@@ -141,7 +142,8 @@ void batch_clear_depth(dsrg_batch b) {
 		void *at = f.depth.data;
 		if (!f.depth.onDevice && !host_mapped(f.depth.data, &at)) continue; // excluded by batch_depth_in_place
 		char *p = static_cast<char *>(at);
-		if (first && p == first + (size_t)rows * strideBytes && f.depth.strideBytes == strideBytes && f.width == width) {
+		if (first && p == first + (size_t)rows * strideBytes && f.depth.strideBytes == strideBytes && f.width == width &&
+		    (int64_t)(strideBytes / 4) * (rows + f.height) < (1ll << 31)) {
 			rows += f.height;
 			continue;
 		}
@@ -152,6 +154,7 @@ void batch_clear_depth(dsrg_batch b) {
 		rows = f.height;
 	}
 	flush();
+	enqueue_fill_rects(rects.data(), rects.size(), b->context->stream);
 }
 
 dsrg_context batch_context(dsrg_batch b) { return b->context; }

@@ -325,8 +325,16 @@ int renderer_upload_given(dsrg_renderer r);
 // The device address of page-locked (or registered) host memory, which kernels then read and write
 // in place; false for pageable memory, which is staged through device buffers.
 bool host_mapped(const void *p, void **devicePointer);
-// Queues a fill of a rectangle of 32-bit words (device or mapped memory) with one value.
-void enqueue_fill_words(void *image, int32_t strideWords, int32_t width, int32_t height, uint32_t value, cudaStream_t stream);
+// Queues fills of rectangles of 32-bit words (device or mapped memory), each with one value.
+static const int FILL_RECTS = 32; // rectangles of one launch
+struct FillRect {
+	uint32_t *words;
+	uint32_t stride, width, height; // in words
+	uint32_t value;
+	int32_t vector;                 // set by enqueue_fill_rects
+};
+FillRect fill_rect(void *image, int32_t strideWords, int32_t width, int32_t height, uint32_t value);
+void enqueue_fill_rects(const FillRect *rects, size_t count, cudaStream_t stream);
 // Whether every depth image of a batch is reachable by kernels without staging (device or page-locked memory).
 bool batch_depth_in_place(dsrg_batch b);
 // Queues zeroing of every depth image of a batch (CubeMapF32::clear for a batch of cube faces).

@@ -14,6 +14,7 @@
 // which restart the sweep.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <map>
@@ -368,10 +369,33 @@ __global__ void root_check_kernel(uint32_t firstBits, uint32_t count, unsigned l
 	if (bad) atomicAdd(mismatches, bad);
 }
 
-// A rectangle of 32-bit words set to one value (the frame's clears).
-__global__ void fill_words_kernel(uint32_t *image, int32_t stride, int32_t width, int32_t height, uint32_t value) {
-	const int32_t x = (int32_t)(blockIdx.x * blockDim.x + threadIdx.x), y = (int32_t)blockIdx.y;
-	if (x < width && y < height) image[(size_t)y * stride + x] = value;
+// Rectangles of 32-bit words, each set to one value (a frame's clears), blockIdx.y the rectangle.
+// Bound by the write bandwidth: a thread writes 16 bytes at a time where the rows allow it, four
+// stores in flight, and rows that follow one another in memory are one long row.  The 16 shadow cubes of
+// the 1080p light frame (100 MB) took up to eight launches of a word per thread and 75 to 100 us; they
+// now take 14 us in one (frame 616 -> 571 us).
+struct FillBatch {
+	FillRect rect[FILL_RECTS];
+};
+
+__global__ void __launch_bounds__(256) fill_rects_kernel(FillBatch batch) {
+	const FillRect r = batch.rect[blockIdx.y];
+	const uint32_t stride = gridDim.x * blockDim.x, at = blockIdx.x * blockDim.x + threadIdx.x;
+	if (r.vector) {
+		const uint32_t perRow = r.width / 4u, units = perRow * r.height;
+		const uint4 value = make_uint4(r.value, r.value, r.value, r.value);
+#pragma unroll 4
+		for (uint32_t u = at; u < units; u += stride) {
+			const uint32_t row = r.height == 1u ? 0u : u / perRow;
+			reinterpret_cast<uint4 *>(r.words + (size_t)row * r.stride)[u - row * perRow] = value;
+		}
+		return;
+	}
+	const uint32_t units = r.width * r.height;
+	for (uint32_t u = at; u < units; u += stride) {
+		const uint32_t row = r.height == 1u ? 0u : u / r.width;
+		r.words[(size_t)row * r.stride + (u - row * r.width)] = r.value;
+	}
 }
 
 bool sprite_ok(const dsrg_sprite &s) {
@@ -696,10 +720,10 @@ int sprite_frame_images(dsrg_context ctx, const dsrg_sprite_frame_desc &d, const
 	const dsrg_image &height = img[0], &diffuse = img[1], &normal = img[2], &light = img[3];
 	uint32_t clearHeight;
 	memcpy(&clearHeight, &d.clearHeight, 4);
-	enqueue_fill_words(height.data, height.strideBytes / 4, height.width, height.height, clearHeight, ctx->stream);
-	enqueue_fill_words(diffuse.data, diffuse.strideBytes / 4, diffuse.width, diffuse.height, d.clearDiffuse, ctx->stream);
-	enqueue_fill_words(normal.data, normal.strideBytes / 4, normal.width, normal.height, d.clearNormal, ctx->stream);
-	add_launches(3);
+	const FillRect clears[3] = {fill_rect(height.data, height.strideBytes / 4, height.width, height.height, clearHeight),
+	                            fill_rect(diffuse.data, diffuse.strideBytes / 4, diffuse.width, diffuse.height, d.clearDiffuse),
+	                            fill_rect(normal.data, normal.strideBytes / 4, normal.width, normal.height, d.clearNormal)};
+	enqueue_fill_rects(clears, 3, ctx->stream);
 	DSRG_CUDA_TRY(ctx, cudaGetLastError());
 	const int status = draw_higher_impl(ctx, &height, &diffuse, &normal, sprites, d.spriteCount, false);
 	if (status != DSRG_OK) return status;
@@ -749,12 +773,38 @@ int sprite_frame_steps(dsrg_context ctx, const dsrg_sprite_frame_desc &d, const 
 
 } // namespace
 
-void enqueue_fill_words(void *image, int32_t strideWords, int32_t width, int32_t height, uint32_t value, cudaStream_t stream) {
-	if (width <= 0 || height <= 0) return;
-	for (int32_t first = 0; first < height; first += 65535) { // grid y is limited to 65535 rows per launch
-		const int32_t rows = height - first < 65535 ? height - first : 65535;
-		fill_words_kernel<<<dim3((width + 255) / 256, rows), 256, 0, stream>>>((uint32_t *)image + (size_t)first * strideWords,
-		                                                                      strideWords, width, rows, value);
+FillRect fill_rect(void *image, int32_t strideWords, int32_t width, int32_t height, uint32_t value) {
+	FillRect r;
+	r.words = (uint32_t *)image;
+	r.stride = (uint32_t)strideWords;
+	r.width = (uint32_t)width;
+	r.height = (uint32_t)height;
+	r.value = value;
+	r.vector = 0;
+	return r;
+}
+
+void enqueue_fill_rects(const FillRect *rects, size_t count, cudaStream_t stream) {
+	for (size_t first = 0; first < count; first += FILL_RECTS) {
+		const size_t n = std::min(count - first, (size_t)FILL_RECTS);
+		FillBatch batch;
+		memset(&batch, 0, sizeof(batch));
+		uint64_t largest = 0;
+		for (size_t i = 0; i < n; i++) {
+			FillRect &r = batch.rect[i];
+			r = rects[first + i];
+			// rows without a gap between them are one row (32-bit indices: up to 2^31 words)
+			if (r.stride == r.width && (uint64_t)r.width * r.height < (1ull << 31)) {
+				r.width *= r.height;
+				r.height = 1;
+			}
+			r.vector = ((uintptr_t)r.words & 15u) == 0 && r.width % 4u == 0 && (r.height == 1 || r.stride % 4u == 0);
+			largest = std::max(largest, (uint64_t)r.width * r.height / (r.vector ? 4 : 1));
+		}
+		if (largest == 0) continue;
+		const uint64_t blocks = std::min<uint64_t>((largest + 1023) / 1024, (uint64_t)sm_count() * 8);
+		fill_rects_kernel<<<dim3((unsigned)std::max<uint64_t>(blocks, 1), (unsigned)n), 256, 0, stream>>>(batch);
+		add_launches(1);
 	}
 }
 
