@@ -517,20 +517,23 @@ __device__ __noinline__ void emit_clipped(const BatchParams &b, const FrameBuffe
 // extra slots as numbers 8 * g + 1 .. 8 * g + 6 (record_slot), so that record numbers grow in
 // submission order wherever the records lie, and nothing has to be counted and scanned before they
 // can be written.  The rows, the list of drawn records and the list of big ones are taken from
-// counters, one atomic of each per block of 256 triangles; a record over at most four tiles takes
+// counters, one atomic per warp for the first two together and one for the third where it has any; a record over at most four tiles takes
 // its place in their lists at once (what the atomic on the list's cursor returns).
 // This pass takes the place of a counting pass over the same triangles, two scans (of the
 // triangles' records and of the records' rows) and the atomics of the list-filling pass:
 // a terrain frame of 522,242 triangles went from 304 to 290 us, 64 views of 50,000 triangles (forward,
 // loss and adjoint) from 960 to 938 us, a frame of 400 triangles (64x64) from 114 to 107 us with 7 launches
-// less.  It is bound by the latency of its gathers and atomics, so four blocks per SM with a few
-// spilled registers beat two with none (128 registers: 1,015 us for the 64 views).
-__global__ void __launch_bounds__(256, 4) setup_emit_kernel(BatchParams b, FrameBuffers fb) {
+// less.  It is bound by the latency of its gathers and atomics, so four blocks of 256 per SM with a few
+// spilled registers beat two with none (128 registers: 1,015 us for the 64 views), and warps that take
+// their places on their own beat blocks that met at two barriers for it (64 views 911 -> 874 us, terrain 286
+// -> 281 us).
+static const uint32_t EMIT_THREADS = 128;
+
+__global__ void __launch_bounds__(EMIT_THREADS, 1024 / EMIT_THREADS) setup_emit_kernel(BatchParams b, FrameBuffers fb) {
 	chain_enter();
-	__shared__ uint32_t warpRows[8], warpDrawn[8], warpBig[8], taken[3];
-	const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+	const uint32_t lane = threadIdx.x & 31u;
 	const EmitBuffers &emit = fb.emit;
-	for (uint32_t g0 = blockIdx.x * 256u; g0 < b.totalTriangles; g0 += gridDim.x * 256u) { // uniform per block
+	for (uint32_t g0 = blockIdx.x * EMIT_THREADS; g0 < b.totalTriangles; g0 += gridDim.x * EMIT_THREADS) { // uniform per warp
 		const uint32_t g = g0 + threadIdx.x;
 		Command m;
 		bool drawn = false, big = false;
@@ -555,42 +558,39 @@ __global__ void __launch_bounds__(256, 4) setup_emit_kernel(BatchParams b, Frame
 				big = command_tiles(m, f, tx0, ty0, w) > 4;
 			}
 		}
-		// this block's share of the counters, then each thread's place in it
+		// the warp's share of the counters, then each lane's place in it
 		const uint32_t drawnMask = __ballot_sync(0xFFFFFFFFu, drawn), bigMask = __ballot_sync(0xFFFFFFFFu, big);
+		if (!drawnMask) continue;
 		uint32_t inclusive = rows;
 		for (int o = 1; o < 32; o <<= 1) {
 			const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, inclusive, o);
 			if (lane >= (uint32_t)o) inclusive += v;
 		}
-		if (lane == 31) { warpRows[warp] = inclusive; warpDrawn[warp] = __popc(drawnMask); warpBig[warp] = __popc(bigMask); }
-		__syncthreads();
-		if (threadIdx.x < 3) {
-			const uint32_t *of = threadIdx.x == 0 ? warpRows : (threadIdx.x == 1 ? warpDrawn : warpBig);
-			uint32_t total = 0;
-			for (int i = 0; i < 8; i++) total += of[i];
-			uint32_t *counter = threadIdx.x == 0 ? &emit.counters[EMIT_ROWS] : (threadIdx.x == 1 ? &emit.counters[EMIT_DRAWN] : emit.bigCount);
-			taken[threadIdx.x] = total ? atomicAdd(counter, total) : 0u;
+		unsigned long long taken = 0ull; // rows in the upper word, records in the lower one (EmitCounter)
+		uint32_t bigAt = 0;
+		if (lane == 31) {
+			taken = atomicAdd(reinterpret_cast<unsigned long long *>(emit.counters + EMIT_DRAWN),
+			                  ((unsigned long long)inclusive << 32) | (unsigned long long)__popc(drawnMask));
+			if (bigMask) bigAt = atomicAdd(emit.bigCount, (uint32_t)__popc(bigMask));
 		}
-		__syncthreads();
+		taken = __shfl_sync(0xFFFFFFFFu, taken, 31);
+		bigAt = __shfl_sync(0xFFFFFFFFu, bigAt, 31);
 		if (drawn) {
-			uint32_t rowStart = taken[0] + inclusive - rows, drawnAt = taken[1], bigAt = taken[2];
-			for (uint32_t i = 0; i < warp; i++) { rowStart += warpRows[i]; drawnAt += warpDrawn[i]; bigAt += warpBig[i]; }
 			const uint32_t before = (1u << lane) - 1u;
-			drawnAt += __popc(drawnMask & before);
+			const uint32_t rowStart = (uint32_t)(taken >> 32) + inclusive - rows, drawnAt = (uint32_t)taken + __popc(drawnMask & before);
 			bigAt += __popc(bigMask & before);
 			const TaskParams &task = b.tasks[k];
 			const float one = task.depthOnly ? 0.0f : 1.0f; // depth only: no weights
 			const float subB[3] = {0.0f, one, 0.0f}, subC[3] = {0.0f, 0.0f, one};
 			store_command(b, fb, task, k, b.frames[task.frame], g - task.triangleBase, m, subB, subC, g, rowStart, drawnAt, bigAt);
 		}
-		__syncthreads(); // the shared totals are read before the next round writes them
 	}
 }
 
 void launch_setup_emit(const BatchParams &b, const FrameBuffers &fb, cudaStream_t stream) {
 	if (b.totalTriangles == 0) return;
 	COUNT_LAUNCH();
-	launch_chained(setup_emit_kernel, grid_for(b.totalTriangles, 256), 256, stream, b, fb);
+	launch_chained(setup_emit_kernel, grid_for(b.totalTriangles, EMIT_THREADS), EMIT_THREADS, stream, b, fb);
 }
 
 // One thread per cell of the grid: the cell's run of the top pixel row of its cell row.  The

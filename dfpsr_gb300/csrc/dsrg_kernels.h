@@ -88,7 +88,8 @@ struct ProjectedPoints {
 };
 
 // What setup_emit_kernel writes beside the records.  Counters in device memory, zeroed by the
-// batch's first launch: draw records, row intervals taken, extra slots taken.
+// batch's first launch: draw records, row intervals taken (the two as one 64-bit word, records in the
+// lower half), extra slots taken.
 enum EmitCounter : uint32_t { EMIT_DRAWN = 0, EMIT_ROWS = 1, EMIT_EXTRAS = 2, EMIT_COUNTERS = 3 };
 static const uint32_t ROW_SEGMENT = 16; // rows one thread of rows_segment_kernel computes
 
