@@ -112,7 +112,7 @@ int dsrg_context_destroy(dsrg_context ctx) {
 	if (ctx->branchStream) cudaStreamDestroy(ctx->branchStream);
 	ctx->tileList.release(); ctx->bigList.release(); ctx->binThresholds.release();
 	ctx->tileParts.release(); ctx->tilePartsDone.release();
-	ctx->drawnSlots.release(); ctx->extraBase.release(); ctx->extraIds.release(); ctx->tileHeads.release(); ctx->tileRanks.release();
+	ctx->drawnMarks.release(); ctx->extraBase.release(); ctx->extraIds.release(); ctx->tileHeads.release(); ctx->tileRanks.release();
 	ctx->segmentSlots.release();
 	for (PhaseGraph &g : ctx->graphs) g.reset();
 	cudaEventDestroy(ctx->eventStart);
@@ -576,7 +576,8 @@ static int end_frame(dsrg_renderer r, bool debugWireframe) {
 		if (e != DSRG_OK || !wire || t.records == 0 || !o.fb.records) return e;
 		const size_t lines = ((size_t)wireCount + t.records) * 3;
 		CUDA_TRY(ctx, r->wireLines.reserve(lines + 1, true, (size_t)wireCount * 3, ctx->stream));
-		launch_wire_lines(o.fb.records, o.fb.emit.drawn, t.records, r->wireLines.ptr + (size_t)wireCount * 3, ctx->stream);
+		launch_wire_lines(o.fb.records, o.fb.emit.drawn, o.slots, t.records, ctx->control.ptr + CONTROL_WIRE_LINES,
+		                  r->wireLines.ptr + (size_t)wireCount * 3, ctx->stream);
 		wireCount += t.records;
 		return DSRG_OK;
 	};

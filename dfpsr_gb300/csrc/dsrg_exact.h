@@ -277,6 +277,73 @@ DSRG_HD void edge_step(EdgeStepper &s, int32_t L, int32_t R, int32_t &left, int3
 	}
 }
 
+// The steppers in 32-bit arithmetic, for triangles whose corners lie within NEAR_UNITS sub-pixel units
+// (64 pixels) of the pixel corner (left, top) they are taken relative to, and rows within
+// NEAR_ROWS of it: every product is then below 2^30.  Taking `left` whole pixels off the corners takes
+// exactly `left` off the floor quotient and leaves its remainder, so the quotient of the caller's
+// coordinates, which decides the truncation toward zero, is q + left.
+static const int32_t NEAR_UNITS = 16384, NEAR_ROWS = 16;
+
+DSRG_HD bool near_corners(const int32_t *flat, int32_t left, int32_t top) {
+	for (int i = 0; i < 3; i++) {
+		const int64_t x = (int64_t)flat[2 * i] - 256 * (int64_t)left, y = (int64_t)flat[2 * i + 1] - 256 * (int64_t)top;
+		if (x < -NEAR_UNITS || x > NEAR_UNITS || y < -NEAR_UNITS || y > NEAR_UNITS) return false;
+	}
+	return true;
+}
+
+struct NearEdge {
+	int32_t kind;      // as EdgeStepper
+	int32_t q, r, B;
+	int32_t qd, rd;
+};
+
+DSRG_HD void floor_divide_near(int32_t a, int32_t b, int32_t &q, int32_t &r) {
+	q = (int32_t)floorf(fdiv_estimate((float)a, (float)b)); // within 4 of a / b, and b >= 256
+	r = a - q * b;
+	while (r < 0) { q -= 1; r += b; }
+	while (r >= b) { q += 1; r -= b; }
+}
+
+// The edge from (sx, sy) to (ex, ey), relative to the pixel corner, at row 0.
+DSRG_HD NearEdge near_edge(int32_t sx, int32_t sy, int32_t ex, int32_t ey) {
+	NearEdge e;
+	e.q = e.r = e.B = e.qd = e.rd = 0;
+	const int32_t nx = ey - sy, ny = sx - ex, threshold = (sx > ex || (sx == ex && sy > ey)) ? -1 : 0;
+	if (nx != 0) {
+		int32_t a = threshold - (128 - sx) * nx - (128 - sy) * ny;
+		if (nx < 0) a += 1;
+		e.kind = nx < 0 ? 0 : 1;
+		e.B = 256 * (nx < 0 ? -nx : nx);
+		floor_divide_near(nx < 0 ? -a : a, e.B, e.q, e.r);
+		floor_divide_near(nx < 0 ? 256 * ny : -256 * ny, e.B, e.qd, e.rd);
+	} else if (ny != 0) {
+		e.kind = 2;
+		e.q = (128 - sy) * ny;
+		e.qd = 256 * ny;
+		e.B = threshold;
+	} else {
+		e.kind = 3;
+	}
+	return e;
+}
+
+// edge_step, `offset` being the pixels the corners were moved by; L and R as there.
+DSRG_HD void near_step(NearEdge &e, int32_t offset, int32_t L, int32_t R, int32_t &left, int32_t &right) {
+	if (e.kind <= 1) {
+		const int32_t t = e.q + offset;
+		int32_t v = t + ((t < 0 && e.r != 0) ? 2 : 1); // the quotient truncated toward zero, plus one
+		v = v < L ? L : (v > R ? R : v);
+		if (e.kind == 0) { if (v > left) left = v; } else { if (v < right) right = v; }
+		e.q += e.qd;
+		e.r += e.rd;
+		if (e.r >= e.B) { e.r -= e.B; e.q += 1; }
+	} else if (e.kind == 2) {
+		if (e.q > e.B) { left = R; right = L; }
+		e.q += e.qd;
+	}
+}
+
 // Row intervals of rows [y0, y0 + rows) of a triangle, stepped (equal to row_interval of each row).
 DSRG_HD void row_intervals_stepped(const int32_t *flat, int32_t y0, int32_t rows, int32_t L, int32_t R, int32_t *lefts, int32_t *rights) {
 	const bool degenerate = (flat[0] == flat[2] && flat[1] == flat[3]) || (flat[2] == flat[4] && flat[3] == flat[5]) ||

@@ -26,6 +26,23 @@ void dsrg_host_row_intervals(const int32_t *flat, int32_t y0, int32_t rows, int3
 	for (int32_t r = 0; r < rows; r++) dsrg::row_interval(flat, y0 + r, L, R, lefts[r], rights[r]);
 }
 
+// The same rows in 32-bit arithmetic where the triangle allows it (dsrg::near_edge, near_step), as
+// rows_place_kernel steps them; 0 when it does not.
+int32_t dsrg_host_row_intervals_near(const int32_t *flat, int32_t y0, int32_t rows, int32_t L, int32_t R, int32_t *lefts, int32_t *rights) {
+	if (rows > dsrg::NEAR_ROWS || !dsrg::near_corners(flat, L, y0)) return 0;
+	int32_t p[6];
+	for (int i = 0; i < 3; i++) { p[2 * i] = flat[2 * i] - 256 * L; p[2 * i + 1] = flat[2 * i + 1] - 256 * y0; }
+	const bool degenerate = (p[0] == p[2] && p[1] == p[3]) || (p[2] == p[4] && p[3] == p[5]) || (p[4] == p[0] && p[5] == p[1]);
+	dsrg::NearEdge e[3] = {dsrg::near_edge(p[0], p[1], p[2], p[3]), dsrg::near_edge(p[2], p[3], p[4], p[5]), dsrg::near_edge(p[4], p[5], p[0], p[1])};
+	for (int32_t k = 0; k < rows; k++) {
+		lefts[k] = degenerate ? R : L;
+		rights[k] = degenerate ? L : R;
+		if (!degenerate)
+			for (int i = 0; i < 3; i++) dsrg::near_step(e[i], L, L, R, lefts[k], rights[k]);
+	}
+	return 1;
+}
+
 // The same rows by exact stepping (dsrg::row_intervals_stepped).
 void dsrg_host_row_intervals_stepped(const int32_t *flat, int32_t y0, int32_t rows, int32_t L, int32_t R, int32_t *lefts,
                                      int32_t *rights) {

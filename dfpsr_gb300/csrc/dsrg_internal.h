@@ -173,7 +173,7 @@ struct PhaseGraph {
 };
 
 // Words of a context's control buffer, all zeroed by a batch's first launch.
-enum ControlWord : uint32_t { CONTROL_TILE_QUEUE = 0, CONTROL_ERROR = 1, CONTROL_EMIT = 2, CONTROL_BIG_RECORDS = 5, CONTROL_LISTED_TILES = 6, CONTROL_TILE_PARTS = 7, CONTROL_WORDS = 8 };
+enum ControlWord : uint32_t { CONTROL_TILE_QUEUE = 0, CONTROL_ERROR = 1, CONTROL_EMIT = 2, CONTROL_BIG_RECORDS = 5, CONTROL_LISTED_TILES = 6, CONTROL_TILE_PARTS = 7, CONTROL_WIRE_LINES = 8, CONTROL_WORDS = 9 };
 static_assert(CONTROL_BIG_RECORDS == CONTROL_EMIT + EMIT_COUNTERS, "control words");
 
 struct BatchTotals {
@@ -221,11 +221,12 @@ struct dsrg_context_s {
 	DeviceBuffer<uint32_t> binCounts, binOffsets, binCursors, binLists;
 	DeviceBuffer<uint32_t> bigList;      // records over more than four tiles
 	DeviceBuffer<uint32_t> binThresholds; // per tile: the key that large records must reach to be listed
-	DeviceBuffer<uint32_t> drawnSlots, extraBase, extraIds, segmentSlots; // the one-pass setup (EmitBuffers)
+	DeviceBuffer<uint16_t> drawnMarks;
+	DeviceBuffer<uint32_t> extraBase, extraIds, segmentSlots; // the one-pass setup (EmitBuffers)
 	DeviceBuffer<uint2> tileParts;       // tiles of long lists, drawn in parts
 	DeviceBuffer<uint32_t> tilePartsDone;
-	DeviceBuffer<uint2> tileHeads;
-	DeviceBuffer<uint4> tileRanks;
+	DeviceBuffer<uint4> tileHeads;
+	DeviceBuffer<uint2> tileRanks;
 	DeviceBuffer<TextureData> textureTable;
 	DeviceBuffer<uint32_t> stagingColor;
 	DeviceBuffer<uint32_t> textureStaging;      // texture creation: host images and two-step resize halves
@@ -383,6 +384,7 @@ size_t layout_tables(TaskParams *tasks, size_t taskCount, FrameTarget *frames, s
 struct BatchOutputs {
 	BatchParams params;
 	FrameBuffers fb;
+	uint32_t slots; // of records (EmitBuffers::drawn tells which hold one)
 };
 
 // Runs the phases of the batch on the context's stream (growing its scratch as needed) and

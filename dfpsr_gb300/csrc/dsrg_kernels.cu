@@ -406,12 +406,6 @@ __device__ __forceinline__ bool make_command(const FrameTarget &f, const Corner 
 	return true;
 }
 
-// Rows the command takes: its bound's, in whole segments where segments are listed.
-__device__ __forceinline__ uint32_t command_rows(const Command &m, const EmitBuffers &emit) {
-	const uint32_t rows = (uint32_t)(m.bottom - m.top);
-	return emit.segmentSlots ? (rows + ROW_SEGMENT - 1) / ROW_SEGMENT * ROW_SEGMENT : rows;
-}
-
 __device__ __forceinline__ int32_t command_tiles(const Command &m, const FrameTarget &f, int32_t &tx0, int32_t &ty0, int32_t &w) {
 	tx0 = m.left >> 4;
 	ty0 = m.top >> 4;
@@ -420,19 +414,25 @@ __device__ __forceinline__ int32_t command_tiles(const Command &m, const FrameTa
 	return (w > 0 && h > 0) ? w * h : 0;
 }
 
-// Writes a command's record and what the launches behind it need.  subB, subC: its corners' places
-// in the fan triangle.
+// Writes a command's record and what the launches behind it need (its rows are placed by
+// rows_place_kernel).  subB, subC: its corners' places in the fan triangle.
 __device__ __forceinline__ void store_command(const BatchParams &b, const FrameBuffers &fb, const TaskParams &task, uint32_t taskIndex,
                                               const FrameTarget &f, uint32_t tri, const Command &m, const float *subB, const float *subC,
-                                              uint32_t slot, uint32_t rowStart, uint32_t drawnAt, uint32_t bigAt) {
+                                              uint32_t slot) {
 	const EmitBuffers &emit = fb.emit;
 	int32_t tx0, ty0, w;
 	const int32_t tiles = command_tiles(m, f, tx0, ty0, w);
-	emit.drawn[drawnAt] = slot;
 	if (tiles > 4) {
-		emit.tileHeads[drawnAt] = make_uint2(0u, 0u);
-		emit.bigList[bigAt] = slot;
+		emit.drawn[slot] = drawn_mark(DRAWN_BIG, m.bottom - m.top);
+		// one atomic for the lanes that are here together
+		const unsigned together = __activemask();
+		const uint32_t lane = threadIdx.x & 31u, leader = __ffs(together) - 1;
+		uint32_t at = 0;
+		if (lane == leader) at = atomicAdd(emit.bigCount, (uint32_t)__popc(together));
+		at = __shfl_sync(together, at, leader);
+		emit.bigList[at + __popc(together & ((1u << lane) - 1u))] = slot;
 	} else {
+		emit.drawn[slot] = drawn_mark((uint32_t)tiles + 1u, m.bottom - m.top);
 		// a place in each tile's list: the atomics' answers arrive while the record is made
 		const uint32_t large = (b.depthOnly || !bound_is_small(m.left, m.top, m.right, m.bottom, b.smallRows, b.smallWidth)) ? 1u : 0u;
 		const uint32_t first = 2u * (f.tileBase + (uint32_t)(ty0 * f.tilesX + tx0)) + large;
@@ -443,19 +443,14 @@ __device__ __forceinline__ void store_command(const BatchParams &b, const FrameB
 			const int32_t row = w == 1 ? i : (w == 2 ? i >> 1 : (i >= w ? 1 : 0));
 			if (i < tiles) rank[i] = atomicAdd(&emit.tileCursors[first + 2u * (uint32_t)(row * f.tilesX + i - row * w)], 1u);
 		}
-		emit.tileHeads[drawnAt] = make_uint2(first, (uint32_t)f.tilesX | ((uint32_t)w << 16) | ((uint32_t)tiles << 24));
-		emit.tileRanks[drawnAt] = make_uint4(rank[0], rank[1], rank[2], rank[3]);
+		emit.tileHeads[slot] = make_uint4(first, (uint32_t)f.tilesX | ((uint32_t)w << 16), rank[0], rank[1]);
+		if (tiles > 2) emit.tileRanks[slot] = make_uint2(rank[2], rank[3]);
 	}
-	const uint32_t rows = command_rows(m, emit);
-	if (rowStart + rows > fb.rowCapacity) atomicOr(fb.errorFlag, ERROR_ROW_OVERFLOW);
-	if (emit.segmentSlots)
-		for (uint32_t s = rowStart / ROW_SEGMENT; s < (rowStart + rows) / ROW_SEGMENT && s < fb.rowCapacity / ROW_SEGMENT; s++)
-			emit.segmentSlots[s] = slot;
 	DrawRecord r;
 	for (int i = 0; i < 6; i++) r.flat[i] = m.flat[i];
 	r.left = m.left; r.top = m.top; r.right = m.right; r.bottom = m.bottom;
 	triangle_projection(m.isx, m.isy, m.csz, subB, subC, task.camera.perspective != 0, r.start, r.dx, r.dy);
-	r.rowStart = rowStart;
+	r.rowStart = 0;
 	r.tri = tri;
 	r.task = taskIndex;
 	r.frame = (uint32_t)task.frame;
@@ -464,9 +459,9 @@ __device__ __forceinline__ void store_command(const BatchParams &b, const FrameB
 }
 
 // A fan triangle that crosses a clipping plane: every piece is stored on its own, the first at the
-// triangle's slot (renderTriangleFromData, renderCore.cpp:220-341).  Out of line: few triangles come
+// triangle's slot (renderTriangleFromData, renderCore.cpp:220-341).  Returns whether there was one.  Out of line: few triangles come
 // here, and the polygon would cost the others their registers.
-__device__ __noinline__ void emit_clipped(const BatchParams &b, const FrameBuffers &fb, uint32_t g, uint32_t k, const Corner *corners) {
+__device__ __noinline__ bool emit_clipped(const BatchParams &b, const FrameBuffers &fb, uint32_t g, uint32_t k, const Corner *corners) {
 	const TaskParams &task = b.tasks[k];
 	const FrameTarget &f = b.frames[task.frame];
 	const EmitBuffers &emit = fb.emit;
@@ -479,6 +474,7 @@ __device__ __noinline__ void emit_clipped(const BatchParams &b, const FrameBuffe
 	poly.v[2].subB = 0.0f; poly.v[2].subC = 1.0f;
 	for (int s = 0; s < task.camera.clipCount; s++) poly.clip(task.camera.clip[s]);
 	uint32_t pieces = 0, base = 0;
+	bool first = false;
 	for (int n = 0; n < poly.count - 2; n++) {
 		const SubVertex *sv[3] = {&poly.v[0], &poly.v[1 + n], &poly.v[2 + n]};
 		Corner c[3];
@@ -493,8 +489,11 @@ __device__ __noinline__ void emit_clipped(const BatchParams &b, const FrameBuffe
 		if (!make_command(f, c, fb.errorFlag, m)) continue;
 		uint64_t slot = g;
 		if (pieces == 1) { // extra slots for this piece and all that can follow it
-			base = atomicAdd(&emit.counters[EMIT_EXTRAS], (uint32_t)(poly.count - 2 - n));
+			const uint32_t taken = (uint32_t)(poly.count - 2 - n);
+			base = atomicAdd(&emit.counters[EMIT_EXTRAS], taken);
 			emit.extraBase[g] = base;
+			for (uint32_t i = 0; i < taken; i++)
+				if ((uint64_t)b.totalTriangles + base + i < emit.capacity) emit.drawn[b.totalTriangles + base + i] = 0;
 		}
 		if (pieces > 0) {
 			slot = (uint64_t)b.totalTriangles + base + (pieces - 1);
@@ -505,85 +504,51 @@ __device__ __noinline__ void emit_clipped(const BatchParams &b, const FrameBuffe
 			atomicOr(fb.errorFlag, ERROR_RECORD_OVERFLOW);
 			continue;
 		}
-		int32_t tx0, ty0, w;
-		const bool big = command_tiles(m, f, tx0, ty0, w) > 4;
-		store_command(b, fb, task, k, f, t, m, subB, subC, (uint32_t)slot, atomicAdd(&emit.counters[EMIT_ROWS], command_rows(m, emit)),
-		              atomicAdd(&emit.counters[EMIT_DRAWN], 1u), big ? atomicAdd(emit.bigCount, 1u) : 0u);
+		if (pieces == 1) first = true;
+		store_command(b, fb, task, k, f, t, m, subB, subC, (uint32_t)slot);
 	}
+	return first;
 }
 
 // One thread per fan triangle (renderTriangleFromData, renderCore.cpp:220-341, 400-443).  The record
 // of triangle g goes to slot g and is numbered 8 * g; further pieces of a clipped triangle go to
 // extra slots as numbers 8 * g + 1 .. 8 * g + 6 (record_slot), so that record numbers grow in
 // submission order wherever the records lie, and nothing has to be counted and scanned before they
-// can be written.  The rows, the list of drawn records and the list of big ones are taken from
-// counters, one atomic per warp for the first two together and one for the third where it has any; a record over at most four tiles takes
-// its place in their lists at once (what the atomic on the list's cursor returns).
+// can be written.  `drawn` tells per slot whether there is a record, over how many tiles and rows; a record
+// over at most four tiles takes its place in their lists at once (what the atomic on the list's cursor
+// returns).  The rows are placed by the launch behind it (rows_place_kernel).
 // This pass takes the place of a counting pass over the same triangles, two scans (of the
 // triangles' records and of the records' rows) and the atomics of the list-filling pass:
 // a terrain frame of 522,242 triangles went from 304 to 290 us, 64 views of 50,000 triangles (forward,
 // loss and adjoint) from 960 to 938 us, a frame of 400 triangles (64x64) from 114 to 107 us with 7 launches
-// less.  It is bound by the latency of its gathers and atomics, so four blocks of 256 per SM with a few
-// spilled registers beat two with none (128 registers: 1,015 us for the 64 views), and warps that take
-// their places on their own beat blocks that met at two barriers for it (64 views 911 -> 874 us, terrain 286
-// -> 281 us).
-static const uint32_t EMIT_THREADS = 128;
+// less.  It is bound by the latency of its gathers, so four blocks of 256 per SM with a few spilled
+// registers beat half as many with none.  Counters that every warp adds to are kept out of it: an
+// atomic on one address takes 1.6 to 1.9 ns, and with one per warp of 32 triangles (for a list of the
+// drawn records and their rows) it took
+// exactly that time per warp. Without them: terrain 48 -> 33 us of the setup, the 64 views 162 -> 120 us.
+static const uint32_t EMIT_THREADS = 256;
 
 __global__ void __launch_bounds__(EMIT_THREADS, 1024 / EMIT_THREADS) setup_emit_kernel(BatchParams b, FrameBuffers fb) {
 	chain_enter();
-	const uint32_t lane = threadIdx.x & 31u;
-	const EmitBuffers &emit = fb.emit;
-	for (uint32_t g0 = blockIdx.x * EMIT_THREADS; g0 < b.totalTriangles; g0 += gridDim.x * EMIT_THREADS) { // uniform per warp
-		const uint32_t g = g0 + threadIdx.x;
-		Command m;
-		bool drawn = false, big = false;
-		uint32_t k = 0, rows = 0;
-		if (g < b.totalTriangles) {
-			k = (uint32_t)find_segment(b.taskTriangleBase, b.taskCount, g);
-			const TaskParams &task = b.tasks[k];
-			const FrameTarget &f = b.frames[task.frame];
-			Corner c[3];
-			bool whole;
-			if (load_triangle(task, g - task.triangleBase, fb.points, c, &whole) && (f.color != nullptr || f.depth != nullptr)) {
-				if (whole) {
-					drawn = make_command(f, c, fb.errorFlag, m);
-				} else {
-					Corner copy[3] = {c[0], c[1], c[2]};
-					emit_clipped(b, fb, g, k, copy);
-				}
-			}
-			if (drawn) {
-				int32_t tx0, ty0, w;
-				rows = command_rows(m, emit);
-				big = command_tiles(m, f, tx0, ty0, w) > 4;
+	for (uint32_t g = blockIdx.x * EMIT_THREADS + threadIdx.x; g < b.totalTriangles; g += gridDim.x * EMIT_THREADS) {
+		const uint32_t k = (uint32_t)find_segment(b.taskTriangleBase, b.taskCount, g);
+		const TaskParams &task = b.tasks[k];
+		const FrameTarget &f = b.frames[task.frame];
+		Corner c[3];
+		bool whole, drawn = false;
+		if (load_triangle(task, g - task.triangleBase, fb.points, c, &whole) && (f.color != nullptr || f.depth != nullptr)) {
+			Command m;
+			if (!whole) {
+				Corner copy[3] = {c[0], c[1], c[2]};
+				drawn = emit_clipped(b, fb, g, k, copy);
+			} else if (make_command(f, c, fb.errorFlag, m)) {
+				drawn = true;
+				const float one = task.depthOnly ? 0.0f : 1.0f; // depth only: no weights
+				const float subB[3] = {0.0f, one, 0.0f}, subC[3] = {0.0f, 0.0f, one};
+				store_command(b, fb, task, k, f, g - task.triangleBase, m, subB, subC, g);
 			}
 		}
-		// the warp's share of the counters, then each lane's place in it
-		const uint32_t drawnMask = __ballot_sync(0xFFFFFFFFu, drawn), bigMask = __ballot_sync(0xFFFFFFFFu, big);
-		if (!drawnMask) continue;
-		uint32_t inclusive = rows;
-		for (int o = 1; o < 32; o <<= 1) {
-			const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, inclusive, o);
-			if (lane >= (uint32_t)o) inclusive += v;
-		}
-		unsigned long long taken = 0ull; // rows in the upper word, records in the lower one (EmitCounter)
-		uint32_t bigAt = 0;
-		if (lane == 31) {
-			taken = atomicAdd(reinterpret_cast<unsigned long long *>(emit.counters + EMIT_DRAWN),
-			                  ((unsigned long long)inclusive << 32) | (unsigned long long)__popc(drawnMask));
-			if (bigMask) bigAt = atomicAdd(emit.bigCount, (uint32_t)__popc(bigMask));
-		}
-		taken = __shfl_sync(0xFFFFFFFFu, taken, 31);
-		bigAt = __shfl_sync(0xFFFFFFFFu, bigAt, 31);
-		if (drawn) {
-			const uint32_t before = (1u << lane) - 1u;
-			const uint32_t rowStart = (uint32_t)(taken >> 32) + inclusive - rows, drawnAt = (uint32_t)taken + __popc(drawnMask & before);
-			bigAt += __popc(bigMask & before);
-			const TaskParams &task = b.tasks[k];
-			const float one = task.depthOnly ? 0.0f : 1.0f; // depth only: no weights
-			const float subB[3] = {0.0f, one, 0.0f}, subC[3] = {0.0f, 0.0f, one};
-			store_command(b, fb, task, k, b.frames[task.frame], g - task.triangleBase, m, subB, subC, g, rowStart, drawnAt, bigAt);
-		}
+		if (!drawn) fb.emit.drawn[g] = 0;
 	}
 }
 
@@ -857,95 +822,219 @@ void launch_row_offsets(const FrameBuffers &fb, uint32_t recordCount, uint32_t *
 static const int32_t ROWS_STEPPED_MAX = 16; // records of at most this many rows are stepped by one lane each
 static_assert(ROWS_STEPPED_MAX == ROW_SEGMENT, "a segment is what one lane steps");
 
-// The row intervals of every record, stepped exactly (row_intervals_stepped: two floor divisions
-// per edge start a segment of rows, then one carry step per edge and row).  Each warp takes 32
-// records.  When all of them have at most ROWS_STEPPED_MAX rows (dense meshes) each lane steps its
+// The row intervals of a warp's 32 records (count 0: none in the lane), stepped exactly
+// (row_intervals_stepped: two floor divisions per edge start a segment of rows, then one carry step
+// per edge and row).  a, b and c hold the record's corners and bound, out its first row.  When all of them have at most ROWS_STEPPED_MAX rows (dense meshes) each lane steps its
 // own record; otherwise the records are cut into segments of up to ROWS_STEPPED_MAX rows that are
 // spread over the lanes (a lane finds its record by a search over the warp's prefix sums of
 // segment counts and fetches its corners with shuffles), so tall triangles keep every lane busy.
-// `drawn` lists the records (null: all of the first recordCount).  With rowOffsets (the two-pass
-// setup) the rows lie where that scan put them and rowStart is written; otherwise rowStart holds
-// where setup_emit_kernel put them.
-__global__ void __launch_bounds__(256, 3) rows_group_kernel(DrawRecord *records, uint32_t capacity, const uint32_t *countDevice,
-                                                   const uint32_t *__restrict__ drawn, const uint32_t *__restrict__ rowOffsets,
-                                                   uint32_t *rows, uint32_t rowCapacity, int32_t *errorFlag) {
-	chain_enter();
-	const uint32_t recordCount = device_count(capacity, countDevice);
+__device__ __noinline__ void step_rows(int4 a, int4 b, int2 c, int32_t count, uint32_t out, uint32_t *rows,
+                                          uint32_t rowCapacity, int32_t *errorFlag) {
 	const int lane = threadIdx.x & 31;
-	const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-	for (uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w * 32u < recordCount; w += warps) {
-		uint32_t i = w * 32u + (uint32_t)lane;
-		int32_t count = 0, top = 0, L = 0, R = 0;
-		int32_t f0 = 0, f1 = 0, f2 = 0, f3 = 0, f4 = 0, f5 = 0;
-		uint32_t out = 0;
-		if (i < recordCount) {
-			if (drawn) i = drawn[i];
-			const int4 a = *reinterpret_cast<const int4 *>(&records[i].flat[0]);   // flat[0..3]
-			const int4 b = *reinterpret_cast<const int4 *>(&records[i].flat[4]);   // flat[4..5], left, top
-			const int2 c = *reinterpret_cast<const int2 *>(&records[i].right);     // right, bottom
-			f0 = a.x; f1 = a.y; f2 = a.z; f3 = a.w; f4 = b.x; f5 = b.y;
-			L = b.z; top = b.w; R = c.x;
-			count = c.y - top;
-			if (rowOffsets) records[i].rowStart = rowOffsets[i];
-			out = rowOffsets ? rowOffsets[i] : records[i].rowStart;
+	const int32_t f0 = a.x, f1 = a.y, f2 = a.z, f3 = a.w, f4 = b.x, f5 = b.y, L = b.z, top = b.w, R = c.x;
+	const bool short_ = __all_sync(0xFFFFFFFFu, count <= ROWS_STEPPED_MAX);
+	const int32_t segments = short_ ? 1 : (count + ROWS_STEPPED_MAX - 1) / ROWS_STEPPED_MAX;
+	int32_t inclusive = segments, total = 32;
+	if (!short_) {
+		for (int o = 1; o < 32; o <<= 1) {
+			const int32_t v = __shfl_up_sync(0xFFFFFFFFu, inclusive, o);
+			if (lane >= o) inclusive += v;
 		}
-		const bool short_ = __all_sync(0xFFFFFFFFu, count <= ROWS_STEPPED_MAX);
-		const int32_t segments = short_ ? 1 : (count + ROWS_STEPPED_MAX - 1) / ROWS_STEPPED_MAX;
-		int32_t inclusive = segments, total = 32;
+		total = __shfl_sync(0xFFFFFFFFu, inclusive, 31);
+	}
+	for (int32_t base = 0; base < total; base += 32) {
+		// this lane's segment: the rows [first, first + rowsHere) of the record held by lane k
+		int32_t x0 = f0, y0 = f1, x1 = f2, y1 = f3, x2 = f4, y2 = f5, kTop = top, kL = L, kR = R, kCount = count;
+		uint32_t kOut = out;
+		int32_t first = 0;
+		const int32_t j = base + lane;
 		if (!short_) {
-			for (int o = 1; o < 32; o <<= 1) {
-				const int32_t v = __shfl_up_sync(0xFFFFFFFFu, inclusive, o);
-				if (lane >= o) inclusive += v;
-			}
-			total = __shfl_sync(0xFFFFFFFFu, inclusive, 31);
+			int k = 0; // first lane whose inclusive sum exceeds j
+			for (int step = 16; step >= 1; step >>= 1)
+				if (__shfl_sync(0xFFFFFFFFu, inclusive, k + step - 1) <= j) k += step;
+			const int32_t start = __shfl_sync(0xFFFFFFFFu, inclusive, k) - __shfl_sync(0xFFFFFFFFu, segments, k);
+			x0 = __shfl_sync(0xFFFFFFFFu, f0, k); y0 = __shfl_sync(0xFFFFFFFFu, f1, k);
+			x1 = __shfl_sync(0xFFFFFFFFu, f2, k); y1 = __shfl_sync(0xFFFFFFFFu, f3, k);
+			x2 = __shfl_sync(0xFFFFFFFFu, f4, k); y2 = __shfl_sync(0xFFFFFFFFu, f5, k);
+			kTop = __shfl_sync(0xFFFFFFFFu, top, k); kL = __shfl_sync(0xFFFFFFFFu, L, k);
+			kR = __shfl_sync(0xFFFFFFFFu, R, k); kCount = __shfl_sync(0xFFFFFFFFu, count, k);
+			kOut = __shfl_sync(0xFFFFFFFFu, out, k);
+			first = (j - start) * ROWS_STEPPED_MAX;
 		}
-		for (int32_t base = 0; base < total; base += 32) {
-			// this lane's segment: the rows [first, first + rowsHere) of the record held by lane k
-			int32_t x0 = f0, y0 = f1, x1 = f2, y1 = f3, x2 = f4, y2 = f5, kTop = top, kL = L, kR = R, kCount = count;
-			uint32_t kOut = out;
-			int32_t first = 0;
-			const int32_t j = base + lane;
-			if (!short_) {
-				int k = 0; // first lane whose inclusive sum exceeds j
-				for (int step = 16; step >= 1; step >>= 1)
-					if (__shfl_sync(0xFFFFFFFFu, inclusive, k + step - 1) <= j) k += step;
-				const int32_t start = __shfl_sync(0xFFFFFFFFu, inclusive, k) - __shfl_sync(0xFFFFFFFFu, segments, k);
-				x0 = __shfl_sync(0xFFFFFFFFu, f0, k); y0 = __shfl_sync(0xFFFFFFFFu, f1, k);
-				x1 = __shfl_sync(0xFFFFFFFFu, f2, k); y1 = __shfl_sync(0xFFFFFFFFu, f3, k);
-				x2 = __shfl_sync(0xFFFFFFFFu, f4, k); y2 = __shfl_sync(0xFFFFFFFFu, f5, k);
-				kTop = __shfl_sync(0xFFFFFFFFu, top, k); kL = __shfl_sync(0xFFFFFFFFu, L, k);
-				kR = __shfl_sync(0xFFFFFFFFu, R, k); kCount = __shfl_sync(0xFFFFFFFFu, count, k);
-				kOut = __shfl_sync(0xFFFFFFFFu, out, k);
-				first = (j - start) * ROWS_STEPPED_MAX;
-			}
-			if (j >= total) continue;
-			const int32_t rowsHere = min(ROWS_STEPPED_MAX, kCount - first);
-			if (rowsHere <= 0) continue;
-			const bool degenerate = (x0 == x1 && y0 == y1) || (x1 == x2 && y1 == y2) || (x2 == x0 && y2 == y0);
-			EdgeStepper st[3];
+		if (j >= total) continue;
+		const int32_t rowsHere = min(ROWS_STEPPED_MAX, kCount - first);
+		if (rowsHere <= 0) continue;
+		const bool degenerate = (x0 == x1 && y0 == y1) || (x1 == x2 && y1 == y2) || (x2 == x0 && y2 == y0);
+		EdgeStepper st[3];
+		if (!degenerate) {
+			st[0] = edge_stepper(make_edge(x0, y0, x1, y1), kTop + first);
+			st[1] = edge_stepper(make_edge(x1, y1, x2, y2), kTop + first);
+			st[2] = edge_stepper(make_edge(x2, y2, x0, y0), kTop + first);
+		}
+		for (int32_t r = 0; r < rowsHere; r++) {
+			int32_t left = kR, right = kL;
 			if (!degenerate) {
-				st[0] = edge_stepper(make_edge(x0, y0, x1, y1), kTop + first);
-				st[1] = edge_stepper(make_edge(x1, y1, x2, y2), kTop + first);
-				st[2] = edge_stepper(make_edge(x2, y2, x0, y0), kTop + first);
+				left = kL; right = kR;
+				edge_step(st[0], kL, kR, left, right);
+				edge_step(st[1], kL, kR, left, right);
+				edge_step(st[2], kL, kR, left, right);
 			}
-			for (int32_t r = 0; r < rowsHere; r++) {
-				int32_t left = kR, right = kL;
-				if (!degenerate) {
-					left = kL; right = kR;
-					edge_step(st[0], kL, kR, left, right);
-					edge_step(st[1], kL, kR, left, right);
-					edge_step(st[2], kL, kR, left, right);
-				}
-				const uint32_t at = kOut + (uint32_t)(first + r);
-				if (at < rowCapacity) rows[at] = (uint32_t)(left & 0xFFFF) | ((uint32_t)right << 16);
-				else atomicOr(errorFlag, ERROR_ROW_OVERFLOW);
-			}
+			const uint32_t at = kOut + (uint32_t)(first + r);
+			if (at < rowCapacity) rows[at] = (uint32_t)(left & 0xFFFF) | ((uint32_t)right << 16);
+			else atomicOr(errorFlag, ERROR_ROW_OVERFLOW);
 		}
 	}
 }
 
+// The two-pass setup's rows: one lane per record, placed by the scan of their row counts.
+__global__ void __launch_bounds__(256, 3) rows_group_kernel(DrawRecord *records, uint32_t capacity, const uint32_t *countDevice,
+                                                            const uint32_t *__restrict__ rowOffsets, uint32_t *rows, uint32_t rowCapacity,
+                                                            int32_t *errorFlag) {
+	chain_enter();
+	const uint32_t recordCount = device_count(capacity, countDevice);
+	const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+	for (uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w * 32u < recordCount; w += warps) {
+		const uint32_t i = w * 32u + (threadIdx.x & 31u);
+		int4 a = make_int4(0, 0, 0, 0), b = a;
+		int2 c = make_int2(0, 0);
+		uint32_t out = 0;
+		if (i < recordCount) {
+			a = *reinterpret_cast<const int4 *>(&records[i].flat[0]); // flat[0..3]
+			b = *reinterpret_cast<const int4 *>(&records[i].flat[4]); // flat[4..5], left, top
+			c = *reinterpret_cast<const int2 *>(&records[i].right);   // right, bottom
+			out = rowOffsets[i];
+			records[i].rowStart = out;
+		}
+		step_rows(a, b, c, c.y - b.w, out, rows, rowCapacity, errorFlag);
+	}
+}
+
+// The one-pass setup's rows.  A block takes PLACE_SLOTS slots at a time, makes a dense list of the
+// records among them in shared memory (in a closed mesh half the triangles face away), adds their
+// rows up, takes that many with one atomic and writes each record's first one.  With `segments`
+// (tall triangles) it lists the segments of ROW_SEGMENT rows for rows_segment_kernel; otherwise it
+// computes the rows itself, a warp stepping 32 of the listed records: in 32-bit arithmetic where all are
+// small (a 64-bit product or remainder costs several times as much, and there are three edges), with
+// step_rows otherwise.  With both, placing and computing the rows of the 1.4 M records of
+// 64 views takes 56 to 68 us (computing them alone in 64 bits took 72), and a step of the 64 views went
+// from 874 to 845 us, a terrain frame from 281 to 266 us, 4k from 908 to 872 us.
+static const uint32_t PLACE_BLOCKS = 4; // per SM
+static const uint32_t PLACE_THREADS = 256, PLACE_SLOTS = 4 * PLACE_THREADS;
+
+// Exclusive prefix sums of two values over the block's threads, and their totals.  `sums` holds a pair
+// of values per warp.
+__device__ __forceinline__ uint2 block_prefix(uint2 v, uint2 *sums, uint2 &total) {
+	const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+	uint2 inclusive = v;
+	for (int o = 1; o < 32; o <<= 1) {
+		const uint32_t x = __shfl_up_sync(0xFFFFFFFFu, inclusive.x, o), y = __shfl_up_sync(0xFFFFFFFFu, inclusive.y, o);
+		if (lane >= (uint32_t)o) { inclusive.x += x; inclusive.y += y; }
+	}
+	if (lane == 31) sums[warp] = inclusive;
+	__syncthreads();
+	uint2 before = make_uint2(0u, 0u);
+	total = before;
+	for (uint32_t w = 0; w < PLACE_THREADS / 32; w++) {
+		const uint2 s = sums[w];
+		if (w < warp) { before.x += s.x; before.y += s.y; }
+		total.x += s.x;
+		total.y += s.y;
+	}
+	return make_uint2(before.x + inclusive.x - v.x, before.y + inclusive.y - v.y);
+}
+
+__global__ void __launch_bounds__(PLACE_THREADS, PLACE_BLOCKS) rows_place_kernel(DrawRecord *records, uint32_t triangles, EmitBuffers emit,
+                                                                                 uint32_t *rows, uint32_t rowCapacity, int32_t *errorFlag) {
+	chain_enter();
+	__shared__ uint32_t slots[PLACE_SLOTS], starts[PLACE_SLOTS], taken;
+	__shared__ uint2 sums[PLACE_THREADS / 32];
+	const uint32_t end = min(triangles + emit.counters[EMIT_EXTRAS], emit.capacity);
+	for (uint32_t base = blockIdx.x * PLACE_SLOTS; base < end; base += gridDim.x * PLACE_SLOTS) { // uniform per block
+		// four slots per thread: their records and rows
+		const uint32_t at = base + 4u * threadIdx.x;
+		const ushort4 marks = at < end ? *reinterpret_cast<const ushort4 *>(emit.drawn + at) : make_ushort4(0, 0, 0, 0); // (padded)
+		const uint32_t mark[4] = {marks.x, marks.y, marks.z, marks.w};
+		uint32_t count[4];
+		uint2 mine = make_uint2(0u, 0u);
+#pragma unroll
+		for (uint32_t i = 0; i < 4; i++) {
+			count[i] = 0;
+			if (at + i >= end || (mark[i] & DRAWN_MASK) == 0u) continue;
+			count[i] = 2u * (mark[i] >> DRAWN_BITS);
+			if (count[i] == 2u * DRAWN_ROWS_MAX) count[i] = (uint32_t)(records[at + i].bottom - records[at + i].top);
+			if (emit.segmentSlots) count[i] = (count[i] + ROW_SEGMENT - 1) / ROW_SEGMENT * ROW_SEGMENT;
+			mine.x++;
+			mine.y += count[i];
+		}
+		uint2 total;
+		const uint2 place = block_prefix(mine, sums, total);
+		const uint32_t n = total.x;
+		if (threadIdx.x == 0) {
+			taken = total.y ? atomicAdd(&emit.counters[EMIT_ROWS], total.y) : 0u;
+			if (n) atomicAdd(&emit.counters[EMIT_DRAWN], n);
+			if (taken + total.y > rowCapacity) atomicOr(errorFlag, ERROR_ROW_OVERFLOW);
+		}
+		__syncthreads();
+		uint32_t e = place.x, start = taken + place.y;
+#pragma unroll
+		for (uint32_t i = 0; i < 4; i++) {
+			if (count[i] == 0u) continue; // (a record has two rows at least)
+			slots[e] = at + i;
+			starts[e] = start;
+			records[at + i].rowStart = start;
+			if (emit.segmentSlots)
+				for (uint32_t s = start / ROW_SEGMENT; s < (start + count[i]) / ROW_SEGMENT && s < rowCapacity / ROW_SEGMENT; s++)
+					emit.segmentSlots[s] = at + i;
+			e++;
+			start += count[i];
+		}
+		__syncthreads();
+		if (emit.segmentSlots) continue;
+		for (uint32_t first = threadIdx.x & ~31u; first < n; first += PLACE_THREADS) { // uniform per warp
+			const uint32_t e = first + (threadIdx.x & 31u);
+			int4 a = make_int4(0, 0, 0, 0), b = a;
+			int2 c = make_int2(0, 0);
+			uint32_t out = 0;
+			if (e < n) {
+				const DrawRecord &r = records[slots[e]];
+				a = *reinterpret_cast<const int4 *>(&r.flat[0]); // flat[0..3]
+				b = *reinterpret_cast<const int4 *>(&r.flat[4]); // flat[4..5], left, top
+				c = *reinterpret_cast<const int2 *>(&r.right);   // right, bottom
+				out = starts[e];
+			}
+			const int32_t count = c.y - b.w;
+			const int32_t flat[6] = {a.x, a.y, a.z, a.w, b.x, b.y};
+			if (!__all_sync(0xFFFFFFFFu, count <= NEAR_ROWS && near_corners(flat, b.z, b.w))) {
+				step_rows(a, b, c, count, out, rows, rowCapacity, errorFlag);
+				continue;
+			}
+			// a warp of small triangles: each lane steps its record in 32-bit arithmetic
+			const int32_t dx = 256 * b.z, dy = 256 * b.w;
+			const bool degenerate = (a.x == a.z && a.y == a.w) || (a.z == b.x && a.w == b.y) || (b.x == a.x && b.y == a.y);
+			NearEdge e0 = near_edge(a.x - dx, a.y - dy, a.z - dx, a.w - dy), e1 = near_edge(a.z - dx, a.w - dy, b.x - dx, b.y - dy);
+			NearEdge e2 = near_edge(b.x - dx, b.y - dy, a.x - dx, a.y - dy);
+			for (int32_t r = 0; r < count; r += 2) { // rows come in pairs
+				uint32_t packed[2];
+#pragma unroll
+				for (int j = 0; j < 2; j++) {
+					int32_t left = degenerate ? c.x : b.z, right = degenerate ? b.z : c.x;
+					if (!degenerate) {
+						near_step(e0, b.z, b.z, c.x, left, right);
+						near_step(e1, b.z, b.z, c.x, left, right);
+						near_step(e2, b.z, b.z, c.x, left, right);
+					}
+					packed[j] = (uint32_t)(left & 0xFFFF) | ((uint32_t)right << 16);
+				}
+				// (past the capacity: the block has set the overflow bit and the frame is redone)
+				if (out + (uint32_t)r + 2u <= rowCapacity) *reinterpret_cast<uint2 *>(rows + out + r) = make_uint2(packed[0], packed[1]);
+			}
+		}
+		__syncthreads(); // the lists are done with
+	}
+}
+
 // The rows of frames of tall triangles: one thread per segment of ROW_SEGMENT rows, whose record
-// setup_emit_kernel wrote down (segmentSlots) as it took the rows.  Two floor divisions per edge
+// rows_place_kernel wrote down (segmentSlots) as it placed the rows.  Two floor divisions per edge
 // start the segment and each row then steps, so the work is spread evenly whatever the records'
 // heights and no thread searches for its record.  A kernel that cut the concatenated rows into
 // chunks of 1,024, searched the records of each chunk with one warp and stepped four rows per thread
@@ -992,12 +1081,17 @@ void launch_rows(const FrameBuffers &fb, uint32_t recordCount, cudaStream_t stre
 	if (recordCount == 0) return;
 	COUNT_LAUNCH();
 	const uint32_t rowCapacity = fb.rowCapacity ? fb.rowCapacity : 0xFFFFFFFFu;
-	if (fb.emit.segmentSlots)
+	if (fb.emit.drawn) {
+		launch_chained(rows_place_kernel, grid_for((uint64_t)fb.emit.capacity / 4u + 1u, PLACE_THREADS), PLACE_THREADS, stream, fb.records,
+		               fb.emit.triangles, fb.emit, fb.rows, rowCapacity, fb.errorFlag);
+		if (!fb.emit.segmentSlots) return;
+		COUNT_LAUNCH();
 		launch_chained(rows_segment_kernel, grid_for(fb.rowCapacity / ROW_SEGMENT, 128), 128, stream, fb.records, fb.emit.segmentSlots,
 		               fb.emit.counters + EMIT_ROWS, rowCapacity, fb.rows);
-	else
-		launch_chained(rows_group_kernel, grid_for((uint64_t)((recordCount + 31) / 32) * 32, 256), 256, stream, fb.records, recordCount,
-		               fb.recordCountDevice, fb.emit.drawn, fb.emit.drawn ? nullptr : fb.rowOffsets, fb.rows, rowCapacity, fb.errorFlag);
+		return;
+	}
+	launch_chained(rows_group_kernel, grid_for((uint64_t)((recordCount + 31) / 32) * 32, 256), 256, stream, fb.records, recordCount,
+	               fb.recordCountDevice, fb.rowOffsets, fb.rows, rowCapacity, fb.errorFlag);
 }
 
 // ------------------------------------------------------------------ binning
@@ -1299,19 +1393,22 @@ __global__ void __launch_bounds__(256) bin_big_kernel(BatchParams b, const DrawR
 __global__ void __launch_bounds__(256) bin_fill_kernel(BatchParams b, const DrawRecord *__restrict__ records, TileBins bins, EmitBuffers emit,
                                                        int32_t *errorFlag) {
 	chain_enter();
-	const uint32_t count = min(emit.counters[EMIT_DRAWN], emit.capacity);
-	for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
-		const uint2 head = emit.tileHeads[i];
-		if (head.y == 0u) continue; // a big record
-		const uint4 rank4 = emit.tileRanks[i];
-		const uint32_t id = record_id(b, emit.extraIds, emit.drawn[i]);
-		const uint32_t tilesX = head.y & 0xFFFFu, w = (head.y >> 16) & 0xFFu, tiles = head.y >> 24;
-		const uint32_t rank[4] = {rank4.x, rank4.y, rank4.z, rank4.w};
+	const uint32_t end = min(b.totalTriangles + emit.counters[EMIT_EXTRAS], emit.capacity);
+	for (uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x; slot < end; slot += gridDim.x * blockDim.x) {
+		const uint32_t mark = emit.drawn[slot] & DRAWN_MASK;
+		if (mark == 0u || mark == DRAWN_BIG) continue;
+		const uint32_t tiles = mark - 1u;
+		const uint4 head = emit.tileHeads[slot];
+		const uint2 more = tiles > 2u ? emit.tileRanks[slot] : make_uint2(0u, 0u);
+		const uint32_t id = record_id(b, emit.extraIds, slot);
+		const uint32_t tilesX = head.y & 0xFFFFu, w = head.y >> 16;
+		const uint32_t rank[4] = {head.z, head.w, more.x, more.y};
 #pragma unroll
 		for (uint32_t k = 0; k < 4; k++) {
 			if (k >= tiles) break;
-			const uint32_t slot = bins.offsets[head.x + 2u * (k / w * tilesX + k % w)] + rank[k];
-			if (slot < bins.listCapacity) bins.lists[slot] = id; else atomicOr(errorFlag, ERROR_BIN_OVERFLOW);
+			const uint32_t row = w == 1u ? k : (w == 2u ? k >> 1 : (k >= w ? 1u : 0u));
+			const uint32_t at = bins.offsets[head.x + 2u * (row * tilesX + k - row * w)] + rank[k];
+			if (at < bins.listCapacity) bins.lists[at] = id; else atomicOr(errorFlag, ERROR_BIN_OVERFLOW);
 		}
 	}
 	bin_big<true>(b, records, bins, emit.extraIds, errorFlag);

@@ -87,20 +87,28 @@ struct ProjectedPoints {
 	longlong2 *flat;  // flat x, flat y
 };
 
-// What setup_emit_kernel writes beside the records.  Counters in device memory, zeroed by the
-// batch's first launch: draw records, row intervals taken (the two as one 64-bit word, records in the
-// lower half), extra slots taken.
+// What the one-pass setup writes beside the records.  Counters in device memory, zeroed by the
+// batch's first launch: draw records, row intervals taken, extra slots taken.
 enum EmitCounter : uint32_t { EMIT_DRAWN = 0, EMIT_ROWS = 1, EMIT_EXTRAS = 2, EMIT_COUNTERS = 3 };
 static const uint32_t ROW_SEGMENT = 16; // rows one thread of rows_segment_kernel computes
+// A slot's mark: 0 no record, else its tiles + 1 (of a record over at most four) or DRAWN_BIG, and half
+// its rows (always even) above, DRAWN_ROWS_MAX standing for that many or more.
+static const uint32_t DRAWN_BITS = 3, DRAWN_MASK = 7, DRAWN_BIG = 6, DRAWN_ROWS_MAX = (1u << (16 - DRAWN_BITS)) - 1u;
+__host__ __device__ inline uint16_t drawn_mark(uint32_t tiles, int32_t rows) {
+	const uint32_t half = (uint32_t)rows / 2u;
+	return (uint16_t)(tiles | ((half < DRAWN_ROWS_MAX ? half : DRAWN_ROWS_MAX) << DRAWN_BITS));
+}
 
 struct EmitBuffers {
 	uint32_t *counters;      // EMIT_COUNTERS values
-	uint32_t *drawn;         // the slots of the records, in no order; null: the two-pass setup
-	uint32_t capacity;       // slots: one per fan triangle, then the extra ones
+	uint16_t *drawn;         // per slot: drawn_mark; null: the two-pass setup
+	uint32_t triangles;      // slots of the fan triangles, which come first,
+	uint32_t capacity;       // and all slots
 	uint32_t *extraBase;     // per fan triangle with further pieces: their first extra slot
 	uint32_t *extraIds;      // per extra slot: its record's number
-	uint2 *tileHeads;        // per drawn record: its first tile-list slot, and tilesX | columns << 16 | tiles << 24 (0: a big record)
-	uint4 *tileRanks;        // per drawn record over at most four tiles: its place in each tile's list
+	uint4 *tileHeads;        // per slot of a record over at most four tiles: its first tile-list slot, tilesX | columns << 16,
+	                         // and its places in the first two tiles' lists
+	uint2 *tileRanks;        // over more than two tiles: its places in the third and fourth
 	uint32_t *segmentSlots;  // tall triangles: the record of every segment of ROW_SEGMENT rows; null: rows are packed in pairs
 	uint32_t *tileCursors;   // 2 * totalTiles: the places taken in each tile's lists
 	uint32_t *bigList, *bigCount; // records over more than four tiles, for bin_big_kernel
@@ -189,8 +197,7 @@ enum ErrorBits : int32_t {
 
 // Phase A: projection (zeroing the counters of the launches behind it when `clear` is given).
 void launch_project(const BatchParams &b, const FrameBuffers &fb, cudaStream_t stream, const ClearedCounters *clear = nullptr);
-// The one-pass setup (fb.emit): every fan triangle's records with their rows taken and their tiles
-// counted.  Needs fewer than MAX_EMIT_TRIANGLES fan triangles.
+// The one-pass setup (fb.emit): every fan triangle's records with their places in the tile lists.  Needs fewer than MAX_EMIT_TRIANGLES fan triangles.
 static const uint32_t MAX_EMIT_TRIANGLES = 1u << 29;
 void launch_setup_emit(const BatchParams &b, const FrameBuffers &fb, cudaStream_t stream);
 // The two-pass setup: the count of draw records per fan triangle, scanned so that the record count
@@ -237,7 +244,9 @@ void launch_stable_sort(const uint32_t *keys, const uint32_t *ids, uint64_t n, i
 void launch_alpha(const BatchParams &b, const FrameBuffers &fb, const TileBins &bins, cudaStream_t stream);
 // Debug overlays: the three edges of every record as lines in pixels (flat / 256), and draw_line
 // (api/drawAPI.cpp:176-279) of many lines of one packed colour into a device image.
-void launch_wire_lines(const DrawRecord *records, const uint32_t *drawn, uint32_t count, int4 *lines, cudaStream_t stream);
+// (drawn: the records' marks per slot, null for the first `slots` records; counter: zero, counts them.)
+void launch_wire_lines(const DrawRecord *records, const uint16_t *drawn, uint32_t slots, uint32_t capacity, uint32_t *counter, int4 *lines,
+                       cudaStream_t stream);
 void launch_draw_lines(uint32_t *image, int32_t stride, int32_t width, int32_t height, const int4 *lines, uint32_t count,
                        uint32_t color, cudaStream_t stream);
 // out[0..3] = record count, row count, tile-list entry count, error bits of a batch, and the extra

@@ -16,9 +16,13 @@ namespace dsrg {
 
 namespace {
 
-__global__ void wire_lines_kernel(const DrawRecord *__restrict__ records, const uint32_t *__restrict__ drawn, uint32_t count, int4 *lines) {
-	for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
-		const DrawRecord &r = records[drawn ? drawn[i] : i];
+__global__ void wire_lines_kernel(const DrawRecord *__restrict__ records, const uint16_t *__restrict__ drawn, uint32_t slots,
+                                  uint32_t capacity, uint32_t *counter, int4 *lines) {
+	for (uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x; slot < slots; slot += gridDim.x * blockDim.x) {
+		if (drawn && !drawn[slot]) continue;
+		const uint32_t i = atomicAdd(counter, 1u); // the lines are drawn in any order
+		if (i >= capacity) break;                  // never reached: the records were counted
+		const DrawRecord &r = records[slot];
 		int32_t x[3], y[3];
 		for (int c = 0; c < 3; c++) { x[c] = r.flat[2 * c] / 256; y[c] = r.flat[2 * c + 1] / 256; } // flat / unitsPerPixel
 		for (int e = 0; e < 3; e++) {
@@ -76,9 +80,10 @@ int grid_of(uint64_t threads) {
 
 } // namespace
 
-void launch_wire_lines(const DrawRecord *records, const uint32_t *drawn, uint32_t count, int4 *lines, cudaStream_t stream) {
-	if (count == 0) return;
-	wire_lines_kernel<<<grid_of(count), 256, 0, stream>>>(records, drawn, count, lines);
+void launch_wire_lines(const DrawRecord *records, const uint16_t *drawn, uint32_t slots, uint32_t capacity, uint32_t *counter, int4 *lines,
+                       cudaStream_t stream) {
+	if (slots == 0) return;
+	wire_lines_kernel<<<grid_of(slots), 256, 0, stream>>>(records, drawn, slots, capacity, counter, lines);
 	add_launches(1);
 }
 

@@ -215,7 +215,7 @@ static int enqueue_phases(dsrg_context ctx, BatchJob &job, BatchTotals &totals, 
 	TRY(ctx->pointCsis.reserve(np)); TRY(ctx->pointIsyOut.reserve(np)); TRY(ctx->pointFlat.reserve(np));
 	TRY(ctx->records.reserve((size_t)recordCap + 1));
 	if (onePass) {
-		TRY(ctx->drawnSlots.reserve((size_t)recordCap + 1));
+		TRY(ctx->drawnMarks.reserve((size_t)recordCap + 4)); // read four at a time
 		TRY(ctx->extraBase.reserve(nt + 1));
 		TRY(ctx->extraIds.reserve((size_t)recordCap - nt + 1));
 		TRY(ctx->tileHeads.reserve((size_t)recordCap + 1));
@@ -250,7 +250,8 @@ static int enqueue_phases(dsrg_context ctx, BatchJob &job, BatchTotals &totals, 
 	fb.rowCapacity = rowCap;
 	if (onePass) {
 		fb.emit.counters = ctx->control.ptr + CONTROL_EMIT;
-		fb.emit.drawn = ctx->drawnSlots.ptr;
+		fb.emit.drawn = ctx->drawnMarks.ptr;
+		fb.emit.triangles = (uint32_t)nt;
 		fb.emit.capacity = recordCap;
 		fb.emit.extraBase = ctx->extraBase.ptr;
 		fb.emit.extraIds = ctx->extraIds.ptr;
@@ -378,6 +379,7 @@ static int enqueue_phases(dsrg_context ctx, BatchJob &job, BatchTotals &totals, 
 	if (outputs) {
 		outputs->params = params;
 		outputs->fb = fb;
+		outputs->slots = onePass ? (uint32_t)nt + ctx->pinnedReadback[TOTALS_EXTRAS] : totals.records;
 	}
 	return DSRG_OK;
 }

@@ -153,3 +153,44 @@ def test_stepped_row_intervals_equal_per_row_intervals(host, kind):
         host.dsrg_host_row_intervals_stepped(C.c_void_p(f.ctypes.data), C.c_int32(y0), C.c_int32(rows), C.c_int32(L), C.c_int32(R),
                                              C.c_void_p(lefts.ctypes.data), C.c_void_p(rights.ctypes.data))
         assert np.array_equal(lefts, a[0]) and np.array_equal(rights, a[1]), (f.tolist(), y0, rows, L, R)
+
+
+@pytest.mark.parametrize("kind", ["small", "offscreen_left", "axis_aligned", "at_the_limit", "degenerate"])
+def test_near_row_intervals_match_oracle(host, kind):
+    """The 32-bit stepping of small triangles equals the oracle's rows, with bounds cut at the image's left
+    and top edges (where quotients turn negative), horizontal and vertical edges, and corners up to
+    the limit of its range; triangles beyond it are refused."""
+    from oracle import port
+    r = np.random.default_rng(sum(map(ord, kind)))
+    W, H = 800, 600
+    taken = 0
+    for _ in range(3000):
+        base = r.integers([2000, 2000], [190000, 140000])
+        flat = base + r.integers(-1800, 1800, size=(3, 2))
+        if kind == "offscreen_left":
+            flat = r.integers(-1500, 1500, size=(3, 2))
+        elif kind == "axis_aligned":
+            flat[1, 1] = flat[0, 1]
+            flat[2, 0] = flat[0, 0]
+        elif kind == "at_the_limit":
+            flat = base // 256 * 256 + r.integers(-17000, 17000, size=(3, 2))
+        elif kind == "degenerate":
+            flat[2] = flat[r.integers(0, 2)]
+        flat = flat.astype(np.int32).reshape(-1)
+        L, R = _bound_x(flat, W)
+        top = max(min(int((v + 128) / 256) for v in flat[1::2]) - 1, 0) & ~1
+        bottom = min(max(int((v + 128) / 256) for v in flat[1::2]) + 1, H)
+        rows = min(((bottom + 1) & ~1) - top, 16)
+        if L >= R or rows <= 0:
+            continue
+        lefts, rights = np.zeros(16, np.int32), np.zeros(16, np.int32)
+        ok = host.dsrg_host_row_intervals_near(C.c_void_p(flat.ctypes.data), C.c_int32(top), C.c_int32(rows), C.c_int32(L), C.c_int32(R),
+                                               C.c_void_p(lefts.ctypes.data), C.c_void_p(rights.ctypes.data))
+        relative = np.abs(flat.astype(np.int64).reshape(3, 2) - 256 * np.array([L, top]))
+        assert bool(ok) == bool((relative <= 16384).all())
+        if not ok:
+            continue
+        taken += 1
+        want = _rows(host, flat, top, rows, L, R)
+        assert np.array_equal(lefts[:rows], want[0]) and np.array_equal(rights[:rows], want[1])
+    assert taken > 300
