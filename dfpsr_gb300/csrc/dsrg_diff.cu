@@ -247,6 +247,16 @@ __device__ __forceinline__ void warp_run_add(float4 *base, uint32_t key, float4 
 	if (active && last) atomicAdd(base + key, value);
 }
 
+// Where adjoint_emit_kernel puts the texture's and the vertex colours' contributions: their targets, their
+// values and each target's number.  A vertex colour's target is vertexKeyBase + its point, so that both
+// kinds can be sorted together.
+struct DeterministicSums {
+	uint32_t *texKeys, *vertexKeys;
+	float4 *texValues, *vertexValues;
+	uint32_t *texCounts, *vertexCounts;
+	uint32_t texKeyEnd, vertexKeyBase, vertexKeyEnd;
+};
+
 // Per-pixel gradients: texture (4 taps), vertex colours (3 corners) and light.
 struct PixelGrad {
 	float4 tex[4], vertex[3];
@@ -317,11 +327,11 @@ __global__ void __launch_bounds__(256) adjoint_atomic_kernel(DiffModel m, DiffPa
 	block_light_sums(light, blockLight);
 }
 
-// Deterministic mode, step 1: every contribution as (target, value) in pixel order.
+// Deterministic mode, step 1: every contribution as (target, value) in pixel order, and the number of
+// each target's.  A pixel without a triangle has only the keys texKeyEnd and vertexKeyEnd.
 __global__ void __launch_bounds__(256) adjoint_emit_kernel(DiffModel m, DiffParams q, const uint32_t *__restrict__ visibility,
-                                                           const float4 *__restrict__ grad, uint64_t pixels, uint32_t texKeyEnd,
-                                                           uint32_t vertexKeyEnd, uint32_t *texKeys, float4 *texValues,
-                                                           uint32_t *vertexKeys, float4 *vertexValues, float *blockLight) {
+                                                           const float4 *__restrict__ grad, uint64_t pixels, DeterministicSums sums,
+                                                           float *blockLight) {
 	float light[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 	for (uint64_t base = blockIdx.x * (uint64_t)blockDim.x; base < pixels; base += (uint64_t)gridDim.x * blockDim.x) {
 		const uint64_t i = base + threadIdx.x;
@@ -330,12 +340,17 @@ __global__ void __launch_bounds__(256) adjoint_emit_kernel(DiffModel m, DiffPara
 		PixelGrad pg;
 		const bool active = pixel_gradient(m, q, visibility, i, grad[i], s, pg);
 		for (int k = 0; k < 4; k++) {
-			texKeys[i * 4 + k] = active ? s.taps[k] : texKeyEnd;
-			texValues[i * 4 + k] = active ? pg.tex[k] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+			sums.texKeys[i * 4 + k] = active ? s.taps[k] : sums.texKeyEnd;
+			if (!active) continue;
+			sums.texValues[i * 4 + k] = pg.tex[k];
+			atomicAdd(&sums.texCounts[s.taps[k]], 1u);
 		}
 		for (int c = 0; c < 3; c++) {
-			vertexKeys[i * 3 + c] = active ? (uint32_t)s.point[c] : vertexKeyEnd;
-			vertexValues[i * 3 + c] = active ? pg.vertex[c] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+			const uint32_t key = active ? sums.vertexKeyBase + (uint32_t)s.point[c] : sums.vertexKeyEnd;
+			sums.vertexKeys[i * 3 + c] = key;
+			if (!active) continue;
+			sums.vertexValues[i * 3 + c] = pg.vertex[c];
+			atomicAdd(&sums.vertexCounts[key], 1u);
 		}
 		if (active)
 			for (int j = 0; j < 4; j++) light[j] = fadd(light[j], pg.light[j]);
@@ -346,9 +361,10 @@ __global__ void __launch_bounds__(256) adjoint_emit_kernel(DiffModel m, DiffPara
 // One warp per target key k: the values of the ids sorted into [segment[k], segment[k + 1]),
 // lane l summing entries l, l + 32, ... in order, then a butterfly over the lanes.  Float
 // addition is commutative, so every lane of the butterfly ends with the same bits; the shape of
-// the sum depends only on the segment's length, which makes the result run-independent.
+// the sum depends only on the segment's length, which makes the result run-independent.  Keys from
+// `split` on go to outAbove.
 __global__ void segment_sum_kernel(const uint32_t *__restrict__ segment, const uint32_t *__restrict__ sortedIds,
-                                   const float4 *__restrict__ values, uint32_t keys, float4 *out) {
+                                   const float4 *__restrict__ values, uint32_t keys, float4 *out, uint32_t split, float4 *outAbove) {
 	const uint32_t lane = threadIdx.x & 31;
 	const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
 	for (uint32_t k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < keys; k += warps) {
@@ -364,14 +380,9 @@ __global__ void segment_sum_kernel(const uint32_t *__restrict__ segment, const u
 			s.z = fadd(s.z, __shfl_xor_sync(0xFFFFFFFFu, s.z, o));
 			s.w = fadd(s.w, __shfl_xor_sync(0xFFFFFFFFu, s.w, o));
 		}
-		if (lane == 0) out[k] = s;
-	}
-}
-
-__global__ void key_count_kernel(const uint32_t *__restrict__ keys, uint64_t n, uint32_t keyEnd, uint32_t *counts) {
-	for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-		const uint32_t k = keys[i];
-		if (k < keyEnd) atomicAdd(&counts[k], 1u);
+		if (lane == 0) {
+			if (k < split) out[k] = s; else outAbove[k - split] = s;
+		}
 	}
 }
 
@@ -391,7 +402,7 @@ struct dsrg_diff_s {
 	float ambient;
 	DeviceBuffer<float> depth, normals, blockSums, transform;
 	DeviceBuffer<uint32_t> keysA, keysB, idsA, idsB, hist, offsets, counts, segments, emitted;
-	DeviceBuffer<float4> texValues, vertexValues;
+	DeviceBuffer<float4> values;
 	BatchJob job;
 	int32_t views = 0, width = 0, height = 0;
 };
@@ -409,6 +420,10 @@ static DiffModel diff_model(dsrg_diff d) {
 
 #define TRY(expr) DSRG_CUDA_TRY(ctx, expr)
 
+// Entries (seven per pixel) up to which the deterministic adjoint sorts both kinds of targets at once:
+// three passes instead of five over few entries, which launches and waits decide, not their number.
+static const uint64_t TOGETHER_ENTRIES = 1u << 25;
+
 // Scratch of segmented_sum for n entries and keys below keyEnd, reserved before any launch.
 static int reserve_segmented_sum(dsrg_diff d, uint64_t n, uint32_t keyEnd) {
 	dsrg_context ctx = d->context;
@@ -416,103 +431,28 @@ static int reserve_segmented_sum(dsrg_diff d, uint64_t n, uint32_t keyEnd) {
 	TRY(d->keysA.reserve(n)); TRY(d->keysB.reserve(n)); TRY(d->idsA.reserve(n)); TRY(d->idsB.reserve(n));
 	TRY(d->hist.reserve((size_t)256 * blocks + 1));
 	TRY(d->offsets.reserve((size_t)256 * blocks + 1));
-	TRY(d->counts.reserve((size_t)keyEnd + 1));
 	TRY(d->segments.reserve((size_t)keyEnd + 1));
 	const size_t scanElems = scan_scratch_elems((uint32_t)((size_t)256 * blocks > keyEnd ? (size_t)256 * blocks : keyEnd) + 1);
 	TRY(ctx->scanScratch.reserve(scanElems));
 	return DSRG_OK;
 }
 
-// Entries a block of compact_count_kernel / compact_write_kernel takes (256 threads x 16).
-static const int COMPACT_ITEMS = 16;
-static const uint64_t COMPACT_CHUNK = 256 * COMPACT_ITEMS;
-
-// The entries of each block's chunk with a key below keyEnd (the others are pixels without a
-// triangle), counted.
-__global__ void __launch_bounds__(256) compact_count_kernel(const uint32_t *__restrict__ keys, uint64_t n, uint32_t keyEnd,
-                                                            uint32_t *blockCounts) {
-	__shared__ uint32_t warpSums[8];
-	const uint64_t begin = (uint64_t)blockIdx.x * COMPACT_CHUNK;
-	uint32_t c = 0;
-	for (int r = 0; r < COMPACT_ITEMS; r++) {
-		const uint64_t i = begin + (uint64_t)r * 256 + threadIdx.x;
-		if (i < n && keys[i] < keyEnd) c++;
-	}
-	for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xFFFFFFFFu, c, o);
-	if ((threadIdx.x & 31) == 0) warpSums[threadIdx.x >> 5] = c;
-	__syncthreads();
-	if (threadIdx.x == 0) {
-		uint32_t total = 0;
-		for (int w = 0; w < 8; w++) total += warpSums[w];
-		blockCounts[blockIdx.x] = total;
-	}
-}
-
-// Those entries as (key, entry index) pairs, in entry order, each block from its scanned offset.
-__global__ void __launch_bounds__(256) compact_write_kernel(const uint32_t *__restrict__ keys, uint64_t n, uint32_t keyEnd,
-                                                            const uint32_t *__restrict__ blockOffsets, uint32_t *outKeys,
-                                                            uint32_t *outIds) {
-	__shared__ uint32_t warpCounts[8];
-	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-	const uint64_t begin = (uint64_t)blockIdx.x * COMPACT_CHUNK;
-	uint32_t running = blockOffsets[blockIdx.x];
-	for (int r = 0; r < COMPACT_ITEMS; r++) {
-		const uint64_t i = begin + (uint64_t)r * 256 + threadIdx.x;
-		const uint32_t k = i < n ? keys[i] : keyEnd;
-		const bool keep = k < keyEnd;
-		const uint32_t kept = __ballot_sync(0xFFFFFFFFu, keep);
-		if (lane == 0) warpCounts[warp] = __popc(kept);
-		__syncthreads();
-		uint32_t before = running, total = 0;
-		for (int w = 0; w < 8; w++) {
-			if (w < warp) before += warpCounts[w];
-			total += warpCounts[w];
-		}
-		if (keep) {
-			const uint32_t at = before + __popc(kept & ((1u << lane) - 1u));
-			outKeys[at] = k;
-			outIds[at] = (uint32_t)i;
-		}
-		running += total;
-		__syncthreads(); // warpCounts is read before the next round writes it
-	}
-}
-
-// Sums `values` per key in [0, keyEnd) into out (keyEnd float4), in the order of the entries:
-// count and scan the keys, keep the entries with a key (in entry order), stable-sort their ids by
-// key, then one ordered sum per key.  Its scratch must have been reserved (reserve_segmented_sum).
-static int segmented_sum(dsrg_diff d, const uint32_t *keys, const float4 *values, uint64_t n, uint32_t keyEnd, float4 *out) {
+// Sums `values` per key in [0, keyEnd) in the order of the entries, keys below `split` into out and the
+// others into outAbove: the keys' counts (at `counts`) are scanned into segments, the indices of the
+// entries with a key are stable-sorted by it (n entries in all), then one ordered sum per key.  Its
+// scratch must have been reserved (reserve_segmented_sum).  Nothing comes back to the host.
+static int segmented_sum(dsrg_diff d, const uint32_t *keys, const float4 *values, const uint32_t *counts, uint64_t n, uint32_t keyEnd,
+                         float4 *out, uint32_t split, float4 *outAbove) {
 	dsrg_context ctx = d->context;
 	cudaStream_t stream = ctx->stream;
-	int bits = 1;
-	while ((1ull << bits) <= (uint64_t)keyEnd) bits++;
-	// segment starts per key
-	TRY(cudaMemsetAsync(d->counts.ptr, 0, sizeof(uint32_t) * keyEnd, stream));
-	key_count_kernel<<<grid_for(n, 256), 256, 0, stream>>>(keys, n, keyEnd, d->counts.ptr);
-	add_launches(1);
-	launch_scan(d->counts.ptr, d->segments.ptr, keyEnd, ctx->scanScratch.ptr, ctx->scanScratch.capacity, stream);
-	// the entries with a key, in entry order, into the sort's second buffers (its first pass reads
-	// them from there); their number comes back to the host for the sort's launch shape
-	const uint32_t blocks = (uint32_t)((n + COMPACT_CHUNK - 1) / COMPACT_CHUNK);
-	uint32_t kept = 0;
-	if (blocks > 0) {
-		compact_count_kernel<<<blocks, 256, 0, stream>>>(keys, n, keyEnd, d->hist.ptr);
-		launch_scan(d->hist.ptr, d->offsets.ptr, blocks, ctx->scanScratch.ptr, ctx->scanScratch.capacity, stream);
-		compact_write_kernel<<<blocks, 256, 0, stream>>>(keys, n, keyEnd, d->offsets.ptr, d->keysB.ptr, d->idsB.ptr);
-		add_launches(2);
-		TRY(cudaGetLastError());
-		TRY(cudaMemcpyAsync(ctx->pinnedReadback + 8, d->offsets.ptr + blocks, sizeof(uint32_t), cudaMemcpyDeviceToHost, stream));
-		TRY(cudaStreamSynchronize(stream));
-		kept = ctx->pinnedReadback[8];
-	}
-	// the kept entries' ids sorted by key, entries of one key in entry order
+	launch_scan(counts, d->segments.ptr, keyEnd, ctx->scanScratch.ptr, ctx->scanScratch.capacity, stream);
 	SortBuffers sb;
 	sb.keysA = d->keysA.ptr; sb.keysB = d->keysB.ptr; sb.idsA = d->idsA.ptr; sb.idsB = d->idsB.ptr;
 	sb.hist = d->hist.ptr; sb.offsets = d->offsets.ptr;
 	sb.scanScratch = ctx->scanScratch.ptr; sb.scanScratchElems = ctx->scanScratch.capacity;
-	const uint32_t *sortedKeys = nullptr, *iin = nullptr;
-	launch_stable_sort(d->keysB.ptr, d->idsB.ptr, kept, bits, sb, stream, &sortedKeys, &iin);
-	segment_sum_kernel<<<grid_for((uint64_t)keyEnd * 32, 256), 256, 0, stream>>>(d->segments.ptr, iin, values, keyEnd, out);
+	const uint32_t *sorted = nullptr;
+	launch_stable_sort(keys, n, keyEnd, d->segments.ptr + keyEnd, sb, stream, &sorted);
+	segment_sum_kernel<<<grid_for((uint64_t)keyEnd * 32, 256), 256, 0, stream>>>(d->segments.ptr, sorted, values, keyEnd, out, split, outAbove);
 	add_launches(1);
 	TRY(cudaGetLastError());
 	return DSRG_OK;
@@ -563,8 +503,7 @@ int dsrg_diff_destroy(dsrg_diff d) {
 	for (auto *b : f) b->release();
 	DeviceBuffer<uint32_t> *u[] = {&d->keysA, &d->keysB, &d->idsA, &d->idsB, &d->hist, &d->offsets, &d->counts, &d->segments, &d->emitted};
 	for (auto *b : u) b->release();
-	d->texValues.release();
-	d->vertexValues.release();
+	d->values.release();
 	delete d;
 	return DSRG_OK;
 }
@@ -700,19 +639,36 @@ int dsrg_diff_adjoint(dsrg_diff d, int32_t views, int32_t width, int32_t height,
 		                                                  reinterpret_cast<float4 *>(gradVertexColors), blockLight);
 		add_launches(1);
 	} else {
-		TRY(d->texValues.reserve(pixels * 4));
-		TRY(d->vertexValues.reserve(pixels * 3));
+		TRY(d->values.reserve(pixels * 7));
 		TRY(d->emitted.reserve(pixels * 7));
-		status = reserve_segmented_sum(d, pixels * 4, texels > points ? texels : points);
+		TRY(d->counts.reserve((size_t)texels + points + 2));
+		// both kinds of targets sorted together where that saves passes and launches; large images keep the
+		// smaller scratch of one kind at a time
+		const bool together = pixels * 7 <= TOGETHER_ENTRIES;
+		status = together ? reserve_segmented_sum(d, pixels * 7, texels + points) : reserve_segmented_sum(d, pixels * 4, texels > points ? texels : points);
 		if (status != DSRG_OK) return status;
-		uint32_t *texKeys = d->emitted.ptr, *vertexKeys = d->emitted.ptr + pixels * 4;
-		adjoint_emit_kernel<<<blocks, 256, 0, stream>>>(diff_model(d), q, visibility, grad, pixels, texels, points, texKeys,
-		                                                d->texValues.ptr, vertexKeys, d->vertexValues.ptr, blockLight);
+		DeterministicSums sums;
+		sums.texKeys = d->emitted.ptr;
+		sums.vertexKeys = d->emitted.ptr + pixels * 4;
+		sums.texValues = d->values.ptr;
+		sums.vertexValues = d->values.ptr + pixels * 4;
+		sums.texCounts = d->counts.ptr;
+		sums.vertexCounts = together ? d->counts.ptr : d->counts.ptr + texels;
+		sums.vertexKeyBase = together ? texels : 0u;
+		sums.texKeyEnd = together ? texels + points : texels;
+		sums.vertexKeyEnd = sums.vertexKeyBase + points;
+		TRY(cudaMemsetAsync(d->counts.ptr, 0, sizeof(uint32_t) * ((size_t)texels + points), stream));
+		adjoint_emit_kernel<<<blocks, 256, 0, stream>>>(diff_model(d), q, visibility, grad, pixels, sums, blockLight);
 		add_launches(1);
 		TRY(cudaGetLastError());
-		status = segmented_sum(d, texKeys, d->texValues.ptr, pixels * 4, texels, reinterpret_cast<float4 *>(gradTexture));
-		if (status == DSRG_OK)
-			status = segmented_sum(d, vertexKeys, d->vertexValues.ptr, pixels * 3, points, reinterpret_cast<float4 *>(gradVertexColors));
+		float4 *texOut = reinterpret_cast<float4 *>(gradTexture), *vertexOut = reinterpret_cast<float4 *>(gradVertexColors);
+		if (together) {
+			status = segmented_sum(d, sums.texKeys, sums.texValues, sums.texCounts, pixels * 7, texels + points, texOut, texels, vertexOut);
+		} else {
+			status = segmented_sum(d, sums.texKeys, sums.texValues, sums.texCounts, pixels * 4, texels, texOut, texels, nullptr);
+			if (status == DSRG_OK)
+				status = segmented_sum(d, sums.vertexKeys, sums.vertexValues, sums.vertexCounts, pixels * 3, points, vertexOut, points, nullptr);
+		}
 		if (status != DSRG_OK) {
 			cudaStreamSynchronize(stream);
 			return status;

@@ -211,7 +211,7 @@ struct dsrg_context_s {
 	DeviceBuffer<uint32_t> control;      // a batch's counters (ControlWord)
 	DeviceBuffer<uint4> tileList;        // the tiles of a batch that have tile-list entries
 	uint32_t *pinnedReadback = nullptr;  // page-locked: the gathered totals (written there by the GPU), the fragment count,
-	                                     // [8] the entries a deterministic adjoint's sums keep, [9] TOTALS_EXTRAS
+	                                     // [9] TOTALS_EXTRAS
 	uint32_t *readbackDevice = nullptr;  // its device address
 	bool timingPending = false;          // stats' times not yet read from the events of the last call
 	bool timingHasRaster = false;

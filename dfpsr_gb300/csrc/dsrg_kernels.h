@@ -234,11 +234,12 @@ struct SortBuffers {
 	uint32_t *scanScratch;
 	size_t scanScratchElems;
 };
-uint32_t sort_blocks(uint64_t n);
-// Stable LSD radix sort of the ids (the item indices when ids is null) by the low keyBits bits of
-// their keys; *sortedKeys and *sortedIds point at the buffers holding the result (the inputs when n is 0).
-void launch_stable_sort(const uint32_t *keys, const uint32_t *ids, uint64_t n, int keyBits, const SortBuffers &b,
-                        cudaStream_t stream, const uint32_t **sortedKeys, const uint32_t **sortedIds);
+uint32_t sort_blocks(uint64_t n); // n >= 1
+// Stable LSD radix sort of the indices of the n >= 1 items by their keys, leaving out the items whose
+// key is not below keyEnd; *keptDevice is the number of the others.  *sortedIds points at the buffer
+// holding the result.
+void launch_stable_sort(const uint32_t *keys, uint64_t n, uint32_t keyEnd, const uint32_t *keptDevice, const SortBuffers &b,
+                        cudaStream_t stream, const uint32_t **sortedIds);
 // The alpha filter over the binned records (in place of launch_raster): colour blends in
 // submission order, depth read only.
 void launch_alpha(const BatchParams &b, const FrameBuffers &fb, const TileBins &bins, cudaStream_t stream);

@@ -183,3 +183,30 @@ def test_forward_matches_reference_rgbamultiply_with_unit_light(ctx):
     diff = np.abs(ours - ref)[covered]
     assert diff.max() <= 3.0, f"max {diff.max()}"
     assert diff.mean() < 1.0
+
+
+@pytest.mark.parametrize("views,width,height,major,minor,texture", [
+    (1, 9, 7, 12, 8, 4),        # fewer entries than one block of the sort, three-bit keys
+    (20, 201, 151, 40, 16, 64),  # above the size from which a thread sorts more items
+    (80, 256, 256, 60, 24, 512)  # too many entries to sort both kinds of targets together
+])
+def test_deterministic_sums_of_any_size(ctx, views, width, height, major, minor, texture):
+    """The deterministic adjoint equals the atomic one up to the rounding of its sums, and itself bit for
+    bit.  A target sums n terms in either order with an error of at most n 2^-24 of their magnitudes each;
+    at these sizes a target has fewer than 1000 terms on average, so the two differ by less than 1.2e-4."""
+    import torch
+    from diff_harness import make_renderer
+    from dfpsr_gb300 import scenes
+    problem = scenes.diff_problem(seed=views, views=views, size=256, texture_size=texture, major=major, minor=minor)
+    problem.mesh.width = problem.width = width
+    problem.mesh.height = problem.height = height
+    _, renderer, cameras, params = make_renderer(ctx, problem)
+    images, vis = run_forward(renderer, cameras, problem, params)
+    grad = torch.rand(images.shape, device="cuda", generator=torch.Generator(device="cuda").manual_seed(3)) / images.numel()
+    atomic = gpu_adjoint(renderer, problem, params, vis, grad, False)
+    sums = gpu_adjoint(renderer, problem, params, vis, grad, True)
+    again = gpu_adjoint(renderer, problem, params, vis, grad, True)
+    for name in atomic:
+        assert np.array_equal(sums[name].view(np.uint32), again[name].view(np.uint32)), name
+        a, b = atomic[name].astype(np.float64), sums[name].astype(np.float64)
+        assert np.linalg.norm(a) > 0 and np.linalg.norm(a - b) < 1.2e-4 * np.linalg.norm(a), name
