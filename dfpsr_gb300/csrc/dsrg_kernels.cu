@@ -1119,17 +1119,21 @@ __device__ __forceinline__ bool tile_may_overlap(const DrawRecord &r, int32_t px
 // The corner test above is exact only when no row of the record makes the reference cast a
 // quotient beyond 32 bits (a nearly horizontal edge whose row crossings lie 2^30 pixels away),
 // because such a row's interval comes from the wrapped value, not from the edge.
+__device__ __forceinline__ bool edge_test_is_exact(const Edge &e, int32_t top, int32_t bottom) {
+	if (e.nx == 0) return true;
+	const float den = fabsf(i64_to_float(e.nx * 256));
+	for (int k = 0; k < 2; k++) {
+		const int64_t y = k ? (int64_t)bottom : (int64_t)top;
+		const int64_t limit = e.threshold - (128 - e.sx) * e.nx - (128 + 256 * y - e.sy) * e.ny;
+		if (fabsf(i64_to_float(limit)) >= 5.0e8f * den) return false;
+	}
+	return true;
+}
+
 __device__ __forceinline__ bool tile_test_is_exact(const DrawRecord &r) {
 	for (int i = 0; i < 3; i++) {
 		const int j = (i + 1) % 3;
-		const Edge e = make_edge(r.flat[i * 2], r.flat[i * 2 + 1], r.flat[j * 2], r.flat[j * 2 + 1]);
-		if (e.nx == 0) continue;
-		const float den = fabsf(i64_to_float(e.nx * 256));
-		for (int k = 0; k < 2; k++) {
-			const int64_t y = k ? (int64_t)r.bottom : (int64_t)r.top;
-			const int64_t limit = e.threshold - (128 - e.sx) * e.nx - (128 + 256 * y - e.sy) * e.ny;
-			if (fabsf(i64_to_float(limit)) >= 5.0e8f * den) return false;
-		}
+		if (!edge_test_is_exact(make_edge(r.flat[i * 2], r.flat[i * 2 + 1], r.flat[j * 2], r.flat[j * 2 + 1]), r.top, r.bottom)) return false;
 	}
 	return true;
 }
@@ -1236,40 +1240,56 @@ __device__ __forceinline__ uint32_t plane_hi(float s, float dx, float dy, float 
 	return affine ? ~hi : hi;
 }
 
-// The records over more than four tiles, which setup_emit_kernel listed.  A block takes BIG_GROUP of them at a time and its threads share
-// the (record, tile) pairs of their bounds evenly, so that one record spanning a whole frame is
-// spread over the block instead of keeping a single warp busy while the rest of the grid idles.
+// The records over more than four tiles, which setup_emit_kernel listed.  A block takes BIG_GROUP of
+// them at a time.  Four lanes load each record (one per edge, one for the plane), the (record, tile
+// row) pairs are dealt to the warps in turn, each lane finds the columns of one row, and the warp's
+// lanes share the (record, tile) pairs of its 32 rows evenly: one record spanning a whole frame is
+// spread over the block, and no lane is spent on the tiles of a bound that the triangle misses.
 //
-// The edge test of tile_may_overlap is a linear function of the tile's column and row, so the
-// loading thread writes each edge as base + column * stepX + row * stepY (the value at the tile's
-// most inside corner less the threshold, at most 0 when the edge admits it) and a pair costs two
-// multiply-adds per edge.  Adding `full`, the function's change from that corner to the opposite one,
-// gives the same test for the most outside corner: a tile whose grown rectangle passes it for all
-// three edges is covered by the record completely (the growth by two pixels also keeps clear of the
-// column where the reference's truncating division rejects a pixel that is inside).
+// The edge test of tile_may_overlap is a linear function of the tile's column and row, so an edge is
+// kept as base + row * stepY + column * stepX (the value at the tile's most inside corner less the
+// threshold, at most 0 when the edge admits it), and in one row it admits the columns on one side of
+// a crossing.  Adding `full`, the function's change from that corner to the opposite one, gives the
+// same for the most outside corner: a tile whose grown rectangle passes it for all three edges is
+// covered by the record completely (the growth by two pixels also keeps clear of the column where
+// the reference's truncating division rejects a pixel that is inside).  The row's value is exact; the
+// crossing is a binary32 quotient (four roundings, under 2^-21 of itself) widened by 2^-20 of itself
+// and 2^-10 of a tile, towards listing a tile too many and towards covering one too few.
 //
 // Culling while binning: the count pass raises a tile's threshold to the worst key (plane_hi) of
-// each record that covers it completely, and the fill pass, which runs when every record has been
-// counted, lists a large record only where its best key reaches that threshold.  Every pixel of the
-// tile then holds a better key than a record left out could give.  Scenes of large triangles drawn
-// over one another keep a few entries per tile of hundreds or thousands: of the 1.07 M entries of
-// 20,000 random triangles at 800x600, which the tile kernel fetched and rejected one by one, about
-// 62,000 are listed and a frame takes 277 us instead of 375; a batch of 32 mixed frames 8.7 ms
-// instead of 10.4.
-static const int BIG_GROUP = 8;
+// each record that covers it completely and leaves out a large record whose best key does not reach
+// the threshold so far.  The fill pass runs when every record has been counted and tests against the
+// final threshold, so what it lists was counted, whatever the order; the count is an upper bound that
+// differs from run to run.  Every pixel of the tile then holds a better key than a record left out
+// could give.  Scenes of large triangles drawn over one another keep a few entries per tile of
+// hundreds or thousands: of the 1.07 M entries of 20,000 random triangles at 800x600, which the tile
+// kernel fetched and rejected one by one, about 62,000 are listed and a frame takes 277 us instead of
+// 375; a batch of 32 mixed frames 8.7 ms instead of 10.4.
+static const int BIG_GROUP = 16;
+static const int BIG_WARPS = 8; // warps of a block
 
 struct BigEdge {
-	long long base, stepX, stepY, full;
+	long long base, stepY, full;
+	float recip; // 1 / stepX
+	int32_t side; // sign of stepX
 };
 
 struct BigRecord {
 	BigEdge edge[3];
 	float start, dx, dy, margin;
-	uint32_t id, tileBase, large;
 	int32_t left, top, right, bottom;
-	int32_t tx0, ty0, bw, tilesX, exact, affine, width, height;
+	uint32_t id, tileBase, large;
+	int32_t tx0, tx1, ty0, tilesX, exact, affine, width, height;
+	int32_t coverLeft, coverRight; // columns within the record's bounds
 	int32_t cullRows; // tile rows from the top in which keys decide (0: none)
-	float recip;      // 1 / bw
+};
+
+// One row of tiles of a big record, as its warp's lanes read it.
+struct __align__(16) BigRow {
+	int32_t shift;   // column of a pair less its number
+	uint32_t covers; // first column covered completely, and the last one << 16
+	uint32_t place;  // the row, its record in the group << 16, and whether keys decide << 31
+	uint32_t tile;   // tile number of column 0
 };
 
 // Tile rows of a frame in which the largest key decides every pixel, so that records may be culled:
@@ -1280,102 +1300,166 @@ __device__ __forceinline__ int32_t key_decided_rows(const FrameTarget &f, bool d
 	return (!depthOnly && (f.height & 1)) ? f.tilesY - 1 : f.tilesY;
 }
 
+// Columns of the tile row ty that the record may touch (lo..hi) and that it covers (cl..ch).
+__device__ __forceinline__ void big_row_columns(const BigRecord &h, int32_t ty, int32_t &lo, int32_t &hi, int32_t &cl, int32_t &ch) {
+	lo = h.tx0; hi = h.tx1;
+	cl = h.coverLeft; ch = h.coverRight;
+	const int32_t py0 = ty * TILE_H;
+	if (!h.exact || ty >= h.cullRows || h.top > py0 || h.bottom < min(py0 + TILE_H, h.height)) ch = -1;
+	if (!h.exact) return;
+#pragma unroll
+	for (int e = 0; e < 3; e++) {
+		const BigEdge &edge = h.edge[e];
+		const long long outer = edge.base + (long long)ty * edge.stepY, inner = outer + edge.full;
+		if (edge.side == 0) {
+			if (outer > 0) hi = -1;
+			if (inner > 0) ch = -1;
+			continue;
+		}
+		const float qo = -__fmul_rn(i64_to_float(outer), edge.recip), qi = -__fmul_rn(i64_to_float(inner), edge.recip);
+		const float mo = __fadd_rn(__fmul_rn(fabsf(qo), 9.5367431640625e-7f), 9.765625e-4f);
+		const float mi = __fadd_rn(__fmul_rn(fabsf(qi), 9.5367431640625e-7f), 9.765625e-4f);
+		if (edge.side > 0) {
+			hi = min(hi, __float2int_rd(__fadd_rn(qo, mo)));
+			ch = min(ch, __float2int_rd(__fsub_rn(qi, mi)));
+		} else {
+			lo = max(lo, __float2int_ru(__fsub_rn(qo, mo)));
+			cl = max(cl, __float2int_ru(__fadd_rn(qi, mi)));
+		}
+	}
+}
+
 template <bool FILL>
 __device__ __forceinline__ void bin_big(const BatchParams &b, const DrawRecord *__restrict__ records, const TileBins &bins,
                                         const uint32_t *extraIds, int32_t *errorFlag) {
 	__shared__ BigRecord held[BIG_GROUP];
-	__shared__ int32_t firstPair[BIG_GROUP + 1];
+	__shared__ BigRow heldRows[BIG_WARPS][32];
+	__shared__ int32_t firstRow[BIG_GROUP + 1];
 	const uint32_t count = *bins.bigCount;
+	const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+	const uint32_t upTo = 0xFFFFFFFFu >> (31u - lane); // this lane and those before
 	for (uint32_t first = blockIdx.x * BIG_GROUP; first < count; first += gridDim.x * BIG_GROUP) { // uniform per block
-		if (threadIdx.x < BIG_GROUP) {
-			const uint32_t w = first + threadIdx.x;
-			int32_t pairs = 0;
-			if (w < count) {
-				BigRecord &h = held[threadIdx.x];
-				const uint32_t slot = bins.bigList[w];
-				h.id = record_id(b, extraIds, slot);
-				const DrawRecord rec = records[slot];
-				const FrameTarget &f = b.frames[rec.frame];
-				h.large = (b.depthOnly || !record_is_small(rec, b.smallRows, b.smallWidth)) ? 1u : 0u;
-				h.left = rec.left; h.top = rec.top; h.right = rec.right; h.bottom = rec.bottom;
-				h.tx0 = rec.left >> 4;
-				h.ty0 = rec.top >> 4;
-				const int32_t tx1 = min((rec.right - 1) >> 4, f.tilesX - 1), ty1 = min((rec.bottom - 1) >> 4, f.tilesY - 1);
-				h.bw = tx1 - h.tx0 + 1;
-				h.recip = 1.0f / (float)max(h.bw, 1);
-				h.tilesX = f.tilesX;
-				h.tileBase = f.tileBase;
-				h.width = f.width;
-				h.height = f.height;
-				h.affine = f.affine;
-				h.cullRows = bins.thresholds ? key_decided_rows(f, b.depthOnly != 0) : 0;
-				h.start = rec.start[0]; h.dx = rec.dx[0]; h.dy = rec.dy[0];
-				h.margin = plane_margin(rec, b.depthOnly != 0);
-				h.exact = tile_test_is_exact(rec) ? 1 : 0;
-				for (int i = 0; i < 3; i++) {
-					const int j = (i + 1) % 3;
-					const Edge e = make_edge(rec.flat[i * 2], rec.flat[i * 2 + 1], rec.flat[j * 2], rec.flat[j * 2 + 1]);
+		const uint32_t taken = min((uint32_t)BIG_GROUP, count - first);
+		if (threadIdx.x < BIG_GROUP * 4) {
+			const uint32_t q = threadIdx.x >> 2, role = threadIdx.x & 3u;
+			bool wrapped = false; // an edge whose test is not exact
+			if (q < taken) {
+				BigRecord &h = held[q];
+				const uint32_t slot = bins.bigList[first + q];
+				const DrawRecord &rec = records[slot];
+				if (role < 3u) {
+					const uint32_t j = role == 2u ? 0u : role + 1u;
+					const Edge e = make_edge(rec.flat[role * 2], rec.flat[role * 2 + 1], rec.flat[j * 2], rec.flat[j * 2 + 1]);
 					// the grown rectangle of tile (0, 0): pixel centres -2 .. TILE_W + 1 and -2 .. TILE_H + 1
 					const long long x = 128 + 256 * (long long)(e.nx >= 0 ? -2 : TILE_W + 1);
 					const long long y = 128 + 256 * (long long)(e.ny >= 0 ? -2 : TILE_H + 1);
-					h.edge[i].base = (x - e.sx) * e.nx + (y - e.sy) * e.ny - e.threshold;
-					h.edge[i].stepX = 256 * TILE_W * (long long)e.nx;
-					h.edge[i].stepY = 256 * TILE_H * (long long)e.ny;
-					h.edge[i].full = 256 * (TILE_W + 3) * (long long)(e.nx >= 0 ? e.nx : -e.nx) + 256 * (TILE_H + 3) * (long long)(e.ny >= 0 ? e.ny : -e.ny);
+					BigEdge &edge = h.edge[role];
+					edge.base = (x - e.sx) * e.nx + (y - e.sy) * e.ny - e.threshold;
+					edge.stepY = 256 * TILE_H * (long long)e.ny;
+					edge.full = 256 * (TILE_W + 3) * (long long)(e.nx >= 0 ? e.nx : -e.nx) + 256 * (TILE_H + 3) * (long long)(e.ny >= 0 ? e.ny : -e.ny);
+					edge.side = e.nx > 0 ? 1 : (e.nx < 0 ? -1 : 0);
+					edge.recip = e.nx != 0 ? __fdiv_rn(1.0f, i64_to_float(256 * TILE_W * (long long)e.nx)) : 0.0f;
+					wrapped = !edge_test_is_exact(e, rec.top, rec.bottom);
+				} else {
+					const FrameTarget &f = b.frames[rec.frame];
+					h.id = record_id(b, extraIds, slot);
+					h.large = (b.depthOnly || !record_is_small(rec, b.smallRows, b.smallWidth)) ? 1u : 0u;
+					h.left = rec.left; h.top = rec.top; h.right = rec.right; h.bottom = rec.bottom;
+					h.tx0 = rec.left >> 4;
+					h.ty0 = rec.top >> 4;
+					h.tx1 = min((rec.right - 1) >> 4, f.tilesX - 1);
+					h.tilesX = f.tilesX;
+					h.tileBase = f.tileBase;
+					h.width = f.width;
+					h.height = f.height;
+					h.affine = f.affine;
+					h.coverLeft = (rec.left + TILE_W - 1) >> 4;
+					h.coverRight = rec.right >= f.width ? f.tilesX - 1 : (rec.right >> 4) - 1;
+					h.cullRows = bins.thresholds ? key_decided_rows(f, b.depthOnly != 0) : 0;
+					h.start = rec.start[0]; h.dx = rec.dx[0]; h.dy = rec.dy[0];
+					h.margin = plane_margin(rec, b.depthOnly != 0);
 				}
-				pairs = (h.bw > 0 && ty1 >= h.ty0) ? h.bw * (ty1 - h.ty0 + 1) : 0;
 			}
-			// prefix sums of the group's pair counts within the first BIG_GROUP lanes
-			int32_t inclusive = pairs;
-			for (int o = 1; o < BIG_GROUP; o <<= 1) {
-				const int32_t v = __shfl_up_sync((1u << BIG_GROUP) - 1u, inclusive, o);
-				if ((int)threadIdx.x >= o) inclusive += v;
-			}
-			firstPair[threadIdx.x + 1] = inclusive;
-			if (threadIdx.x == 0) firstPair[0] = 0;
+			const uint32_t wrappedMask = __ballot_sync(0xFFFFFFFFu, wrapped);
+			if (q < taken && role == 3u) held[q].exact = (wrappedMask >> (lane & 28u) & 7u) == 0u ? 1 : 0;
 		}
 		__syncthreads();
-		const int32_t total = firstPair[BIG_GROUP];
-		int k = 0;
-		for (int32_t i = (int32_t)threadIdx.x; i < total; i += (int32_t)blockDim.x) {
-			while (firstPair[k + 1] <= i) k++;
-			const BigRecord &h = held[k];
-			const int32_t local = i - firstPair[k];
-			// local / bw from a binary32 estimate, corrected (at most 2048 x 2048 tiles)
-			int32_t row = (int32_t)((float)local * h.recip), column = local - row * h.bw;
-			if (column < 0) { row--; column += h.bw; }
-			if (column >= h.bw) { row++; column -= h.bw; }
-			const int32_t tx = h.tx0 + column, ty = h.ty0 + row;
-			bool covered = h.exact != 0;
-			if (h.exact) {
-				bool outside = false;
-#pragma unroll
-				for (int e = 0; e < 3; e++) {
-					const long long value = h.edge[e].base + (long long)tx * h.edge[e].stepX + (long long)ty * h.edge[e].stepY;
-					outside = outside || value > 0;
-					covered = covered && value + h.edge[e].full <= 0;
-				}
-				if (outside) continue;
+		if (threadIdx.x < 32) { // the group's rows
+			int32_t rows = 0;
+			if (lane < taken) {
+				const BigRecord &h = held[lane];
+				const int32_t ty1 = min((h.bottom - 1) >> 4, ((h.height + TILE_H - 1) >> 4) - 1);
+				if (h.tx1 >= h.tx0 && ty1 >= h.ty0) rows = ty1 - h.ty0 + 1;
 			}
-			const uint32_t at = h.tileBase + (uint32_t)(ty * h.tilesX + tx);
-			const uint32_t slotOf = 2u * at + h.large;
-			const int32_t px0 = tx * TILE_W, py0 = ty * TILE_H;
-			const bool decided = ty < h.cullRows;
-			if (!FILL) {
-				atomicAdd(&bins.counts[slotOf], 1u);
-				const int32_t px1 = min(px0 + TILE_W, h.width), py1 = min(py0 + TILE_H, h.height);
-				if (decided && covered && h.left <= px0 && h.top <= py0 && h.right >= px1 && h.bottom >= py1) {
-					const uint32_t worst = plane_hi<false>(h.start, h.dx, h.dy, h.margin, px0, px1 - 1, py0, py1 - 1, h.affine != 0);
-					if (worst) atomicMax(&bins.thresholds[at], worst);
-				}
-			} else {
-				if (decided && h.large &&
-				    plane_hi<true>(h.start, h.dx, h.dy, h.margin, max(px0, h.left), min(px0 + TILE_W, h.right) - 1, max(py0, h.top),
-				                   min(py0 + TILE_H, h.bottom) - 1, h.affine != 0) < bins.thresholds[at])
-					continue;
-				const uint32_t slot = bins.offsets[slotOf] + atomicAdd(&bins.cursors[slotOf], 1u);
-				if (slot < bins.listCapacity) bins.lists[slot] = h.id; else atomicOr(errorFlag, ERROR_BIN_OVERFLOW);
+			int32_t inclusive = rows;
+			for (int o = 1; o < BIG_GROUP; o <<= 1) {
+				const int32_t v = __shfl_up_sync(0xFFFFFFFFu, inclusive, o);
+				if ((int)lane >= o) inclusive += v;
 			}
+			if (lane < BIG_GROUP) firstRow[lane + 1] = inclusive;
+			if (lane == 0) firstRow[0] = 0;
+		}
+		__syncthreads();
+		const int32_t totalRows = firstRow[BIG_GROUP];
+		for (int32_t item0 = (int32_t)warp; item0 < totalRows; item0 += 32 * BIG_WARPS) { // uniform per warp
+			const int32_t item = item0 + (int32_t)lane * BIG_WARPS;
+			int32_t lo = 0, hi = -1, cl = 0, ch = -1, ty = 0, q = 0;
+			if (item < totalRows) {
+				for (int o = BIG_GROUP / 2; o > 0; o >>= 1) // the record: firstRow[q] <= item < firstRow[q + 1]
+					if (firstRow[q + o] <= item) q += o;
+				ty = held[q].ty0 + item - firstRow[q];
+				big_row_columns(held[q], ty, lo, hi, cl, ch);
+			}
+			const int32_t length = max(hi - lo + 1, 0);
+			int32_t inclusive = length;
+			for (int o = 1; o < 32; o <<= 1) {
+				const int32_t v = __shfl_up_sync(0xFFFFFFFFu, inclusive, o);
+				if ((int)lane >= o) inclusive += v;
+			}
+			const int32_t total = __shfl_sync(0xFFFFFFFFu, inclusive, 31), begin = inclusive - length;
+			const uint32_t some = __ballot_sync(0xFFFFFFFFu, length > 0);
+			if (length > 0) {
+				const BigRecord &h = held[q];
+				BigRow row;
+				row.shift = lo - begin;
+				row.covers = ch >= cl ? (uint32_t)cl | (uint32_t)ch << 16 : 0x0000FFFFu;
+				row.place = (uint32_t)ty | (uint32_t)q << 16 | (ty < h.cullRows ? 0x80000000u : 0u);
+				row.tile = h.tileBase + (uint32_t)(ty * h.tilesX);
+				heldRows[warp][__popc(some & (upTo >> 1))] = row;
+			}
+			__syncwarp();
+			int32_t before = -1; // rows begun so far, less one
+			for (int32_t base = 0; base < total; base += 32) {
+				// which of the next 32 pairs begin a row
+				const uint32_t at = (uint32_t)(begin - base);
+				const uint32_t starts = __reduce_or_sync(0xFFFFFFFFu, length > 0 && at < 32u ? 1u << at : 0u);
+				const int32_t i = base + (int32_t)lane;
+				const int32_t mine = before + __popc(starts & upTo);
+				before += __popc(starts);
+				if (i >= total) continue;
+				const BigRow row = heldRows[warp][mine];
+				const BigRecord &h = held[row.place >> 16 & 0x7FFFu];
+				const int32_t tx = i + row.shift, py0 = (int32_t)(row.place & 0xFFFFu) * TILE_H, px0 = tx * TILE_W;
+				const uint32_t tile = row.tile + (uint32_t)tx, slotOf = 2u * tile + h.large;
+				if ((row.place >> 31) && h.large) {
+					const uint32_t best =
+						plane_hi<true>(h.start, h.dx, h.dy, h.margin, max(px0, h.left), min(px0 + TILE_W, h.right) - 1, max(py0, h.top),
+						               min(py0 + TILE_H, h.bottom) - 1, h.affine != 0);
+					if (best < bins.thresholds[tile]) continue;
+				}
+				if (!FILL) {
+					atomicAdd(&bins.counts[slotOf], 1u);
+					if ((uint32_t)tx >= (row.covers & 0xFFFFu) && (uint32_t)tx <= row.covers >> 16) {
+						const uint32_t worst = plane_hi<false>(h.start, h.dx, h.dy, h.margin, px0, min(px0 + TILE_W, h.width) - 1, py0,
+						                                       min(py0 + TILE_H, h.height) - 1, h.affine != 0);
+						if (worst > bins.thresholds[tile]) atomicMax(&bins.thresholds[tile], worst);
+					}
+				} else {
+					const uint32_t slot = bins.offsets[slotOf] + atomicAdd(&bins.cursors[slotOf], 1u);
+					if (slot < bins.listCapacity) bins.lists[slot] = h.id; else atomicOr(errorFlag, ERROR_BIN_OVERFLOW);
+				}
+			}
+			__syncwarp(); // the rows are done with before the next ones are written
 		}
 		__syncthreads(); // the group is done with before the next one is loaded
 	}

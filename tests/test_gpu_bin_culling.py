@@ -92,3 +92,24 @@ def test_depth_only_images_of_any_shape(ctx, w, h, stride, perspective):
         same = (got.view(np.uint32) == expected.view(np.uint32)) | (np.isnan(got) & np.isnan(expected))
         assert same.all(), np.argwhere(~same)[:5].tolist()
     assert (host.numpy()[:, w:] == 0).all() and bool((device[:, w:] == 0).all())
+
+
+@pytest.mark.parametrize("perspective", [True, False])
+@pytest.mark.parametrize("w,h", [(1000, 16), (16, 900), (700, 90), (333, 257)])
+def test_slivers_over_many_tiles(ctx, w, h, perspective):
+    """Triangles over many tiles whose edges are nearly horizontal, nearly vertical or exactly so, thin
+    ones that touch few tiles of their bounds among them: the columns found for each row of tiles."""
+    rng = np.random.default_rng(w * 7 + h)
+    s = scenes.random_triangles(seed=w, triangles=300, width=w, height=h, texture_size=32)
+    p = s.positions.reshape(-1, 3, 3).copy()
+    k = np.arange(300)
+    p[:, :, :2] = rng.uniform(-9.0, 9.0, (300, 3, 2))
+    p[k % 6 == 0, 1, 1] = p[k % 6 == 0, 0, 1]                                  # a horizontal edge
+    p[k % 6 == 1, 1, 0] = p[k % 6 == 1, 0, 0]                                  # a vertical edge
+    for way, axis in ((2, 0), (3, 1)):                                         # slivers along each axis
+        p[k % 6 == way, :, axis] = p[k % 6 == way, :1, axis] + rng.uniform(-0.01, 0.01, (50, 3))
+    p[k % 6 == 4, 2, :2] = p[k % 6 == 4, :2, :2].mean(1) + rng.uniform(-0.02, 0.02, (50, 2))  # diagonal slivers
+    s.positions = p.reshape(-1, 3).astype(np.float32)
+    if not perspective:
+        s = dataclasses.replace(s, perspective=False, slope=2.0)
+    run_case(ctx, s, f"{w}x{h}")
