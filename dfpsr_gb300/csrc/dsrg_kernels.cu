@@ -1591,8 +1591,7 @@ __device__ __forceinline__ uint32_t warp_tile_threshold(const unsigned long long
 			m = min(m, max(keyHi, initialHi));
 		}
 	}
-	for (int o = 16; o > 0; o >>= 1) m = min(m, __shfl_xor_sync(0xFFFFFFFFu, m, o));
-	return m;
+	return __reduce_min_sync(0xFFFFFFFFu, m);
 }
 
 // Largest key hi any fragment of the record can have inside the tile (plane_hi over the pixels of
@@ -1890,16 +1889,23 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) raster_kernel(BatchPa
 			uint32_t largeMask = __ballot_sync(0xFFFFFFFFu, valid && !culled);
 			int sinceRefresh = 0;
 			while (largeMask) {
-				const int src = __ffs(largeMask) - 1;
-				largeMask &= largeMask - 1;
+				int src = __ffs(largeMask) - 1;
 				if (cull) {
-					// the threshold only rises while the tile is drawn: refresh it every few records
-					if (++sinceRefresh == 4) {
+					// the threshold only rises while the tile is drawn: refresh it every few records (8: against
+					// 4, a batch of 32 mixed frames takes 4.03 ms instead of 4.16; 1 costs more than it culls)
+					if (++sinceRefresh == 8) {
 						sinceRefresh = 0;
 						tileMin = max(tileFloor, warp_tile_threshold(keys, initialDepth, lane, validW, validH, affine));
 					}
-					if (__shfl_sync(0xFFFFFFFFu, myBest, src) < tileMin) continue;
+					// nearest first, until the nearest one left is below the threshold: what is drawn early hides
+					// what would have come before it in the list (277 us of a frame of 20,000 random triangles
+					// were 250 with the list's order and spans while binning, and are 231 in this order)
+					const bool left = (largeMask >> lane & 1u) != 0u;
+					const uint32_t nearest = __reduce_max_sync(0xFFFFFFFFu, left ? myBest : 0u);
+					if (nearest < tileMin) break;
+					src = __ffs(__ballot_sync(0xFFFFFFFFu, left && myBest == nearest)) - 1;
 				}
+				largeMask &= ~(1u << src);
 				const uint32_t ri = __shfl_sync(0xFFFFFFFFu, myRecord, src);
 				const DrawRecord r = records[record_slot(b, ri)];
 				// every lane reads one of the tile's 16 rows (lanes 16..31 repeat 0..15)
