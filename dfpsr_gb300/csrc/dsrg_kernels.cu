@@ -1662,35 +1662,97 @@ __device__ __forceinline__ void resolve_pixel(const BatchParams &b, const FrameT
 	write_lane(b, f, r, pair, y1, x, lane4, px, py, affine);
 }
 
-// The winner of pixel (px, py) when all four pixels of its 2x2 quad have that winner, evaluated by
-// the four lanes of the quad together (lanes 4q..4q+3 of `quadLanes` hold quad q, lane l4 its
-// position): each lane computes the running sums of its own position only (quad_lane), and the
-// vertex weights of positions 0..2, which every position's mip level needs, come from the other
-// lanes by shuffles.  The values are those of resolve_pixel; the quad's sums are evaluated once
-// instead of four times.
-__device__ __forceinline__ void resolve_shared_quad(const BatchParams &b, const FrameTarget &f, const DrawRecord *__restrict__ records,
-                                                    const uint32_t *__restrict__ rows, int32_t px, int32_t py, unsigned long long key, int l4, unsigned quadLanes) {
+// The winners of the eight quads that a warp holds (lanes 4q..4q+3 the positions of quad q), shaded and
+// written; the values are those of resolve_pixel.  A pixel's mip level needs the vertex weights of
+// three positions of its quad besides its own.  Far from a triangle's left end the running sums are
+// most of what a pixel costs (up to 18 chains of additions when one lane evaluates its whole quad),
+// so there the quad's lanes work together: in each round they take one winner of their quad, every
+// lane evaluates the sums (quad_lane, up to 6 chains) and weights of its own position for it, and the
+// pixels with that winner collect the positions' weights by shuffles.  There are as many rounds as
+// the warp's most divided quad has winners.  One round is always the better way; of several, only
+// where the tile has large triangles (largeCount) and a pixel of the warp lies LONG_CHAIN from its
+// triangle's left bound: in meshes of small triangles the chains are short and the rounds' own work
+// costs more than they save.
+// 20,000 random triangles at 800x600: 228 us when every divided quad's pixels go alone, 204 with
+// rounds; 32 mixed frames 4.03 and 3.55 ms.  Limits of 16, 32, 64 and 128 pixels: the batch 3.59, 3.59,
+// 3.64 and 3.73 ms, the random triangles 206, 203, 210 and 216 us.
+// `key` 0: nothing to write.  All 32 lanes call it.
+static const int LONG_CHAIN = 32; // pixels from the record's left bound
+
+__device__ __forceinline__ void resolve_quads(const BatchParams &b, const FrameTarget &f, const DrawRecord *__restrict__ records,
+                                              const uint32_t *__restrict__ rows, int32_t px, int32_t py, unsigned long long key,
+                                              const uint32_t *largeCount) {
 	const bool depthTest = f.depth != nullptr, affine = f.affine != 0;
-	const DrawRecord r = records[record_slot(b, key_record(key, depthTest))];
+	const bool oddRow = odd_last_row(py, f.height);
+	const int lane = (int)(threadIdx.x & 31u), base = lane & ~3;
+	const bool mine = key != 0ull && !(oddRow && depthTest); // that row's depth-tested pixels are odd_row_kernel's
+	const uint32_t winner = mine ? key_record(key, depthTest) : 0u;
 	const int32_t y1 = py & ~1, x = px & ~1;
-	const RowPair pair = record_row_pair(r, rows, y1, f.height);
-	const float depthValue = quad_lane(r.start[0], r.dx[0], r.dy[0], pair, y1, x, l4);
-	if (f.color) {
-		float a, bw, c;
-		lane_weight(depthValue, quad_lane(r.start[1], r.dx[1], r.dy[1], pair, y1, x, l4),
-		            quad_lane(r.start[2], r.dx[2], r.dy[2], pair, y1, x, l4), affine, a, bw, c);
-		const int base = (int)(threadIdx.x & 31u) & ~3;
-		float wa[4], wb[4], wc[4];
-		for (int l = 0; l < 3; l++) {
-			wa[l] = __shfl_sync(quadLanes, a, base + l);
-			wb[l] = __shfl_sync(quadLanes, bw, base + l);
-			wc[l] = __shfl_sync(quadLanes, c, base + l);
+	float depthValue = 0.0f;
+	float wa[4], wb[4], wc[4]; // of positions 0..2, and of the pixel's own
+	const uint32_t drawn = __ballot_sync(0xFFFFFFFFu, mine);
+	bool first = mine; // no earlier position of the quad has the pixel's winner
+#pragma unroll
+	for (int l = 1; l < 4; l++) {
+		const int other = lane ^ l;
+		const uint32_t theirs = __shfl_sync(0xFFFFFFFFu, winner, other);
+		if (other < lane && (drawn >> other & 1u) && theirs == winner) first = false;
+	}
+	const int winners = __popc(__ballot_sync(0xFFFFFFFFu, first) >> base & 15u);
+	const DrawRecord &r = records[record_slot(b, winner)];
+	const uint32_t rounds = __reduce_max_sync(0xFFFFFFFFu, (uint32_t)winners);
+	const bool distant = rounds > 1u && *largeCount != 0u && __any_sync(0xFFFFFFFFu, mine && x - r.left >= LONG_CHAIN);
+	if (rounds > 1u && !distant) { // every pixel for itself
+		if (!mine) return;
+		const RowPair pair = record_row_pair(r, rows, y1, f.height);
+		float w[3][4];
+		const int components = f.color ? 3 : 1;
+		for (int c = 0; c < components; c++) quad_lanes(r.start[c], r.dx[c], r.dy[c], pair, y1, x, w[c]);
+		const int at = (lane & 3) | (oddRow && full_quad(pair, x) ? 2 : 0);
+		depthValue = pick4(w[0], at);
+		if (f.color) {
+			lane_weights(w, affine, wa, wb, wc);
+			wa[3] = pick4(wa, at); wb[3] = pick4(wb, at); wc[3] = pick4(wc, at);
 		}
-		wa[3] = a; wb[3] = bw; wc[3] = c; // position 3 reads only its own weights
+	} else {
+		bool waiting = mine;
+		for (;;) {
+			const uint32_t pending = __ballot_sync(0xFFFFFFFFu, waiting);
+			if (!pending) break;
+			const uint32_t quad = pending >> base & 15u;
+			const uint32_t round = __shfl_sync(0xFFFFFFFFu, winner, base + (quad ? __ffs(quad) - 1 : 0));
+			float z = 0.0f, a = 0.0f, bw = 0.0f, c = 0.0f;
+			int at = lane;
+			if (quad) {
+				const DrawRecord &t = records[record_slot(b, round)];
+				const RowPair pair = record_row_pair(t, rows, y1, f.height);
+				// without a depth buffer the last row of an odd height holds the lower lanes of full quads
+				if (oddRow && full_quad(pair, x)) at |= 2;
+				z = quad_lane(t.start[0], t.dx[0], t.dy[0], pair, y1, x, lane & 3);
+				if (f.color)
+					lane_weight(z, quad_lane(t.start[1], t.dx[1], t.dy[1], pair, y1, x, lane & 3),
+					            quad_lane(t.start[2], t.dx[2], t.dy[2], pair, y1, x, lane & 3), affine, a, bw, c);
+			}
+			const bool taken = waiting && winner == round;
+#pragma unroll
+			for (int l = 0; l < 4; l++) {
+				const int from = l < 3 ? base + l : at;
+				const float va = __shfl_sync(0xFFFFFFFFu, a, from), vb = __shfl_sync(0xFFFFFFFFu, bw, from);
+				const float vc = __shfl_sync(0xFFFFFFFFu, c, from);
+				if (taken) { wa[l] = va; wb[l] = vb; wc[l] = vc; }
+			}
+			if (taken) {
+				depthValue = z;
+				waiting = false;
+			}
+		}
+		if (!mine) return;
+	}
+	if (f.color) {
 		ShadeRecord shade;
 		make_shade(b.tasks[r.task], r.source, shade);
 		float rgba[4];
-		shade_lane_inline(shade, b.textures, wa, wb, wc, l4, rgba);
+		shade_lane_inline(shade, b.textures, wa, wb, wc, 3, rgba);
 		f.color[(size_t)py * f.colorStride + px] = pack_saturated(rgba, f.packOrder);
 	}
 	if (f.depth) f.depth[(size_t)py * f.depthStride + px] = depthValue;
@@ -2033,19 +2095,8 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) raster_kernel(BatchPa
 					f.depth[(size_t)py * f.depthStride + px] = depth_from_key(b, key, affine, records, rows, px, py);
 			}
 			if (!RESOLVE || DEPTH_ONLY_1X1) continue;
-			// the tile's winners shaded right away (resolve_pixels_kernel fused into the tile pass): a
-			// warp whose quads each have one winner (or none) shares each quad's sums among its lanes;
-			// other warps, and every quad touching the image's edge or an odd height's last row (whose
-			// missing pixels have no key), resolve pixel by pixel
-			const int same = key == __shfl_sync(0xFFFFFFFFu, key, lane & ~3) ? 1 : 0;
-			const bool quadSame = (same & __shfl_xor_sync(0xFFFFFFFFu, same, 1) & __shfl_xor_sync(0xFFFFFFFFu, same, 2) &
-			                       __shfl_xor_sync(0xFFFFFFFFu, same, 3)) != 0;
-			const unsigned drawn = __ballot_sync(0xFFFFFFFFu, key != 0ull);
-			if (__all_sync(0xFFFFFFFFu, quadSame || key == 0ull)) {
-				if (key != 0ull) resolve_shared_quad(b, f, records, rows, px, py, key, l4, drawn);
-			} else if (key != 0ull) {
-				resolve_pixel(b, f, records, rows, px, py, key);
-			}
+			// the tile's winners shaded right away (resolve_pixels_kernel fused into the tile pass)
+			if (__any_sync(0xFFFFFFFFu, key != 0ull)) resolve_quads(b, f, records, rows, px, py, key, &bins.cursors[2 * tile + 1]);
 		}
 		if (tid == 0 && fragmentSum) {
 			if (b.fragments) atomicAdd(b.fragments, fragmentSum);
