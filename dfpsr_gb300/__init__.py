@@ -360,17 +360,13 @@ class Context:
     def point_lights(lights):
         """A dsrg_point_light array from dicts with position, radius, intensity, color and optionally
         cube (cubeWidth*6 x cubeWidth floats)."""
-        arr = (PointLight * max(1, len(lights)))()
-        for i, l in enumerate(lights):
-            for k in range(3):
-                arr[i].position[k] = float(l["position"][k])
-                arr[i].color[k] = int(l["color"][k])
-            arr[i].radius = float(l["radius"])
-            arr[i].intensity = float(l["intensity"])
-            cube = l.get("cube")
-            arr[i].shadowCube = _ptr(cube) if cube is not None else None
-            arr[i].cubeWidth = int(cube.shape[1]) if cube is not None else 0
-        return arr
+        rows = []
+        for l in lights:
+            position, color, cube = l["position"], l["color"], l.get("cube")
+            rows.append(((float(position[0]), float(position[1]), float(position[2])), float(l["radius"]), float(l["intensity"]),
+                         (int(color[0]), int(color[1]), int(color[2])), _ptr(cube) if cube is not None else None,
+                         int(cube.shape[1]) if cube is not None else 0))
+        return (PointLight * max(1, len(rows)))(*rows)
 
     def light_points(self, view: "OrthoView", center, light, normal, height, lights, reference_threads: int = 0):
         """lights: dicts with position, radius, intensity, color and optionally cube (cubeWidth*6 x cubeWidth floats)."""
@@ -434,11 +430,21 @@ class Context:
     def dense_render_many(self, instances, view: "OrthoView", height, diffuse, normal, high_quality: bool = False):
         """instances: (DenseModel, origin, model_to_world) in drawing order, drawn as that many
         dense_render calls would draw them, in one call."""
-        arr = (DenseInstance * max(len(instances), 1))()
-        for i, (model, origin, transform) in enumerate(instances):
-            arr[i].model = model.handle
-            arr[i].originX, arr[i].originY = float(origin[0]), float(origin[1])
-            arr[i].modelToWorld[:] = [float(v) for v in np.asarray(transform, np.float32).reshape(12)]
+        # column by column: set value by value, the table of 64 instances took longer than drawing them
+        # (277 to 288 us a call, 218 this way)
+        table = np.zeros(max(len(instances), 1), DENSE_INSTANCE)
+        models, origins, transforms = [], [], []
+        for model, origin, transform in instances:
+            handle = model.handle
+            models.append(handle.value or 0 if handle else 0)
+            origins += (float(origin[0]), float(origin[1]))
+            transforms.append(np.asarray(transform, np.float32).reshape(12))
+        if models:
+            table["model"] = models
+            with np.errstate(over="ignore"):
+                table["origin"] = np.array(origins).reshape(-1, 2)
+            table["modelToWorld"] = np.concatenate(transforms).reshape(-1, 12)
+        arr = (DenseInstance * len(table)).from_buffer(table)
         hi, di, ni = image_struct(height), image_struct(diffuse), image_struct(normal)
         _torch_sync()
         self._check(self._l.dsrg_dense_render_many(self.handle, arr, len(instances), C.byref(view), C.byref(hi), C.byref(di),
@@ -471,6 +477,10 @@ class Context:
 
 class DenseInstance(C.Structure):
     _fields_ = [("model", C.c_void_p), ("originX", C.c_float), ("originY", C.c_float), ("modelToWorld", C.c_float * 12)]
+
+
+DENSE_INSTANCE = np.dtype([("model", np.uint64), ("origin", np.float32, 2), ("modelToWorld", np.float32, 12)])
+assert DENSE_INSTANCE.itemsize == C.sizeof(DenseInstance)
 
 
 class DenseModel:

@@ -7,6 +7,7 @@
 
 #include <cmath>
 #include <cstring>
+#include <functional>
 #include <string>
 #include <vector>
 
@@ -237,6 +238,7 @@ struct dsrg_context_s {
 	DeviceBuffer<unsigned long long> spriteKeys; // draw_higher's per-pixel keys and its sprite table, apart from the
 	DeviceBuffer<unsigned char> spriteTables;    // pipeline's, so that a sprite frame can draw sprites beside its shadows
 	cudaStream_t sideStream = nullptr;           // a sprite frame's second stream (created on first use)
+	std::function<void()> beforeWait;            // host work that the next batch does between queueing its launches and waiting for them
 	cudaStream_t branchStream = nullptr;         // a batch's second branch: the row intervals beside the tile lists
 	cudaEvent_t branchFork = nullptr, branchJoin = nullptr;
 	cudaEvent_t sideStart = nullptr, sideDone = nullptr;

@@ -357,6 +357,11 @@ static int enqueue_phases(dsrg_context ctx, BatchJob &job, BatchTotals &totals, 
 	if (ctx->counting)
 		TRY(cudaMemcpyAsync(ctx->pinnedReadback + 4, ctx->fragmentCounter.ptr, sizeof(unsigned long long), cudaMemcpyDeviceToHost,
 		                    stream));
+	if (ctx->beforeWait) { // once, also when the batch is redone
+		const std::function<void()> work = std::move(ctx->beforeWait);
+		ctx->beforeWait = nullptr;
+		work();
+	}
 	TRY(cudaStreamSynchronize(stream));
 	ctx->stopRecorded = true;
 	totals.records = ctx->pinnedReadback[0];
