@@ -143,14 +143,15 @@ __global__ void normals_kernel(DiffModel m, const float *__restrict__ modelToWor
 }
 
 // One thread per pixel of every view: the winning fragment's vertex weights, re-evaluated
-// exactly as the resolve pass does, then the float shading and the visibility buffer.
+// exactly as the resolve pass does, then the float shading and the visibility buffer.  No mip level
+// is chosen here, so only the pixel's own position of its quad is evaluated.
 __global__ void __launch_bounds__(256) diff_forward_kernel(BatchParams b, const DrawRecord *__restrict__ records,
                                                            const uint32_t *__restrict__ rows, const unsigned long long *__restrict__ keys, DiffModel m, DiffParams q,
                                                            int32_t width, int32_t height, uint64_t pixels, float4 *images,
                                                            uint32_t *visibility) {
 	for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < pixels; i += (uint64_t)gridDim.x * blockDim.x) {
 		const uint64_t hw = (uint64_t)width * height;
-		const uint32_t view = (uint32_t)(i / hw);
+		const uint32_t view = pixels <= 0xFFFFFFFFull ? (uint32_t)i / (uint32_t)hw : (uint32_t)(i / hw); // hw <= pixels
 		const uint32_t rem = (uint32_t)(i - (uint64_t)view * hw);
 		const int32_t py = (int32_t)(rem / (uint32_t)width), px = (int32_t)(rem - (uint32_t)py * (uint32_t)width);
 		const unsigned long long key = keys ? keys[i] : 0ull;
@@ -166,11 +167,9 @@ __global__ void __launch_bounds__(256) diff_forward_kernel(BatchParams b, const 
 		const int32_t y1 = py & ~1, x = px & ~1;
 		const int lane4 = ((py & 1) << 1) | (px & 1);
 		const RowPair pair = record_row_pair(r, rows, y1, height);
-		float w[3][4], wa[4], wb[4], wc[4];
-		for (int c = 0; c < 3; c++) quad_lanes(r.start[c], r.dx[c], r.dy[c], pair, y1, x, w[c]);
-		lane_weights(w, affine, wa, wb, wc);
-		const float pb = lane4 == 0 ? wb[0] : lane4 == 1 ? wb[1] : lane4 == 2 ? wb[2] : wb[3];
-		const float pc = lane4 == 0 ? wc[0] : lane4 == 1 ? wc[1] : lane4 == 2 ? wc[2] : wc[3];
+		float pa, pb, pc;
+		lane_weight(quad_lane(r.start[0], r.dx[0], r.dy[0], pair, y1, x, lane4), quad_lane(r.start[1], r.dx[1], r.dy[1], pair, y1, x, lane4),
+		            quad_lane(r.start[2], r.dx[2], r.dy[2], pair, y1, x, lane4), affine, pa, pb, pc);
 		PixelShade s;
 		shade_pixel(m, q, r.tri, pb, pc, s);
 		images[i] = make_float4(fmul(fmul(s.texel.x, s.vertex.x), s.light), fmul(fmul(s.texel.y, s.vertex.y), s.light),
@@ -187,7 +186,19 @@ __global__ void l2_loss_kernel(const float *__restrict__ images, const float *__
                                float scale, float *blockSums) {
 	__shared__ float partial[8];
 	float sum = 0.0f;
-	for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < count; i += (uint64_t)gridDim.x * blockDim.x) {
+	// bound by memory: four values at a time where the three arrays are aligned for it (64 views of
+	// 256x256: 41 -> 28 us, 7.1 TB/s of the 201 MB read and written)
+	const bool vector = (((uintptr_t)images | (uintptr_t)targets | (uintptr_t)grad) & 15u) == 0;
+	const uint64_t fours = vector ? count >> 2 : 0u;
+	const uint64_t first = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x, stride = (uint64_t)gridDim.x * blockDim.x;
+	for (uint64_t i = first; i < fours; i += stride) {
+		const float4 a = reinterpret_cast<const float4 *>(images)[i], t = reinterpret_cast<const float4 *>(targets)[i];
+		const float4 d = make_float4(a.x - t.x, a.y - t.y, a.z - t.z, a.w - t.w);
+		reinterpret_cast<float4 *>(grad)[i] = make_float4(fmul(fmul(2.0f, d.x), scale), fmul(fmul(2.0f, d.y), scale),
+		                                                  fmul(fmul(2.0f, d.z), scale), fmul(fmul(2.0f, d.w), scale));
+		sum = fadd(sum, fadd(fadd(fmul(d.x, d.x), fmul(d.y, d.y)), fadd(fmul(d.z, d.z), fmul(d.w, d.w))));
+	}
+	for (uint64_t i = 4u * fours + first; i < count; i += stride) {
 		const float d = images[i] - targets[i];
 		grad[i] = fmul(fmul(2.0f, d), scale);
 		sum = fadd(sum, fmul(d, d));
@@ -225,22 +236,23 @@ __global__ void fixed_order_sum_kernel(const float *blockSums, int32_t blocks, i
 // Adds `value` to base[key] (a float4) once per run of consecutive lanes holding the same key:
 // a segmented scan over the run (shuffles up, only within the run) and one vector atomic from
 // its last lane.  Consecutive pixels mostly share their triangle's corners and often a texel, so
-// runs catch nearly all repeats; equal keys in separate runs each add their own sum.
+// runs catch nearly all repeats; equal keys in separate runs each add their own sum.  The scan goes
+// as far as the warp's longest run, which in fine meshes is a few pixels, and warps of empty pixels skip
+// it: 64 views of 256x256 took 125 us and take 81.
 __device__ __forceinline__ void warp_run_add(float4 *base, uint32_t key, float4 value, bool active) {
 	const uint32_t k = active ? key : 0xFFFFFFFFu;
 	const int lane = threadIdx.x & 31;
 	const uint32_t previous = __shfl_up_sync(0xFFFFFFFFu, k, 1);
-	const bool head = lane == 0 || previous != k;
+	const bool head = lane == 0 || previous != k || !active;
 	const uint32_t heads = __ballot_sync(0xFFFFFFFFu, head);
 	const int start = 31 - __clz(heads & (0xFFFFFFFFu >> (31 - lane))); // this lane's run begins here
-	if (heads != 0xFFFFFFFFu) { // some run holds more than one lane
-		for (int d = 1; d < 32; d <<= 1) {
-			const float ox = __shfl_up_sync(0xFFFFFFFFu, value.x, d), oy = __shfl_up_sync(0xFFFFFFFFu, value.y, d);
-			const float oz = __shfl_up_sync(0xFFFFFFFFu, value.z, d), ow = __shfl_up_sync(0xFFFFFFFFu, value.w, d);
-			if (lane - d >= start) {
-				value.x = fadd(value.x, ox); value.y = fadd(value.y, oy);
-				value.z = fadd(value.z, oz); value.w = fadd(value.w, ow);
-			}
+	const int longest = (int)__reduce_max_sync(0xFFFFFFFFu, (uint32_t)(lane - start));
+	for (int d = 1; d <= longest; d <<= 1) {
+		const float ox = __shfl_up_sync(0xFFFFFFFFu, value.x, d), oy = __shfl_up_sync(0xFFFFFFFFu, value.y, d);
+		const float oz = __shfl_up_sync(0xFFFFFFFFu, value.z, d), ow = __shfl_up_sync(0xFFFFFFFFu, value.w, d);
+		if (lane - d >= start) {
+			value.x = fadd(value.x, ox); value.y = fadd(value.y, oy);
+			value.z = fadd(value.z, oz); value.w = fadd(value.w, ow);
 		}
 	}
 	const bool last = lane == 31 || ((heads >> (lane + 1)) & 1u) != 0;
@@ -264,9 +276,10 @@ struct PixelGrad {
 };
 
 __device__ __forceinline__ bool pixel_gradient(const DiffModel &m, const DiffParams &q, const uint32_t *visibility, uint64_t i,
-                                               float4 g, PixelShade &s, PixelGrad &out) {
+                                               const float4 *__restrict__ grad, PixelShade &s, PixelGrad &out) {
 	const uint32_t tri = visibility[i * 3];
 	if (tri >= (uint32_t)m.triangleCount) return false; // uncovered (or not a triangle of this model)
+	const float4 g = grad[i];
 	shade_pixel(m, q, tri, bitsf(visibility[i * 3 + 1]), bitsf(visibility[i * 3 + 2]), s);
 	// d out / d texel: vertex colour times light (alpha unlit)
 	const float4 gt = make_float4(fmul(fmul(g.x, s.vertex.x), s.light), fmul(fmul(g.y, s.vertex.y), s.light),
@@ -318,7 +331,8 @@ __global__ void __launch_bounds__(256) adjoint_atomic_kernel(DiffModel m, DiffPa
 		const uint64_t i = base + threadIdx.x;
 		PixelShade s;
 		PixelGrad pg;
-		const bool active = i < pixels && pixel_gradient(m, q, visibility, i, grad[i < pixels ? i : 0], s, pg);
+		const bool active = i < pixels && pixel_gradient(m, q, visibility, i, grad, s, pg);
+		if (!__any_sync(0xFFFFFFFFu, active)) continue;
 		for (int k = 0; k < 4; k++) warp_run_add(gradTexture, active ? s.taps[k] : 0u, pg.tex[k], active);
 		for (int c = 0; c < 3; c++) warp_run_add(gradVertex, active ? (uint32_t)s.point[c] : 0u, pg.vertex[c], active);
 		if (active)
@@ -338,7 +352,7 @@ __global__ void __launch_bounds__(256) adjoint_emit_kernel(DiffModel m, DiffPara
 		if (i >= pixels) continue;
 		PixelShade s;
 		PixelGrad pg;
-		const bool active = pixel_gradient(m, q, visibility, i, grad[i], s, pg);
+		const bool active = pixel_gradient(m, q, visibility, i, grad, s, pg);
 		for (int k = 0; k < 4; k++) {
 			sums.texKeys[i * 4 + k] = active ? s.taps[k] : sums.texKeyEnd;
 			if (!active) continue;

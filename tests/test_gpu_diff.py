@@ -210,3 +210,27 @@ def test_deterministic_sums_of_any_size(ctx, views, width, height, major, minor,
         assert np.array_equal(sums[name].view(np.uint32), again[name].view(np.uint32)), name
         a, b = atomic[name].astype(np.float64), sums[name].astype(np.float64)
         assert np.linalg.norm(a) > 0 and np.linalg.norm(a - b) < 1.2e-4 * np.linalg.norm(a), name
+
+
+@pytest.mark.parametrize("count", [1, 3, 4, 5, 1023, 700001])
+@pytest.mark.parametrize("shift", [(0, 0, 0), (1, 0, 0), (0, 0, 3)])
+def test_l2_loss_of_any_length_and_alignment(ctx, count, shift):
+    """Arrays at 16-byte addresses are read four values at a time, with a remainder; others singly.
+    The gradient is exact; the sum of n squares loses at most a rounding per addition in a row (a
+    thread has under 8 values, then 5 + 8 + 18 levels of sums): 40 x 2^-24 of it, plus the squares' own."""
+    import torch
+    from diff_harness import make_renderer
+    _, renderer, _, _ = make_renderer(ctx, small_problem())
+    rng = np.random.default_rng(count)
+    a, t = (rng.uniform(-1.0, 2.0, count).astype(np.float32) for _ in range(2))
+    held = [torch.zeros(count + 4, device="cuda") for _ in range(3)]
+    images, targets, grad = (h[s:s + count] for h, s in zip(held, shift))
+    images.copy_(torch.tensor(a))
+    targets.copy_(torch.tensor(t))
+    loss = torch.empty(1, device="cuda")
+    renderer.l2_loss(images, targets, grad, loss)
+    d = a - t
+    assert np.array_equal(grad.cpu().numpy(), np.float32(2.0) * d * (np.float32(1.0) / np.float32(count)))
+    exact = np.sum(d.astype(np.float64) ** 2) / count
+    assert abs(float(loss) - exact) <= 45 * 2.0**-24 * exact
+    assert not held[2][:shift[2]].any() and not held[2][shift[2] + count:].any()  # nothing written outside
