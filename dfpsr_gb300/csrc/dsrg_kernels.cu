@@ -1265,7 +1265,7 @@ __device__ __forceinline__ uint32_t plane_hi(float s, float dx, float dy, float 
 // hundreds or thousands: of the 1.07 M entries of 20,000 random triangles at 800x600, which the tile
 // kernel fetched and rejected one by one, about 62,000 are listed and a frame takes 277 us instead of
 // 375; a batch of 32 mixed frames 8.7 ms instead of 10.4.
-static const int BIG_GROUP = 16;
+static const int BIG_GROUP = 32;
 static const int BIG_WARPS = 8; // warps of a block
 
 struct BigEdge {
@@ -1338,8 +1338,12 @@ __device__ __forceinline__ void bin_big(const BatchParams &b, const DrawRecord *
 	const uint32_t count = *bins.bigCount;
 	const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
 	const uint32_t upTo = 0xFFFFFFFFu >> (31u - lane); // this lane and those before
-	for (uint32_t first = blockIdx.x * BIG_GROUP; first < count; first += gridDim.x * BIG_GROUP) { // uniform per block
-		const uint32_t taken = min((uint32_t)BIG_GROUP, count - first);
+	// two groups per block where that leaves a group 8 to BIG_GROUP records: fewer barriers per record where
+	// there are many (32 mixed frames: groups of 8, 16 and 32 take 3.73, 3.58 and 3.52 ms), more blocks at
+	// work where there are few (20,000 random triangles: 205, 211 and 213 us)
+	const uint32_t group = min(max(count / (gridDim.x * 2u), 8u), (uint32_t)BIG_GROUP);
+	for (uint32_t first = blockIdx.x * group; first < count; first += gridDim.x * group) { // uniform per block
+		const uint32_t taken = min(group, count - first);
 		if (threadIdx.x < BIG_GROUP * 4) {
 			const uint32_t q = threadIdx.x >> 2, role = threadIdx.x & 3u;
 			bool wrapped = false; // an edge whose test is not exact
