@@ -133,9 +133,11 @@ DSRG_HD_CALL float chain_add(float s, float d, int32_t n) {
 		const float lo = bitsf(exponent), a = bitsf(b2 & 0x7FFFFFFFu), step = bitsf(fbits(inc) & 0x7FFFFFFFu);
 		const bool up = ((fbits(inc) ^ b2) >> 31) == 0u;
 		// Steps left in the binade: the value after k of them keeps one increment's distance from its
-		// end when k <= room / step - 1.  The estimate is less than 4 off (2 ulp of a quotient below 2^23).
+		// end when k <= room / step - 1.  The estimate is 2 ulp off: less than 4 for a quotient below 2^23,
+		// less than 1/8 below 2^18.
 		const float room = up ? fsub(fadd(lo, lo), a) : fsub(a, lo);
-		int32_t k = (int32_t)fdiv_estimate(room, step) - 5;
+		const float steps = fdiv_estimate(room, step);
+		int32_t k = (int32_t)steps - (steps < 262144.0f ? 2 : 5);
 		k = k < n ? k : n;
 		if (k > 0) {
 			s = fadd(s2, fmul((float)k, inc));
