@@ -1263,8 +1263,10 @@ __device__ __forceinline__ uint32_t plane_hi(float s, float dx, float dy, float 
 // differs from run to run.  Every pixel of the tile then holds a better key than a record left out
 // could give.  Scenes of large triangles drawn over one another keep a few entries per tile of
 // hundreds or thousands: of the 1.07 M entries of 20,000 random triangles at 800x600, which the tile
-// kernel fetched and rejected one by one, about 62,000 are listed and a frame takes 277 us instead of
-// 375; a batch of 32 mixed frames 8.7 ms instead of 10.4.
+// kernel fetched and rejected one by one, about 62,000 are listed (frame 375 -> 277 us, a batch of 32 mixed
+// frames 10.4 -> 8.7 ms).  With every tile of a bound tested by itself and culling in the fill pass
+// only, the batch's two passes took 970 and 940 us; they take 350 and 320 (frame 277 -> 250 us, batch
+// 5.73 -> 4.72 ms).
 static const int BIG_GROUP = 32;
 static const int BIG_WARPS = 8; // warps of a block
 
@@ -1964,8 +1966,8 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) raster_kernel(BatchPa
 						tileMin = max(tileFloor, warp_tile_threshold(keys, initialDepth, lane, validW, validH, affine));
 					}
 					// nearest first, until the nearest one left is below the threshold: what is drawn early hides
-					// what would have come before it in the list (277 us of a frame of 20,000 random triangles
-					// were 250 with the list's order and spans while binning, and are 231 in this order)
+					// what would have come before it in the list (a frame of 20,000 random triangles took
+					// 250 us in the list's order and 231 in this one, 32 mixed frames 4.72 and 4.07 ms)
 					const bool left = (largeMask >> lane & 1u) != 0u;
 					const uint32_t nearest = __reduce_max_sync(0xFFFFFFFFu, left ? myBest : 0u);
 					if (nearest < tileMin) break;
@@ -2549,7 +2551,7 @@ __device__ __forceinline__ void alpha_count(const uint32_t *__restrict__ lists, 
 // work on different records at the same time, and the four lanes of a quad evaluate one position
 // each and share the weights by shuffles.  What bounds it is instruction issue, and most records of a
 // tile (small particles) cover a small part of it: when the whole warp walked every record of the
-// tile, each lane evaluating the four positions of its quad, a frame of 3,000 particles over a
+// tile, each lane evaluating the four positions of its quad, a frame of 1,500 particles over a
 // 1281x719 image spent 474 us here and 160 us in four global sorting passes before it; it now
 // takes 140 us in all (frame 834 -> 358 us).
 __global__ void __launch_bounds__(256) alpha_kernel(BatchParams b, const DrawRecord *__restrict__ records, TileBins bins,
