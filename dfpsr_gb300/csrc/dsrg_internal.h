@@ -174,7 +174,7 @@ struct PhaseGraph {
 };
 
 // Words of a context's control buffer, all zeroed by a batch's first launch.
-enum ControlWord : uint32_t { CONTROL_TILE_QUEUE = 0, CONTROL_ERROR = 1, CONTROL_EMIT = 2, CONTROL_BIG_RECORDS = 5, CONTROL_LISTED_TILES = 6, CONTROL_TILE_PARTS = 7, CONTROL_WIRE_LINES = 8, CONTROL_WORDS = 9 };
+enum ControlWord : uint32_t { CONTROL_TILE_QUEUE = 0, CONTROL_ERROR = 1, CONTROL_EMIT = 2, CONTROL_BIG_RECORDS = 5, CONTROL_LISTED_TILES = 6, CONTROL_TILE_PARTS = 7, CONTROL_WIRE_LINES = 8, CONTROL_CULLED = 9, CONTROL_WORDS = 10 };
 static_assert(CONTROL_BIG_RECORDS == CONTROL_EMIT + EMIT_COUNTERS, "control words");
 
 struct BatchTotals {
@@ -212,7 +212,7 @@ struct dsrg_context_s {
 	DeviceBuffer<uint32_t> control;      // a batch's counters (ControlWord)
 	DeviceBuffer<uint4> tileList;        // the tiles of a batch that have tile-list entries
 	uint32_t *pinnedReadback = nullptr;  // page-locked: the gathered totals (written there by the GPU), the fragment count,
-	                                     // [9] TOTALS_EXTRAS
+	                                     // [9] TOTALS_EXTRAS, [10] TOTALS_CULLED
 	uint32_t *readbackDevice = nullptr;  // its device address
 	bool timingPending = false;          // stats' times not yet read from the events of the last call
 	bool timingHasRaster = false;

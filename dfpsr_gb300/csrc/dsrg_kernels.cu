@@ -732,6 +732,7 @@ __global__ void gather_totals_kernel(BatchParams b, TotalsSources from, TileBins
 		out[2] = binOffsets[2 * tiles];
 		out[3] = (uint32_t)*from.errorFlag;
 		out[TOTALS_EXTRAS] = from.extras ? *from.extras : 0u;
+		out[TOTALS_CULLED] = from.culled ? *from.culled : 0u;
 	}
 	const uint32_t lane = threadIdx.x & 31u;
 	if (bins.parts) {
@@ -1254,13 +1255,14 @@ __device__ __forceinline__ uint32_t plane_hi(float s, float dx, float dy, float 
 // covered by the record completely (the growth by two pixels also keeps clear of the column where
 // the reference's truncating division rejects a pixel that is inside).  The row's value is exact; the
 // crossing is a binary32 quotient (four roundings, under 2^-21 of itself) widened by 2^-20 of itself
-// and 2^-10 of a tile, towards listing a tile too many and towards covering one too few.
+// and 2^-10 of a tile: towards a tile too many to list, which the exact value at that tile then settles,
+// and towards covering one too few.
 //
 // Culling while binning: the count pass raises a tile's threshold to the worst key (plane_hi) of
 // each record that covers it completely and leaves out a large record whose best key does not reach
 // the threshold so far.  The fill pass runs when every record has been counted and tests against the
 // final threshold, so what it lists was counted, whatever the order; the count is an upper bound that
-// differs from run to run.  Every pixel of the tile then holds a better key than a record left out
+// differs from run to run.  (The pairs left out are counted apart, for the statistics.)  Every pixel of the tile then holds a better key than a record left out
 // could give.  Scenes of large triangles drawn over one another keep a few entries per tile of
 // hundreds or thousands: of the 1.07 M entries of 20,000 random triangles at 800x600, which the tile
 // kernel fetched and rejected one by one, about 62,000 are listed (frame 375 -> 277 us, a batch of 32 mixed
@@ -1271,7 +1273,7 @@ static const int BIG_GROUP = 32;
 static const int BIG_WARPS = 8; // warps of a block
 
 struct BigEdge {
-	long long base, stepY, full;
+	long long base, stepX, stepY, full;
 	float recip; // 1 / stepX
 	int32_t side; // sign of stepX
 };
@@ -1322,10 +1324,12 @@ __device__ __forceinline__ void big_row_columns(const BigRecord &h, int32_t ty, 
 		const float mo = __fadd_rn(__fmul_rn(fabsf(qo), 9.5367431640625e-7f), 9.765625e-4f);
 		const float mi = __fadd_rn(__fmul_rn(fabsf(qi), 9.5367431640625e-7f), 9.765625e-4f);
 		if (edge.side > 0) {
-			hi = min(hi, __float2int_rd(__fadd_rn(qo, mo)));
+			const int32_t x = max(__float2int_rd(__fadd_rn(qo, mo)), -1);
+			if (x <= hi) hi = outer + x * edge.stepX > 0 ? x - 1 : x;
 			ch = min(ch, __float2int_rd(__fsub_rn(qi, mi)));
 		} else {
-			lo = max(lo, __float2int_ru(__fsub_rn(qo, mo)));
+			const int32_t x = min(__float2int_ru(__fsub_rn(qo, mo)), h.tx1 + 1);
+			if (x >= lo) lo = outer + x * edge.stepX > 0 ? x + 1 : x;
 			cl = max(cl, __float2int_ru(__fadd_rn(qi, mi)));
 		}
 	}
@@ -1344,6 +1348,7 @@ __device__ __forceinline__ void bin_big(const BatchParams &b, const DrawRecord *
 	// there are many (32 mixed frames: groups of 8, 16 and 32 take 3.73, 3.58 and 3.52 ms), more blocks at
 	// work where there are few (20,000 random triangles: 205, 211 and 213 us)
 	const uint32_t group = min(max(count / (gridDim.x * 2u), 8u), (uint32_t)BIG_GROUP);
+	uint32_t culled = 0;
 	for (uint32_t first = blockIdx.x * group; first < count; first += gridDim.x * group) { // uniform per block
 		const uint32_t taken = min(group, count - first);
 		if (threadIdx.x < BIG_GROUP * 4) {
@@ -1361,6 +1366,7 @@ __device__ __forceinline__ void bin_big(const BatchParams &b, const DrawRecord *
 					const long long y = 128 + 256 * (long long)(e.ny >= 0 ? -2 : TILE_H + 1);
 					BigEdge &edge = h.edge[role];
 					edge.base = (x - e.sx) * e.nx + (y - e.sy) * e.ny - e.threshold;
+					edge.stepX = 256 * TILE_W * (long long)e.nx;
 					edge.stepY = 256 * TILE_H * (long long)e.ny;
 					edge.full = 256 * (TILE_W + 3) * (long long)(e.nx >= 0 ? e.nx : -e.nx) + 256 * (TILE_H + 3) * (long long)(e.ny >= 0 ? e.ny : -e.ny);
 					edge.side = e.nx > 0 ? 1 : (e.nx < 0 ? -1 : 0);
@@ -1451,7 +1457,10 @@ __device__ __forceinline__ void bin_big(const BatchParams &b, const DrawRecord *
 					const uint32_t best =
 						plane_hi<true>(h.start, h.dx, h.dy, h.margin, max(px0, h.left), min(px0 + TILE_W, h.right) - 1, max(py0, h.top),
 						               min(py0 + TILE_H, h.bottom) - 1, h.affine != 0);
-					if (best < bins.thresholds[tile]) continue;
+					if (best < bins.thresholds[tile]) {
+						culled++;
+						continue;
+					}
 				}
 				if (!FILL) {
 					atomicAdd(&bins.counts[slotOf], 1u);
@@ -1468,6 +1477,15 @@ __device__ __forceinline__ void bin_big(const BatchParams &b, const DrawRecord *
 			__syncwarp(); // the rows are done with before the next ones are written
 		}
 		__syncthreads(); // the group is done with before the next one is loaded
+	}
+	if (!FILL && bins.culled && blockIdx.x * group < count) { // uniform per block: one that had a group
+		culled = __reduce_add_sync(0xFFFFFFFFu, culled);
+		if (lane == 0) firstRow[warp] = (int32_t)culled;
+		__syncthreads();
+		if (threadIdx.x == 0) {
+			for (int w = 1; w < BIG_WARPS; w++) culled += (uint32_t)firstRow[w];
+			if (culled) atomicAdd(bins.culled, culled);
+		}
 	}
 }
 

@@ -154,6 +154,7 @@ struct TileBins {
 	// per tile: a key (upper word) that every pixel of the tile reaches, from the big records covering it
 	// completely; large records below it are not listed.  null: nothing is culled while binning
 	uint32_t *thresholds;
+	uint32_t *culled; // (tile, record) pairs left out of the count; null: nothing is culled
 	// tiles weighing more than partWeight as (tile, part) items, and per tile the parts done; null: every
 	// tile is drawn by one CTA
 	uint2 *parts;
@@ -251,10 +252,10 @@ void launch_wire_lines(const DrawRecord *records, const uint16_t *drawn, uint32_
 void launch_draw_lines(uint32_t *image, int32_t stride, int32_t width, int32_t height, const int4 *lines, uint32_t count,
                        uint32_t color, cudaStream_t stream);
 // out[0..3] = record count, row count, tile-list entry count, error bits of a batch, and the extra
-// slots at out[TOTALS_EXTRAS].
-static const uint32_t TOTALS_EXTRAS = 9;
+// slots at out[TOTALS_EXTRAS], the pairs that binning culled before counting at out[TOTALS_CULLED].
+static const uint32_t TOTALS_EXTRAS = 9, TOTALS_CULLED = 10;
 struct TotalsSources {
-	const uint32_t *records, *rows, *extras;
+	const uint32_t *records, *rows, *extras, *culled;
 	const uint32_t *rowOffsets;   // the two-pass setup: the row count is rowOffsets[records]
 	uint32_t recordCapacity;
 	const int32_t *errorFlag;

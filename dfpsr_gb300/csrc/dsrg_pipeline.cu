@@ -211,7 +211,7 @@ static int enqueue_phases(dsrg_context ctx, BatchJob &job, BatchTotals &totals, 
 	const uint32_t recordCap = onePass ? (uint32_t)(nt + std::max<uint64_t>(ctx->extraCapacity, nt / 8 + 1024))
 	                                   : (uint32_t)std::max<uint64_t>(ctx->recordCapacity, nt + nt / 8 + 1024);
 	const uint32_t rowCap = (uint32_t)std::max<uint64_t>(ctx->rowCapacity, (uint64_t)recordCap * 4);
-	const uint32_t binCap = (uint32_t)std::max<uint64_t>(ctx->binCapacity, (uint64_t)recordCap * 2);
+	const uint32_t binCap = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(ctx->binCapacity, (uint64_t)recordCap * 2), 0xFFFFFFF0u);
 	TRY(ctx->pointCsis.reserve(np)); TRY(ctx->pointIsyOut.reserve(np)); TRY(ctx->pointFlat.reserve(np));
 	TRY(ctx->records.reserve((size_t)recordCap + 1));
 	if (onePass) {
@@ -283,6 +283,7 @@ static int enqueue_phases(dsrg_context ctx, BatchJob &job, BatchTotals &totals, 
 	// records are culled while binning where only the best key of a pixel counts: not where every
 	// fragment is counted, nor for the alpha filter, which blends them all
 	bins.thresholds = (job.alpha || params.fragments) ? nullptr : ctx->binThresholds.ptr;
+	bins.culled = bins.thresholds ? ctx->control.ptr + CONTROL_CULLED : nullptr;
 	if (!job.alpha) {
 		bins.parts = ctx->tileParts.ptr;
 		bins.partCount = ctx->control.ptr + CONTROL_TILE_PARTS;
@@ -303,6 +304,7 @@ static int enqueue_phases(dsrg_context ctx, BatchJob &job, BatchTotals &totals, 
 	from.records = fb.recordCountDevice;
 	from.rows = onePass ? fb.emit.counters + EMIT_ROWS : nullptr;
 	from.extras = onePass ? fb.emit.counters + EMIT_EXTRAS : nullptr;
+	from.culled = ctx->control.ptr + CONTROL_CULLED;
 	from.rowOffsets = fb.rowOffsets;
 	from.recordCapacity = recordCap;
 	from.errorFlag = fb.errorFlag;
@@ -366,7 +368,8 @@ static int enqueue_phases(dsrg_context ctx, BatchJob &job, BatchTotals &totals, 
 	ctx->stopRecorded = true;
 	totals.records = ctx->pinnedReadback[0];
 	totals.rows = ctx->pinnedReadback[1];
-	totals.binEntries = ctx->pinnedReadback[2];
+	const uint32_t counted = ctx->pinnedReadback[2]; // the tile lists' entries
+	totals.binEntries = counted + ctx->pinnedReadback[TOTALS_CULLED];
 	const uint32_t errorBits = ctx->pinnedReadback[3];
 	if (errorBits & ERROR_OVERFLOW_BITS) {
 		// the capacities the totals ask for; a total counted past an overflowed buffer is a lower bound
@@ -376,7 +379,10 @@ static int enqueue_phases(dsrg_context ctx, BatchJob &job, BatchTotals &totals, 
 		else ctx->recordCapacity = std::max<uint64_t>(ctx->recordCapacity, (uint64_t)totals.records + totals.records / 4 + 1024);
 		if (!recordsOver) {
 			ctx->rowCapacity = std::max<uint64_t>(ctx->rowCapacity, (uint64_t)totals.rows + totals.rows / 4 + 1024);
-			ctx->binCapacity = std::max<uint64_t>(ctx->binCapacity, (uint64_t)totals.binEntries + totals.binEntries / 4 + 1024);
+			// the entries counted depend on how early the tiles' thresholds rose (bin_big_kernel), by a third from
+			// run to run for 20,000 random triangles at 800x600: twice the total, so that a frame that has
+			// been drawn once is not redone for it
+			ctx->binCapacity = std::max<uint64_t>(ctx->binCapacity, (uint64_t)counted * 2 + 1024);
 		}
 		return DSRG_RETRY;
 	}

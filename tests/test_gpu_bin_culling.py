@@ -113,3 +113,21 @@ def test_slivers_over_many_tiles(ctx, w, h, perspective):
     if not perspective:
         s = dataclasses.replace(s, perspective=False, slope=2.0)
     run_case(ctx, s, f"{w}x{h}")
+
+
+def test_statistics_count_every_pair_whatever_is_culled(ctx):
+    """binEntries counts the pairs of tiles and triangles that touch them, culled ones too, and is the same
+    from run to run; with fragments counted nothing is culled and it is the same again."""
+    import dfpsr_gb300 as d
+    s = _layers(257, 131, 500, seed=3, tilt=0.3, perspective=True)
+    seen = set()
+    for _ in range(4):
+        d.render_scene(ctx, s)
+        seen.add(ctx.stats()["bin_entries"])
+    ctx.set_counting(True)
+    try:
+        d.render_scene(ctx, s)
+        seen.add(ctx.stats()["bin_entries"])
+    finally:
+        ctx.set_counting(False)
+    assert len(seen) == 1 and seen.pop() > 500
