@@ -92,8 +92,7 @@ int dsrg_context_destroy(dsrg_context ctx) {
 	DeviceBuffer<float> *fbufs[] = {&ctx->stagingDepth};
 	for (auto *b : fbufs) b->release();
 	ctx->pointCsis.release(); ctx->pointIsyOut.release(); ctx->pointFlat.release();
-	DeviceBuffer<uint32_t> *ubufs[] = {&ctx->triCounts, &ctx->triOffsets, &ctx->scanScratch, &ctx->control, &ctx->binCounts,
-	                                   &ctx->binOffsets, &ctx->binCursors, &ctx->binLists, &ctx->stagingColor};
+	DeviceBuffer<uint32_t> *ubufs[] = {&ctx->triCounts, &ctx->triOffsets, &ctx->scanScratch, &ctx->control, &ctx->binLists, &ctx->stagingColor};
 	for (auto *b : ubufs) b->release();
 	ctx->records.release(); ctx->tables.release(); ctx->keys.release(); ctx->denseKeys.release(); ctx->denseInstances.release();
 	if (ctx->pinnedTables) cudaFreeHost(ctx->pinnedTables);
@@ -110,10 +109,7 @@ int dsrg_context_destroy(dsrg_context ctx) {
 	if (ctx->branchFork) cudaEventDestroy(ctx->branchFork);
 	if (ctx->branchJoin) cudaEventDestroy(ctx->branchJoin);
 	if (ctx->branchStream) cudaStreamDestroy(ctx->branchStream);
-	ctx->tileList.release(); ctx->bigList.release(); ctx->binThresholds.release();
-	ctx->tileParts.release(); ctx->tilePartsDone.release();
-	ctx->drawnMarks.release(); ctx->extraBase.release(); ctx->extraIds.release(); ctx->tileHeads.release(); ctx->tileRanks.release();
-	ctx->segmentSlots.release();
+	ctx->tileList.release(); ctx->batchScratch.release();
 	for (PhaseGraph &g : ctx->graphs) g.reset();
 	cudaEventDestroy(ctx->eventStart);
 	cudaEventDestroy(ctx->eventStop);

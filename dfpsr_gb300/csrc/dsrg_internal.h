@@ -219,15 +219,8 @@ struct dsrg_context_s {
 	bool stopRecorded = false;           // the last batch recorded eventStop before its host wait
 	// capacities of the buffers sized before their totals are known (largest totals seen, with slack)
 	uint64_t extraCapacity = 0, recordCapacity = 0, rowCapacity = 0, binCapacity = 0;
-	DeviceBuffer<uint32_t> binCounts, binOffsets, binCursors, binLists;
-	DeviceBuffer<uint32_t> bigList;      // records over more than four tiles
-	DeviceBuffer<uint32_t> binThresholds; // per tile: the key that large records must reach to be listed
-	DeviceBuffer<uint16_t> drawnMarks;
-	DeviceBuffer<uint32_t> extraBase, extraIds, segmentSlots; // the one-pass setup (EmitBuffers)
-	DeviceBuffer<uint2> tileParts;       // tiles of long lists, drawn in parts
-	DeviceBuffer<uint32_t> tilePartsDone;
-	DeviceBuffer<uint4> tileHeads;
-	DeviceBuffer<uint2> tileRanks;
+	DeviceBuffer<uint32_t> binLists;
+	DeviceBuffer<uint4> batchScratch;    // a batch's other arrays, one after another (enqueue_phases)
 	DeviceBuffer<TextureData> textureTable;
 	DeviceBuffer<uint32_t> stagingColor;
 	DeviceBuffer<uint32_t> textureStaging;      // texture creation: host images and two-step resize halves

@@ -157,7 +157,7 @@ static int enqueue_phases(dsrg_context ctx, BatchJob &job, BatchTotals &totals, 
 	const size_t tableBytes = layout_tables(job, nullptr, nullptr, nullptr, params, totals);
 	if (totals.pixels > 0) TRY(ctx->keys.reserve(totals.pixels));
 	TRY(ctx->tables.reserve(tableBytes));
-	TRY(ctx->tileList.reserve((size_t)totals.tiles + 1));
+	if (job.depthOnly) TRY(ctx->tileList.reserve((size_t)totals.tiles + 1));
 	if (ctx->pinnedCapacity < tableBytes) {
 		if (ctx->pinnedTables) cudaFreeHost(ctx->pinnedTables);
 		ctx->pinnedTables = nullptr;
@@ -212,58 +212,71 @@ static int enqueue_phases(dsrg_context ctx, BatchJob &job, BatchTotals &totals, 
 	                                   : (uint32_t)std::max<uint64_t>(ctx->recordCapacity, nt + nt / 8 + 1024);
 	const uint32_t rowCap = (uint32_t)std::max<uint64_t>(ctx->rowCapacity, (uint64_t)recordCap * 4);
 	const uint32_t binCap = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(ctx->binCapacity, (uint64_t)recordCap * 2), 0xFFFFFFF0u);
-	TRY(ctx->pointCsis.reserve(np)); TRY(ctx->pointIsyOut.reserve(np)); TRY(ctx->pointFlat.reserve(np));
 	TRY(ctx->records.reserve((size_t)recordCap + 1));
-	if (onePass) {
-		TRY(ctx->drawnMarks.reserve((size_t)recordCap + 4)); // read four at a time
-		TRY(ctx->extraBase.reserve(nt + 1));
-		TRY(ctx->extraIds.reserve((size_t)recordCap - nt + 1));
-		TRY(ctx->tileHeads.reserve((size_t)recordCap + 1));
-		TRY(ctx->tileRanks.reserve((size_t)recordCap + 1));
-		if (tallTriangles) TRY(ctx->segmentSlots.reserve((size_t)rowCap / ROW_SEGMENT + 1));
-	} else {
+	if (!onePass) {
 		TRY(ctx->triCounts.reserve(nt + 1));
 		TRY(ctx->triOffsets.reserve(nt + 1));
 		TRY(ctx->rowCounts.reserve((size_t)recordCap + 1));
 		TRY(ctx->rowOffsets.reserve((size_t)recordCap + 1));
 	}
 	TRY(ctx->rows.reserve((size_t)rowCap + 2));
-	TRY(ctx->binCounts.reserve(2 * (size_t)totals.tiles + 1));
-	TRY(ctx->binOffsets.reserve(2 * (size_t)totals.tiles + 1));
-	TRY(ctx->binCursors.reserve(2 * (size_t)totals.tiles + 1));
 	TRY(ctx->binLists.reserve((size_t)binCap + 1));
-	TRY(ctx->bigList.reserve((size_t)recordCap + 1));
-	TRY(ctx->binThresholds.reserve((size_t)totals.tiles + 1));
+	// the smaller arrays of a batch lie in one allocation: a buffer for each made the first frame of a context
+	// 100 us longer
+	size_t scratchBytes = 0;
+	const auto part = [&](size_t bytes) {
+		const size_t at = scratchBytes;
+		scratchBytes = (at + bytes + 255) & ~(size_t)255;
+		return at;
+	};
 	const uint32_t partWeight = job.depthOnly ? DEPTH_PART_WEIGHT : PART_WEIGHT;
-	TRY(ctx->tileParts.reserve((size_t)max_parts(binCap, partWeight) + 1));
-	TRY(ctx->tilePartsDone.reserve((size_t)totals.tiles + 1));
+	const size_t slots = 2 * (size_t)totals.tiles + 1;
+	const size_t csisAt = part(np * sizeof(*ctx->pointCsis.ptr)), isyOutAt = part(np * sizeof(*ctx->pointIsyOut.ptr));
+	const size_t flatAt = part(np * sizeof(*ctx->pointFlat.ptr));
+	const size_t countsAt = part(slots * sizeof(uint32_t)), offsetsAt = part(slots * sizeof(uint32_t)), cursorsAt = part(slots * sizeof(uint32_t));
+	const size_t bigListAt = part(((size_t)recordCap + 1) * sizeof(uint32_t)), thresholdsAt = part(((size_t)totals.tiles + 1) * sizeof(uint32_t));
+	const size_t partsAt = part(((size_t)max_parts(binCap, partWeight) + 1) * sizeof(uint2)), partsDoneAt = part(((size_t)totals.tiles + 1) * sizeof(uint32_t));
+	size_t marksAt = 0, extraBaseAt = 0, extraIdsAt = 0, headsAt = 0, ranksAt = 0, segmentsAt = 0;
+	if (onePass) {
+		marksAt = part(((size_t)recordCap + 4) * sizeof(uint16_t)); // read four at a time
+		extraBaseAt = part((nt + 1) * sizeof(uint32_t));
+		extraIdsAt = part(((size_t)recordCap - nt + 1) * sizeof(uint32_t));
+		headsAt = part(((size_t)recordCap + 1) * sizeof(uint4));
+		ranksAt = part(((size_t)recordCap + 1) * sizeof(uint2));
+		if (tallTriangles) segmentsAt = part(((size_t)rowCap / ROW_SEGMENT + 1) * sizeof(uint32_t));
+	}
 	const uint64_t scanned = std::max<uint64_t>(onePass ? 0 : recordCap, 2 * (uint64_t)totals.tiles);
-	TRY(ctx->scanScratch.reserve(scan_scratch_elems((uint32_t)scanned + 1)));
+	const size_t scanElems = scan_scratch_elems((uint32_t)scanned + 1), scanAt = part(scanElems * sizeof(uint32_t));
+	TRY(ctx->batchScratch.reserve(scratchBytes / sizeof(uint4)));
+	uint8_t *scratch = reinterpret_cast<uint8_t *>(ctx->batchScratch.ptr);
+	const auto words = [&](size_t at) { return reinterpret_cast<uint32_t *>(scratch + at); };
 	FrameBuffers fb;
 	memset(&fb, 0, sizeof(fb));
-	fb.points.csis = ctx->pointCsis.ptr; fb.points.isyOut = ctx->pointIsyOut.ptr; fb.points.flat = ctx->pointFlat.ptr;
+	fb.points.csis = reinterpret_cast<decltype(fb.points.csis)>(scratch + csisAt);
+	fb.points.isyOut = reinterpret_cast<decltype(fb.points.isyOut)>(scratch + isyOutAt);
+	fb.points.flat = reinterpret_cast<decltype(fb.points.flat)>(scratch + flatAt);
 	fb.records = ctx->records.ptr;
 	fb.rows = ctx->rows.ptr;
 	fb.errorFlag = (int32_t *)(ctx->control.ptr + CONTROL_ERROR);
-	fb.scanScratch = ctx->scanScratch.ptr;
-	fb.scanScratchElems = ctx->scanScratch.capacity;
+	fb.scanScratch = words(scanAt);
+	fb.scanScratchElems = scanElems;
 	fb.rowCapacity = rowCap;
 	if (onePass) {
 		fb.emit.counters = ctx->control.ptr + CONTROL_EMIT;
-		fb.emit.drawn = ctx->drawnMarks.ptr;
+		fb.emit.drawn = reinterpret_cast<uint16_t *>(scratch + marksAt);
 		fb.emit.triangles = (uint32_t)nt;
 		fb.emit.capacity = recordCap;
-		fb.emit.extraBase = ctx->extraBase.ptr;
-		fb.emit.extraIds = ctx->extraIds.ptr;
-		fb.emit.tileHeads = ctx->tileHeads.ptr;
-		fb.emit.tileRanks = ctx->tileRanks.ptr;
-		fb.emit.segmentSlots = tallTriangles ? ctx->segmentSlots.ptr : nullptr;
-		fb.emit.tileCursors = ctx->binCursors.ptr;
-		fb.emit.bigList = ctx->bigList.ptr;
+		fb.emit.extraBase = words(extraBaseAt);
+		fb.emit.extraIds = words(extraIdsAt);
+		fb.emit.tileHeads = reinterpret_cast<uint4 *>(scratch + headsAt);
+		fb.emit.tileRanks = reinterpret_cast<uint2 *>(scratch + ranksAt);
+		fb.emit.segmentSlots = tallTriangles ? words(segmentsAt) : nullptr;
+		fb.emit.tileCursors = words(cursorsAt);
+		fb.emit.bigList = words(bigListAt);
 		fb.emit.bigCount = ctx->control.ptr + CONTROL_BIG_RECORDS;
 		fb.recordCountDevice = fb.emit.counters + EMIT_DRAWN;
 		params.recordShift = 3;
-		params.extraBase = ctx->extraBase.ptr;
+		params.extraBase = words(extraBaseAt);
 	} else {
 		fb.triCounts = ctx->triCounts.ptr;
 		fb.triOffsets = ctx->triOffsets.ptr;
@@ -272,24 +285,24 @@ static int enqueue_phases(dsrg_context ctx, BatchJob &job, BatchTotals &totals, 
 	}
 	TileBins bins;
 	memset(&bins, 0, sizeof(bins));
-	bins.counts = ctx->binCounts.ptr;
-	bins.offsets = ctx->binOffsets.ptr;
-	bins.cursors = ctx->binCursors.ptr;
+	bins.counts = words(countsAt);
+	bins.offsets = words(offsetsAt);
+	bins.cursors = words(cursorsAt);
 	bins.lists = ctx->binLists.ptr;
 	bins.listCapacity = binCap;
-	bins.bigList = ctx->bigList.ptr;
+	bins.bigList = words(bigListAt);
 	bins.bigCount = ctx->control.ptr + CONTROL_BIG_RECORDS;
 	bins.cleared = 1; // by the first launch of phase A
 	// records are culled while binning where only the best key of a pixel counts: not where every
 	// fragment is counted, nor for the alpha filter, which blends them all
-	bins.thresholds = (job.alpha || params.fragments) ? nullptr : ctx->binThresholds.ptr;
+	bins.thresholds = (job.alpha || params.fragments) ? nullptr : words(thresholdsAt);
 	bins.culled = bins.thresholds ? ctx->control.ptr + CONTROL_CULLED : nullptr;
 	if (!job.alpha) {
-		bins.parts = ctx->tileParts.ptr;
+		bins.parts = reinterpret_cast<uint2 *>(scratch + partsAt);
 		bins.partCount = ctx->control.ptr + CONTROL_TILE_PARTS;
 		bins.partWeight = partWeight;
 		bins.partCapacity = max_parts(binCap, partWeight);
-		bins.partsDone = ctx->tilePartsDone.ptr;
+		bins.partsDone = words(partsDoneAt);
 	}
 	ClearedCounters clear;
 	memset(&clear, 0, sizeof(clear));
