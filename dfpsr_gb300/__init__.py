@@ -431,7 +431,7 @@ class Context:
         """instances: (DenseModel, origin, model_to_world) in drawing order, drawn as that many
         dense_render calls would draw them, in one call."""
         # transforms row by row through a view of the table's words: set value by value, the table of 64
-        # instances took longer than drawing them (277 to 288 us a call, 218 this way)
+        # instances took longer than drawing them (277 to 288 us a call, 208 this way)
         arr = (DenseInstance * max(len(instances), 1))()
         words = np.frombuffer(arr, np.float32).reshape(len(arr), -1)
         for i, (model, origin, transform) in enumerate(instances):
