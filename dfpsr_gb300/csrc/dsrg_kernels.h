@@ -148,6 +148,7 @@ struct TileBins {
 	uint32_t *cursors;  // 2 * totalTiles: places taken in each list
 	uint32_t *lists;
 	size_t listCapacity;
+	uint32_t *scratch;  // alpha filter: as long as lists, where long ones are sorted
 	// records over more than four tiles, listed by setup_emit_kernel and binned by whole blocks
 	uint32_t *bigList;
 	uint32_t *bigCount;

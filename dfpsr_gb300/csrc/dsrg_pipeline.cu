@@ -236,6 +236,7 @@ static int enqueue_phases(dsrg_context ctx, BatchJob &job, BatchTotals &totals, 
 	const size_t countsAt = part(slots * sizeof(uint32_t)), offsetsAt = part(slots * sizeof(uint32_t)), cursorsAt = part(slots * sizeof(uint32_t));
 	const size_t bigListAt = part(((size_t)recordCap + 1) * sizeof(uint32_t)), thresholdsAt = part(((size_t)totals.tiles + 1) * sizeof(uint32_t));
 	const size_t partsAt = part(((size_t)max_parts(binCap, partWeight) + 1) * sizeof(uint2)), partsDoneAt = part(((size_t)totals.tiles + 1) * sizeof(uint32_t));
+	const size_t sortAt = job.alpha ? part((size_t)binCap * sizeof(uint32_t)) : 0;
 	size_t marksAt = 0, extraBaseAt = 0, extraIdsAt = 0, headsAt = 0, ranksAt = 0, segmentsAt = 0;
 	if (onePass) {
 		marksAt = part(((size_t)recordCap + 4) * sizeof(uint16_t)); // read four at a time
@@ -290,6 +291,7 @@ static int enqueue_phases(dsrg_context ctx, BatchJob &job, BatchTotals &totals, 
 	bins.cursors = words(cursorsAt);
 	bins.lists = ctx->binLists.ptr;
 	bins.listCapacity = binCap;
+	bins.scratch = job.alpha ? words(sortAt) : nullptr;
 	bins.bigList = words(bigListAt);
 	bins.bigCount = ctx->control.ptr + CONTROL_BIG_RECORDS;
 	bins.cleared = 1; // by the first launch of phase A

@@ -150,3 +150,63 @@ def test_alpha_lists_around_the_shared_sort(ctx, w, h, triangles, perspective):
     if not perspective:
         depth = (depth * 5.0 + 2.5).astype(np.float32)
     _check(_gpu(ctx, s, color, depth), port.render(s, color, depth, coverage=True), f"{w}x{h} {triangles}")
+
+
+def _layers_over_one_tile(n):
+    """n alpha-filtered triangles that each cover a whole 16x16 image, every one facing the camera."""
+    s = _alpha_scene(n, triangles=n, width=16, height=16)
+    z = np.random.default_rng(n).uniform(-1.0, 1.0, n).astype(np.float32)
+    corners = np.array([[-90.0, -60.0], [0.0, 120.0], [90.0, -60.0]], np.float32)
+    s.positions[:] = np.concatenate([np.broadcast_to(corners, (n, 3, 2)), np.broadcast_to(z[:, None, None], (n, 3, 1))], axis=2).reshape(-1, 3)
+    return s
+
+
+@pytest.mark.parametrize("n", [2047, 2048, 2049, 4096, 4099])
+def test_alpha_lists_of_exact_lengths(ctx, n):
+    """Lists that just fit the sort in shared memory, that just do not, and that end on a step of the
+    sort of long lists."""
+    from oracle import port
+    s = _layers_over_one_tile(n)
+    color, _ = _prefilled(4, 16, 16)
+    depth = np.zeros((16, 16), np.float32)
+    ref = port.render(s, color, depth, coverage=True)
+    assert ref[2]["fragments"] == n * 256
+    _check(_gpu(ctx, s, color, depth), ref, f"{n} layers")
+
+
+@pytest.mark.parametrize("seen,hidden", [(6000, 0), (5001, 60000), (6002, 2150000)])
+def test_alpha_long_lists_of_far_apart_numbers(ctx, seen, hidden):
+    """Long lists whose record numbers take two, three and four digits: `hidden` triangles behind the
+    camera stand between the first and the last of those that are seen."""
+    from oracle import port
+    s = _alpha_scene(seen, triangles=seen + hidden, width=33, height=17)
+    s.positions[3 * (seen // 2):3 * (seen // 2 + hidden), 2] -= 10.0  # the camera stands at z = -3
+    color, depth = _prefilled(6, 17, 33)
+    gpu = _gpu(ctx, s, color, depth)
+    assert gpu[2]["draw_records"] > 2048
+    _check(gpu, port.render(s, color, depth, coverage=True), f"{seen} of {seen + hidden}")
+
+
+def test_alpha_time_grows_no_faster_than_the_list(ctx):
+    """Small triangles over one tile: eight times as many take at most sixteen times as long (when long
+    lists were taken in windows, each found by reading the whole list some twenty times, it was more)."""
+    import time
+    import torch
+    import dfpsr_gb300 as d
+    seconds = {}
+    for n in (60000, 480000):
+        s = _alpha_scene(9, triangles=n, width=16, height=16)
+        rng = np.random.default_rng(n)
+        s.positions[:] = (rng.uniform(-1.0, 1.0, (n, 1, 3)) + 0.08 * rng.normal(size=(n, 3, 3))).reshape(-1, 3).astype(np.float32)
+        model = d.Model(ctx, s)
+        c = torch.zeros((16, 16), dtype=torch.int32, device="cuda")
+        z = torch.zeros((16, 16), dtype=torch.float32, device="cuda")
+        times = []
+        for _ in range(6):
+            torch.cuda.synchronize()
+            t = time.perf_counter()
+            ctx.render(model, model.camera, c, z)
+            times.append(time.perf_counter() - t)
+        seconds[n] = min(times)
+        model.destroy()
+    assert seconds[480000] <= 16 * seconds[60000], seconds
