@@ -2656,7 +2656,9 @@ __device__ __noinline__ const uint32_t *sort_long_list(uint32_t *list, uint32_t 
 __global__ void __launch_bounds__(ALPHA_THREADS) alpha_kernel(BatchParams b, const DrawRecord *__restrict__ records, TileBins bins,
                                                     const uint32_t *__restrict__ rows) {
 	chain_enter();
-	if (overflowed(b)) return;
+	// lists or rows that overflowed (the run is redone), or a coordinate out of range (the call fails): nothing
+	// is blended over the image
+	if (b.errorFlag && *(volatile const int32_t *)b.errorFlag != 0) return;
 	__shared__ uint32_t ids[ALPHA_LIST];
 	__shared__ DrawRecord staged[ALPHA_CHUNK];
 	__shared__ ShadeRecord shades[ALPHA_CHUNK];

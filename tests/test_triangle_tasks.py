@@ -122,3 +122,40 @@ def test_gpu_triangle_tasks_match_oracle(ctx):
         r.give_triangles(corners(t2[0][:1]), t2[1][:1], t2[2][:1], None, None, 0, cam)
     assert e.value.status == 4
     r.destroy()
+
+
+@pytest.mark.gpu
+def test_alpha_triangle_out_of_the_coordinate_range_blends_nothing(ctx):
+    """An alpha-filtered run holding a corner more than 2^30 sub-pixel units away fails, and leaves the
+    image as the runs before it made it."""
+    import torch
+    import dfpsr_gb300 as d
+    scene = scenes.random_triangles(seed=8, triangles=200, width=64, height=48, texture_size=16)
+    alpha = dataclasses.replace(scenes.random_triangles(seed=9, triangles=200, width=64, height=48, texture_size=16), filter=1)
+    far = np.zeros((1, 3), d.PROJECTED_POINT)
+    far["cs"] = (0.0, 0.0, 1.0)
+    far["is"] = 1.0
+    far["flat"] = [[(-(1 << 30) - 256, 0), (1 << 14, 0), (0, 1 << 14)]]
+    ones = np.ones((1, 3, 4), np.float32)
+    images = {}
+    for fails in (False, True):
+        c = torch.zeros((48, 64), dtype=torch.int32, device="cuda")
+        z = torch.zeros((48, 64), dtype=torch.float32, device="cuda")
+        solid_model, alpha_model = d.Model(ctx, scene), d.Model(ctx, alpha)
+        r = d.Renderer(ctx)
+        r.begin(c, z)
+        r.give_task(solid_model, solid_model.camera)
+        if fails:
+            r.give_task(alpha_model, alpha_model.camera)
+            for order in ([0, 1, 2], [0, 2, 1]):  # one of the two faces the camera
+                r.give_triangles(far[:, order], ones, np.zeros((1, 3, 4), np.float32), None, None, 1, alpha_model.camera)
+            with pytest.raises(d.DsrgError) as e:
+                r.end()
+            assert "error bits" in str(e.value)
+        else:
+            r.end()
+        torch.cuda.synchronize()
+        images[fails] = c.cpu().numpy()
+        r.destroy()
+    assert np.count_nonzero(images[False])
+    assert np.array_equal(images[True], images[False])
