@@ -59,14 +59,18 @@ DSRG_HD float frcp(float x) {
 	return 1.0f / x;
 #endif
 }
-// An estimate of a / b for quotients that exact integer products correct afterwards: within 2 ulp
-// on the device (|b| < 2^126, which int64 operands satisfy).  A host build may define
-// DSRG_HOST_ESTIMATE_ERROR to push its estimates that far off, so that host checks exercise the
-// corrections as the device does.
+// An estimate of a / b, within 2 ulp on the device for 2^-126 <= |b| <= 2^126, which every nonzero int64
+// satisfies and chain_add sees to; beyond it is 0, below (subnormal divisors) it can be infinite.  Integer
+// quotients are corrected by exact products afterwards, chain_add leaves room for the error.  A host
+// build may define DSRG_HOST_ESTIMATE_ERROR to push its estimates that far off, and out of that range as
+// far as they can be, so that host checks exercise what the device does.
 DSRG_HD float fdiv_estimate(float a, float b) {
 #if defined(__CUDA_ARCH__)
 	return __fdividef(a, b);
 #elif defined(DSRG_HOST_ESTIMATE_ERROR)
+	const float size = b < 0.0f ? -b : b;
+	if (a != 0.0f && size < 1.17549435e-38f) return ((a < 0.0f) == (b < 0.0f) ? 1.0f : -1.0f) / 0.0f;
+	if (size > 8.50705917e37f) return 0.0f;
 	const float q = a / b;
 	return q + q * DSRG_HOST_ESTIMATE_ERROR;
 #else
@@ -125,7 +129,9 @@ DSRG_HD_CALL float chain_add(float s, float d, int32_t n) {
 		if (b1 == b2) return s; // a fixed point: d is too small to move s, or an infinity
 		if ((((b0 ^ b1) | (b1 ^ b2)) & 0xFF800000u) != 0u) continue; // another binade or sign: only the plain steps
 		const uint32_t exponent = b2 & 0x7F800000u;
-		if (exponent == 0u || exponent >= 0x7F000000u) { // subnormal, near-overflow or NaN: plain steps
+		// plain steps near overflow, for NaN, and below 2^-103, where the ulp and so the increment can be
+		// subnormal, a divisor that the estimate below does not take
+		if (exponent - 0x0C000000u >= 0x7F000000u - 0x0C000000u) {
 			if (exponent == 0x7F800000u) return s;
 			continue;
 		}

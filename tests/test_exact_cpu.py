@@ -76,6 +76,23 @@ def test_chain_add_long_chains(host, mantissa_bits):
     assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
 
 
+@pytest.mark.parametrize("low,high", [(-126, -98), (100, 126)])
+def test_chain_add_near_the_ends_of_the_exponent_range(host, low, high):
+    """Chains whose increments can be subnormal, or whose sums come near the largest float: there the
+    estimated quotient is out of its bounds (the host build makes it as wrong as it may be)."""
+    r = np.random.default_rng(high + 1000)
+    N = 6000
+    e = r.integers(low, high + 1, N)
+    s = np.ldexp(r.uniform(0.5, 1.0, N), e) * r.choice([1, -1], N)
+    d = np.ldexp(r.uniform(0.5, 1.0, N), np.maximum(e - r.integers(0, 26, N), -148)) * r.choice([1, -1], N)
+    n = r.integers(0, 4096, N)
+    with np.errstate(over="ignore"):
+        s, d, n = s.astype(np.float32), d.astype(np.float32), n.astype(np.int32)
+        a, b = _chain(host, s, d, n), _serial(s, d, n)
+    assert np.isfinite(b).any()
+    assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
+
+
 def _rows(host, flat, y0, rows, L, R):
     fl = np.ascontiguousarray(flat, np.int32)
     lefts, rights = np.zeros(rows, np.int32), np.zeros(rows, np.int32)
