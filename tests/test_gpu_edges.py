@@ -101,3 +101,35 @@ def test_fresh_context_outgrows_its_buffers(built):
             _assert_same(got, expect, label)
     finally:
         fresh.close()
+
+
+def _torus_frame(size, width, height):
+    rng = np.random.default_rng(size)
+    s = scenes.torus(2 * size, size, width=width, height=height)
+    s.colors = rng.uniform(0.4, 1.0, size=s.colors.shape).astype(np.float32)
+    s.diffuse, s.diffuse_levels = scenes.noise_texture(rng, 64), 16
+    s.model_to_world = np.concatenate([[0, 0, 0], scenes.random_rotation(rng).reshape(-1)]).astype(np.float32)
+    return s
+
+
+@pytest.mark.parametrize("size,width,height", [(20, 320, 200), (50, 640, 480), (120, 1281, 719)])
+def test_first_frame_of_a_mesh_is_drawn_once(built, size, width, height):
+    """The first large frame of a context takes as many launches as the next one: its rows, rounded up
+    to whole segments, fit the buffer that the context starts with."""
+    import dfpsr_gb300 as d
+    from oracle import port
+    fresh = d.Context(0)
+    try:
+        scene = _torus_frame(size, width, height)
+        small = _torus_frame(4, 32, 32)
+        model, small_model = d.Model(fresh, scene), d.Model(fresh, small)
+        d.render_scene(fresh, small, model=small_model)
+        launches = [fresh.stats()["kernel_launches"]]
+        for _ in range(2):
+            color, depth = d.render_scene(fresh, scene, model=model)
+            launches.append(fresh.stats()["kernel_launches"])
+        assert launches[1] - launches[0] == launches[2] - launches[1]
+        rc, rz, _ = port.render(scene)
+        assert np.array_equal(color, rc) and np.array_equal(depth.view(np.uint32), rz.view(np.uint32))
+    finally:
+        fresh.close()
