@@ -7,6 +7,7 @@
 // exercise the exact corrections that follow them.
 #define DSRG_HOST_ESTIMATE_ERROR 4.76837158203125e-7f
 #include "dsrg_exact.h"
+#include "dsrg_fill.h"
 #include "dsrg_geometry.h"
 
 extern "C" {
@@ -47,6 +48,19 @@ int32_t dsrg_host_row_intervals_near(const int32_t *flat, int32_t y0, int32_t ro
 void dsrg_host_row_intervals_stepped(const int32_t *flat, int32_t y0, int32_t rows, int32_t L, int32_t R, int32_t *lefts,
                                      int32_t *rights) {
 	dsrg::row_intervals_stepped(flat, y0, rows, L, R, lefts, rights);
+}
+
+// The pieces that a rectangle is filled in (dsrg::add_fill_pieces): per piece its first byte, stride, width
+// and height in words, and whether it is written 16 bytes at a time.  Returns their number.
+int32_t dsrg_host_fill_pieces(uint64_t address, int32_t strideWords, int32_t width, int32_t height, uint64_t *out, int32_t capacity) {
+	std::vector<dsrg::FillRect> pieces;
+	dsrg::add_fill_pieces(dsrg::fill_rect((void *)(uintptr_t)address, strideWords, width, height, 0u), pieces);
+	for (size_t i = 0; i < pieces.size() && (int32_t)i < capacity; i++) {
+		const dsrg::FillRect &p = pieces[i];
+		const uint64_t row[5] = {(uint64_t)(uintptr_t)p.words, p.stride, p.width, p.height, (uint64_t)p.vector};
+		for (int k = 0; k < 5; k++) out[5 * i + k] = row[k];
+	}
+	return (int32_t)pieces.size();
 }
 
 } // extern "C"

@@ -12,6 +12,7 @@
 #include <vector>
 
 #include "../../include/dsrg.h"
+#include "dsrg_fill.h"
 #include "dsrg_geometry.h"
 #include "dsrg_kernels.h"
 
@@ -322,15 +323,7 @@ int renderer_upload_given(dsrg_renderer r);
 // in place; false for pageable memory, which is staged through device buffers.
 bool host_mapped(const void *p, void **devicePointer);
 // Queues fills of rectangles of 32-bit words (device or mapped memory), each with one value.
-static const int FILL_RECTS = 32; // rectangles of one launch
-struct FillRect {
-	uint32_t *words;
-	uint32_t stride, width, height; // in words
-	uint32_t value;
-	int32_t vector;                 // set by enqueue_fill_rects
-};
-FillRect fill_rect(void *image, int32_t strideWords, int32_t width, int32_t height, uint32_t value);
-void enqueue_fill_rects(const FillRect *rects, size_t count, cudaStream_t stream);
+void enqueue_fill_rects(const dsrg::FillRect *rects, size_t count, cudaStream_t stream);
 // Whether every depth image of a batch is reachable by kernels without staging (device or page-locked memory).
 bool batch_depth_in_place(dsrg_batch b);
 // Queues zeroing of every depth image of a batch (CubeMapF32::clear for a batch of cube faces).

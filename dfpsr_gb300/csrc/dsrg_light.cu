@@ -371,7 +371,8 @@ __global__ void root_check_kernel(uint32_t firstBits, uint32_t count, unsigned l
 
 // Rectangles of 32-bit words, each set to one value (a frame's clears), blockIdx.y the rectangle.
 // Bound by the write bandwidth: a thread writes 16 bytes at a time where the rows allow it, four
-// stores in flight, and rows that follow one another in memory are one long row.  The 16 shadow cubes of
+// stores in flight, and rows that follow one another in memory are one long row.  Words are counted in
+// 32 bits: add_fill_pieces keeps every rectangle below 2^31.  The 16 shadow cubes of
 // the 1080p light frame (100 MB) took up to eight launches of a word per thread and 75 to 100 us; they
 // now take 14 us in one (frame 616 -> 571 us).
 struct FillBatch {
@@ -786,35 +787,18 @@ int sprite_frame_steps(dsrg_context ctx, const dsrg_sprite_frame_desc &d, const 
 
 } // namespace
 
-FillRect fill_rect(void *image, int32_t strideWords, int32_t width, int32_t height, uint32_t value) {
-	FillRect r;
-	r.words = (uint32_t *)image;
-	r.stride = (uint32_t)strideWords;
-	r.width = (uint32_t)width;
-	r.height = (uint32_t)height;
-	r.value = value;
-	r.vector = 0;
-	return r;
-}
-
 void enqueue_fill_rects(const FillRect *rects, size_t count, cudaStream_t stream) {
-	for (size_t first = 0; first < count; first += FILL_RECTS) {
-		const size_t n = std::min(count - first, (size_t)FILL_RECTS);
+	std::vector<FillRect> pieces;
+	for (size_t i = 0; i < count; i++) add_fill_pieces(rects[i], pieces);
+	for (size_t first = 0; first < pieces.size(); first += FILL_RECTS) {
+		const size_t n = std::min(pieces.size() - first, (size_t)FILL_RECTS);
 		FillBatch batch;
 		memset(&batch, 0, sizeof(batch));
 		uint64_t largest = 0;
 		for (size_t i = 0; i < n; i++) {
-			FillRect &r = batch.rect[i];
-			r = rects[first + i];
-			// rows without a gap between them are one row (32-bit indices: up to 2^31 words)
-			if (r.stride == r.width && (uint64_t)r.width * r.height < (1ull << 31)) {
-				r.width *= r.height;
-				r.height = 1;
-			}
-			r.vector = ((uintptr_t)r.words & 15u) == 0 && r.width % 4u == 0 && (r.height == 1 || r.stride % 4u == 0);
+			const FillRect &r = batch.rect[i] = pieces[first + i];
 			largest = std::max(largest, (uint64_t)r.width * r.height / (r.vector ? 4 : 1));
 		}
-		if (largest == 0) continue;
 		const uint64_t blocks = std::min<uint64_t>((largest + 1023) / 1024, (uint64_t)sm_count() * 8);
 		fill_rects_kernel<<<dim3((unsigned)std::max<uint64_t>(blocks, 1), (unsigned)n), 256, 0, stream>>>(batch);
 		add_launches(1);

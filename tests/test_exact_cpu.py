@@ -211,3 +211,31 @@ def test_near_row_intervals_match_oracle(host, kind):
         want = _rows(host, flat, top, rows, L, R)
         assert np.array_equal(lefts[:rows], want[0]) and np.array_equal(rights[:rows], want[1])
     assert taken > 300
+
+
+@pytest.mark.parametrize("address,stride,width,height", [
+    (4096, 64, 64, 64), (4096, 70, 64, 9), (4100, 64, 64, 3), (4096, 7, 5, 11), (4096, 1, 1, 1), (4096, 8, 8, 0),
+    (4096, 32767, 32767, 32767), (4096, 65536, 65536, 65535), (4096, 70000, 70000, 62000), (4100, 50001, 50000, 50003),
+    (4096, 1 << 29, 1 << 29, 9), (4096, (1 << 29) - 1, (1 << 29) - 4, 5)])
+def test_fills_of_large_rectangles_are_cut(host, address, stride, width, height):
+    """The pieces that a clear is queued in hold every word of the rectangle once, in order, and fewer
+    than 2^31 words each, so that the kernel's 32-bit count neither wraps nor runs on for ever."""
+    capacity = 64
+    out = np.zeros((capacity, 5), np.uint64)
+    n = host.dsrg_host_fill_pieces(C.c_uint64(address), C.c_int32(stride), C.c_int32(width), C.c_int32(height),
+                                   C.c_void_p(out.ctypes.data), C.c_int32(capacity))
+    assert 0 <= n <= capacity and (n == 0) == (height == 0)
+    row = 0
+    for first, piece_stride, piece_width, piece_height, vector in out[:n].tolist():
+        assert 0 < piece_width * piece_height < 2 ** 31
+        assert first == address + 4 * row * stride
+        if piece_height == 1 and piece_width != width:  # rows without a gap as one
+            assert stride == width and piece_width % width == 0
+            rows = piece_width // width
+        else:
+            assert (piece_stride, piece_width) == (stride, width)
+            rows = piece_height
+        row += rows
+        aligned = first % 16 == 0 and piece_width % 4 == 0 and (piece_height == 1 or piece_stride % 4 == 0)
+        assert vector == aligned
+    assert row == height
