@@ -624,16 +624,26 @@ int light_blend_impl(dsrg_context ctx, const dsrg_image *target, const dsrg_imag
 	return finish(ctx, mem, images, wait);
 }
 
-int draw_higher_impl(dsrg_context ctx, const dsrg_image *targetHeight, const dsrg_image *targetA, const dsrg_image *targetB,
-                     const dsrg_sprite *sprites, int32_t count, bool wait) {
-	if (!ctx) return DSRG_ERROR_INVALID_ARGUMENT;
-	if (count < 0 || (count > 0 && !sprites)) return fail(ctx, DSRG_ERROR_INVALID_ARGUMENT, "dsrg_draw_higher: null sprites");
+// What draw_higher refuses of its targets, and its buffers for `count` sprites: nothing is queued here.
+int draw_higher_ready(dsrg_context ctx, const dsrg_image *targetHeight, const dsrg_image *targetA, const dsrg_image *targetB, int32_t count) {
 	if (!valid_image(targetHeight) || !valid_image(targetA) || !valid_image(targetB) || targetHeight->width != targetA->width ||
 	    targetHeight->height != targetA->height || targetHeight->width != targetB->width || targetHeight->height != targetB->height ||
 	    targetA->packOrder < 0 || targetA->packOrder > 3 || targetB->packOrder < 0 || targetB->packOrder > 3)
 		return fail(ctx, DSRG_ERROR_INVALID_ARGUMENT, "dsrg_draw_higher: targets must be images of one size");
 	cudaSetDevice(ctx->device);
 	if (count == 0) return DSRG_OK;
+	DSRG_CUDA_TRY(ctx, ctx->spriteKeys.reserve((size_t)targetHeight->width * targetHeight->height));
+	DSRG_CUDA_TRY(ctx, ctx->spriteTables.reserve(sizeof(SpriteData) * (size_t)count));
+	DSRG_CUDA_TRY(ctx, ctx->spriteTableHost.reserve(sizeof(SpriteData) * (size_t)count));
+	return DSRG_OK;
+}
+
+int draw_higher_impl(dsrg_context ctx, const dsrg_image *targetHeight, const dsrg_image *targetA, const dsrg_image *targetB,
+                     const dsrg_sprite *sprites, int32_t count, bool wait) {
+	if (!ctx) return DSRG_ERROR_INVALID_ARGUMENT;
+	if (count < 0 || (count > 0 && !sprites)) return fail(ctx, DSRG_ERROR_INVALID_ARGUMENT, "dsrg_draw_higher: null sprites");
+	const int ready = draw_higher_ready(ctx, targetHeight, targetA, targetB, count);
+	if (ready != DSRG_OK || count == 0) return ready;
 	std::vector<SpriteData> table(count);
 	int32_t tallest = 1;
 	for (int32_t i = 0; i < count; i++) {
@@ -679,9 +689,6 @@ int draw_higher_impl(dsrg_context ctx, const dsrg_image *targetHeight, const dsr
 	}
 	const int32_t width = targetHeight->width, height = targetHeight->height;
 	const size_t pixels = (size_t)width * height;
-	DSRG_CUDA_TRY(ctx, ctx->spriteKeys.reserve(pixels));
-	DSRG_CUDA_TRY(ctx, ctx->spriteTables.reserve(sizeof(SpriteData) * table.size()));
-	DSRG_CUDA_TRY(ctx, ctx->spriteTableHost.reserve(sizeof(SpriteData) * table.size()));
 	memcpy(ctx->spriteTableHost.ptr, table.data(), sizeof(SpriteData) * table.size());
 	DSRG_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->spriteTables.ptr, ctx->spriteTableHost.ptr, sizeof(SpriteData) * table.size(), cudaMemcpyHostToDevice,
 	                                   ctx->stream));
@@ -745,6 +752,9 @@ int sprite_frame_steps(dsrg_context ctx, const dsrg_sprite_frame_desc &d, const 
 			DSRG_CUDA_TRY(ctx, cudaEventCreateWithFlags(&ctx->sideStart, cudaEventDisableTiming));
 			DSRG_CUDA_TRY(ctx, cudaEventCreateWithFlags(&ctx->sideDone, cudaEventDisableTiming));
 		}
+		// what the sprites would be refused for stops the frame before its shadow cubes are touched
+		const int ready = draw_higher_ready(ctx, &height, &diffuse, &normal, d.spriteCount);
+		if (ready != DSRG_OK) return ready;
 		cudaStream_t mainStream = ctx->stream;
 		DSRG_CUDA_TRY(ctx, cudaEventRecord(ctx->sideStart, mainStream)); // after the frame's images were placed
 		DSRG_CUDA_TRY(ctx, cudaStreamWaitEvent(ctx->sideStream, ctx->sideStart, 0));
@@ -768,12 +778,15 @@ int sprite_frame_steps(dsrg_context ctx, const dsrg_sprite_frame_desc &d, const 
 		} else {
 			status = fail(ctx, DSRG_ERROR_CUDA, "sprite frame: clearing the shadow cubes failed");
 		}
-		if (status == DSRG_OK && !imagesQueued) queueImages(); // a batch without triangles does not wait
+		// a batch without triangles does not wait, and one that fails may not have come to it: the images are
+		// drawn whatever became of the shadows, whose error is the one reported
+		const std::string shadowError = status != DSRG_OK ? ctx->lastError : std::string();
+		if (!imagesQueued) queueImages();
 		// the main stream waits for the side stream whatever happened, so that a wait for the main
 		// stream covers both
-		const cudaError_t joined = !imagesQueued ? cudaSuccess : recorded == cudaSuccess ? cudaStreamWaitEvent(mainStream, ctx->sideDone, 0) : recorded;
-		if (status == DSRG_OK) status = imagesStatus;
-		if (status != DSRG_OK) return status;
+		const cudaError_t joined = recorded == cudaSuccess ? cudaStreamWaitEvent(mainStream, ctx->sideDone, 0) : recorded;
+		if (status != DSRG_OK) return fail(ctx, status, shadowError);
+		if (imagesStatus != DSRG_OK) return imagesStatus;
 		DSRG_CUDA_TRY(ctx, joined);
 	} else {
 		status = sprite_frame_images(ctx, d, img, sprites);

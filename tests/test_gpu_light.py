@@ -338,3 +338,79 @@ def test_sprite_frame_without_sprites_lights_or_shadows(ctx):
     ctx.light_blend(out, images[1], light)
     assert np.array_equal(host(images[4], np.uint32), host(out, np.uint32))
     assert ctx.check_float_roots(0x3F800000, 0) == 0
+
+
+def _shadowed_pass(context, seed=12):
+    import dfpsr_gb300 as d
+    from dfpsr_gb300.sprite_pass import DeferredLightPass
+    m, _ = d.ortho_view(-0.7, 64, 0).arrays()
+    scene = scenes.light_scene(seed=seed, width=128, height=96, sprites=20, sprite_types=2, lights=2, radius_px=(40, 60),
+                               caster_triangles=60, cube_resolution=32, light_space=(m[9:18], m[0:9]))
+    return DeferredLightPass(context, scene, THREADS), scene
+
+
+def test_sprite_frame_refused_for_its_sprites_leaves_the_shadow_cubes(built):
+    """A frame whose sprites cannot be drawn (a target's pack order, an exhausted GPU) stops before its
+    shadow cubes are cleared; the next frame is the oracle's."""
+    import dfpsr_gb300 as d
+    from oracle import light_pass
+    fresh = d.Context(0)
+    try:
+        gpu, scene = _shadowed_pass(fresh)
+        gpu.shadows.render()  # the batch's own buffers are there: the next allocation is the sprites'
+        for cube in gpu.cubes:
+            cube.fill_(7.0)
+        d.lib().dsrg_debug_fail_allocation(0)
+        try:
+            with pytest.raises(d.DsrgError) as e:
+                gpu.run()
+        finally:
+            d.lib().dsrg_debug_fail_allocation(-1)
+        assert e.value.status == 3
+        assert all((host(cube, np.float32) == 7.0).all() for cube in gpu.cubes)
+        assert np.array_equal(host(gpu.run(), np.uint32), light_pass.run(scene, THREADS)[0])
+        for cube in gpu.cubes:
+            cube.fill_(7.0)
+        original = d.image_struct
+        d.image_struct = lambda array, pack_order=0: original(array, 9 if array is gpu.diffuse else pack_order)
+        try:
+            with pytest.raises(d.DsrgError) as e:
+                gpu.run()
+        finally:
+            d.image_struct = original
+        assert e.value.status == 1
+        assert all((host(cube, np.float32) == 7.0).all() for cube in gpu.cubes)
+        gpu.destroy()
+    finally:
+        fresh.close()
+
+
+def test_sprite_frame_draws_its_images_when_the_shadows_fail(built):
+    """A shadow batch that fails before its launches are queued leaves the frame's images cleared, with
+    the sprites and the directed light drawn; the error is the batch's."""
+    import dfpsr_gb300 as d
+    from dfpsr_gb300.sprite_pass import BACKGROUND_HEIGHT
+    fresh = d.Context(0)
+    try:
+        gpu, scene = _shadowed_pass(fresh, seed=13)
+        s = scene
+        sun = (s.sun_direction, s.sun_intensity, s.sun_color)
+        images = (gpu.height, gpu.diffuse, gpu.normal, gpu.light, gpu.output)
+        # the sprites' own buffers are there: the next allocation is the batch's
+        fresh.sprite_frame(gpu.view, s.center, images, (BACKGROUND_HEIGHT, 0, 0), gpu.sprites, sun, None, [], THREADS)
+        expected = [host(i, np.uint32).copy() for i in images[:4]]
+        assert np.count_nonzero(expected[1])
+        for i in images:
+            i.fill_(1)
+        d.lib().dsrg_debug_fail_allocation(0)
+        try:
+            with pytest.raises(d.DsrgError) as e:
+                gpu.run()
+        finally:
+            d.lib().dsrg_debug_fail_allocation(-1)
+        assert e.value.status == 3 and e.value.message
+        for got, want in zip(images, expected):
+            assert np.array_equal(host(got, np.uint32), want)
+        gpu.destroy()
+    finally:
+        fresh.close()
