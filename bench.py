@@ -51,7 +51,7 @@ def parse_args():
     p.add_argument("--light-sprites", type=int, default=4096, help="sprites of the deferred-light pass (0 skips it)")
     p.add_argument("--c0", type=int, default=1, help="also measure the 800x600 random-triangle workload (0 skips it)")
     p.add_argument("--shadow-tuning", default="auto",
-                   help="the light pass's shadow batch: auto (the autotuner on that batch) or TxCxRxWxM like --tuning")
+                   help="the light pass's shadow batch: auto (the context's configuration) or TxCxRxWxM like --tuning")
     p.add_argument("--tuning", default="auto",
                    help="tile kernel launch shape THREADSxCTAS_PER_SMxSMALL_ROWSxSMALL_WIDTH[xRESOLVE] (e.g. 128x8x8x16x1), or auto")
     return p.parse_args()
@@ -371,7 +371,8 @@ def light_section(ctx, args):
     scene = scenes.light_scene(seed=2024, sprites=args.light_sprites, light_space=(m[9:18], m[0:9]))
     threads = os.cpu_count() or 1
     gpu = DeferredLightPass(ctx, scene, threads)
-    # the shadow batch's own tile-kernel shape, chosen by the autotuner on it (the context's stays)
+    # the shadow batch keeps a configuration of its own (depth-only batches draw a tile per warp: the
+    # autotuner leaves it as it is, and a given shape counts only while fragments are counted)
     if args.shadow_tuning == "auto":
         shadow_tuning = gpu.tune_shadows(rounds=2)
     else:  # a given shape (profiling runs keep the autotuner's trial launches out of the launch list)

@@ -433,6 +433,12 @@ int dsrg_batch_autotune(dsrg_batch b, int32_t rounds, dsrg_tuning *best) {
 			if (own) dsrg_context_set_tuning(context, &tuning);
 		}
 	} restore{b, ctx, contextTuning, own};
+	if (b->depthOnly && !ctx->counting) {
+		// raster_depth_kernel draws a tile per warp whatever the configuration: there is nothing to search
+		const int status = dsrg_batch_render(b);
+		if (status == DSRG_OK && best) *best = start;
+		return status;
+	}
 	struct Shape { int32_t threads, perSm; };
 	const Shape shapes[] = {{256, 4}, {256, 2}, {128, 8}, {128, 4}, {64, 16}};
 	const int32_t smalls[][2] = {{8, 16}, {0, 0}, {4, 8}};

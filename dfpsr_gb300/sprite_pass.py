@@ -55,9 +55,9 @@ class DeferredLightPass:
         self.light_list = [dict(l, cube=self.cubes[k]) for k, l in enumerate(scene.lights)]
 
     def tune_shadows(self, rounds: int = 2) -> dict:
-        """Gives the shadow batch a tile-kernel configuration of its own, the autotuner's choice for
-        it (cube faces of large triangles suit other shapes than the frames drawn with the
-        context's configuration, which stays as it is)."""
+        """Gives the shadow batch a configuration of its own, the context's present one (depth-only
+        batches are drawn by one warp per tile: the autotuner finds nothing to choose for them), so
+        that later changes of the context's leave it alone."""
         self.shadows.set_tuning(self.ctx.tuning())
         return self.shadows.autotune(rounds)
 

@@ -279,7 +279,10 @@ int dsrg_batch_give_task(dsrg_batch batch, int32_t frameIndex, dsrg_model model,
  * batch keeps its frames and tasks, so rendering it again redraws the same scenes. */
 int dsrg_batch_render(dsrg_batch batch);
 
-/* Launch configuration of the tile kernel, chosen per context by dsrg_batch_autotune.
+/* Launch configuration of the tile kernel, chosen per context by dsrg_batch_autotune.  Depth-only
+ * work (dsrg_batch_set_depth_only, dsrg_model_render_depth) has a kernel of its own that draws each
+ * tile with one warp: of these values it uses `graphs` alone (all of them while fragments are
+ * counted, dsrg_context_set_counting).
  *   threadsPerTile   threads of one tile's CTA (64, 128 or 256)
  *   ctasPerSm        persistent CTAs per SM pulling tiles from the queue (1 to 1024 / threadsPerTile)
  *   smallRows/Width  triangles whose raster bound is at most smallRows x smallWidth pixels are
@@ -301,13 +304,13 @@ int dsrg_context_set_tuning(dsrg_context context, const dsrg_tuning *tuning);
 /* Renders the batch once per candidate configuration (rounds times each, each timed render
  * starting from a cold L2 cache), keeps the fastest and returns it in *best (may be null): for the
  * batch when it has a configuration of its own (dsrg_batch_set_tuning), the context's staying as
- * it was, else for the context.  The images end up holding the batch's rendered frames. */
+ * it was, else for the context.  The images end up holding the batch's rendered frames.  A
+ * depth-only batch is rendered once and keeps the configuration that it has. */
 int dsrg_batch_autotune(dsrg_batch batch, int32_t rounds, dsrg_tuning *best);
 
 /* A tile-kernel configuration for this batch alone (no counterpart in the reference): its renders
  * use *tuning and leave the context's configuration as it is, so that batches of different
- * workloads (a frame of small triangles, shadow faces of large ones) each keep the shape that
- * suits them.  tuning = null returns the batch to the context's configuration. */
+ * workloads (frames of small triangles, frames of large ones) each keep the shape that suits them.  tuning = null returns the batch to the context's configuration. */
 int dsrg_batch_set_tuning(dsrg_batch batch, const dsrg_tuning *tuning);
 
 /* ---- differentiable rendering; no counterpart in the reference.

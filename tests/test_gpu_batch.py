@@ -364,3 +364,34 @@ def test_depth_only_tiles_drawn_in_parts(ctx):
     m = d.Model(ctx, s)
     ctx.render_depth(m, m.camera, z)
     assert np.array_equal(z.view(np.uint32), port.render_depth(s)[0].view(np.uint32))
+
+
+def test_autotune_of_a_depth_only_batch_draws_it_once(ctx):
+    """Depth-only tiles are drawn by one warp each whatever the configuration: the autotuner renders the
+    batch once, keeps the configuration, and leaves the frames in the images."""
+    import torch
+    import dfpsr_gb300 as d
+    s = scenes.random_triangles(seed=31, triangles=300, width=96, height=64, texture_size=16)
+    model = d.Model(ctx, s)
+    batch = d.Batch(ctx)
+    batch.set_depth_only(True)
+    image = torch.zeros((64, 96), dtype=torch.float32, device="cuda")
+    batch.add_frame(None, image)
+    batch.give_task(0, model)
+    launches = []
+    for _ in range(3):
+        batch.render()
+        launches.append(ctx.stats()["kernel_launches"])
+    expected = image.cpu().numpy().copy()
+    image.zero_()
+    for own in (None, dict(ctx.tuning(), threads_per_tile=64, ctas_per_sm=16)):
+        if own:
+            batch.set_tuning(own)
+        before = ctx.tuning()
+        assert batch.autotune(rounds=3) == (own or before)
+        assert ctx.tuning() == before
+        assert np.array_equal(image.cpu().numpy().view(np.uint32), expected.view(np.uint32))
+        launches.append(ctx.stats()["kernel_launches"])
+        assert launches[-1] - launches[-2] <= launches[2] - launches[1]
+    batch.destroy()
+    model.destroy()
