@@ -47,6 +47,12 @@ int dsrg_debug_fail_allocation(int64_t after) {
 	return DSRG_OK;
 }
 
+int dsrg_internal_set_one_pass_limit(dsrg_context ctx, uint32_t triangles) {
+	if (!ctx) return DSRG_ERROR_INVALID_ARGUMENT;
+	ctx->onePassLimit = triangles < MAX_EMIT_TRIANGLES ? triangles : MAX_EMIT_TRIANGLES;
+	return DSRG_OK;
+}
+
 int dsrg_context_create(int32_t device, dsrg_context *out) {
 	if (!out) return DSRG_ERROR_INVALID_ARGUMENT;
 	*out = nullptr;

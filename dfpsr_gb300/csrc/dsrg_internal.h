@@ -219,6 +219,7 @@ struct dsrg_context_s {
 	bool timingHasRaster = false;
 	bool stopRecorded = false;           // the last batch recorded eventStop before its host wait
 	// capacities of the buffers sized before their totals are known (largest totals seen, with slack)
+	uint32_t onePassLimit = dsrg::MAX_EMIT_TRIANGLES; // fan triangles from which on a batch is set up in two passes
 	uint64_t extraCapacity = 0, recordCapacity = 0, rowCapacity = 0, binCapacity = 0;
 	DeviceBuffer<uint32_t> binLists;
 	DeviceBuffer<uint4> batchScratch;    // a batch's other arrays, one after another (enqueue_phases)
@@ -317,6 +318,10 @@ struct dsrg_renderer_s {
 	DeviceBuffer<int4> debugLinesDevice;
 };
 
+// Batches of this context of `triangles` fan triangles and more are set up in two passes (at most, and
+// without a call, MAX_EMIT_TRIANGLES, which no batch of ordinary size has).  Not part of the API: for tests
+// of the two-pass setup.
+extern "C" int dsrg_internal_set_one_pass_limit(dsrg_context ctx, uint32_t triangles);
 // Uploads the frame's renderer_giveTask_triangle data and points its tasks at it.
 int renderer_upload_given(dsrg_renderer r);
 // The device address of page-locked (or registered) host memory, which kernels then read and write

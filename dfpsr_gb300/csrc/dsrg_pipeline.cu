@@ -207,7 +207,7 @@ static int enqueue_phases(dsrg_context ctx, BatchJob &job, BatchTotals &totals, 
 	const size_t np = totals.points, nt = totals.triangles;
 	// the one-pass setup keeps a slot per fan triangle and extra ones for the pieces of clipped
 	// triangles; beyond its record numbers' range the two-pass setup counts first
-	const bool onePass = nt < MAX_EMIT_TRIANGLES;
+	const bool onePass = nt < ctx->onePassLimit;
 	const uint32_t recordCap = onePass ? (uint32_t)(nt + std::max<uint64_t>(ctx->extraCapacity, nt / 8 + 1024))
 	                                   : (uint32_t)std::max<uint64_t>(ctx->recordCapacity, nt + nt / 8 + 1024);
 	// Four rows per record at first, and where rows are placed in whole segments (tall triangles) what rounding
