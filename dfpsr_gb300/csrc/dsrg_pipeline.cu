@@ -396,12 +396,17 @@ static int enqueue_phases(dsrg_context ctx, BatchJob &job, BatchTotals &totals, 
 		const bool recordsOver = onePass ? nt + extras > recordCap : totals.records > recordCap;
 		if (onePass) ctx->extraCapacity = std::max<uint64_t>(ctx->extraCapacity, extras + extras / 4 + 1024);
 		else ctx->recordCapacity = std::max<uint64_t>(ctx->recordCapacity, (uint64_t)totals.records + totals.records / 4 + 1024);
-		if (!recordsOver) {
-			ctx->rowCapacity = std::max<uint64_t>(ctx->rowCapacity, (uint64_t)totals.rows + totals.rows / 4 + 1024);
+		// rows and entries of the pieces that found no slot: as many each as the others have, so that one redo
+		// is mostly enough (the two-pass setup's own totals say nothing about them)
+		const uint64_t missing = onePass && recordsOver ? nt + extras - recordCap : 0;
+		const double scale = missing && totals.records ? 1.0 + (double)missing / totals.records : 1.0;
+		if (!recordsOver || missing) {
+			const uint64_t rows = (uint64_t)(scale * totals.rows), entries = (uint64_t)(scale * counted);
+			ctx->rowCapacity = std::max<uint64_t>(ctx->rowCapacity, rows + rows / 4 + 1024);
 			// the entries counted depend on how early the tiles' thresholds rose (bin_big_kernel), by a third from
 			// run to run for 20,000 random triangles at 800x600: twice the total, so that a frame that has
 			// been drawn once is not redone for it
-			ctx->binCapacity = std::max<uint64_t>(ctx->binCapacity, (uint64_t)counted * 2 + 1024);
+			ctx->binCapacity = std::max<uint64_t>(ctx->binCapacity, entries * 2 + 1024);
 		}
 		return DSRG_RETRY;
 	}

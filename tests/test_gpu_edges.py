@@ -133,3 +133,38 @@ def test_first_frame_of_a_mesh_is_drawn_once(built, size, width, height):
         assert np.array_equal(color, rc) and np.array_equal(depth.view(np.uint32), rz.view(np.uint32))
     finally:
         fresh.close()
+
+
+@pytest.mark.parametrize("first", ["small", "large"])
+@pytest.mark.parametrize("kind", ["solid", "alpha", "depth only"])
+def test_more_pieces_of_clipped_triangles_than_a_new_context_expects(built, kind, first):
+    """A camera among 24,000 triangles, most of them across a clipping plane: the further pieces outgrow
+    the slots that a context starts with (an eighth of the triangles), and after a small frame the rows
+    and lists too; after a large one seen from outside the slots alone.  Either way the frame is redone
+    once inside the call and equals the oracle's."""
+    import dfpsr_gb300 as d
+    from oracle import port
+    s = scenes.random_triangles(seed=67, triangles=24000, width=200, height=121, texture_size=32)
+    s.camera_location = scenes.camera_location((0.1, 0.2, -0.3), (0.0, 0.0, 1.0))
+    s = dataclasses.replace(s, filter=1 if kind == "alpha" else 0)
+    triangles, width, height = (200, 96, 64) if first == "small" else (25000, 500, 400)
+    other = dataclasses.replace(scenes.random_triangles(seed=65, triangles=triangles, width=width, height=height), filter=s.filter)
+    fresh = d.Context(0)
+    try:
+        model = d.Model(fresh, s)
+        d.render_scene(fresh, other, model=d.Model(fresh, other))
+        launches = [fresh.stats()["kernel_launches"]]
+        for _ in range(2):
+            if kind == "depth only":
+                z = np.zeros((s.height, s.width), np.float32)
+                fresh.render_depth(model, model.camera, z)
+                assert np.array_equal(z.view(np.uint32), port.render_depth(s)[0].view(np.uint32))
+            else:
+                got = d.render_scene(fresh, s, model=model)
+                expected = port.render(s)
+                assert np.array_equal(got[0], expected[0])
+                assert np.array_equal(got[1].view(np.uint32), expected[1].view(np.uint32))
+            launches.append(fresh.stats()["kernel_launches"])
+        assert launches[1] - launches[0] == 2 * (launches[2] - launches[1])
+    finally:
+        fresh.close()
