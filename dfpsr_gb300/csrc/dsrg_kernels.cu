@@ -2669,17 +2669,8 @@ __global__ void __launch_bounds__(ALPHA_THREADS) alpha_kernel(BatchParams b, con
 	if (begin == end) return; // the same for the whole CTA, as every condition around a barrier below
 	const FrameTarget &f = b.frames[find_segment(b.frameTileBase, b.frameCount, tile)];
 	if (!f.color) return;
-	const int tid = threadIdx.x, lane = tid & 31, l4 = tid & 3, quadBase = lane & ~3;
-	const int32_t local = (int32_t)(tile - f.tileBase), tx0 = (local % f.tilesX) * TILE_W, ty0 = (local / f.tilesX) * TILE_H;
-	const int32_t width = f.width, height = f.height, packOrder = f.packOrder;
-	const int q = tid >> 2;
-	const int32_t x = tx0 + 2 * (q & 7), y1 = ty0 + 2 * (q >> 3), px = x + (l4 & 1), py = y1 + (l4 >> 1);
-	const bool inside = px < width && py < height;
-	const bool depthTest = f.depth != nullptr, affine = f.affine != 0, oddRow = odd_last_row(y1, height);
-	const float stored = (depthTest && inside) ? f.depth[(size_t)py * f.depthStride + px] : 0.0f;
-	uint32_t *target = f.color + (size_t)py * f.colorStride + px;
-	uint32_t packed = inside ? *target : 0u;
-	uint32_t fragments = 0;
+	// the list in submission order, before the pixels take their registers
+	const int tid = threadIdx.x;
 	const uint32_t n = end - begin;
 	const uint32_t *order = ids;
 	if (n > ALPHA_LIST) {
@@ -2702,6 +2693,17 @@ __global__ void __launch_bounds__(ALPHA_THREADS) alpha_kernel(BatchParams b, con
 			}
 		}
 	}
+	const int lane = tid & 31, l4 = tid & 3, quadBase = lane & ~3;
+	const int32_t local = (int32_t)(tile - f.tileBase), tx0 = (local % f.tilesX) * TILE_W, ty0 = (local / f.tilesX) * TILE_H;
+	const int32_t width = f.width, height = f.height, packOrder = f.packOrder;
+	const int q = tid >> 2;
+	const int32_t x = tx0 + 2 * (q & 7), y1 = ty0 + 2 * (q >> 3), px = x + (l4 & 1), py = y1 + (l4 >> 1);
+	const bool inside = px < width && py < height;
+	const bool depthTest = f.depth != nullptr, affine = f.affine != 0, oddRow = odd_last_row(y1, height);
+	const float stored = (depthTest && inside) ? f.depth[(size_t)py * f.depthStride + px] : 0.0f;
+	uint32_t *target = f.color + (size_t)py * f.colorStride + px;
+	uint32_t packed = inside ? *target : 0u;
+	uint32_t fragments = 0;
 	for (uint32_t base = 0; base < n; base += ALPHA_CHUNK) {
 		const uint32_t m = min(ALPHA_CHUNK, n - base);
 		__syncthreads(); // the chunk before is done with
