@@ -435,7 +435,9 @@ static DiffModel diff_model(dsrg_diff d) {
 #define TRY(expr) DSRG_CUDA_TRY(ctx, expr)
 
 // Entries (seven per pixel) up to which the deterministic adjoint sorts both kinds of targets at once:
-// three passes instead of five over few entries, which launches and waits decide, not their number.
+// three passes instead of five.  One view of 64x64 (28,672 entries) takes 88 us together and 123 apart, 64
+// views of 256x256 (29 M) 688 and 729.  Beyond the line it is still 2 to 4 % faster (100 views, 46 M:
+// 1,009 and 1,048 us), but the sort's arrays then hold seven entries per pixel instead of four at a time.
 static const uint64_t TOGETHER_ENTRIES = 1u << 25;
 
 // Scratch of segmented_sum for n entries and keys below keyEnd, reserved before any launch.
@@ -660,6 +662,7 @@ int dsrg_diff_adjoint(dsrg_diff d, int32_t views, int32_t width, int32_t height,
 		// smaller scratch of one kind at a time
 		const bool together = pixels * 7 <= TOGETHER_ENTRIES;
 		status = together ? reserve_segmented_sum(d, pixels * 7, texels + points) : reserve_segmented_sum(d, pixels * 4, texels > points ? texels : points);
+		if (status == DSRG_OK && !together) status = reserve_segmented_sum(d, pixels * 3, points); // fewer items can take more blocks
 		if (status != DSRG_OK) return status;
 		DeterministicSums sums;
 		sums.texKeys = d->emitted.ptr;
