@@ -98,12 +98,12 @@ int dsrg_context_destroy(dsrg_context ctx) {
 	DeviceBuffer<float> *fbufs[] = {&ctx->stagingDepth};
 	for (auto *b : fbufs) b->release();
 	ctx->pointCsis.release(); ctx->pointIsyOut.release(); ctx->pointFlat.release();
-	DeviceBuffer<uint32_t> *ubufs[] = {&ctx->triCounts, &ctx->triOffsets, &ctx->scanScratch, &ctx->control, &ctx->binLists, &ctx->stagingColor};
+	DeviceBuffer<uint32_t> *ubufs[] = {&ctx->triCounts, &ctx->triOffsets, &ctx->scanScratch, &ctx->control, &ctx->stagingColor};
 	for (auto *b : ubufs) b->release();
-	ctx->records.release(); ctx->tables.release(); ctx->keys.release(); ctx->denseKeys.release(); ctx->denseInstances.release();
+	ctx->tables.release(); ctx->keys.release(); ctx->denseKeys.release(); ctx->denseInstances.release();
 	if (ctx->pinnedTables) cudaFreeHost(ctx->pinnedTables);
 	if (ctx->pinnedReadback) cudaFreeHost(ctx->pinnedReadback);
-	ctx->rowCounts.release(); ctx->rowOffsets.release(); ctx->rows.release(); ctx->textureTable.release(); ctx->fragmentCounter.release();
+	ctx->rowCounts.release(); ctx->rowOffsets.release(); ctx->textureTable.release(); ctx->fragmentCounter.release();
 	ctx->lightStaging.release();
 	ctx->spriteTableHost.release();
 	ctx->lightTableHost.release();

@@ -43,6 +43,19 @@ struct DeviceBuffer {
 		capacity = newCapacity;
 		return cudaSuccess;
 	}
+	// reserve for a large block whose contents nobody needs any more: the old memory goes first, so that both
+	// never have to fit, and from 1 GB on an eighth of slack takes the place of the next power of two.
+	cudaError_t replace(size_t n) {
+		if (n <= capacity) return cudaSuccess;
+		size_t newCapacity = 1024;
+		while (newCapacity < n) newCapacity *= 2;
+		if (n * sizeof(T) > ((size_t)1 << 30)) newCapacity = n + n / 8;
+		release();
+		const cudaError_t err = device_alloc((void **)&ptr, newCapacity * sizeof(T));
+		if (err != cudaSuccess) { ptr = nullptr; return err; }
+		capacity = newCapacity;
+		return cudaSuccess;
+	}
 	void release() {
 		if (ptr) cudaFree(ptr);
 		ptr = nullptr;
@@ -206,7 +219,6 @@ struct dsrg_context_s {
 	DeviceBuffer<uint32_t> triCounts, triOffsets, scanScratch;
 	DeviceBuffer<unsigned long long> denseKeys; // per-pixel winners of dsrg_dense_render
 	DeviceBuffer<unsigned char> denseInstances; // the instance table of one dense-model call
-	DeviceBuffer<DrawRecord> records;
 	DeviceBuffer<unsigned char> tables;  // the batch's task, frame and texture tables
 	unsigned char *pinnedTables = nullptr; // host staging of the tables (page-locked)
 	size_t pinnedCapacity = 0;
@@ -221,8 +233,7 @@ struct dsrg_context_s {
 	// capacities of the buffers sized before their totals are known (largest totals seen, with slack)
 	uint32_t onePassLimit = dsrg::MAX_EMIT_TRIANGLES; // fan triangles from which on a batch is set up in two passes
 	uint64_t extraCapacity = 0, recordCapacity = 0, rowCapacity = 0, binCapacity = 0;
-	DeviceBuffer<uint32_t> binLists;
-	DeviceBuffer<uint4> batchScratch;    // a batch's other arrays, one after another (enqueue_phases)
+	DeviceBuffer<uint4> batchScratch;    // a batch's arrays, one after another (enqueue_phases)
 	DeviceBuffer<TextureData> textureTable;
 	DeviceBuffer<uint32_t> stagingColor;
 	DeviceBuffer<uint32_t> textureStaging;      // texture creation: host images and two-step resize halves
@@ -239,7 +250,7 @@ struct dsrg_context_s {
 	cudaEvent_t sideStart = nullptr, sideDone = nullptr;
 	DeviceBuffer<unsigned long long> fragmentCounter;
 	DeviceBuffer<unsigned long long> keys;
-	DeviceBuffer<uint32_t> rowCounts, rowOffsets, rows;
+	DeviceBuffer<uint32_t> rowCounts, rowOffsets;
 	int32_t smallRows = 8, smallWidth = 16; // one lane walks records whose raster bound is at most 8 x 16 pixels
 	int32_t ctasPerSm = 4;                  // resident CTAs per SM of the persistent tile kernel
 	int32_t threadsPerTile = 256;           // threads of one tile's CTA

@@ -86,3 +86,39 @@ def test_failed_batch_and_texture_allocations_leave_the_context_usable(ctx, no_i
         rc, rd, _ = port.render(s, bands=12, threads=os.cpu_count() or 1)
         assert np.array_equal(c, rc) and np.array_equal(z.view(np.uint32), rd.view(np.uint32))
     batch.destroy()
+
+
+def test_a_first_frame_allocates_its_buffers_in_few_blocks(built, no_injection):
+    """A new context's first frame into device images allocates its tables, its keys and one block for
+    everything between them; whichever of them fails, the frame after the failure is right."""
+    import torch
+    d = no_injection
+    from oracle import port
+    scene = scenes.random_triangles(seed=82, triangles=4000, width=96, height=64, texture_size=32)
+    rc, rd, _ = port.render(scene)
+    for k in range(8):
+        ctx = d.Context(0)
+        try:
+            model = d.Model(ctx, scene)
+            color = torch.zeros((64, 96), dtype=torch.int32, device="cuda")
+            depth = torch.zeros((64, 96), dtype=torch.float32, device="cuda")
+            d.lib().dsrg_debug_fail_allocation(k)
+            try:
+                ctx.render(model, model.camera, color, depth)
+                failed = False
+            except d.DsrgError as e:
+                assert e.status == OUT_OF_MEMORY
+                failed = True
+            d.lib().dsrg_debug_fail_allocation(-1)
+            if failed:
+                color.zero_()
+                depth.zero_()
+                ctx.render(model, model.camera, color, depth)
+            assert np.array_equal(color.cpu().numpy().view(np.uint32), rc)
+            assert np.array_equal(depth.cpu().numpy().view(np.uint32), rd.view(np.uint32))
+        finally:
+            ctx.close()
+        if not failed:
+            break
+    # three, and the block once more when the rows or lists of this scene outgrow it
+    assert not failed and k <= 4
