@@ -374,7 +374,7 @@ __global__ void root_check_kernel(uint32_t firstBits, uint32_t count, unsigned l
 // stores in flight, and rows that follow one another in memory are one long row.  Words are counted in
 // 32 bits: add_fill_pieces keeps every rectangle below 2^31.  The 16 shadow cubes of
 // the 1080p light frame (100 MB) took up to eight launches of a word per thread and 75 to 100 us; they
-// now take 14 us in one (frame 616 -> 571 us).
+// now take 14 us in one.
 struct FillBatch {
 	FillRect rect[FILL_RECTS];
 };

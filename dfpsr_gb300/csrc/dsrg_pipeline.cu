@@ -1,7 +1,7 @@
-// Host side of one batch through the kernels: table layout, scratch sizing and the three
-// launch phases, shared by the renderer (one frame), the batch API (many frames) and the
-// differentiable renderer.  Between the phases the host reads two totals (draw records, then
-// row intervals and tile-list entries) to size the next phase's buffers exactly.
+// Host side of one batch through the kernels: table layout, scratch sizing and the launch phases,
+// shared by the renderer (one frame), the batch API (many frames) and the differentiable renderer.
+// All phases are queued before the host reads their totals, once: buffers are sized from the largest
+// totals seen, and a batch that outgrows them is redone.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -427,7 +427,7 @@ static int enqueue_phases(dsrg_context ctx, BatchJob &job, BatchTotals &totals, 
 int batch_enqueue(dsrg_context ctx, BatchJob &job, BatchTotals &totals, BatchOutputs *outputs) {
 	if (outputs) memset(outputs, 0, sizeof(*outputs));
 	int status = DSRG_RETRY;
-	// a batch whose totals outgrow the capacities is redone once per buffer that was too small
+	// a batch whose totals outgrow the capacities is redone with larger ones
 	for (int attempt = 0; attempt < 4 && status == DSRG_RETRY; attempt++) status = enqueue_phases(ctx, job, totals, outputs);
 	if (status == DSRG_RETRY) return fail(ctx, DSRG_ERROR_DEVICE, "batch buffers kept overflowing");
 	if (status == DSRG_OK && !ctx->stopRecorded) TRY(cudaEventRecord(ctx->eventStop, ctx->stream));

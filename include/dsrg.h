@@ -270,9 +270,8 @@ int dsrg_batch_destroy(dsrg_batch batch);
 int dsrg_batch_clear(dsrg_batch batch);
 /* Adds a frame (renderer_begin, api/rendererAPI.cpp:151-168); *frameIndex receives its index. */
 int dsrg_batch_add_frame(dsrg_batch batch, const dsrg_image *color, const dsrg_image *depth, int32_t *frameIndex);
-/* renderer_giveTask (api/modelAPI.h:299-301) for one frame of the batch.  Alpha-filtered models
- * on a frame with a colour target are rejected with DSRG_ERROR_UNSUPPORTED (draw them with
- * dsrg_renderer_* or dsrg_model_render). */
+/* renderer_giveTask (api/modelAPI.h:299-301) for one frame of the batch.  A frame's solid and
+ * alpha-filtered tasks, of either projection, are drawn in the order given. */
 int dsrg_batch_give_task(dsrg_batch batch, int32_t frameIndex, dsrg_model model, const float *modelToWorld,
                          const dsrg_camera *camera);
 /* Draws every frame (renderer_end of each); returns when all results are in the images.  The
